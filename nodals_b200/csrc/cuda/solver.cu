@@ -29,6 +29,7 @@
 #include "kernels.cuh"
 #include "krylov.cuh"
 #include "mpnn.hpp"
+#include "split.cuh"
 
 namespace nds {
 
@@ -456,6 +457,149 @@ class Solver final : public ISolver {
     }
 
     tm.mark("momentum_and_cells");
+    // The pressure operator: in split form, or as assembled rows (SELL) for
+    // the smoothers that read a row's entries.
+    split_ = o_.amg_smoother == NDS_SM_CHEB2 || o_.amg_smoother == NDS_SM_JACOBI;
+    const FineTopo& F = S.fine;
+    if (split_) upload_split();
+    else upload_sell(tm);
+    tm.mark("sell_layout");
+    fdiag_.upload(H.fine_diag);
+    const bool l1 = o_.amg_smoother == NDS_SM_L1JACOBI;
+    if (l1) fl1_.alloc((size_t)nc_);
+    if (o_.amg_smoother == NDS_SM_MCGS) {
+      std::vector<int32_t> rows;
+      greedy_color(nc_, F.row, F.col, rows, fine_coff_);
+      fine_crows_.upload(rows);
+    }
+    for (auto* b : {&x_, &r_, &z_, &pp_, &q_, &rhs_}) b->alloc((size_t)nc_);
+    for (auto* b : {&fr_, &ftmp_, &fcorr_, &frhs_, &fpong_}) b->alloc((size_t)nc_);
+    if (!kSame) {
+      rA_.alloc((size_t)nc_);
+      zA_.alloc((size_t)nc_);
+    }
+
+    // AMG levels and transfers
+    L_.resize(H.A.size());
+    for (size_t l = 0; l < H.A.size(); ++l) {
+      const CsrHost& A = H.A[l];
+      Level& Lv = L_[l];
+      Lv.n = A.n;
+      Lv.row.upload(to_i32(A.row, "AMG level CSR"));
+      Lv.col.upload(A.col);
+      Lv.val.upload(A.val);
+      Lv.diag.upload(A.diag);
+      std::vector<double> l1h((size_t)A.n);
+#pragma omp parallel for schedule(static)
+      for (int i = 0; i < A.n; ++i) {
+        double ss = 0.0;
+        for (int64_t k = A.row[(size_t)i]; k < A.row[(size_t)i + 1]; ++k) ss += std::abs(A.val[(size_t)k]);
+        l1h[(size_t)i] = ss;
+      }
+      Lv.l1.upload(l1h);
+      for (auto* b : {&Lv.b, &Lv.x, &Lv.r, &Lv.tmp, &Lv.corr, &Lv.pong}) b->alloc((size_t)A.n);
+      // the mixed path's V-cycle reads FP16 copies of the explicit levels
+      // (the terminal level goes through its dense inverse)
+      if (!kSame && o_.precision == NDS_MIXED && o_.amg_half && l + 1 < H.A.size()) level_to_half(Lv, A);
+      if (o_.amg_smoother == NDS_SM_MCGS && l + 1 < H.A.size()) {
+        std::vector<int32_t> rows;
+        std::vector<int32_t> r32 = to_i32(A.row, "AMG level CSR");
+        greedy_color(A.n, r32, A.col, rows, Lv.coff);
+        Lv.crows.upload(rows);
+      }
+    }
+    X_.resize(H.P.size());
+    for (size_t l = 0; l < H.P.size(); ++l) {
+      const Transfer& Ph = H.P[l];
+      Xfer& X = X_[l];
+      X.nf = Ph.nf;
+      X.nc = Ph.nc;
+      {
+        // P in ELL, entry k of fine row i at k nf + i (coalesced across rows);
+        // padding entries carry value 0 and coarse column 0
+        int pw = 0;
+        for (int i = 0; i < Ph.nf; ++i) pw = std::max<int>(pw, (int)(Ph.row[(size_t)i + 1] - Ph.row[(size_t)i]));
+        std::vector<int32_t> ec((size_t)pw * Ph.nf, 0);
+        std::vector<double> ev((size_t)pw * Ph.nf, 0.0);
+#pragma omp parallel for schedule(static)
+        for (int i = 0; i < Ph.nf; ++i)
+          for (int64_t q = Ph.row[(size_t)i]; q < Ph.row[(size_t)i + 1]; ++q) {
+            const size_t o = (size_t)(q - Ph.row[(size_t)i]) * Ph.nf + i;
+            ec[o] = Ph.col[(size_t)q];
+            ev[o] = Ph.val[(size_t)q];
+          }
+        X.pw = pw;
+        X.pcol.upload(ec);
+        X.pval.upload(ev);
+      }
+      // R = P^T, entries of each coarse row in ascending fine row
+      std::vector<int32_t> rr((size_t)Ph.nc + 1, 0), rc(Ph.col.size());
+      std::vector<double> rv(Ph.col.size());
+      for (int32_t c : Ph.col) ++rr[(size_t)c + 1];
+      for (int c = 0; c < Ph.nc; ++c) rr[(size_t)c + 1] += rr[(size_t)c];
+      std::vector<int32_t> pos(rr.begin(), rr.end() - 1);
+      for (int i = 0; i < Ph.nf; ++i)
+        for (int64_t k = Ph.row[(size_t)i]; k < Ph.row[(size_t)i + 1]; ++k) {
+          const int c = Ph.col[(size_t)k];
+          rc[(size_t)pos[(size_t)c]] = i;
+          rv[(size_t)pos[(size_t)c]++] = Ph.val[(size_t)k];
+        }
+      X.rrow.upload(rr);
+      X.rcol.upload(rc);
+      X.rval.upload(rv);
+    }
+    tinv_.upload(H.terminal_inv);
+    fine_lambda_ = H.fine_lambda;
+    level_lambda_ = H.level_lambda;
+    level_lambda_.resize(L_.size(), 0.0);
+
+    part_.alloc((size_t)kMaxPartBlocks * 8);
+    sc_.alloc(kScalars);
+    flags_.alloc(1);
+    ctl_.alloc(4);
+    NDS_CUDA(cudaMallocHost((void**)&hsc_, sizeof(double) * kScalars));
+    NDS_CUDA(cudaMallocHost((void**)&hflags_, sizeof(int) * 8));
+    NDS_CUDA(cudaMemsetAsync(flags_.p, 0, sizeof(int), st_));
+
+    if constexpr (!kSame) {
+      mixed_ = o_.precision == NDS_MIXED;
+      if (mixed_) alloc_mixed();
+    }
+    // setup-time state: fine CSR refreshed with the initial rAU
+    tm.mark("levels_and_transfers");
+    refresh_fine(rau_.p);
+    if (mixed_ && o_.amg_half) {
+      // FP16 copy: scale by a power of two that puts the largest setup-time
+      // diagonal at 2^11 (the diagonal dominates its row; 2^4 headroom below
+      // the FP16 maximum for later growth of rAU, values beyond saturate)
+      std::vector<TA> d((size_t)nc_);
+      NDS_CUDA(cudaMemcpyAsync(d.data(), fdiag_.p, sizeof(TA) * d.size(), cudaMemcpyDeviceToHost, st_));
+      NDS_CUDA(cudaStreamSynchronize(st_));
+      double dmax = 0.0;
+      for (TA v : d) dmax = std::max(dmax, std::abs((double)v));
+      if (!(dmax > 0.0) || !std::isfinite(dmax)) throw std::runtime_error("FP16 operator copy: no positive diagonal");
+      hscale_ = std::ldexp(1.0, (int)std::floor(std::log2(2048.0 / dmax)));
+      half_on_ = true;
+      if (!split_) fvalH_.alloc(fval_.n);
+      refresh_fine(rau_.p);
+    }
+    if (P_.power_its > 0) {
+      fine_lambda_ = power_fine(P_.power_its, o_.amg_lambda_safety);
+      for (size_t l = 0; l + 1 < L_.size(); ++l) level_lambda_[l] = power_level(L_[l], P_.power_its, o_.amg_lambda_safety);
+    } else {
+      fine_lambda_ = 1.0;
+      for (auto& v : level_lambda_) v = 1.0;
+    }
+    if (o_.pressure_solver == NDS_P_CHEB) p_cheb_lambda_ = precond_power(o_.p_power_its, o_.p_power_safety);
+    NDS_CUDA(cudaStreamSynchronize(st_));
+    tm.mark("refresh_and_spectrum");
+    reset();
+  }
+
+  // assembled fine operator: refresh contributions and SELL layout
+  void upload_sell(StageTimer& tm) {
+    const Setup& S = P_.setup;
+    const FineTopo& F = S.fine;
     // fine Schur refresh contributions, regrouped by destination slot in the
     // reference's order and laid out in runs (one run per fine entry, the
     // longest first) that never straddle a 32-contribution chunk of the row: a run that would
@@ -463,7 +607,6 @@ class Solver final : public ISolver {
     // pad entries.  Per contribution: the code word cs (basis a bits 0-2,
     // position in its run bits 3-5, run tail bit 6, slot bits 7-15; pads are
     // 0xFFFF) and the packed incidence (c2 << 3 | b) for the geometry.
-    const FineTopo& F = S.fine;
     {
       std::vector<int32_t> plen((size_t)nc_ + 1, 0);
       std::vector<int32_t> poff((size_t)nc_ + 1, 0);
@@ -622,136 +765,186 @@ class Solver final : public ISolver {
       }
       sell_nnz_ = (long long)scol.size();
     }
-    tm.mark("sell_layout");
-    fdiag_.upload(H.fine_diag);
-    const bool l1 = o_.amg_smoother == NDS_SM_L1JACOBI;
-    if (l1) fl1_.alloc((size_t)nc_);
-    if (o_.amg_smoother == NDS_SM_MCGS) {
-      std::vector<int32_t> rows;
-      greedy_color(nc_, F.row, F.col, rows, fine_coff_);
-      fine_crows_.upload(rows);
-    }
-    for (auto* b : {&x_, &r_, &z_, &pp_, &q_, &rhs_}) b->alloc((size_t)nc_);
-    for (auto* b : {&fr_, &ftmp_, &fcorr_, &frhs_, &fpong_}) b->alloc((size_t)nc_);
-    if (!kSame) {
-      rA_.alloc((size_t)nc_);
-      zA_.alloc((size_t)nc_);
-    }
-
-    // AMG levels and transfers
-    L_.resize(H.A.size());
-    for (size_t l = 0; l < H.A.size(); ++l) {
-      const CsrHost& A = H.A[l];
-      Level& Lv = L_[l];
-      Lv.n = A.n;
-      Lv.row.upload(to_i32(A.row, "AMG level CSR"));
-      Lv.col.upload(A.col);
-      Lv.val.upload(A.val);
-      Lv.diag.upload(A.diag);
-      std::vector<double> l1h((size_t)A.n);
-#pragma omp parallel for schedule(static)
-      for (int i = 0; i < A.n; ++i) {
-        double ss = 0.0;
-        for (int64_t k = A.row[(size_t)i]; k < A.row[(size_t)i + 1]; ++k) ss += std::abs(A.val[(size_t)k]);
-        l1h[(size_t)i] = ss;
-      }
-      Lv.l1.upload(l1h);
-      for (auto* b : {&Lv.b, &Lv.x, &Lv.r, &Lv.tmp, &Lv.corr, &Lv.pong}) b->alloc((size_t)A.n);
-      // the mixed path's V-cycle reads FP16 copies of the explicit levels
-      // (the terminal level goes through its dense inverse)
-      if (!kSame && o_.precision == NDS_MIXED && o_.amg_half && l + 1 < H.A.size()) level_to_half(Lv, A);
-      if (o_.amg_smoother == NDS_SM_MCGS && l + 1 < H.A.size()) {
-        std::vector<int32_t> rows;
-        std::vector<int32_t> r32 = to_i32(A.row, "AMG level CSR");
-        greedy_color(A.n, r32, A.col, rows, Lv.coff);
-        Lv.crows.upload(rows);
-      }
-    }
-    X_.resize(H.P.size());
-    for (size_t l = 0; l < H.P.size(); ++l) {
-      const Transfer& Ph = H.P[l];
-      Xfer& X = X_[l];
-      X.nf = Ph.nf;
-      X.nc = Ph.nc;
-      {
-        // P in ELL, entry k of fine row i at k nf + i (coalesced across rows);
-        // padding entries carry value 0 and coarse column 0
-        int pw = 0;
-        for (int i = 0; i < Ph.nf; ++i) pw = std::max<int>(pw, (int)(Ph.row[(size_t)i + 1] - Ph.row[(size_t)i]));
-        std::vector<int32_t> ec((size_t)pw * Ph.nf, 0);
-        std::vector<double> ev((size_t)pw * Ph.nf, 0.0);
-#pragma omp parallel for schedule(static)
-        for (int i = 0; i < Ph.nf; ++i)
-          for (int64_t q = Ph.row[(size_t)i]; q < Ph.row[(size_t)i + 1]; ++q) {
-            const size_t o = (size_t)(q - Ph.row[(size_t)i]) * Ph.nf + i;
-            ec[o] = Ph.col[(size_t)q];
-            ev[o] = Ph.val[(size_t)q];
+  }
+  // fine operator in split form (split.cuh): the free vertices' incidences,
+  // the cells' vertices, face neighbours and gradients, in the precisions in
+  // use; rAU-dependent parts are written by refresh_fine
+  void upload_split() {
+    const Setup& S = P_.setup;
+    const FineTopo& F = S.fine;
+    int nvert = 0;
+    for (int v = 0; v < S.n_vert; ++v) nvert += S.g2free[(size_t)v] >= 0;
+    svert_.n = nvert;
+    const std::vector<int32_t> off(F.inc_off.begin(), F.inc_off.begin() + nvert + 1);
+    const size_t nz = (size_t)off[(size_t)nvert];
+    sp_off_.upload(off);
+    svert_.off = sp_off_.p;
+    const size_t n = (size_t)nc_;
+    const bool half = !kSame && o_.precision == NDS_MIXED && o_.amg_half;
+    auto vert = [&](int c, int a, int d) { return S.bco[24 * (size_t)c + 3 * (size_t)a + (size_t)d]; };
+    std::vector<int4> vid(n), nid(n);
+    std::vector<T> g4(4 * n);
+    int too_far = 0;
+#pragma omp parallel for schedule(static) reduction(| : too_far)
+    for (int c = 0; c < nc_; ++c) {
+      int v[4], nb[4];
+      for (int a = 0; a < 4; ++a) {
+        const int g = S.ref[8 * (size_t)c + (size_t)a], f = S.ref[8 * (size_t)c + 4 + (size_t)a];
+        v[a] = g >= 0 ? g : nvert;
+        nb[a] = -1;
+        if (f >= 0)
+          for (int k = F.inc_off[(size_t)f]; k < F.inc_off[(size_t)f + 1]; ++k) {
+            const int q = (int)(F.packed[(size_t)k] >> 3);
+            if (q != c) nb[a] = q;
           }
-        X.pw = pw;
-        X.pcol.upload(ec);
-        X.pval.upload(ev);
+        if (nb[a] >= 0 && std::abs(nb[a] - c) > 32767) too_far = 1;
+        double b2 = 0.0;
+        for (int d = 0; d < 3; ++d) b2 += vert(c, a, d) * vert(c, a, d);
+        g4[(size_t)a * n + (size_t)c] = (T)b2;
       }
-      // R = P^T, entries of each coarse row in ascending fine row
-      std::vector<int32_t> rr((size_t)Ph.nc + 1, 0), rc(Ph.col.size());
-      std::vector<double> rv(Ph.col.size());
-      for (int32_t c : Ph.col) ++rr[(size_t)c + 1];
-      for (int c = 0; c < Ph.nc; ++c) rr[(size_t)c + 1] += rr[(size_t)c];
-      std::vector<int32_t> pos(rr.begin(), rr.end() - 1);
-      for (int i = 0; i < Ph.nf; ++i)
-        for (int64_t k = Ph.row[(size_t)i]; k < Ph.row[(size_t)i + 1]; ++k) {
-          const int c = Ph.col[(size_t)k];
-          rc[(size_t)pos[(size_t)c]] = i;
-          rv[(size_t)pos[(size_t)c]++] = Ph.val[(size_t)k];
-        }
-      X.rrow.upload(rr);
-      X.rcol.upload(rc);
-      X.rval.upload(rv);
+      vid[(size_t)c] = make_int4(v[0], v[1], v[2], v[3]);
+      nid[(size_t)c] = make_int4(nb[0], nb[1], nb[2], nb[3]);
     }
-    tinv_.upload(H.terminal_inv);
-    fine_lambda_ = H.fine_lambda;
-    level_lambda_ = H.level_lambda;
-    level_lambda_.resize(L_.size(), 0.0);
-
-    part_.alloc((size_t)kMaxPartBlocks * 8);
-    sc_.alloc(kScalars);
-    flags_.alloc(1);
-    ctl_.alloc(4);
-    NDS_CUDA(cudaMallocHost((void**)&hsc_, sizeof(double) * kScalars));
-    NDS_CUDA(cudaMallocHost((void**)&hflags_, sizeof(int) * 8));
-    NDS_CUDA(cudaMemsetAsync(flags_.p, 0, sizeof(int), st_));
-
-    if constexpr (!kSame) {
-      mixed_ = o_.precision == NDS_MIXED;
-      if (mixed_) alloc_mixed();
-    }
-    // setup-time state: fine CSR refreshed with the initial rAU
-    tm.mark("levels_and_transfers");
-    refresh_fine(rau_.p);
-    if (mixed_ && o_.amg_half) {
-      // FP16 copy: scale by a power of two that puts the largest setup-time
-      // diagonal at 2^11 (the diagonal dominates its row; 2^4 headroom below
-      // the FP16 maximum for later growth of rAU, values beyond saturate)
-      std::vector<TA> d((size_t)nc_);
-      NDS_CUDA(cudaMemcpyAsync(d.data(), fdiag_.p, sizeof(TA) * d.size(), cudaMemcpyDeviceToHost, st_));
-      NDS_CUDA(cudaStreamSynchronize(st_));
-      double dmax = 0.0;
-      for (TA v : d) dmax = std::max(dmax, std::abs((double)v));
-      if (!(dmax > 0.0) || !std::isfinite(dmax)) throw std::runtime_error("FP16 operator copy: no positive diagonal");
-      hscale_ = std::ldexp(1.0, (int)std::floor(std::log2(2048.0 / dmax)));
-      fvalH_.alloc(fval_.n);
-      refresh_fine(rau_.p);
-    }
-    if (P_.power_its > 0) {
-      fine_lambda_ = power_fine(P_.power_its, o_.amg_lambda_safety);
-      for (size_t l = 0; l + 1 < L_.size(); ++l) level_lambda_[l] = power_level(L_[l], P_.power_its, o_.amg_lambda_safety);
+    sp_vid_.upload(vid);
+    scell_.n = nc_;
+    scell_.vid = sp_vid_.p;
+    if (!too_far && !std::getenv("NDS_SELL_COL32")) {
+      std::vector<short4> d16(n);
+#pragma omp parallel for schedule(static)
+      for (int c = 0; c < nc_; ++c) {
+        const int4 q = nid[(size_t)c];
+        auto d = [&](int j) { return (short)(j >= 0 ? j - c : 0); };
+        d16[(size_t)c] = make_short4(d(q.x), d(q.y), d(q.z), d(q.w));
+      }
+      sp_nd16_.upload(d16);
+      scell_.nd16 = sp_nd16_.p;
     } else {
-      fine_lambda_ = 1.0;
-      for (auto& v : level_lambda_) v = 1.0;
+      sp_nid_.upload(nid);
+      scell_.nid = sp_nid_.p;
     }
-    if (o_.pressure_solver == NDS_P_CHEB) p_cheb_lambda_ = precond_power(o_.p_power_its, o_.p_power_safety);
-    NDS_CUDA(cudaStreamSynchronize(st_));
-    tm.mark("refresh_and_spectrum");
-    reset();
+    sp_g4_.upload(g4);
+    // double: component arrays; float: 16-byte records (x, y, z, cell)
+    auto records16 = [&](DBuf<float4>& out, auto&& value) {
+      std::vector<float4> r(nz);
+#pragma omp parallel for schedule(static)
+      for (size_t z = 0; z < nz; ++z) {
+        const uint32_t pa = F.packed[z];
+        const int c = (int)(pa >> 3), a = (int)(pa & 7u);
+        float cf;
+        std::memcpy(&cf, &c, sizeof(cf));
+        r[z] = make_float4(value(vert(c, a, 0)), value(vert(c, a, 1)), value(vert(c, a, 2)), cf);
+      }
+      out.upload(r);
+    };
+    auto geo_float = [&](DBuf<float4>& o4, DBuf<float>& o1) {
+      std::vector<float4> q(2 * n);
+      std::vector<float> l(n);
+#pragma omp parallel for schedule(static)
+      for (int c = 0; c < nc_; ++c) {
+        float b[9];
+        for (int k = 0; k < 9; ++k) b[k] = (float)vert(c, 1 + k / 3, k % 3);
+        q[(size_t)c] = make_float4(b[0], b[1], b[2], b[3]);
+        q[n + (size_t)c] = make_float4(b[4], b[5], b[6], b[7]);
+        l[(size_t)c] = b[8];
+      }
+      o4.upload(q);
+      o1.upload(l);
+    };
+    if constexpr (std::is_same<T, double>::value) {
+      std::vector<double> b[3];
+      std::vector<int32_t> cell(nz);
+      for (auto& v : b) v.resize(nz);
+#pragma omp parallel for schedule(static)
+      for (size_t z = 0; z < nz; ++z) {
+        const uint32_t pa = F.packed[z];
+        const int c = (int)(pa >> 3), a = (int)(pa & 7u);
+        cell[z] = c;
+        for (int d = 0; d < 3; ++d) b[d][z] = vert(c, a, d);
+      }
+      for (int d = 0; d < 3; ++d) sp_b_[d].upload(b[d]);
+      sp_cell_.upload(cell);
+      svert_.bx = sp_b_[0].p;
+      svert_.by = sp_b_[1].p;
+      svert_.bz = sp_b_[2].p;
+      svert_.cell = sp_cell_.p;
+      std::vector<double2> q(4 * n);
+      std::vector<double> l(n);
+#pragma omp parallel for schedule(static)
+      for (int c = 0; c < nc_; ++c) {
+        for (int k = 0; k < 4; ++k)
+          q[(size_t)k * n + (size_t)c] = make_double2(vert(c, 1 + 2 * k / 3, 2 * k % 3), vert(c, 1 + (2 * k + 1) / 3, (2 * k + 1) % 3));
+        l[(size_t)c] = vert(c, 3, 2);
+      }
+      sp_gd2_.upload(q);
+      sp_gd1_.upload(l);
+    }
+    if (std::is_same<TA, float>::value) {
+      records16(sp_rec16_, [](double v) { return (float)v; });
+      geo_float(sp_gf4_, sp_gf1_);
+    }
+    sp_rv_.alloc((size_t)std::max(nvert, 1));
+    sp_tau_.alloc(4 * n);
+    sp_w_.alloc(4 * (size_t)(nvert + 1));
+    NDS_CUDA(cudaMemset(sp_w_.p, 0, sp_w_.bytes()));
+    if (!kSame) {
+      sp_rvA_.alloc((size_t)std::max(nvert, 1));
+      sp_tauA_.alloc(4 * n);
+      sp_wA_.alloc(4 * (size_t)(nvert + 1));
+      NDS_CUDA(cudaMemset(sp_wA_.p, 0, sp_wA_.bytes()));
+    }
+    if (half) {
+      // B scaled by the power of two that puts its largest component at
+      // 2^14 .. 2^15 (the smallest normal half is 2^29 below)
+      double bmax = 0.0;
+#pragma omp parallel for schedule(static) reduction(max : bmax)
+      for (size_t z = 0; z < nz; ++z)
+        for (int d = 0; d < 3; ++d) bmax = std::max(bmax, std::abs(vert((int)(F.packed[z] >> 3), (int)(F.packed[z] & 7u), d)));
+      if (!std::isfinite(bmax)) throw std::runtime_error("FP16 operator copy: non-finite gradients");
+      bscale_ = bmax > 0.0 ? std::ldexp(1.0, 14 - (int)std::floor(std::log2(bmax))) : 1.0;
+      auto h = [&](double v) { return __float2half((float)(v * bscale_)); };
+      auto bits = [](__half x) {
+        unsigned short u;
+        std::memcpy(&u, &x, sizeof(u));
+        return (unsigned)u;
+      };
+      std::vector<int32_t> base((size_t)std::max(nvert, 1), 0);
+      int wide = 0;
+#pragma omp parallel for schedule(static) reduction(| : wide)
+      for (int v = 0; v < nvert; ++v) {
+        const int zb = off[(size_t)v], ze = off[(size_t)v + 1];
+        if (zb == ze) continue;
+        base[(size_t)v] = (int)(F.packed[(size_t)zb] >> 3);  // cells ascend
+        if ((int)(F.packed[(size_t)ze - 1] >> 3) - base[(size_t)v] > 65535) wide = 1;
+      }
+      if (!wide && !std::getenv("NDS_SELL_COL32")) {
+        std::vector<uint2> r(nz);
+#pragma omp parallel for schedule(static)
+        for (int v = 0; v < nvert; ++v)
+          for (int z = off[(size_t)v]; z < off[(size_t)v + 1]; ++z) {
+            const uint32_t pa = F.packed[(size_t)z];
+            const int c = (int)(pa >> 3), a = (int)(pa & 7u);
+            r[(size_t)z] = make_uint2(bits(h(vert(c, a, 0))) | bits(h(vert(c, a, 1))) << 16,
+                                      bits(h(vert(c, a, 2))) | (unsigned)(c - base[(size_t)v]) << 16);
+          }
+        sp_rec8_.upload(r);
+        sp_base_.upload(base);
+      } else {
+        records16(sp_rec16h_, [&](double v) { return __half2float(h(v)); });
+      }
+      std::vector<uint4> p(n);
+      std::vector<uint2> q(n);
+#pragma omp parallel for schedule(static)
+      for (int c = 0; c < nc_; ++c) {
+        unsigned w[6];
+        for (int k = 0; k < 6; ++k)
+          w[k] = bits(h(vert(c, 2 * k / 3, 2 * k % 3))) | bits(h(vert(c, (2 * k + 1) / 3, (2 * k + 1) % 3))) << 16;
+        p[(size_t)c] = make_uint4(w[0], w[1], w[2], w[3]);
+        q[(size_t)c] = make_uint2(w[4], w[5]);
+      }
+      sp_h4_.upload(p);
+      sp_h2_.upload(q);
+      sp_tauH_.alloc(4 * n);
+    }
   }
 
   // ------------------------------------------------------------------ helpers
@@ -929,9 +1122,48 @@ class Solver final : public ISolver {
     const __half* vh = nullptr;  // FP16 copy of the values, scaled by 1 / vinv
     double vinv = 1.0;
     const int16_t* ch = nullptr;  // CSR levels with vh: columns as deltas to the row
+    // fine operator in split form (sell is set too)
+    bool split = false, half = false;
+    k::SplitVerts sv{};
+    k::SplitCells sc{};
+    const V* rv = nullptr;
+    V* w = nullptr;
+    double wscale = 1.0, tinv = 1.0;
   };
+  // the two steps of a product in split form
+  template <int MODE, class V>
+  void split_launch(const OpView<V>& A, int grid, const V* x, const V* b, const V* den, double w, V* y, V* y2) {
+    const int gv = grid_for(8LL * A.sv.n);
+    if (A.sv.n > 0) {
+      if constexpr (std::is_same<V, double>::value)
+        k::split_vertex<V, k::REC_SOA><<<gv, kBlock, 0, st_>>>(A.sv, A.rv, x, A.w, V(A.wscale));
+      else if (A.sv.rec8)
+        k::split_vertex<V, k::REC_8><<<gv, kBlock, 0, st_>>>(A.sv, A.rv, x, A.w, V(A.wscale));
+      else
+        k::split_vertex<V, k::REC_16><<<gv, kBlock, 0, st_>>>(A.sv, A.rv, x, A.w, V(A.wscale));
+      NDS_LAUNCH();
+    }
+    auto cells = [&](auto mt) {
+      using MT = decltype(mt);
+      if (A.sc.nd16)
+        k::split_cell<V, MODE, true, MT><<<grid, kBlock, 0, st_>>>(A.sc, A.w, x, b, den, V(w), y, y2, part_.p, V(A.tinv));
+      else
+        k::split_cell<V, MODE, false, MT><<<grid, kBlock, 0, st_>>>(A.sc, A.w, x, b, den, V(w), y, y2, part_.p, V(A.tinv));
+    };
+    if constexpr (std::is_same<V, float>::value) {
+      if (A.half) {
+        cells(__half{});
+        return;
+      }
+    }
+    cells(V{});
+  }
   template <int MODE, class V>
   void sell_launch(const OpView<V>& A, int grid, const V* x, const V* b, const V* den, double w, V* y, V* y2) {
+    if (A.split) {
+      split_launch<MODE, V>(A, grid, x, b, den, w, y, y2);
+      return;
+    }
     if constexpr (std::is_same<V, float>::value) {
       if (A.vh) {
         if (A.s.dcol)
@@ -949,15 +1181,60 @@ class Solver final : public ISolver {
       k::sell_spmv<V, MODE, false><<<grid, kBlock, 0, st_>>>(A.s, A.v, x, b, den, V(w), y, y2, part_.p);
   }
   // physical operator (precision T) and the AMG's fine operator (precision TA)
-  OpView<T> fine_op() const { return {nc_, true, sell_, nullptr, nullptr, fval_.p, P_FINE_SPMV}; }
-  OpView<TA> fine_opA() const {
+  OpView<T> fine_op() {
+    OpView<T> A{nc_, true, sell_, nullptr, nullptr, fval_.p, P_FINE_SPMV};
+    if (split_) set_split(A, sp_rv_.p, sp_w_.p, sp_tau_.p);
+    return A;
+  }
+  // the split form in the precision of V (FP64 or FP32 data)
+  template <class V>
+  void set_split(OpView<V>& A, const V* rv, V* w, const V* tau) {
+    A.split = true;
+    A.sv = svert_;
+    A.sc = scell_;
+    A.rv = rv;
+    A.w = w;
+    A.sc.tau = tau;
+    if constexpr (std::is_same<V, double>::value) {
+      A.sc.g0 = sp_gd2_.p;
+      A.sc.g2 = sp_gd1_.p;
+    } else {
+      A.sv.rec16 = sp_rec16_.p;
+      A.sc.g0 = sp_gf4_.p;
+      A.sc.g1 = sp_gf4_.p + nc_;
+      A.sc.g2 = sp_gf1_.p;
+    }
+  }
+  OpView<TA> fine_opA() {
+    if (split_) {
+      if constexpr (kSame) {
+        OpView<TA> A = fine_op();
+        A.cat = P_FINE_AMG;
+        return A;
+      } else {
+        OpView<TA> A{nc_, true, sell_, nullptr, nullptr, nullptr, P_FINE_AMG};
+        set_split(A, (const TA*)sp_rvA_.p, sp_wA_.p, (const TA*)sp_tauA_.p);
+        return A;
+      }
+    }
     if constexpr (kSame) return {nc_, true, sell_, nullptr, nullptr, fval_.p, P_FINE_AMG};
     else return {nc_, true, sell_, nullptr, nullptr, fvalA_.p, P_FINE_AMG};
   }
   // the fine operator of the V-cycle: the FP16 copy when amg_half is on
-  OpView<TA> fine_opV() const {
+  OpView<TA> fine_opV() {
     OpView<TA> A = fine_opA();
-    if (fvalH_.p) {
+    if (split_ && half_on_) {
+      A.half = true;
+      A.sv.rec16 = sp_rec16h_.p;
+      A.sv.rec8 = sp_rec8_.p;
+      A.sv.base = sp_base_.p;
+      A.sc.g0 = sp_h4_.p;
+      A.sc.g1 = sp_h2_.p;
+      A.sc.tau = sp_tauH_.p;
+      A.wscale = 1.0 / (bscale_ * bscale_);
+      A.tinv = 1.0 / hscale_;
+      A.cat = P_FINE_HALF;
+    } else if (fvalH_.p) {
       A.vh = fvalH_.p;
       A.vinv = 1.0 / hscale_;
       A.cat = P_FINE_HALF;
@@ -1084,6 +1361,13 @@ class Solver final : public ISolver {
   void refresh_fine(const T* rau, cudaStream_t s = nullptr) {
     if (!s) s = st_;
     ProfScope ps(prof, s, P_REFRESH);
+    if (split_) {
+      k::split_refresh<T, TA><<<grid_for(std::max(nc_, svert_.n)), kBlock, 0, s>>>(
+          nc_, svert_.n, ref_.p, sp_g4_.p, rau, sp_rv_.p, kSame ? nullptr : sp_rvA_.p, sp_tau_.p,
+          kSame ? nullptr : sp_tauA_.p, half_on_ ? sp_tauH_.p : nullptr, (float)hscale_, fdiag_.p);
+      NDS_LAUNCH();
+      return;
+    }
     k::sell_refresh<T, TA><<<(nc_ + 31) / 32, k::kRefreshBlock, refresh_smem_, s>>>(
         nc_, fcoff_.p, fcs_.p, fgeo_.p, ref_.p, rau, fdslot_.p, sbase_.p, swidth_.p, fval_.p,
         kSame ? nullptr : fvalA_.p, fdiag_.p, fl1_.p, fvalH_.p, (float)hscale_);
@@ -1615,9 +1899,22 @@ class Solver final : public ISolver {
       add(M.owner[f], M.neighbour[f]);
       add(M.neighbour[f], M.owner[f]);
     }
+    if (split_) {
+      // position of each face in its cell (the edge weights' face couplings)
+      std::vector<uint8_t> face(4 * (size_t)nc_, 0);
+      std::vector<int> at((size_t)nc_, 0);
+      auto local = [&](int c, size_t f) {
+        for (int a = 0; a < 4; ++a)
+          if ((size_t)M.opp[(size_t)c][(size_t)a] == f) return (uint8_t)a;
+        throw std::runtime_error("learned stage: a face missing from its cell");
+      };
+      for (size_t f = 0; f < M.neighbour.size(); ++f)
+        for (const int c : {M.owner[f], M.neighbour[f]}) face[4 * (size_t)c + (size_t)at[(size_t)c]++] = local(c, f);
+      sg_face_.upload(face);
+    }
     std::vector<int32_t> base((size_t)(nc_ + 31) / 32 + 1);
-    NDS_CUDA(cudaMemcpy(base.data(), sbase_.p, sizeof(int32_t) * base.size(), cudaMemcpyDeviceToHost));
-    for (int i = 0; i < nc_; ++i)
+    if (!split_) NDS_CUDA(cudaMemcpy(base.data(), sbase_.p, sizeof(int32_t) * base.size(), cudaMemcpyDeviceToHost));
+    for (int i = 0; i < nc_ && !split_; ++i)
       for (int k = 0; k < 4; ++k) {
         const int j = nbr[4 * (size_t)i + k];
         if (j < 0) continue;
@@ -1628,7 +1925,7 @@ class Solver final : public ISolver {
         off[4 * (size_t)i + k] = base[(size_t)(i >> 5)] + 128 * (pos >> 2) + 4 * (i & 31) + (pos & 3);
       }
     sg_nbr_.upload(nbr);
-    sg_off_.upload(off);
+    if (!split_) sg_off_.upload(off);
     sg_ew_.alloc(4 * (size_t)nc_);
     sg_dscale_.alloc((size_t)nc_);
     st_z1_.alloc((size_t)nc_);
@@ -1641,7 +1938,11 @@ class Solver final : public ISolver {
     if constexpr (!kSame) {
       stage_dscale<<<grid_for(nc_), kBlock, 0, st_>>>(nc_, fdiag_.p, sg_dscale_.p);
       NDS_LAUNCH();
-      stage_edges<<<grid_for(4LL * nc_), kBlock, 0, st_>>>(nc_, sg_nbr_.p, sg_off_.p, fvalA_.p, sg_dscale_.p, sg_ew_.p);
+      if (split_)
+        k::split_edges<T><<<grid_for(4LL * nc_), kBlock, 0, st_>>>(nc_, sg_nbr_.p, sg_face_.p, ref_.p, bco_.p,
+                                                                   sp_rv_.p, sp_tau_.p, sg_dscale_.p, sg_ew_.p);
+      else
+        stage_edges<<<grid_for(4LL * nc_), kBlock, 0, st_>>>(nc_, sg_nbr_.p, sg_off_.p, fvalA_.p, sg_dscale_.p, sg_ew_.p);
       NDS_LAUNCH();
     }
   }
@@ -2417,6 +2718,23 @@ class Solver final : public ISolver {
   k::Sell sell_{};
   long long sell_nnz_ = 0;
   std::vector<int> fine_coff_;
+  // split form of the pressure operator
+  bool split_ = false, half_on_ = false;
+  k::SplitVerts svert_{};
+  k::SplitCells scell_{};
+  double bscale_ = 1.0;
+  DBuf<int32_t> sp_off_, sp_cell_, sp_base_;
+  DBuf<int4> sp_vid_, sp_nid_;
+  DBuf<short4> sp_nd16_;
+  DBuf<T> sp_g4_, sp_rv_, sp_tau_, sp_w_;
+  DBuf<TA> sp_rvA_, sp_tauA_, sp_wA_;
+  DBuf<double> sp_b_[3], sp_gd1_;
+  DBuf<double2> sp_gd2_;
+  DBuf<float4> sp_rec16_, sp_rec16h_, sp_gf4_;
+  DBuf<float> sp_gf1_;
+  DBuf<uint2> sp_rec8_, sp_h2_;
+  DBuf<uint4> sp_h4_;
+  DBuf<__half> sp_tauH_;
   DBuf<uint16_t> fcs_;
   DBuf<int> ctl_;
 
@@ -2439,6 +2757,7 @@ class Solver final : public ISolver {
   // the edges, edge weights, Jacobi scaling), work vectors, counters
   MpnnPtr stage_;
   DBuf<int32_t> sg_nbr_, sg_off_;
+  DBuf<uint8_t> sg_face_;
   DBuf<float> sg_ew_, sg_dscale_, st_z1_, st_t_;
   DBuf<unsigned long long> st_cnt_;
   DBuf<double> part_, sc_;

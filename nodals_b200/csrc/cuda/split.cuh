@@ -1,0 +1,367 @@
+// The fine Schur operator A = B diag(rAU) B^T in split form.
+//
+// A pressure cell reaches its neighbours through two kinds of velocity
+// unknowns (B[c][a][d], gpu/serial_cuda/g2_host.hpp:67-76):
+//  * a face bubble belongs to the two cells of its face and to nothing else,
+//    and the two rows of B are opposite (the face's area vector), so the
+//    bubbles give a face Laplacian with tau_f = rAU_f |B[c][f]|^2:
+//    sum_f tau_f (x_c - x_neighbour), or tau_f x_c on an outlet face;
+//  * a vertex function's rows are V grad(lambda_a): w_v = rAU_v sum_(c,a at v)
+//    B[c][a] x_c per free vertex, then sum_a B[c][a] . w_v(a) per cell.
+// The product is taken in these two steps (split_vertex, split_cell) instead
+// of from assembled rows.  An assembled row of the pipe meshes has 69.5
+// entries (nearly all through the vertices: 24 cells around each), that is
+// 278 bytes a cell in FP16 with 16-bit column deltas, 417 in FP32 and 695 in
+// FP64; the two steps read 32 + 56, 64 + 84 and 112 + 136 bytes a cell, and
+// the refresh writes 4 tau a cell where the assembled form rewrites every
+// entry.  Smoothers that need the entries of a row (multicolour Gauss-Seidel,
+// L1-Jacobi) keep the assembled SELL form.
+//
+// Both steps are bound by HBM on large meshes and by their two dependent
+// memory round trips on small ones: every load of a step that does not
+// depend on another is issued first.
+#pragma once
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include <cstdint>
+#include <type_traits>
+
+#include "common.cuh"
+#include "kernels.cuh"
+
+namespace nds {
+namespace k {
+
+// |B of a face bubble|^2 / |B of the opposite vertex|^2
+constexpr double kBubble2 = (27.0 / 20.0) * (27.0 / 20.0);
+
+// Incidences of the free vertices, CSR by vertex (off), ascending cell; per
+// incidence the vector B[c][a] and the cell.
+//  double: component arrays bx, by, bz and the cells
+//  float:  one 16-byte record (x, y, z, cell)
+//  __half: one 8-byte record of three scaled halves and the cell's 16-bit
+//          offset from the vertex's first cell (base); meshes whose
+//          numbering does not allow that keep the halves' values in the
+//          16-byte records (rec8 null)
+struct SplitVerts {
+  int n = 0;
+  const int32_t* off = nullptr;
+  const double* bx = nullptr;
+  const double* by = nullptr;
+  const double* bz = nullptr;
+  const int32_t* cell = nullptr;
+  const float4* rec16 = nullptr;
+  const uint2* rec8 = nullptr;
+  const int32_t* base = nullptr;
+};
+enum SplitRec { REC_SOA = 0, REC_16 = 1, REC_8 = 2 };
+
+// w_v = scale rAU_v sum B x over the vertex's cells, eight lanes a vertex
+// (24 incidences on average: four records in flight per lane cover 32 in one
+// round).  w holds 4 values a vertex; entry n stays zero (fixed vertices).
+constexpr int kSplitAhead = 4;
+template <class V, int REC>
+__global__ void __launch_bounds__(kBlock) split_vertex(SplitVerts a, const V* __restrict__ rau,
+                                                       const V* __restrict__ x, V* __restrict__ w, V scale) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int g = t >> 3, lane = t & 7;
+  if (g >= a.n) return;
+  const unsigned mask = group8_mask();
+  const int zb = a.off[g], ze = a.off[g + 1];
+  int c0 = 0;
+  if (REC == REC_8) c0 = a.base[g];
+  V r = 0;
+  if (lane == 0) r = scale * rau[g];
+  V s0 = 0, s1 = 0, s2 = 0;
+  for (int z0 = zb + lane; z0 < ze; z0 += 8 * kSplitAhead) {
+    V b0[kSplitAhead], b1[kSplitAhead], b2[kSplitAhead], xv[kSplitAhead];
+    int c[kSplitAhead];
+#pragma unroll
+    for (int u = 0; u < kSplitAhead; ++u) {
+      const int z = z0 + 8 * u;
+      const bool ok = z < ze;
+      c[u] = -1;
+      b0[u] = b1[u] = b2[u] = V(0);
+      if constexpr (REC == REC_SOA) {
+        if (ok) {
+          b0[u] = V(a.bx[z]);
+          b1[u] = V(a.by[z]);
+          b2[u] = V(a.bz[z]);
+          c[u] = a.cell[z];
+        }
+      } else if constexpr (REC == REC_16) {
+        if (ok) {
+          const float4 q = a.rec16[z];
+          b0[u] = q.x;
+          b1[u] = q.y;
+          b2[u] = q.z;
+          c[u] = __float_as_int(q.w);
+        }
+      } else {
+        if (ok) {
+          const uint2 q = a.rec8[z];
+          const float2 xy = __half22float2(*reinterpret_cast<const __half2*>(&q.x));
+          b0[u] = xy.x;
+          b1[u] = xy.y;
+          b2[u] = __half2float(__ushort_as_half((unsigned short)(q.y & 0xFFFFu)));
+          c[u] = c0 + (int)(q.y >> 16);
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kSplitAhead; ++u) xv[u] = c[u] >= 0 ? x[c[u]] : V(0);
+#pragma unroll
+    for (int u = 0; u < kSplitAhead; ++u) {
+      s0 += b0[u] * xv[u];
+      s1 += b1[u] * xv[u];
+      s2 += b2[u] * xv[u];
+    }
+  }
+  s0 = group_sum<8>(s0, mask);
+  s1 = group_sum<8>(s1, mask);
+  s2 = group_sum<8>(s2, mask);
+  if (lane == 0) {
+    if constexpr (std::is_same<V, float>::value) {
+      reinterpret_cast<float4*>(w)[g] = make_float4(r * s0, r * s1, r * s2, 0.f);
+    } else {
+      reinterpret_cast<double2*>(w)[2 * (size_t)g] = make_double2(r * s0, r * s1);
+      w[4 * (size_t)g + 2] = r * s2;
+    }
+  }
+}
+
+// Cell data of the second step, structure of arrays of vector loads:
+//  vid: the four vertices (n_vertices for a fixed one); nid / nd16: the four
+//  face neighbours, absolute (-1: none) or as 16-bit deltas to the cell (0:
+//  none) when they all fit; tau: the four face couplings (0 on a fixed face).
+//  geo: B of the vertices 1, 2, 3 (the four sum to zero): float 4 + 4 + 1,
+//  double 2 + 2 + 2 + 2 + 1; __half: all four, scaled, in 8 + 4 values, each
+//  rounded as in the vertex records, so that the FP16 operator is symmetric.
+//  A free face without a neighbour (outlet) couples as tau x_c.
+struct SplitCells {
+  int n = 0;
+  const int4* vid = nullptr;
+  const int4* nid = nullptr;
+  const short4* nd16 = nullptr;
+  const void* g0 = nullptr;
+  const void* g1 = nullptr;
+  const void* g2 = nullptr;
+  const void* tau = nullptr;
+};
+
+// sum of cell c's row products: vertices from w, faces from x (xc = x[c])
+template <class V, class MT, bool D16>
+__device__ __forceinline__ V split_row(const SplitCells& a, const V* __restrict__ x, const V* __restrict__ w, int c,
+                                       V xc, V tinv) {
+  const int4 vi = a.vid[c];
+  int nb[4];
+  if (D16) {
+    const short4 d = a.nd16[c];
+    nb[0] = d.x ? c + d.x : -1;
+    nb[1] = d.y ? c + d.y : -1;
+    nb[2] = d.z ? c + d.z : -1;
+    nb[3] = d.w ? c + d.w : -1;
+  } else {
+    const int4 d = a.nid[c];
+    nb[0] = d.x;
+    nb[1] = d.y;
+    nb[2] = d.z;
+    nb[3] = d.w;
+  }
+  V t[4];
+  V s = 0;
+  if constexpr (std::is_same<MT, __half>::value) {
+    const uint2 th = static_cast<const uint2*>(a.tau)[c];
+    const uint4 p = static_cast<const uint4*>(a.g0)[c];
+    const uint2 q = static_cast<const uint2*>(a.g1)[c];
+    float4 wv[4];
+    const float4* w4 = reinterpret_cast<const float4*>(w);
+    wv[0] = w4[vi.x];
+    wv[1] = w4[vi.y];
+    wv[2] = w4[vi.z];
+    wv[3] = w4[vi.w];
+    V xn[4];
+#pragma unroll
+    for (int f = 0; f < 4; ++f) xn[f] = nb[f] >= 0 ? x[nb[f]] : V(0);
+    auto h2 = [](unsigned u) { return __half22float2(*reinterpret_cast<const __half2*>(&u)); };
+    const float2 b01 = h2(p.x), b23 = h2(p.y), b45 = h2(p.z), b67 = h2(p.w), b89 = h2(q.x), bab = h2(q.y);
+    s = b01.x * wv[0].x + b01.y * wv[0].y + b23.x * wv[0].z;
+    s += b23.y * wv[1].x + b45.x * wv[1].y + b45.y * wv[1].z;
+    s += b67.x * wv[2].x + b67.y * wv[2].y + b89.x * wv[2].z;
+    s += b89.y * wv[3].x + bab.x * wv[3].y + bab.y * wv[3].z;
+    const float2 t01 = h2(th.x), t23 = h2(th.y);
+    t[0] = t01.x;
+    t[1] = t01.y;
+    t[2] = t23.x;
+    t[3] = t23.y;
+    V f = 0;
+#pragma unroll
+    for (int q4 = 0; q4 < 4; ++q4) f += t[q4] * (xc - xn[q4]);
+    s += tinv * f;
+  } else {
+    V b[9], wv[4][3];
+    if constexpr (std::is_same<V, float>::value) {
+      const float4 p = static_cast<const float4*>(a.g0)[c], q = static_cast<const float4*>(a.g1)[c];
+      b[0] = p.x; b[1] = p.y; b[2] = p.z; b[3] = p.w;
+      b[4] = q.x; b[5] = q.y; b[6] = q.z; b[7] = q.w;
+      b[8] = static_cast<const float*>(a.g2)[c];
+      const float4 tt = static_cast<const float4*>(a.tau)[c];
+      t[0] = tt.x; t[1] = tt.y; t[2] = tt.z; t[3] = tt.w;
+      const float4* w4 = reinterpret_cast<const float4*>(w);
+      const int vv[4] = {vi.x, vi.y, vi.z, vi.w};
+#pragma unroll
+      for (int q4 = 0; q4 < 4; ++q4) {
+        const float4 u = w4[vv[q4]];
+        wv[q4][0] = u.x; wv[q4][1] = u.y; wv[q4][2] = u.z;
+      }
+    } else {
+      const double2* g = static_cast<const double2*>(a.g0);
+      const size_t n = (size_t)a.n;
+#pragma unroll
+      for (int q4 = 0; q4 < 4; ++q4) {
+        const double2 p = g[q4 * n + c];
+        b[2 * q4] = p.x;
+        b[2 * q4 + 1] = p.y;
+      }
+      b[8] = static_cast<const double*>(a.g2)[c];
+      const double2* tp = static_cast<const double2*>(a.tau) + 2 * (size_t)c;
+      const double2 ta = tp[0], tb = tp[1];
+      t[0] = ta.x; t[1] = ta.y; t[2] = tb.x; t[3] = tb.y;
+      const double2* w2 = reinterpret_cast<const double2*>(w);
+      const int vv[4] = {vi.x, vi.y, vi.z, vi.w};
+#pragma unroll
+      for (int q4 = 0; q4 < 4; ++q4) {
+        const double2 u = w2[2 * (size_t)vv[q4]];
+        wv[q4][0] = u.x; wv[q4][1] = u.y;
+        wv[q4][2] = w[4 * (size_t)vv[q4] + 2];
+      }
+    }
+    V xn[4];
+#pragma unroll
+    for (int f = 0; f < 4; ++f) xn[f] = nb[f] >= 0 ? x[nb[f]] : V(0);
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+#pragma unroll
+      for (int d = 0; d < 3; ++d) s += b[3 * j + d] * (wv[j + 1][d] - wv[0][d]);
+    V f = 0;
+#pragma unroll
+    for (int q4 = 0; q4 < 4; ++q4) f += t[q4] * (xc - xn[q4]);
+    s += f;
+  }
+  return s;
+}
+
+// The modes of sell_spmv on the split form (w from split_vertex on the same
+// x); MODE SELL_DOT walks the cells grid-stride and leaves partials of x.y.
+template <class V, int MODE, bool D16, class MT = V>
+__global__ void __launch_bounds__(kBlock) split_cell(SplitCells a, const V* __restrict__ w, const V* __restrict__ x,
+                                                     const V* __restrict__ b, const V* __restrict__ den, V wt,
+                                                     V* __restrict__ y, V* __restrict__ y2, double* __restrict__ part,
+                                                     V tinv) {
+  if (MODE == SELL_DOT) {
+    double acc[1] = {0.0};
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < a.n; c += gridDim.x * blockDim.x) {
+      const V xc = x[c];
+      const V s = split_row<V, MT, D16>(a, x, w, c, xc, tinv);
+      y[c] = s;
+      acc[0] += (double)xc * (double)s;
+    }
+    write_partials<1>(acc, part);
+    return;
+  }
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= a.n) return;
+  const V xc = x[c];
+  V bc = 0, dc = 1;
+  if (MODE != SELL_Y) {
+    bc = b[c];
+    if (MODE == SELL_SMOOTH || den) dc = den[c];
+  }
+  const V s = split_row<V, MT, D16>(a, x, w, c, xc, tinv);
+  if (MODE == SELL_Y) {
+    y[c] = s;
+  } else if (MODE == SELL_RESID) {
+    const V q = bc - s;
+    y[c] = q;
+    if (den) y2[c] = wt * q / dc;
+    else if (y2) y2[c] = q;
+  } else {
+    const V val = xc + wt * (bc - s) / dc;
+    if (y2) y2[c] += val;
+    else y[c] = val;
+  }
+}
+
+// Refresh of the split form from rAU: thread c writes cell c's face couplings
+// in the precisions in use (g4: |B|^2 of the four vertices, static) and the
+// diagonal A_cc = sum_i |B_i|^2 (rAU_vertex + kBubble2 rAU_face); threads
+// below nvert also copy the vertices' rAU.  rv and tau in the operator's
+// precision T; rvA and tauA (FP32, the mixed modes) and tauH (FP16, scaled
+// and saturated) may be null.
+template <class T, class TA>
+__global__ void __launch_bounds__(kBlock) split_refresh(int nc, int nvert, const int32_t* __restrict__ ref,
+                                                        const T* __restrict__ g4, const T* __restrict__ rau,
+                                                        T* __restrict__ rv, TA* __restrict__ rvA,
+                                                        T* __restrict__ tau, TA* __restrict__ tauA,
+                                                        __half* __restrict__ tauH, float hscale,
+                                                        TA* __restrict__ diag) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c < nvert) {
+    const T r = rau[c];
+    rv[c] = r;
+    if (rvA) rvA[c] = TA(r);
+  }
+  if (c >= nc) return;
+  const int4* r4 = reinterpret_cast<const int4*>(ref + 8 * (size_t)c);
+  const int4 v = r4[0], f = r4[1];
+  const int vi[4] = {v.x, v.y, v.z, v.w}, fi[4] = {f.x, f.y, f.z, f.w};
+  T g[4], rvv[4], rf[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    g[i] = g4[(size_t)i * nc + c];
+    rvv[i] = vi[i] >= 0 ? rau[vi[i]] : T(0);
+    rf[i] = fi[i] >= 0 ? rau[fi[i]] : T(0);
+  }
+  T d = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const T t = T(kBubble2) * g[i] * rf[i];
+    d += rvv[i] * g[i] + t;
+    tau[4 * (size_t)c + i] = t;
+    if (tauA) tauA[4 * (size_t)c + i] = TA(t);
+    if (tauH) tauH[4 * (size_t)c + i] = __float2half_rn(fminf((float)t * hscale, 65504.f));
+  }
+  diag[c] = TA(d);
+}
+
+// a_ij of the face neighbours of each cell, off[4 i + k] = face k's position
+// in the cell (its opposite vertex): the face coupling plus the shared
+// vertices' part, from the operator's own data in its precision
+template <class T>
+__global__ void split_edges(int n, const int32_t* __restrict__ nbr, const uint8_t* __restrict__ face,
+                            const int32_t* __restrict__ ref, const T* __restrict__ bco, const T* __restrict__ rv,
+                            const T* __restrict__ tau, const float* __restrict__ dscale, float* __restrict__ ew) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 4 * n) return;
+  const int i = t >> 2, j = nbr[t];
+  if (j < 0) {
+    ew[t] = 0.f;
+    return;
+  }
+  T s = -tau[4 * (size_t)i + face[t]];
+  for (int a = 0; a < 4; ++a) {
+    const int g = ref[8 * (size_t)i + a];
+    if (g < 0) continue;
+    for (int b = 0; b < 4; ++b)
+      if (ref[8 * (size_t)j + b] == g) {
+        const T* p = bco + 24 * (size_t)i + 3 * a;
+        const T* q = bco + 24 * (size_t)j + 3 * b;
+        s += rv[g] * (p[0] * q[0] + p[1] * q[1] + p[2] * q[2]);
+      }
+  }
+  ew[t] = (float)s * dscale[i] * dscale[j];
+}
+
+}  // namespace k
+}  // namespace nds

@@ -898,17 +898,109 @@ __global__ void prolong_add(int nf, int pw, const int32_t* __restrict__ pc, cons
   }
   f[i] += s;
 }
-// x = Ainv b, dense row-major, warp per row
+// ---------------------------------------------------------------------------
+// Dense form of the V-cycle from a level down: the explicit levels never
+// change after setup, so the cycle from level l on is one constant matrix
+// M_l.  Its columns are the cycle applied to the unit vectors, all at once on
+// row-major n x m blocks (column j of the block is the vector of unit vector
+// j): a row of the level matrix is read once for all columns, and the columns
+// lie contiguous for the threads.
+// ---------------------------------------------------------------------------
+// epilogues of block_spmm: the modes of spmv / spmv_resid / spmv_smooth and
+// of the transfers
+enum { BLK_Y = 0, BLK_RESID = 1, BLK_SMOOTH = 2, BLK_ADD = 3 };
+template <class T, class MT, class CT, int MODE>
+__global__ void __launch_bounds__(kBlock) block_spmm(int n, int m, const int32_t* __restrict__ rp,
+                                                     const CT* __restrict__ ci, const MT* __restrict__ v, T vinv,
+                                                     const T* __restrict__ x, const T* __restrict__ b,
+                                                     const T* __restrict__ den, T w, T* __restrict__ y) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= m) return;
+  for (int i = blockIdx.y; i < n; i += gridDim.y) {
+    T s = 0;
+    for (int k = rp[i]; k < rp[i + 1]; ++k) s += load_val<T, MT>(v, k) * x[(size_t)col_at(ci, k, i) * m + j];
+    if constexpr (!std::is_same<MT, T>::value) s *= vinv;
+    const size_t o = (size_t)i * m + j;
+    if (MODE == BLK_Y) y[o] = s;
+    else if (MODE == BLK_ADD) y[o] += s;
+    else if (MODE == BLK_RESID) y[o] = b[o] - s;
+    else y[o] = x[o] + w * (b[o] - s) / den[i];
+  }
+}
+// y += P x, P in ELL (entry k of row i at k n + i)
 template <class T>
-__global__ void __launch_bounds__(kBlock) dense_mv(int n, const T* __restrict__ A, const T* __restrict__ b,
-                                                   T* __restrict__ x) {
-  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (i >= n) return;
-  const T* a = A + (size_t)i * n;
+__global__ void __launch_bounds__(kBlock) block_prolong_add(int n, int m, int pw, const int32_t* __restrict__ pc,
+                                                            const T* __restrict__ pv, const T* __restrict__ x,
+                                                            T* __restrict__ y) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= m) return;
+  for (int i = blockIdx.y; i < n; i += gridDim.y) {
+    T s = 0;
+    for (int k = 0; k < pw; ++k) s += pv[(size_t)k * n + i] * x[(size_t)pc[(size_t)k * n + i] * m + j];
+    y[(size_t)i * m + j] += s;
+  }
+}
+// y = A x with a dense n x n A (row stride ld)
+template <class T>
+__global__ void __launch_bounds__(kBlock) block_dense(int n, int ld, int m, const T* __restrict__ A, const T* __restrict__ x,
+                                                      T* __restrict__ y) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= m) return;
+  for (int i = blockIdx.y; i < n; i += gridDim.y) {
+    T s = 0;
+    for (int k = 0; k < n; ++k) s += A[(size_t)i * ld + k] * x[(size_t)k * m + j];
+    y[(size_t)i * m + j] = s;
+  }
+}
+// y = w b / den by rows; unit blocks; y += x
+template <class T>
+__global__ void block_jacobi(size_t total, int m, T w, const T* __restrict__ b, const T* __restrict__ den,
+                             T* __restrict__ y) {
+  const size_t o = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (o < total) y[o] = w * b[o] / den[o / m];
+}
+template <class T>
+__global__ void block_unit(size_t total, int m, T* __restrict__ y) {
+  const size_t o = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (o < total) y[o] = T(o / m == o % m ? 1 : 0);
+}
+template <class T>
+__global__ void block_add(size_t total, const T* __restrict__ x, T* __restrict__ y) {
+  const size_t o = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (o < total) y[o] += x[o];
+}
+
+// y = A x with a dense row-major n x ld A (ld a multiple of 4, rows padded
+// with zeros, x readable up to ld): a block of kDenseWarps warps per row, so
+// that a few thousand rows of 10 to 40 KB keep every SM's loads in flight;
+// 16-byte loads.  Fixed order: lanes, then warps.
+constexpr int kDenseWarps = 4;
+template <class T>
+__global__ void __launch_bounds__(32 * kDenseWarps) dense_rows(int n, int ld, const T* __restrict__ A,
+                                                               const T* __restrict__ b, T* __restrict__ x) {
+  constexpr int W = 16 / sizeof(T);
+  using V = typename std::conditional<std::is_same<T, float>::value, float4, double2>::type;
+  __shared__ T part[kDenseWarps];
+  const int i = blockIdx.x;
+  const V* a = reinterpret_cast<const V*>(A + (size_t)i * ld);
+  const V* bb = reinterpret_cast<const V*>(b);
   T s = 0;
-  for (int j = lane; j < n; j += 32) s += a[j] * b[j];
+  const int nv = ld / W;
+#pragma unroll 4
+  for (int k = threadIdx.x; k < nv; k += 32 * kDenseWarps) {
+    const V p = a[k], q = bb[k];
+    if constexpr (W == 4) s += p.x * q.x + p.y * q.y + p.z * q.z + p.w * q.w;
+    else s += p.x * q.x + p.y * q.y;
+  }
   s = warp_sum(s);
-  if (lane == 0) x[i] = s;
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    T r = part[0];
+#pragma unroll
+    for (int q = 1; q < kDenseWarps; ++q) r += part[q];
+    x[i] = r;
+  }
 }
 
 // multicolour GS colour pass on an AMG level (h8_main_base.cu:205-223)

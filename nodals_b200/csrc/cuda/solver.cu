@@ -497,7 +497,9 @@ class Solver final : public ISolver {
         l1h[(size_t)i] = ss;
       }
       Lv.l1.upload(l1h);
-      for (auto* b : {&Lv.b, &Lv.x, &Lv.r, &Lv.tmp, &Lv.corr, &Lv.pong}) b->alloc((size_t)A.n);
+      for (auto* b : {&Lv.x, &Lv.r, &Lv.tmp, &Lv.corr, &Lv.pong}) b->alloc((size_t)A.n);
+      Lv.b.alloc(dense_ld(A.n));  // the dense form reads up to the padding, which stays zero
+      NDS_CUDA(cudaMemset(Lv.b.p, 0, Lv.b.bytes()));
       // the mixed path's V-cycle reads FP16 copies of the explicit levels
       // (the terminal level goes through its dense inverse)
       if (!kSame && o_.precision == NDS_MIXED && o_.amg_half && l + 1 < H.A.size()) level_to_half(Lv, A);
@@ -548,7 +550,14 @@ class Solver final : public ISolver {
       X.rcol.upload(rc);
       X.rval.upload(rv);
     }
-    tinv_.upload(H.terminal_inv);
+    if (!L_.empty()) {  // rows padded for 16-byte loads
+      const int n = L_.back().n;
+      const size_t ld = dense_ld(n);
+      std::vector<double> t(ld * (size_t)n, 0.0);
+      for (int i = 0; i < n; ++i)
+        std::copy_n(H.terminal_inv.begin() + (size_t)i * n, (size_t)n, t.begin() + (size_t)i * ld);
+      tinv_.upload(t);
+    }
     fine_lambda_ = H.fine_lambda;
     level_lambda_ = H.level_lambda;
     level_lambda_.resize(L_.size(), 0.0);
@@ -590,6 +599,7 @@ class Solver final : public ISolver {
       fine_lambda_ = 1.0;
       for (auto& v : level_lambda_) v = 1.0;
     }
+    build_dense_level();
     if (o_.pressure_solver == NDS_P_CHEB) p_cheb_lambda_ = precond_power(o_.p_power_its, o_.p_power_safety);
     NDS_CUDA(cudaStreamSynchronize(st_));
     tm.mark("refresh_and_spectrum");
@@ -1482,7 +1492,7 @@ class Solver final : public ISolver {
   }
   // whether the pre-smoother of level l can take its diagonal step in the
   // restriction that feeds it (a polynomial smoother, not the terminal level)
-  bool fuse_pre(int l) const { return o_.amg_smoother != NDS_SM_MCGS && l < (int)L_.size() - 1; }
+  bool fuse_pre(int l) const { return o_.amg_smoother != NDS_SM_MCGS && l < (int)L_.size() - 1 && l != dense_level_; }
   // lanes per coarse row of the restriction (the FP16 levels' count on the
   // mixed FP16 path, a warp otherwise)
   int restrict_lanes() const { return mixed_ && o_.amg_half ? level_lanes_ : 32; }
@@ -1520,14 +1530,120 @@ class Solver final : public ISolver {
     NDS_LAUNCH();
   }
 
+  // ------------------------------------------- dense form of coarse levels
+  // The first level whose V-cycle matrix takes at most kDenseBytes is applied
+  // as that matrix (polynomial smoothers; not the terminal level, which is
+  // dense already).  One product replaces the level's four SpMVs and all
+  // launches below it.  Microseconds of a PCG iteration, level by level /
+  // dense: 278 rows (0.3 MB) 66.5 / 51.9, 2,090 FP64 (35 MB) 72.5 / 58.3,
+  // 2,893 FP32 (33 MB) 81.4 / 65.1, 1,449 FP32 below 23,192 (8 MB) 195 / 179,
+  // 2,893 FP64 (67 MB) 75.6 / 72.9, 4,660 FP32 (87 MB) 390 / 382; nothing
+  // gained at 104 MB (3,614 FP64) and 174 MB (4,660 FP64), hence the limit.
+  // NDS_DENSE_MB overrides it (0: none).
+  static constexpr size_t kDenseBytes = (size_t)96 << 20;
+  static size_t dense_ld(int n) { return ((size_t)n + 3) / 4 * 4; }
+  void build_dense_level() {
+    dense_level_ = -1;
+    if (o_.amg_smoother == NDS_SM_MCGS) return;
+    const size_t lim = std::getenv("NDS_DENSE_MB") ? (size_t)std::atoi(std::getenv("NDS_DENSE_MB")) << 20 : kDenseBytes;
+    int l = 0;
+    const int last = (int)L_.size() - 1;
+    while (l < last && dense_ld(L_[(size_t)l].n) * (size_t)L_[(size_t)l].n * sizeof(TA) > lim) ++l;
+    if (l >= last) return;
+    const int m = L_[(size_t)l].n;
+    std::vector<DBuf<TA>> B((size_t)(last - l + 1)), X((size_t)(last - l + 1));
+    for (int q = l; q <= last; ++q) {
+      B[(size_t)(q - l)].alloc((size_t)L_[(size_t)q].n * m);
+      X[(size_t)(q - l)].alloc((size_t)L_[(size_t)q].n * m);
+    }
+    DBuf<TA> r, t0, t1;
+    for (auto* b : {&r, &t0, &t1}) b->alloc((size_t)m * m);
+    const size_t total = (size_t)m * m;
+    k::block_unit<TA><<<grid_for((long long)total), kBlock, 0, st_>>>(total, m, B[0].p);
+    NDS_LAUNCH();
+    block_cycle(l, l, m, B, X, r.p, t0.p, t1.p);
+    const size_t ld = dense_ld(m);
+    dense_.alloc(ld * (size_t)m);
+    NDS_CUDA(cudaMemsetAsync(dense_.p, 0, dense_.bytes(), st_));
+    NDS_CUDA(cudaMemcpy2DAsync(dense_.p, ld * sizeof(TA), X[0].p, (size_t)m * sizeof(TA), (size_t)m * sizeof(TA),
+                               (size_t)m, cudaMemcpyDeviceToDevice, st_));
+    NDS_CUDA(cudaStreamSynchronize(st_));
+    dense_level_ = l;
+  }
+  dim3 block_grid(int n, int m) const { return dim3((unsigned)grid_for(m), (unsigned)std::min(n, 65535)); }
+  // y = epilogue(A x) of level q on m columns, with the values the level's SpMVs read
+  template <int MODE>
+  void block_op(const Level& A, int m, const TA* x, const TA* b, const TA* den, double w, TA* y) {
+    const dim3 g = block_grid(A.n, m);
+    auto run = [&](auto* ci, auto* v, double vinv) {
+      using CT = std::remove_const_t<std::remove_pointer_t<decltype(ci)>>;
+      using MT = std::remove_const_t<std::remove_pointer_t<decltype(v)>>;
+      k::block_spmm<TA, MT, CT, MODE><<<g, kBlock, 0, st_>>>(A.n, m, A.row.p, ci, v, TA(vinv), x, b, den, TA(w), y);
+    };
+    if (A.hval.p && A.hcol.p) run(A.hcol.p, A.hval.p, A.hinv);
+    else if (A.hval.p) run(A.col.p, A.hval.p, A.hinv);
+    else run(A.col.p, A.val.p, 1.0);
+    NDS_LAUNCH();
+  }
+  // x = S b of level q (poly_smooth on m columns; t the second buffer).  The
+  // last step writes x.
+  void block_smooth(int q, int m, const TA* b, TA* x, TA* t) {
+    const Level& A = L_[(size_t)q];
+    const PolyPlan pl = level_plan(q);
+    const bool cheb = o_.amg_smoother == NDS_SM_CHEB2;
+    const double lam = level_lambda_[(size_t)q], lo = cheb ? o_.amg_lambda_low_fraction * lam : 0.0;
+    const size_t total = (size_t)A.n * m;
+    TA* cur = poly_first(pl, x, t);
+    TA* nxt = cur == x ? t : x;
+    k::block_jacobi<TA><<<grid_for((long long)total), kBlock, 0, st_>>>(total, m, TA(pl.w0), b, pl.den0, cur);
+    NDS_LAUNCH();
+    for (int kk = 1; kk <= pl.m; ++kk) {
+      const double w = cheb ? 1.0 / cheb_root(lam, lo, kk, o_.amg_cheb_degree) : o_.amg_jacobi_omega;
+      block_op<k::BLK_SMOOTH>(A, m, cur, b, pl.den0, w, nxt);
+      std::swap(cur, nxt);
+    }
+  }
+  // vcycle(q, ...) on m columns; B[q - l], X[q - l]: right-hand sides and results
+  void block_cycle(int l, int q, int m, std::vector<DBuf<TA>>& B, std::vector<DBuf<TA>>& X, TA* r, TA* t0, TA* t1) {
+    const Level& A = L_[(size_t)q];
+    TA* b = B[(size_t)(q - l)].p;
+    TA* x = X[(size_t)(q - l)].p;
+    if (q == (int)L_.size() - 1) {
+      k::block_dense<TA><<<block_grid(A.n, m), kBlock, 0, st_>>>(A.n, (int)dense_ld(A.n), m, tinv_.p, b, x);
+      NDS_LAUNCH();
+      return;
+    }
+    const size_t total = (size_t)A.n * m;
+    block_smooth(q, m, b, x, t0);
+    block_op<k::BLK_RESID>(A, m, x, b, nullptr, 0.0, r);
+    const Xfer& P = X_[(size_t)q + 1];
+    k::block_spmm<TA, TA, int32_t, k::BLK_Y><<<block_grid(P.nc, m), kBlock, 0, st_>>>(
+        P.nc, m, P.rrow.p, P.rcol.p, P.rval.p, TA(1), r, nullptr, nullptr, TA(0), B[(size_t)(q - l) + 1].p);
+    NDS_LAUNCH();
+    block_cycle(l, q + 1, m, B, X, r, t0, t1);
+    k::block_prolong_add<TA><<<block_grid(P.nf, m), kBlock, 0, st_>>>(P.nf, m, P.pw, P.pcol.p, P.pval.p,
+                                                                      X[(size_t)(q - l) + 1].p, x);
+    NDS_LAUNCH();
+    block_op<k::BLK_RESID>(A, m, x, b, nullptr, 0.0, r);
+    block_smooth(q, m, r, t1, t0);
+    k::block_add<TA><<<grid_for((long long)total), kBlock, 0, st_>>>(total, t1, x);
+    NDS_LAUNCH();
+  }
+
   // -------------------------------------------------------------- V-cycle
   // pre_done: the diagonal step of this level's pre-smoother is already in
   // place (taken by the restriction that produced b)
   void vcycle(int l, const TA* b, TA* x, bool pre_done = false) {
     Level& A = L_[(size_t)l];
+    if (l == dense_level_) {
+      ProfScope ps(prof, st_, P_TERMINAL);
+      k::dense_rows<TA><<<A.n, 32 * k::kDenseWarps, 0, st_>>>(A.n, (int)dense_ld(A.n), dense_.p, b, x);
+      NDS_LAUNCH();
+      return;
+    }
     if (l == (int)L_.size() - 1) {
       ProfScope ps(prof, st_, P_TERMINAL);
-      k::dense_mv<TA><<<grid_for((long long)A.n * 32), kBlock, 0, st_>>>(A.n, tinv_.p, b, x);
+      k::dense_rows<TA><<<A.n, 32 * k::kDenseWarps, 0, st_>>>(A.n, (int)dense_ld(A.n), tinv_.p, b, x);
       NDS_LAUNCH();
       return;
     }
@@ -2741,6 +2857,8 @@ class Solver final : public ISolver {
   DBuf<T> fval_, x_, r_, z_, pp_, q_, rhs_;
   DBuf<TA> fvalA_, fdiag_, fl1_, fr_, ftmp_, fcorr_, frhs_, fpong_, tinv_, rA_, zA_;
   std::vector<Level> L_;
+  int dense_level_ = -1;  // the level applied as its V-cycle matrix dense_ (-1: none)
+  DBuf<TA> dense_;
   std::vector<Xfer> X_;
   // mixed precision (NDS_MIXED): inner FP32 Krylov vectors, FGMRES basis
   // V (m+1 vectors) and preconditioned vectors Z (m), its FP64 work array,

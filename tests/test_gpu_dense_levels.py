@@ -1,0 +1,44 @@
+"""The coarse levels applied as one dense matrix against the level-by-level
+V-cycle (NDS_DENSE_MB=0): the same operator up to rounding, for every
+polynomial smoother, hierarchy depth and precision.  FP64: the iterates agree
+to rounding amplified by the solves (1e-9 relative, equal iteration counts);
+FP32 state: 1e-3 on relCont as for the FP32 path against FP64; mixed: every
+solve meets its own target p_rtol = 1e-6, as do the fields.
+"""
+from __future__ import annotations
+
+import pytest
+
+from conftest import rel_l2
+
+CFG = dict(re=20.0, alpha_u=0.7, alpha_p=0.3, p_rtol=1e-6, p_max=400, amg_terminal=16, max_outer=10,
+           pressure_solver="pcg")
+SA = dict(amg_hierarchy="sa", amg_smoother="cheb2")
+CF = dict(amg_hierarchy="cf", cf_interp="exti", cf_pmax=8, amg_jacobi_omega=0.5)
+CASES = {
+    "cheb2": (dict(SA), 1e-9, 1e-9),
+    "cheb_degree3": (dict(SA, amg_cheb_degree=3), 1e-9, 1e-9),
+    "jacobi_two_sweeps": (dict(CF, amg_smoother="jacobi", amg_jacobi_fine_sweeps=2, amg_jacobi_coarse_sweeps=2), 1e-9, 1e-9),
+    "l1jacobi": (dict(CF, amg_smoother="l1jacobi"), 1e-9, 1e-9),
+    "fp32": (dict(SA, precision="fp32", p_rtol=1e-4), 1e-3, 1e-3),
+    "mixed_half": (dict(SA, precision="mixed", amg_half=1), 1e-5, 1e-6),
+    "mixed_fgmres": (dict(SA, precision="mixed", p_krylov="fgmres"), 1e-5, 1e-6),
+}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mesh", ["pipe_tiny", "pipe_small"])
+@pytest.mark.parametrize("case", sorted(CASES))
+def test_dense_levels_match(native, meshes, monkeypatch, case, mesh):
+    kw, tol_cont, tol_field = CASES[case]
+    P = native.Problem(native.Mesh.from_tetmesh(meshes(mesh)), **dict(CFG, **kw))
+    A = native.Solver(P)
+    monkeypatch.setenv("NDS_DENSE_MB", "0")
+    B = native.Solver(P)
+    for _ in range(4):
+        a, b = A.step(), B.step()
+        assert abs(a.rel_cont - b.rel_cont) <= tol_cont * abs(b.rel_cont), (a.it, a.rel_cont, b.rel_cont)
+        if tol_field == 1e-9:
+            assert a.p_its == b.p_its
+    for x, y in zip(A.fields(), B.fields()):
+        assert rel_l2(x, y) <= tol_field

@@ -23,6 +23,31 @@ inline void cuda_check(cudaError_t e, const char* what, const char* file, int li
 extern unsigned long long g_launches;
 #define NDS_LAUNCH() (++::nds::g_launches, ::nds::cuda_check(cudaGetLastError(), "kernel launch", __FILE__, __LINE__))
 
+// Launch of a kernel that begins with pdl_begin(): the grid may be set up
+// while the kernel before it in the stream still runs (programmatic dependent
+// launch), which takes about a microsecond off every step of a chain of short
+// kernels.  pdl_begin() lets the next kernel be set up and then waits for the
+// whole of the previous one, so nothing is read or written early; every kernel
+// launched this way must call it before it touches memory.
+__device__ __forceinline__ void pdl_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <class... P, class... A>
+inline void pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  NDS_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+}
+
 constexpr int kBlock = 256;
 constexpr int kWarps = kBlock / 32;
 

@@ -27,16 +27,21 @@ namespace k {
 // y = float(s x)
 // y = s x in FP32; with x1 also the first (diagonal) step of the fine
 // pre-smoother on y, x1 = w0 y / den0 (the expression of jacobi_zero)
+// and with y2 also y2 = y
 __global__ void scale_to_float(int n, const double* __restrict__ x, double s, float* __restrict__ y,
-                               const float* __restrict__ den0 = nullptr, float w0 = 0.f, float* __restrict__ x1 = nullptr) {
+                               const float* __restrict__ den0 = nullptr, float w0 = 0.f, float* __restrict__ x1 = nullptr,
+                               float* __restrict__ y2 = nullptr) {
+  pdl_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float v = (float)(s * x[i]);
   y[i] = v;
+  if (y2) y2[i] = v;
   if (x1) x1[i] = w0 * v / den0[i];
 }
 // x += s y (y in FP32, x in FP64)
 __global__ void axpy_from_float(int n, double s, const float* __restrict__ y, double* __restrict__ x) {
+  pdl_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) x[i] += s * (double)y[i];
 }
@@ -59,63 +64,31 @@ struct FgLayout {
   __host__ __device__ int size() const { return (m + 1) * m + 4 * m + 1; }
 };
 
-// out = V[ctl[0]]   (the preconditioner's input, a fixed buffer)
-__global__ void fg_fetch(int n, const float* __restrict__ V, const int* __restrict__ ctl, float* __restrict__ out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = V[(size_t)ctl[0] * n + i];
-}
 // Z[ctl[0]] = z
 __global__ void fg_store(int n, const float* __restrict__ z, const int* __restrict__ ctl, float* __restrict__ Z) {
+  pdl_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) Z[(size_t)ctl[0] * n + i] = z[i];
-}
-// block partials of V_i . w for i = blockIdx.y <= ctl[0]: part[i gridDim.x + block]
-__global__ void __launch_bounds__(kBlock) fg_dots(int n, const float* __restrict__ V, const float* __restrict__ w,
-                                                  const int* __restrict__ ctl, double* __restrict__ part) {
-  const int vi = blockIdx.y;
-  if (vi > ctl[0]) return;
-  const float* v = V + (size_t)vi * n;
-  double acc[1] = {0.0};
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    acc[0] += (double)v[i] * (double)w[i];
-  block_sum<1>(acc);
-  if (threadIdx.x == 0) part[(size_t)vi * gridDim.x + blockIdx.x] = acc[0];
-}
-// H[i][j] = sum of the partials of V_i . w (one block per i <= j)
-__global__ void __launch_bounds__(kBlock) fg_reduce_h(const double* __restrict__ part, int nblocks,
-                                                      const int* __restrict__ ctl, FgLayout L,
-                                                      double* __restrict__ fg) {
-  const int vi = blockIdx.x, j = ctl[0];
-  if (vi > j) return;
-  double v[1] = {0.0};
-  for (int b = threadIdx.x; b < nblocks; b += blockDim.x) v[0] += part[(size_t)vi * nblocks + b];
-  block_sum<1>(v);
-  if (threadIdx.x == 0) fg[L.H(vi, j)] = v[0];
-}
-// w -= sum_{i <= j} H[i][j] V_i (FP64 sums, FP32 storage); partials of ||w||^2
-__global__ void __launch_bounds__(kBlock) fg_orth(int n, const float* __restrict__ V, const double* __restrict__ fg,
-                                                  FgLayout L, const int* __restrict__ ctl, float* __restrict__ w,
-                                                  double* __restrict__ part) {
-  const int j = ctl[0];
-  const double* h = fg + L.H(0, j);
-  double acc[1] = {0.0};
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    double s = (double)w[i];
-    for (int q = 0; q <= j; ++q) s -= h[q] * (double)V[(size_t)q * n + i];
-    const float f = (float)s;
-    w[i] = f;
-    acc[0] += (double)f * (double)f;
-  }
-  write_partials<1>(acc, part);
 }
 // Hessenberg column j: H[j+1][j] = ||w||, the earlier rotations, a new one;
 // g and the residual estimate |g[j+1]| (relative: the pass starts from a
 // unit vector, g[0] = 1).  Counts the vector, stores ||w|| for fg_normalize,
 // and stops the loop on convergence (|g[j+1]| <= tol), at the cap, on a
 // happy breakdown (||w|| = 0) or on a non-finite value.
-__global__ void fg_givens(double* __restrict__ fg, FgLayout L, double* __restrict__ sc, int wn2_slot, int wn_slot,
-                          int tol_slot, int* __restrict__ ctl, int* __restrict__ flags,
-                          cudaGraphConditionalHandle loop, int in_graph) {
+struct FgScalars {
+  double* sc;
+  int wn2_slot, wn_slot, tol_slot;
+  int* ctl;
+  int* flags;
+  cudaGraphConditionalHandle loop;
+  int in_graph;
+};
+__device__ __forceinline__ void fg_givens(double* __restrict__ fg, const FgLayout& L, const FgScalars& p) {
+  double* const sc = p.sc;
+  int* const ctl = p.ctl;
+  int* const flags = p.flags;
+  const int wn2_slot = p.wn2_slot, wn_slot = p.wn_slot, tol_slot = p.tol_slot, in_graph = p.in_graph;
+  const cudaGraphConditionalHandle loop = p.loop;
   const double tol = sc[tol_slot];
   const int j = ctl[0];
   const double wn = sqrt(sc[wn2_slot]);
@@ -153,13 +126,89 @@ __global__ void fg_givens(double* __restrict__ fg, FgLayout L, double* __restric
   const bool stop = conv || bad || j + 1 >= ctl[3];
   if (in_graph) cudaGraphSetConditional(loop, stop ? 0u : 1u);
 }
-// V[ctl[0]] = w / ||w|| (zero when ||w|| = 0)
+// H[i][j] = V_i . w for i <= j = ctl[0]: blockIdx.y takes the vectors y, y +
+// gridDim.y, ...; each vector's block partials (part[i gridDim.x + block]) are
+// added in order by the vector's last block (tickets, zero between launches)
+constexpr int kDotRows = 8;
+__global__ void __launch_bounds__(kBlock) fg_dots(int n, const float* __restrict__ V, const float* __restrict__ w,
+                                                  const int* __restrict__ ctl, double* __restrict__ part,
+                                                  unsigned* __restrict__ tickets, FgLayout L, double* __restrict__ fg) {
+  pdl_begin();
+  __shared__ bool last;
+  const int j = ctl[0];
+  for (int vi = blockIdx.y; vi <= j; vi += gridDim.y) {
+    const float* v = V + (size_t)vi * n;
+    double acc[1] = {0.0};
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+      acc[0] += (double)v[i] * (double)w[i];
+    block_sum<1>(acc);
+    if (threadIdx.x == 0) {
+      part[(size_t)vi * gridDim.x + blockIdx.x] = acc[0];
+      __threadfence();
+      last = atomicAdd(tickets + vi, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (last) {
+      __threadfence();
+      acc[0] = 0.0;
+      for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) acc[0] += __ldcg(part + (size_t)vi * gridDim.x + b);
+      block_sum<1>(acc);
+      if (threadIdx.x == 0) {
+        tickets[vi] = 0u;
+        fg[L.H(vi, j)] = acc[0];
+      }
+    }
+    __syncthreads();
+  }
+}
+// w -= sum_{i <= j} H[i][j] V_i (FP64 sums, FP32 storage) and ||w||^2, whose
+// last block then takes the Givens step
+__global__ void __launch_bounds__(kBlock) fg_orth(int n, const float* __restrict__ V, double* __restrict__ fg,
+                                                  FgLayout L, float* __restrict__ w, double* __restrict__ part,
+                                                  unsigned* __restrict__ ticket, FgScalars a) {
+  pdl_begin();
+  __shared__ bool last;
+  const int j = a.ctl[0];
+  const double* h = fg + L.H(0, j);
+  double acc[1] = {0.0};
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    double s = (double)w[i];
+    for (int q = 0; q <= j; ++q) s -= h[q] * (double)V[(size_t)q * n + i];
+    const float f = (float)s;
+    w[i] = f;
+    acc[0] += (double)f * (double)f;
+  }
+  block_sum<1>(acc);
+  if (threadIdx.x == 0) {
+    part[blockIdx.x] = acc[0];
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  acc[0] = 0.0;
+  for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) acc[0] += __ldcg(part + b);
+  block_sum<1>(acc);
+  if (threadIdx.x == 0) {
+    *ticket = 0u;
+    a.sc[a.wn2_slot] = acc[0];
+    fg_givens(fg, L, a);
+  }
+}
+// v = w / ||w|| (zero when ||w|| = 0) into V[ctl[0]] and into the next
+// preconditioner input; with x1 also the first step of its fine pre-smoother
 __global__ void fg_normalize(int n, const float* __restrict__ w, const double* __restrict__ sc, int wn_slot,
-                             const int* __restrict__ ctl, float* __restrict__ V) {
+                             const int* __restrict__ ctl, float* __restrict__ V, float* __restrict__ in,
+                             const float* __restrict__ den0, float w0, float* __restrict__ x1) {
+  pdl_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double wn = sc[wn_slot];
-  V[(size_t)ctl[0] * n + i] = wn > 0.0 ? (float)((double)w[i] / wn) : 0.0f;
+  const float v = wn > 0.0 ? (float)((double)w[i] / wn) : 0.0f;
+  V[(size_t)ctl[0] * n + i] = v;
+  in[i] = v;
+  if (x1) x1[i] = w0 * v / den0[i];
 }
 // start of a pass: g = (1, 0, ...), j = 0
 __global__ void fg_start(double* __restrict__ fg, FgLayout L, int* __restrict__ ctl, int cap) {
@@ -205,6 +254,7 @@ constexpr int kMaxGuess = 8;
 template <int K>
 __global__ void __launch_bounds__(kBlock) guess_dots(int n, const double* __restrict__ Y, const double* __restrict__ W,
                                                      const double* __restrict__ b, double* __restrict__ part) {
+  pdl_begin();
   constexpr int NG = K * (K + 1) / 2 + K;
   double acc[NG];
 #pragma unroll
@@ -231,6 +281,7 @@ __global__ void __launch_bounds__(kBlock) guess_dots(int n, const double* __rest
 template <int K>
 __global__ void guess_combine(int n, const double* __restrict__ Y, const double* __restrict__ coef,
                               double* __restrict__ x) {
+  pdl_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double xs = 0.0;
@@ -241,6 +292,7 @@ __global__ void guess_combine(int n, const double* __restrict__ Y, const double*
 // the stored product of a new correction: w = b - r (= A x for r = b - A x)
 __global__ void guess_store(int n, const double* __restrict__ x, const double* __restrict__ b,
                             const double* __restrict__ r, double* __restrict__ y, double* __restrict__ w) {
+  pdl_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   y[i] = x[i];

@@ -473,6 +473,9 @@ class Solver final : public ISolver {
       fine_crows_.upload(rows);
     }
     for (auto* b : {&x_, &r_, &z_, &pp_, &q_, &rhs_}) b->alloc((size_t)nc_);
+    tailpart_.alloc((size_t)std::max(grid_for(nc_), 1));
+    ticket_.alloc(1);
+    NDS_CUDA(cudaMemset(ticket_.p, 0, sizeof(unsigned)));
     for (auto* b : {&fr_, &ftmp_, &fcorr_, &frhs_, &fpong_}) b->alloc((size_t)nc_);
     if (!kSame) {
       rA_.alloc((size_t)nc_);
@@ -1003,9 +1006,9 @@ class Solver final : public ISolver {
     g_launches += g.kernels;
   }
   bool use_graphs_ = std::getenv("NDS_NO_GRAPHS") == nullptr;
-  Graph g_amg_, g_pcg2_;
-  // the whole PCG iteration loop as one graph: a conditional while node whose
-  // body is one iteration and ends with pcg_check, which sets the condition
+  Graph g_amg_;
+  // a whole Krylov loop as one graph: a conditional while node whose body is
+  // one iteration; its last kernel sets the condition
   struct LoopGraph {
     cudaGraphExec_t exec = nullptr;
     unsigned long long body_kernels = 0;
@@ -1015,47 +1018,6 @@ class Solver final : public ISolver {
     }
   };
   LoopGraph g_loop_;
-  bool build_pcg_loop() {
-    const bool was = prof.on;
-    prof.on = false;
-    cudaGraph_t graph = nullptr;
-    bool ok = cudaGraphCreate(&graph, 0) == cudaSuccess;
-    cudaGraphConditionalHandle h{};
-    cudaGraphNodeParams cp{};
-    cudaGraphNode_t node{};
-    if (ok) ok = cudaGraphConditionalHandleCreate(&h, graph, 1, cudaGraphCondAssignDefault) == cudaSuccess;
-    if (ok) {
-      cp.type = cudaGraphNodeTypeConditional;
-      cp.conditional.handle = h;
-      cp.conditional.type = cudaGraphCondTypeWhile;
-      cp.conditional.size = 1;
-      ok = cudaGraphAddNode(&node, graph, nullptr, 0, &cp) == cudaSuccess;
-    }
-    const unsigned long long l0 = g_launches;
-    if (ok) ok = cudaStreamBeginCaptureToGraph(st_, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                               cudaStreamCaptureModeThreadLocal) == cudaSuccess;
-    if (ok) {
-      bool body_ok = true;
-      try {
-        pcg_loop_body(h);
-      } catch (...) {
-        body_ok = false;
-      }
-      ok = cudaStreamEndCapture(st_, nullptr) == cudaSuccess && body_ok;
-    }
-    g_loop_.body_kernels = g_launches - l0;
-    g_launches = l0;
-    if (ok) ok = cudaGraphInstantiate(&g_loop_.exec, graph, 0) == cudaSuccess;
-    if (graph) cudaGraphDestroy(graph);
-    if (!ok) {
-      if (g_loop_.exec) cudaGraphExecDestroy(g_loop_.exec);
-      g_loop_.exec = nullptr;
-      g_loop_.failed = true;
-      cudaGetLastError();  // the fallback path runs instead
-    }
-    prof.on = was;
-    return ok;
-  }
   // z = M b with b, z in the state precision (casts around the V-cycle in
   // the mixed mode)
   void amg_T(const T* b, T* z) {
@@ -1064,17 +1026,17 @@ class Solver final : public ISolver {
     } else if (o_.amg_smoother != NDS_SM_MCGS) {
       // the cast also takes the fine pre-smoother's diagonal step
       const PolyPlan pl = fine_plan();
-      k::cast_jacobi<T, TA><<<grid_for(nc_), kBlock, 0, st_>>>(nc_, b, rA_.p, TA(pl.w0), pl.den0,
-                                                               poly_first(pl, zA_.p, fpong_.p));
+      pdl_launch(k::cast_jacobi<T, TA>, grid_for(nc_), kBlock, 0, st_, nc_, b, rA_.p, TA(pl.w0), pl.den0,
+                 fine_first(zA_.p));
       NDS_LAUNCH();
       amg_apply(rA_.p, zA_.p, true);
-      k::cast_copy<TA, T><<<grid_for(nc_), kBlock, 0, st_>>>(nc_, zA_.p, z);
+      pdl_launch(k::cast_copy<TA, T>, grid_for(nc_), kBlock, 0, st_, nc_, zA_.p, z);
       NDS_LAUNCH();
     } else {
-      k::cast_copy<T, TA><<<grid_for(nc_), kBlock, 0, st_>>>(nc_, b, rA_.p);
+      pdl_launch(k::cast_copy<T, TA>, grid_for(nc_), kBlock, 0, st_, nc_, b, rA_.p);
       NDS_LAUNCH();
       amg_apply(rA_.p, zA_.p);
-      k::cast_copy<TA, T><<<grid_for(nc_), kBlock, 0, st_>>>(nc_, zA_.p, z);
+      pdl_launch(k::cast_copy<TA, T>, grid_for(nc_), kBlock, 0, st_, nc_, zA_.p, z);
       NDS_LAUNCH();
     }
   }
@@ -1088,14 +1050,14 @@ class Solver final : public ISolver {
   int red_grid(long long n, int per = kBlock) const { return std::min(grid_for(n, per), kMaxPartBlocks); }
   template <int NV>
   void reduce_to(int nblocks, int slot) {
-    k::reduce_partials<NV><<<1, kBlock, 0, st_>>>(part_.p, nblocks, sc_.p + slot);
+    pdl_launch(k::reduce_partials<NV>, 1, kBlock, 0, st_, part_.p, nblocks, sc_.p + slot);
     NDS_LAUNCH();
   }
   // reduction of one value into sc[slot], then the PCG scalar step STEP
   template <int STEP>
   void reduce_pcg(int nblocks, int slot, int max_its = 0, cudaGraphConditionalHandle h = {}, int in_graph = 1) {
     const k::PcgScalars ps{sc_.p, flags_.p, ctl_.p, S_RN2, S_R0, S_TARGET, max_its, h, in_graph};
-    k::reduce_pcg<STEP><<<1, kBlock, 0, st_>>>(part_.p, nblocks, sc_.p + slot, ps);
+    pdl_launch(k::reduce_pcg<STEP>, 1, kBlock, 0, st_, part_.p, nblocks, sc_.p + slot, ps);
     NDS_LAUNCH();
   }
   void fetch(int first, int count) {
@@ -1105,7 +1067,7 @@ class Solver final : public ISolver {
   template <class V>
   double dot_fetch(const V* x, const V* y, int n, int slot) {
     const int g = red_grid(n);
-    k::dot<V><<<g, kBlock, 0, st_>>>(n, x, y, part_.p);
+    pdl_launch(k::dot<V>, g, kBlock, 0, st_, n, x, y, part_.p);
     NDS_LAUNCH();
     reduce_to<1>(g, slot);
     fetch(slot, 1);
@@ -1114,7 +1076,7 @@ class Solver final : public ISolver {
   template <class V>
   void dot_dev(const V* x, const V* y, int n, int slot) {
     const int g = red_grid(n);
-    k::dot<V><<<g, kBlock, 0, st_>>>(n, x, y, part_.p);
+    pdl_launch(k::dot<V>, g, kBlock, 0, st_, n, x, y, part_.p);
     NDS_LAUNCH();
     reduce_to<1>(g, slot);
   }
@@ -1142,53 +1104,96 @@ class Solver final : public ISolver {
   };
   // the two steps of a product in split form
   template <int MODE, class V>
-  void split_launch(const OpView<V>& A, int grid, const V* x, const V* b, const V* den, double w, V* y, V* y2) {
+  void split_launch(const OpView<V>& A, const V* x, const V* b, const V* den, double w, V* y, V* y2) {
+    static_assert(MODE != k::SELL_DOT, "split_dot forms p.q");
+    split_vertices(A, x);
+    split_types(A, [&](auto mt, auto d16) {
+      pdl_launch(k::split_cell<V, MODE, decltype(d16)::value, decltype(mt)>, grid_for(A.n), kBlock, 0, st_, A.sc,
+                 A.w, x, b, den, V(w), y, y2, V(A.tinv),
+                 (const V*)nullptr, k::ReduceTail{}, (const int*)nullptr);
+    });
+  }
+  template <class V>
+  void split_vertices(const OpView<V>& A, const V* x) {
     const int gv = grid_for(8LL * A.sv.n);
     if (A.sv.n > 0) {
       if constexpr (std::is_same<V, double>::value)
-        k::split_vertex<V, k::REC_SOA><<<gv, kBlock, 0, st_>>>(A.sv, A.rv, x, A.w, V(A.wscale));
+        pdl_launch(k::split_vertex<V, k::REC_SOA>, gv, kBlock, 0, st_, A.sv, A.rv, x, A.w, V(A.wscale));
       else if (A.sv.rec8)
-        k::split_vertex<V, k::REC_8><<<gv, kBlock, 0, st_>>>(A.sv, A.rv, x, A.w, V(A.wscale));
+        pdl_launch(k::split_vertex<V, k::REC_8>, gv, kBlock, 0, st_, A.sv, A.rv, x, A.w, V(A.wscale));
       else
-        k::split_vertex<V, k::REC_16><<<gv, kBlock, 0, st_>>>(A.sv, A.rv, x, A.w, V(A.wscale));
+        pdl_launch(k::split_vertex<V, k::REC_16>, gv, kBlock, 0, st_, A.sv, A.rv, x, A.w, V(A.wscale));
       NDS_LAUNCH();
     }
-    auto cells = [&](auto mt) {
-      using MT = decltype(mt);
-      if (A.sc.nd16)
-        k::split_cell<V, MODE, true, MT><<<grid, kBlock, 0, st_>>>(A.sc, A.w, x, b, den, V(w), y, y2, part_.p, V(A.tinv));
-      else
-        k::split_cell<V, MODE, false, MT><<<grid, kBlock, 0, st_>>>(A.sc, A.w, x, b, den, V(w), y, y2, part_.p, V(A.tinv));
+  }
+  // f(value type of the cells' data, 16-bit neighbour deltas)
+  template <class V, class F>
+  void split_types(const OpView<V>& A, F&& f) {
+    auto width = [&](auto mt) {
+      if (A.sc.nd16) f(mt, std::true_type{});
+      else f(mt, std::false_type{});
     };
     if constexpr (std::is_same<V, float>::value) {
       if (A.half) {
-        cells(__half{});
+        width(__half{});
         return;
       }
     }
-    cells(V{});
+    width(V{});
+  }
+  // the last smoothing step of the V-cycle, z = x + w (b - A x) / den or
+  // (add_to given) add_to += that, with r.z and the step rho of PCG
+  template <class V, class R>
+  void split_smooth_rho(const OpView<V>& A, const V* x, const V* b, const V* den, double w, V* z, V* add_to,
+                        const R* r) {
+    ProfScope ps(prof, st_, A.cat);
+    split_vertices(A, x);
+    split_types(A, [&](auto mt, auto d16) {
+      pdl_launch(k::split_cell<V, k::SELL_SMOOTH, decltype(d16)::value, decltype(mt), k::PCG_RHO, R>, grid_for(A.n),
+                 kBlock, 0, st_, A.sc, A.w, x, b, den, V(w), z, add_to, V(A.tinv), r, tail(S_RHON),
+                 (const int*)nullptr);
+    });
+    NDS_LAUNCH();
+  }
+  // q = A p with p.q and the step alpha of PCG
+  template <class V>
+  void split_dot(const OpView<V>& A, const V* p, V* q) {
+    ProfScope ps(prof, st_, A.cat);
+    split_vertices(A, p);
+    if (A.sc.nd16)
+      pdl_launch(k::split_cell_dot<V, true>, red_grid(A.n), kBlock, 0, st_, A.sc, A.w, p, q, V(A.tinv), tail(S_PQ));
+    else
+      pdl_launch(k::split_cell_dot<V, false>, red_grid(A.n), kBlock, 0, st_, A.sc, A.w, p, q, V(A.tinv), tail(S_PQ));
+    NDS_LAUNCH();
+  }
+  // a reduction into sc[slot] taken by the producing kernel's last block
+  k::ReduceTail tail(int slot, cudaGraphConditionalHandle h = {}) {
+    return k::ReduceTail{tailpart_.p, ticket_.p, sc_.p + slot,
+                         k::PcgScalars{sc_.p, flags_.p, ctl_.p, S_RN2, S_R0, S_TARGET, -1, h, in_graph_}};
   }
   template <int MODE, class V>
   void sell_launch(const OpView<V>& A, int grid, const V* x, const V* b, const V* den, double w, V* y, V* y2) {
-    if (A.split) {
-      split_launch<MODE, V>(A, grid, x, b, den, w, y, y2);
-      return;
+    if constexpr (MODE != k::SELL_DOT) {
+      if (A.split) {
+        split_launch<MODE, V>(A, x, b, den, w, y, y2);
+        return;
+      }
     }
     if constexpr (std::is_same<V, float>::value) {
       if (A.vh) {
         if (A.s.dcol)
-          k::sell_spmv<V, MODE, true, __half><<<grid, kBlock, 0, st_>>>(A.s, A.vh, x, b, den, V(w), y, y2, part_.p,
-                                                                          V(A.vinv));
+          pdl_launch(k::sell_spmv<V, MODE, true, __half>, grid, kBlock, 0, st_, A.s, A.vh, x, b, den, V(w), y, y2,
+                     part_.p, V(A.vinv));
         else
-          k::sell_spmv<V, MODE, false, __half><<<grid, kBlock, 0, st_>>>(A.s, A.vh, x, b, den, V(w), y, y2, part_.p,
-                                                                           V(A.vinv));
+          pdl_launch(k::sell_spmv<V, MODE, false, __half>, grid, kBlock, 0, st_, A.s, A.vh, x, b, den, V(w), y, y2,
+                     part_.p, V(A.vinv));
         return;
       }
     }
     if (A.s.dcol)
-      k::sell_spmv<V, MODE, true><<<grid, kBlock, 0, st_>>>(A.s, A.v, x, b, den, V(w), y, y2, part_.p);
+      pdl_launch(k::sell_spmv<V, MODE, true>, grid, kBlock, 0, st_, A.s, A.v, x, b, den, V(w), y, y2, part_.p, V(1));
     else
-      k::sell_spmv<V, MODE, false><<<grid, kBlock, 0, st_>>>(A.s, A.v, x, b, den, V(w), y, y2, part_.p);
+      pdl_launch(k::sell_spmv<V, MODE, false>, grid, kBlock, 0, st_, A.s, A.v, x, b, den, V(w), y, y2, part_.p, V(1));
   }
   // physical operator (precision T) and the AMG's fine operator (precision TA)
   OpView<T> fine_op() {
@@ -1300,16 +1305,17 @@ class Solver final : public ISolver {
     else if (A.vh && A.ch && std::is_same<V, float>::value)
       level_half_launch(A, [&](auto gl) {
         constexpr int GL = decltype(gl)::value;
-        k::spmv<V, __half, int16_t, GL><<<grid_for((long long)A.n * GL), kBlock, 0, st_>>>(A.n, A.rp, A.ch, A.vh, x,
-                                                                                             y, V(A.vinv));
+        pdl_launch(k::spmv<V, __half, int16_t, GL>, grid_for((long long)A.n * GL), kBlock, 0, st_, A.n, A.rp, A.ch,
+                   A.vh, x, y, V(A.vinv));
       });
     else if (A.vh && std::is_same<V, float>::value)
       level_half_launch(A, [&](auto gl) {
         constexpr int GL = decltype(gl)::value;
-        k::spmv<V, __half, int32_t, GL><<<grid_for((long long)A.n * GL), kBlock, 0, st_>>>(A.n, A.rp, A.ci, A.vh, x,
-                                                                                             y, V(A.vinv));
+        pdl_launch(k::spmv<V, __half, int32_t, GL>, grid_for((long long)A.n * GL), kBlock, 0, st_, A.n, A.rp, A.ci,
+                   A.vh, x, y, V(A.vinv));
       });
-    else k::spmv<V><<<grid_for((long long)A.n * k::kRowLanes), kBlock, 0, st_>>>(A.n, A.rp, A.ci, A.v, x, y);
+    else pdl_launch(k::spmv<V>, grid_for((long long)A.n * k::kRowLanes), kBlock, 0, st_, A.n, A.rp, A.ci, A.v, x, y,
+                    V(1));
     NDS_LAUNCH();
   }
   // r = b - A x; r2 = r, or (den given) the first Jacobi step w r / den
@@ -1321,17 +1327,18 @@ class Solver final : public ISolver {
     else if (A.vh && A.ch && std::is_same<V, float>::value)
       level_half_launch(A, [&](auto gl) {
         constexpr int GL = decltype(gl)::value;
-        k::spmv_resid<V, __half, int16_t, GL><<<grid_for((long long)A.n * GL), kBlock, 0, st_>>>(
-            A.n, A.rp, A.ch, A.vh, x, b, r, r2, den, V(w), V(A.vinv));
+        pdl_launch(k::spmv_resid<V, __half, int16_t, GL>, grid_for((long long)A.n * GL), kBlock, 0, st_, A.n, A.rp,
+                   A.ch, A.vh, x, b, r, r2, den, V(w), V(A.vinv));
       });
     else if (A.vh && std::is_same<V, float>::value)
       level_half_launch(A, [&](auto gl) {
         constexpr int GL = decltype(gl)::value;
-        k::spmv_resid<V, __half, int32_t, GL><<<grid_for((long long)A.n * GL), kBlock, 0, st_>>>(
-            A.n, A.rp, A.ci, A.vh, x, b, r, r2, den, V(w), V(A.vinv));
+        pdl_launch(k::spmv_resid<V, __half, int32_t, GL>, grid_for((long long)A.n * GL), kBlock, 0, st_, A.n, A.rp,
+                   A.ci, A.vh, x, b, r, r2, den, V(w), V(A.vinv));
       });
     else
-      k::spmv_resid<V><<<grid_for((long long)A.n * k::kRowLanes), kBlock, 0, st_>>>(A.n, A.rp, A.ci, A.v, x, b, r, r2, den, V(w));
+      pdl_launch(k::spmv_resid<V>, grid_for((long long)A.n * k::kRowLanes), kBlock, 0, st_, A.n, A.rp, A.ci, A.v, x,
+                 b, r, r2, den, V(w), V(1));
     NDS_LAUNCH();
   }
   // xout = xin + w (b - A xin) / den, or (add_to given) add_to += that
@@ -1342,18 +1349,18 @@ class Solver final : public ISolver {
     else if (A.vh && A.ch && std::is_same<V, float>::value)
       level_half_launch(A, [&](auto gl) {
         constexpr int GL = decltype(gl)::value;
-        k::spmv_smooth<V, __half, int16_t, GL><<<grid_for((long long)A.n * GL), kBlock, 0, st_>>>(
-            A.n, A.rp, A.ch, A.vh, xin, b, den, V(w), xout, add_to, V(A.vinv));
+        pdl_launch(k::spmv_smooth<V, __half, int16_t, GL>, grid_for((long long)A.n * GL), kBlock, 0, st_, A.n, A.rp,
+                   A.ch, A.vh, xin, b, den, V(w), xout, add_to, V(A.vinv));
       });
     else if (A.vh && std::is_same<V, float>::value)
       level_half_launch(A, [&](auto gl) {
         constexpr int GL = decltype(gl)::value;
-        k::spmv_smooth<V, __half, int32_t, GL><<<grid_for((long long)A.n * GL), kBlock, 0, st_>>>(
-            A.n, A.rp, A.ci, A.vh, xin, b, den, V(w), xout, add_to, V(A.vinv));
+        pdl_launch(k::spmv_smooth<V, __half, int32_t, GL>, grid_for((long long)A.n * GL), kBlock, 0, st_, A.n, A.rp,
+                   A.ci, A.vh, xin, b, den, V(w), xout, add_to, V(A.vinv));
       });
     else
-      k::spmv_smooth<V><<<grid_for((long long)A.n * k::kRowLanes), kBlock, 0, st_>>>(A.n, A.rp, A.ci, A.v, xin, b, den, V(w), xout,
-                                                                          add_to);
+      pdl_launch(k::spmv_smooth<V>, grid_for((long long)A.n * k::kRowLanes), kBlock, 0, st_, A.n, A.rp, A.ci, A.v,
+                 xin, b, den, V(w), xout, add_to, V(1));
     NDS_LAUNCH();
   }
   template <class V>
@@ -1363,7 +1370,7 @@ class Solver final : public ISolver {
   }
   template <class V>
   void vaxpy(int n, double a, const V* x, V* y) {
-    k::axpy<V><<<grid_for(n), kBlock, 0, st_>>>(n, V(a), x, y);
+    pdl_launch(k::axpy<V>, grid_for(n), kBlock, 0, st_, n, V(a), x, y);
     NDS_LAUNCH();
   }
 
@@ -1417,7 +1424,7 @@ class Solver final : public ISolver {
     TA* cur = poly_first(pl, x, pong);
     TA* nxt = (pl.m % 2 == 0) ? pong : x;
     if (!first_done) {
-      k::jacobi_zero<TA><<<grid_for(n), kBlock, 0, st_>>>(n, TA(pl.w0), b, pl.den0, cur);
+      pdl_launch(k::jacobi_zero<TA>, grid_for(n), kBlock, 0, st_, n, TA(pl.w0), b, pl.den0, cur);
       NDS_LAUNCH();
     }
     const double lo = cheb ? o_.amg_lambda_low_fraction * lambda : 0.0;
@@ -1513,20 +1520,20 @@ class Solver final : public ISolver {
     if (restrict_lanes() != 32) {
       auto run = [&](auto gl) {
         constexpr int GL = decltype(gl)::value;
-        k::restrict_rows<TA, GL><<<grid_for((long long)X.nc * GL), kBlock, 0, st_>>>(X.nc, X.rrow.p, X.rcol.p,
-                                                                                    X.rval.p, f, c, den0, TA(w0), x1);
+        pdl_launch(k::restrict_rows<TA, GL>, grid_for((long long)X.nc * GL), kBlock, 0, st_, X.nc, X.rrow.p,
+                   X.rcol.p, X.rval.p, f, c, den0, TA(w0), x1);
       };
       if (restrict_lanes() == 8) run(std::integral_constant<int, 8>{});
       else run(std::integral_constant<int, 16>{});
     } else {
-      k::restrict_rows<TA><<<grid_for((long long)X.nc * k::kRowLanes), kBlock, 0, st_>>>(
-          X.nc, X.rrow.p, X.rcol.p, X.rval.p, f, c, den0, TA(w0), x1);
+      pdl_launch(k::restrict_rows<TA>, grid_for((long long)X.nc * k::kRowLanes), kBlock, 0, st_, X.nc, X.rrow.p,
+                 X.rcol.p, X.rval.p, f, c, den0, TA(w0), x1);
     }
     NDS_LAUNCH();
   }
   void prolong(const Xfer& X, const TA* c, TA* f) {
     ProfScope ps(prof, st_, P_TRANSFER);
-    k::prolong_add<TA><<<grid_for(X.nf), kBlock, 0, st_>>>(X.nf, X.pw, X.pcol.p, X.pval.p, c, f);
+    pdl_launch(k::prolong_add<TA>, grid_for(X.nf), kBlock, 0, st_, X.nf, X.pw, X.pcol.p, X.pval.p, c, f);
     NDS_LAUNCH();
   }
 
@@ -1637,13 +1644,13 @@ class Solver final : public ISolver {
     Level& A = L_[(size_t)l];
     if (l == dense_level_) {
       ProfScope ps(prof, st_, P_TERMINAL);
-      k::dense_rows<TA><<<A.n, 32 * k::kDenseWarps, 0, st_>>>(A.n, (int)dense_ld(A.n), dense_.p, b, x);
+      pdl_launch(k::dense_rows<TA>, A.n, 32 * k::kDenseWarps, 0, st_, A.n, (int)dense_ld(A.n), dense_.p, b, x);
       NDS_LAUNCH();
       return;
     }
     if (l == (int)L_.size() - 1) {
       ProfScope ps(prof, st_, P_TERMINAL);
-      k::dense_rows<TA><<<A.n, 32 * k::kDenseWarps, 0, st_>>>(A.n, (int)dense_ld(A.n), tinv_.p, b, x);
+      pdl_launch(k::dense_rows<TA>, A.n, 32 * k::kDenseWarps, 0, st_, A.n, (int)dense_ld(A.n), tinv_.p, b, x);
       NDS_LAUNCH();
       return;
     }
@@ -1672,28 +1679,57 @@ class Solver final : public ISolver {
     op_resid(level_op(A), x, b, A.b.p, poly_first(pl, A.corr.p, A.pong.p), pl.den0, pl.w0);
     poly_smooth(level_op(A), A.diag.p, A.b.p, A.corr.p, A.pong.p, lam, cheb, den, o_.amg_jacobi_coarse_sweeps, true, x);
   }
-  // pre_done: the fine pre-smoother's diagonal step is already in place
-  void amg_apply(const TA* b, TA* z, bool pre_done = false) {
-    smooth_fine(b, z, pre_done);
-    op_resid(fine_opV(), z, b, fr_.p);
+  // where the fine pre-smoother's diagonal step goes: with one step only
+  // (m = 0, split form) the cycle works in ftmp_, so that the post-smoothing
+  // step can write z from it in one product
+  TA* fine_first(TA* z) {
+    const PolyPlan pl = fine_plan();
+    return split_ && pl.m == 0 ? ftmp_.p : poly_first(pl, z, fpong_.p);
+  }
+  // z = M b.  pre_done: the fine pre-smoother's diagonal step is already in
+  // fine_first(z).  With r (split form only) the last kernel also takes r.z
+  // and the step rho of PCG.
+  template <class R = TA>
+  void amg_apply(const TA* b, TA* z, bool pre_done = false, const R* r = nullptr) {
+    const int sm = o_.amg_smoother;
+    const bool one = split_ && fine_plan().m == 0;
+    TA* x = one ? ftmp_.p : z;
+    smooth_fine(b, x, pre_done);
+    op_resid(fine_opV(), x, b, fr_.p);
     Level& C = L_[0];
     const bool fuse = fuse_pre(0);
     restrict_to(X_[0], fr_.p, C.b.p, fuse ? 0 : -1);
     vcycle(0, C.b.p, C.x.p, fuse);
-    prolong(X_[0], C.x.p, z);
-    const int sm = o_.amg_smoother;
+    prolong(X_[0], C.x.p, x);
     if (sm == NDS_SM_MCGS) {
       op_resid(fine_opV(), z, b, fr_.p, frhs_.p);
       smooth_fine(frhs_.p, fcorr_.p);
       vaxpy(nc_, 1.0, fcorr_.p, z);
       return;
     }
-    // post-smoothing as on the levels: residual with the diagonal step, last
-    // step added to z
     const bool cheb = sm == NDS_SM_CHEB2;
     const TA* den = sm == NDS_SM_L1JACOBI ? fl1_.p : fdiag_.p;
     const PolyPlan pl = poly_plan(fine_lambda_, cheb, fdiag_.p, den, o_.amg_jacobi_fine_sweeps);
+    if (one) {  // z = x + w0 (b - A x) / den
+      if (r) split_smooth_rho(fine_opV(), (const TA*)x, b, pl.den0, pl.w0, z, (TA*)nullptr, r);
+      else op_smooth(fine_opV(), (const TA*)x, b, pl.den0, pl.w0, z);
+      return;
+    }
+    // post-smoothing as on the levels: residual with the diagonal step, last
+    // step added to z
     op_resid(fine_opV(), z, b, frhs_.p, poly_first(pl, fcorr_.p, fpong_.p), pl.den0, pl.w0);
+    if (r && pl.m >= 1) {
+      TA* cur = poly_first(pl, fcorr_.p, fpong_.p);
+      TA* nxt = cur == fcorr_.p ? fpong_.p : fcorr_.p;
+      const double lo = cheb ? o_.amg_lambda_low_fraction * fine_lambda_ : 0.0;
+      for (int kk = 1; kk <= pl.m; ++kk) {
+        const double w = cheb ? 1.0 / cheb_root(fine_lambda_, lo, kk, o_.amg_cheb_degree) : o_.amg_jacobi_omega;
+        if (kk < pl.m) op_smooth(fine_opV(), (const TA*)cur, (const TA*)frhs_.p, pl.den0, w, nxt);
+        else split_smooth_rho(fine_opV(), (const TA*)cur, (const TA*)frhs_.p, pl.den0, w, (TA*)nullptr, z, r);
+        std::swap(cur, nxt);
+      }
+      return;
+    }
     poly_smooth(fine_opV(), fdiag_.p, frhs_.p, fcorr_.p, fpong_.p, fine_lambda_, cheb, den, o_.amg_jacobi_fine_sweeps,
                 true, z);
   }
@@ -1782,13 +1818,6 @@ class Solver final : public ISolver {
     double rel = 1;
     bool ok = false;
   };
-  void check_flags() {
-    int f = 0;
-    NDS_CUDA(cudaMemcpyAsync(&f, flags_.p, sizeof(int), cudaMemcpyDeviceToHost, st_));
-    NDS_CUDA(cudaStreamSynchronize(st_));
-    if (f & 1) throw SolveFailure(NDS_E_BREAKDOWN, "pressure PCG pAp nonpositive");
-    if (f & 2) throw SolveFailure(NDS_E_BREAKDOWN, "pressure PCG rho nonpositive");
-  }
   // ||r0|| and the zero solution
   double p_start(const T* rhs) {
     x_.zero(st_);
@@ -1797,119 +1826,101 @@ class Solver final : public ISolver {
     if (!std::isfinite(r0)) throw SolveFailure(NDS_E_BREAKDOWN, "pressure initial norm nonfinite");
     return r0;
   }
-  // one PCG iteration, first half: q = A p, pq = p.q, alpha = rho/pq,
-  // x += alpha p, r -= alpha q, rn2 = r.r; then rn2 and the flags to the host
-  void pcg_half1() {
+  // Vectors of a PCG solve in precision S (the preconditioner runs in TA):
+  // rA the residual in TA when the precisions differ.
+  template <class S>
+  struct PcgVecs {
+    S *x, *r, *q, *p;
+    TA *z, *rA;
+  };
+  // the PCG loops take the fine pre-smoother's first step in the kernels that
+  // produce r (plain V-cycle with a polynomial smoother only)
+  bool pre_fused() const { return !stage_ && o_.amg_smoother != NDS_SM_MCGS; }
+  // the pre-smoother's first step on the initial residual
+  template <class S>
+  void pcg_first(const PcgVecs<S>& v) {
+    if constexpr (std::is_same<S, TA>::value) {
+      if (!pre_fused()) return;
+      const PolyPlan pl = fine_plan();
+      pdl_launch(k::jacobi_zero<TA>, grid_for(nc_), kBlock, 0, st_, nc_, TA(pl.w0), v.r, pl.den0, fine_first(v.z));
+    } else if (pre_fused()) {
+      const PolyPlan pl = fine_plan();
+      pdl_launch(k::cast_jacobi<S, TA>, grid_for(nc_), kBlock, 0, st_, nc_, v.r, v.rA, TA(pl.w0), pl.den0,
+                 fine_first(v.z));
+    } else {
+      pdl_launch(k::cast_copy<S, TA>, grid_for(nc_), kBlock, 0, st_, nc_, v.r, v.rA);
+    }
+    NDS_LAUNCH();
+  }
+  // One pass of a PCG loop: z = M r; rho (first pass: p = z) and beta; q = A p;
+  // alpha; x and r; ||r||^2 and the stopping test.  In split form the scalar
+  // steps are taken by the kernels before them.
+  template <class S>
+  void pcg_body(const PcgVecs<S>& v, const OpView<S>& A, cudaGraphConditionalHandle h) {
     const int g = red_grid(nc_);
-    {
-      ProfScope ps(prof, st_, P_FINE_SPMV);
-      sell_launch<k::SELL_DOT, T>(fine_op(), g, pp_.p, nullptr, nullptr, 0.0, q_.p, nullptr);
+    const bool fused = pre_fused();
+    const TA* r = v.rA;
+    if constexpr (std::is_same<S, TA>::value) r = v.r;
+    if (split_) {
+      amg_apply<S>(r, v.z, fused, v.r);
+    } else {
+      amg_apply(r, v.z, fused);
+      pdl_launch(k::dot<S, TA>, g, kBlock, 0, st_, nc_, v.r, v.z, part_.p);
+      NDS_LAUNCH();
+      reduce_pcg<k::PCG_RHO>(g, S_RHON);
+    }
+    pdl_launch(k::p_update_dev<S, TA>, grid_for(nc_), kBlock, 0, st_, nc_, sc_.p + S_BETA, ctl_.p, v.z, v.p);
+    NDS_LAUNCH();
+    if (split_) {
+      split_dot(A, (const S*)v.p, v.q);
+    } else {
+      {
+        ProfScope ps(prof, st_, A.cat);
+        sell_launch<k::SELL_DOT, S>(A, g, v.p, nullptr, nullptr, 0.0, v.q, nullptr);
+        NDS_LAUNCH();
+      }
+      reduce_pcg<k::PCG_ALPHA>(g, S_PQ);
+    }
+    const TA* den0 = nullptr;
+    TA w0 = 0, *x1 = nullptr;
+    if (fused) {
+      const PolyPlan pl = fine_plan();
+      den0 = pl.den0;
+      w0 = TA(pl.w0);
+      x1 = fine_first(v.z);
+    }
+    pdl_launch(k::xr_update<S, TA, k::PCG_CHECK>, g, kBlock, 0, st_, nc_, 0.0, sc_.p + S_ALPHA, v.p, v.q, v.x, v.r,
+               tail(S_RN2, h), den0, w0, x1, v.rA);
+    NDS_LAUNCH();
+    if (!fused && v.rA) {
+      pdl_launch(k::cast_copy<S, TA>, grid_for(nc_), kBlock, 0, st_, nc_, v.r, v.rA);
       NDS_LAUNCH();
     }
-    reduce_to<1>(g, S_PQ);
-    k::pcg_alpha<<<1, 1, 0, st_>>>(sc_.p, flags_.p);
-    NDS_LAUNCH();
-    k::xr_update<T><<<g, kBlock, 0, st_>>>(nc_, 0.0, sc_.p + S_ALPHA, pp_.p, q_.p, x_.p, r_.p, part_.p);
-    NDS_LAUNCH();
-    reduce_to<1>(g, S_RN2);
-    NDS_CUDA(cudaMemcpyAsync(hsc_ + S_RN2, sc_.p + S_RN2, sizeof(double), cudaMemcpyDeviceToHost, st_));
-    NDS_CUDA(cudaMemcpyAsync(hflags_, flags_.p, sizeof(int), cudaMemcpyDeviceToHost, st_));
   }
-  // second half: z = M r, rho_new = r.z, beta = rho_new/rho, p = z + beta p
-  void pcg_half2() {
-    amg_T(r_.p, z_.p);
-    dot_dev(r_.p, z_.p, nc_, S_RHON);
-    k::pcg_beta<<<1, 1, 0, st_>>>(sc_.p, flags_.p);
-    NDS_LAUNCH();
-    k::p_update<T><<<grid_for(nc_), kBlock, 0, st_>>>(nc_, sc_.p + S_BETA, z_.p, pp_.p);
-    NDS_LAUNCH();
-  }
-  // one pass of the device loop: z = M r; rho (first pass: p = z); q = A p;
-  // alpha; x, r update; ||r||^2; check
-  void pcg_loop_body(cudaGraphConditionalHandle h) {
-    amg_T(r_.p, z_.p);
-    const int g = red_grid(nc_);
-    k::dot<T><<<g, kBlock, 0, st_>>>(nc_, r_.p, z_.p, part_.p);
-    NDS_LAUNCH();
-    reduce_pcg<k::PCG_RHO>(g, S_RHON);
-    k::p_update_dev<T><<<grid_for(nc_), kBlock, 0, st_>>>(nc_, sc_.p + S_BETA, ctl_.p, z_.p, pp_.p);
-    NDS_LAUNCH();
-    sell_launch<k::SELL_DOT, T>(fine_op(), g, pp_.p, nullptr, nullptr, 0.0, q_.p, nullptr);
-    NDS_LAUNCH();
-    reduce_pcg<k::PCG_ALPHA>(g, S_PQ);
-    k::xr_update<T><<<g, kBlock, 0, st_>>>(nc_, 0.0, sc_.p + S_ALPHA, pp_.p, q_.p, x_.p, r_.p, part_.p);
-    NDS_LAUNCH();
-    reduce_pcg<k::PCG_CHECK>(g, S_RN2, o_.p_max, h);
+  PcgVecs<T> pcg_vecs() {
+    if constexpr (kSame) return {x_.p, r_.p, q_.p, pp_.p, z_.p, nullptr};
+    else return {x_.p, r_.p, q_.p, pp_.p, zA_.p, rA_.p};
   }
   // PCG with the iteration loop on the device: two host synchronisations per
-  // solve (initial norm, final state) instead of one per iteration.  Same
-  // arithmetic and stopping rule as pcg_host.
-  PRes pcg_device(double r0) {
-    const double target = std::max(o_.p_atol, o_.p_rtol * r0);
-    hsc_[S_R0] = r0;
-    hsc_[S_TARGET] = target;
-    NDS_CUDA(cudaMemcpyAsync(sc_.p + S_R0, hsc_ + S_R0, 2 * sizeof(double), cudaMemcpyHostToDevice, st_));
-    const int init[4] = {0, 0, 1, o_.p_max};
-    std::memcpy(hflags_ + 4, init, sizeof(init));
-    NDS_CUDA(cudaMemcpyAsync(ctl_.p, hflags_ + 4, 4 * sizeof(int), cudaMemcpyHostToDevice, st_));
-    NDS_CUDA(cudaMemsetAsync(flags_.p, 0, sizeof(int), st_));
-    NDS_CUDA(cudaGraphLaunch(g_loop_.exec, st_));
-    NDS_CUDA(cudaMemcpyAsync(hflags_ + 4, ctl_.p, 4 * sizeof(int), cudaMemcpyDeviceToHost, st_));
-    NDS_CUDA(cudaMemcpyAsync(hflags_, flags_.p, sizeof(int), cudaMemcpyDeviceToHost, st_));
-    NDS_CUDA(cudaMemcpyAsync(hsc_ + S_RN2, sc_.p + S_RN2, sizeof(double), cudaMemcpyDeviceToHost, st_));
-    NDS_CUDA(cudaStreamSynchronize(st_));
-    const int its = hflags_[4], f = hflags_[0];
-    g_launches += (unsigned long long)its * g_loop_.body_kernels;
-    if (f & 8) throw SolveFailure(NDS_E_BREAKDOWN, "pressure PCG initial rho nonpositive");
-    if (f & 1) throw SolveFailure(NDS_E_BREAKDOWN, "pressure PCG pAp nonpositive");
-    if (f & 2) throw SolveFailure(NDS_E_BREAKDOWN, "pressure PCG rho nonpositive");
-    PRes R;
-    R.its = its;
-    R.rel = std::sqrt(hsc_[S_RN2]) / std::max(r0, 1e-300);
-    if ((f & 4) || !std::isfinite(R.rel)) throw SolveFailure(NDS_E_BREAKDOWN, "pressure PCG residual nonfinite");
-    R.ok = hflags_[5] != 0;
-    return R;
-  }
+  // solve (initial norm, final state) instead of one per iteration.  With
+  // graphs off or the profiler on the same body runs launch by launch.
   PRes pcg(const T* rhs) {
     const double r0 = p_start(rhs);
     start_readback();
     if (r0 <= o_.p_atol) return {0, 0.0, true};
-    // device loop unless the category profiler needs per-kernel events (or
-    // graphs are off / the conditional graph could not be built)
-    if (use_graphs_ && !prof.on && !g_loop_.failed && o_.p_max >= 1) {
-      if (g_loop_.exec || build_pcg_loop()) return pcg_device(r0);
-    }
-    return pcg_host(r0);
-  }
-  PRes pcg_host(double r0) {
-    amg_rz();
-    vcopy(nc_, z_.p, pp_.p);
-    dot_dev(r_.p, z_.p, nc_, S_RHO);
-    fetch(S_RHO, 1);
-    if (!(hsc_[S_RHO] > 0) || !std::isfinite(hsc_[S_RHO])) throw SolveFailure(NDS_E_BREAKDOWN, "pressure PCG initial rho nonpositive");
-    NDS_CUDA(cudaMemsetAsync(flags_.p, 0, sizeof(int), st_));
-    const double target = std::max(o_.p_atol, o_.p_rtol * r0);
-    // the first half stays a direct launch sequence, so the fine SpMV of the
-    // Krylov step is timed live by the profiler; the AMG half is a graph
-    if (use_graphs_ && !g_pcg2_.exec) capture(g_pcg2_, [&] { pcg_half2(); });
+    pcg_first(pcg_vecs());
+    set_target(std::max(o_.p_atol, o_.p_rtol * r0), r0);
+    set_ctl(0, 0, 1, o_.p_max);
+    run_loop(g_loop_, [&](cudaGraphConditionalHandle h) { pcg_body(pcg_vecs(), fine_op(), h); });
+    const int f = hflags_[0];
+    if (f & 8) throw SolveFailure(NDS_E_BREAKDOWN, "pressure PCG initial rho nonpositive");
+    if (f & 1) throw SolveFailure(NDS_E_BREAKDOWN, "pressure PCG pAp nonpositive");
+    if (f & 2) throw SolveFailure(NDS_E_BREAKDOWN, "pressure PCG rho nonpositive");
     PRes R;
-    for (int kk = 0; kk < o_.p_max; ++kk) {
-      pcg_half1();
-      NDS_CUDA(cudaStreamSynchronize(st_));
-      if (*hflags_ & 1) throw SolveFailure(NDS_E_BREAKDOWN, "pressure PCG pAp nonpositive");
-      if (*hflags_ & 2) throw SolveFailure(NDS_E_BREAKDOWN, "pressure PCG rho nonpositive");
-      const double rn = std::sqrt(hsc_[S_RN2]);
-      R.its = kk + 1;
-      R.rel = rn / std::max(r0, 1e-300);
-      if (!std::isfinite(R.rel)) throw SolveFailure(NDS_E_BREAKDOWN, "pressure PCG residual nonfinite");
-      if (rn <= target) {
-        R.ok = true;
-        break;
-      }
-      if (use_graphs_) replay(g_pcg2_);
-      else pcg_half2();
-    }
-    check_flags();
+    R.its = hflags_[4];
+    R.rel = std::sqrt(hsc_[S_RN2]) / std::max(r0, 1e-300);
+    if ((f & 4) || !std::isfinite(R.rel)) throw SolveFailure(NDS_E_BREAKDOWN, "pressure PCG residual nonfinite");
+    R.ok = hflags_[5] != 0;
     return R;
   }
   // Richardson (omega fixed) and outer Chebyshev (omega = 1/root_k)
@@ -1935,7 +1946,11 @@ class Solver final : public ISolver {
       amg_rz();
       fine_apply(z_.p, q_.p);
       const int g = red_grid(nc_);
-      k::xr_update<T><<<g, kBlock, 0, st_>>>(nc_, omega, nullptr, z_.p, q_.p, x_.p, r_.p, part_.p);
+      k::ReduceTail to{};
+      to.part = part_.p;
+      pdl_launch(k::xr_update<T, T, 0>, g, kBlock, 0, st_, nc_, omega, nullptr, z_.p, q_.p, x_.p, r_.p, to, nullptr,
+                 T(0),
+                 nullptr, nullptr);
       NDS_LAUNCH();
       reduce_to<1>(g, S_RN2);
       fetch(S_RN2, 1);
@@ -1968,6 +1983,8 @@ class Solver final : public ISolver {
       fgV_.alloc((size_t)(fg_m_ + 1) * n);
       fgZ_.alloc((size_t)fg_m_ * n);
       fg_.alloc((size_t)k::FgLayout{fg_m_}.size());
+      fgtick_.alloc((size_t)fg_m_ + 1);
+      NDS_CUDA(cudaMemsetAsync(fgtick_.p, 0, fgtick_.bytes(), st_));
       fg_.zero(st_);
     }
     fgpart_.alloc((size_t)kMaxPartBlocks * std::max(fg_m_ + 1, 48));
@@ -1981,9 +1998,6 @@ class Solver final : public ISolver {
   // learned stage: z1 = N(v), t = v - A z1; the V-cycle then solves for t and
   // z = z1 + V(t) -- or, when the stage did not reduce the residual
   // (||t|| >= ||v||), z = V(v) (the plain preconditioner as fallback).
-  // the inner PCG takes the fine pre-smoother's first step in the kernels
-  // that produce r (plain V-cycle with a polynomial smoother only)
-  bool pre_fused() const { return !stage_ && o_.amg_smoother != NDS_SM_MCGS; }
   void precond_f(const float* v, float* z) {
     if constexpr (!kSame) {
       if (!stage_) {
@@ -2116,58 +2130,39 @@ class Solver final : public ISolver {
     if (applied) *applied = (long long)c[0];
     if (fallbacks) *fallbacks = (long long)c[1];
   }
-  // one pass of the FP32 PCG loop: z = M r; rho; p; q = A p; alpha; x, r; check
-  void pcgf_body(cudaGraphConditionalHandle h) {
-    if constexpr (!kSame) {
-      // the fine pre-smoother's first step on r is already in place (taken
-      // by scale_to_float before the loop and by xr_update after it)
-      if (pre_fused()) amg_apply(rf_.p, zf_.p, true);
-      else precond_f(rf_.p, zf_.p);
-      const int g = red_grid(nc_);
-      k::dot<float><<<g, kBlock, 0, st_>>>(nc_, rf_.p, zf_.p, part_.p);
-      NDS_LAUNCH();
-      reduce_pcg<k::PCG_RHO>(g, S_RHON);
-      k::p_update_dev<float><<<grid_for(nc_), kBlock, 0, st_>>>(nc_, sc_.p + S_BETA, ctl_.p, zf_.p, pf_.p);
-      NDS_LAUNCH();
-      {
-        ProfScope ps(prof, st_, P_FINE_AMG);
-        sell_launch<k::SELL_DOT, float>(fine_opA(), g, pf_.p, nullptr, nullptr, 0.0, qf_.p, nullptr);
-        NDS_LAUNCH();
-      }
-      reduce_pcg<k::PCG_ALPHA>(g, S_PQ);
-      if (pre_fused()) {
-        const PolyPlan pl = fine_plan();
-        k::xr_update<float><<<g, kBlock, 0, st_>>>(nc_, 0.0, sc_.p + S_ALPHA, pf_.p, qf_.p, xf_.p, rf_.p, part_.p,
-                                                    pl.den0, float(pl.w0), poly_first(pl, zf_.p, fpong_.p));
-      } else {
-        k::xr_update<float><<<g, kBlock, 0, st_>>>(nc_, 0.0, sc_.p + S_ALPHA, pf_.p, qf_.p, xf_.p, rf_.p, part_.p);
-      }
-      NDS_LAUNCH();
-      reduce_pcg<k::PCG_CHECK>(g, S_RN2, -1, h, in_graph_);
-    }
-  }
   // one Arnoldi step of FGMRES: z_j = M v_j, w = A z_j, classical Gram-Schmidt
   // with FP64 dot products, Givens update of the least-squares problem
   void fg_body(cudaGraphConditionalHandle h) {
     if constexpr (!kSame) {
       const int g = red_grid(nc_);
       const k::FgLayout L{fg_m_};
-      k::fg_fetch<<<grid_for(nc_), kBlock, 0, st_>>>(nc_, fgV_.p, ctl_.p, rf_.p);
+      // rf_ holds v_j, and with pre_fused() the pre-smoother's first step is taken
+      if (pre_fused()) amg_apply(rf_.p, zf_.p, true);
+      else precond_f(rf_.p, zf_.p);
+      if (split_) {  // w = A z_j, Z_j = z_j
+        const OpView<float> A = fine_opA();
+        ProfScope ps(prof, st_, A.cat);
+        split_vertices(A, (const float*)zf_.p);
+        split_types(A, [&](auto mt, auto d16) {
+          pdl_launch(k::split_cell<float, k::SELL_Y, decltype(d16)::value, decltype(mt)>, grid_for(nc_), kBlock, 0,
+                     st_, A.sc, A.w, zf_.p, nullptr, nullptr, 0.f, qf_.p, fgZ_.p, 1.f, (const float*)nullptr,
+                     k::ReduceTail{}, ctl_.p);
+        });
+        NDS_LAUNCH();
+      } else {
+        pdl_launch(k::fg_store, grid_for(nc_), kBlock, 0, st_, nc_, zf_.p, ctl_.p, fgZ_.p);
+        NDS_LAUNCH();
+        op_spmv(fine_opA(), (const float*)zf_.p, qf_.p);
+      }
+      pdl_launch(k::fg_dots, dim3(g, std::min(fg_m_ + 1, k::kDotRows)), kBlock, 0, st_, nc_, fgV_.p, qf_.p, ctl_.p,
+                 fgpart_.p, fgtick_.p, L, fg_.p);
       NDS_LAUNCH();
-      precond_f(rf_.p, zf_.p);
-      k::fg_store<<<grid_for(nc_), kBlock, 0, st_>>>(nc_, zf_.p, ctl_.p, fgZ_.p);
+      pdl_launch(k::fg_orth, g, kBlock, 0, st_, nc_, fgV_.p, fg_.p, L, qf_.p, part_.p, ticket_.p, k::FgScalars{sc_.p,
+                 S_RN2, S_WN, S_TARGET, ctl_.p, flags_.p, h, in_graph_});
       NDS_LAUNCH();
-      op_spmv(fine_opA(), (const float*)zf_.p, qf_.p);
-      k::fg_dots<<<dim3(g, fg_m_ + 1), kBlock, 0, st_>>>(nc_, fgV_.p, qf_.p, ctl_.p, fgpart_.p);
-      NDS_LAUNCH();
-      k::fg_reduce_h<<<fg_m_ + 1, kBlock, 0, st_>>>(fgpart_.p, g, ctl_.p, L, fg_.p);
-      NDS_LAUNCH();
-      k::fg_orth<<<g, kBlock, 0, st_>>>(nc_, fgV_.p, fg_.p, L, ctl_.p, qf_.p, part_.p);
-      NDS_LAUNCH();
-      reduce_to<1>(g, S_RN2);
-      k::fg_givens<<<1, 1, 0, st_>>>(fg_.p, L, sc_.p, S_RN2, S_WN, S_TARGET, ctl_.p, flags_.p, h, in_graph_);
-      NDS_LAUNCH();
-      k::fg_normalize<<<grid_for(nc_), kBlock, 0, st_>>>(nc_, qf_.p, sc_.p, S_WN, ctl_.p, fgV_.p);
+      const PolyPlan pl = pre_fused() ? fine_plan() : PolyPlan{};
+      pdl_launch(k::fg_normalize, grid_for(nc_), kBlock, 0, st_, nc_, qf_.p, sc_.p, S_WN, ctl_.p, fgV_.p, rf_.p,
+                 pl.den0, float(pl.w0), pre_fused() ? fine_first(zf_.p) : nullptr);
       NDS_LAUNCH();
     }
   }
@@ -2224,6 +2219,7 @@ class Solver final : public ISolver {
       NDS_CUDA(cudaGraphLaunch(G.exec, st_));
       NDS_CUDA(cudaMemcpyAsync(hflags_ + 4, ctl_.p, 4 * sizeof(int), cudaMemcpyDeviceToHost, st_));
       NDS_CUDA(cudaMemcpyAsync(hflags_, flags_.p, sizeof(int), cudaMemcpyDeviceToHost, st_));
+      NDS_CUDA(cudaMemcpyAsync(hsc_ + S_RN2, sc_.p + S_RN2, sizeof(double), cudaMemcpyDeviceToHost, st_));
       NDS_CUDA(cudaStreamSynchronize(st_));
       g_launches += (unsigned long long)hflags_[4] * G.body_kernels;
       return;
@@ -2234,6 +2230,7 @@ class Solver final : public ISolver {
       body(cudaGraphConditionalHandle{});
       NDS_CUDA(cudaMemcpyAsync(hflags_ + 4, ctl_.p, 4 * sizeof(int), cudaMemcpyDeviceToHost, st_));
       NDS_CUDA(cudaMemcpyAsync(hflags_, flags_.p, sizeof(int), cudaMemcpyDeviceToHost, st_));
+      NDS_CUDA(cudaMemcpyAsync(hsc_ + S_RN2, sc_.p + S_RN2, sizeof(double), cudaMemcpyDeviceToHost, st_));
       NDS_CUDA(cudaStreamSynchronize(st_));
       prof.collect();
       const int its = hflags_[4], conv = hflags_[5], cap = hflags_[7];
@@ -2257,7 +2254,10 @@ class Solver final : public ISolver {
     xf_.zero(st_);
     set_target(tol, 1.0);
     set_ctl(0, 0, 1, cap);
-    run_loop(g_loopf_, [&](cudaGraphConditionalHandle h) { pcgf_body(h); });
+    if constexpr (!kSame) {
+      const PcgVecs<float> v{xf_.p, rf_.p, qf_.p, pf_.p, zf_.p, nullptr};
+      run_loop(g_loopf_, [&](cudaGraphConditionalHandle h) { pcg_body(v, fine_opA(), h); });
+    }
     const int f = hflags_[0];
     if (f & 8) throw SolveFailure(NDS_E_BREAKDOWN, "inner FP32 PCG initial rho nonpositive");
     if (f & 1) throw SolveFailure(NDS_E_BREAKDOWN, "inner FP32 PCG pAp nonpositive");
@@ -2269,7 +2269,11 @@ class Solver final : public ISolver {
   // Arnoldi steps taken
   int inner_fgmres(double rn, double tol, int cap) {
     const k::FgLayout L{fg_m_};
-    k::scale_to_float<<<grid_for(nc_), kBlock, 0, st_>>>(nc_, r_.p, 1.0 / rn, fgV_.p);
+    if constexpr (!kSame) {
+      const PolyPlan pl = pre_fused() ? fine_plan() : PolyPlan{};
+      pdl_launch(k::scale_to_float, grid_for(nc_), kBlock, 0, st_, nc_, r_.p, 1.0 / rn, fgV_.p, pl.den0,
+                 float(pl.w0), pre_fused() ? fine_first(zf_.p) : nullptr, rf_.p);
+    }
     NDS_LAUNCH();
     set_target(tol, 1.0);
     set_ctl(0, 0, 0, cap);
@@ -2297,14 +2301,14 @@ class Solver final : public ISolver {
         const size_t n = (size_t)nc_;
         for (int a = 0; a < K; ++a) {
           op_spmv(fine_opA(), (const float*)(gYf_.p + a * n), qf_.p);
-          k::cast_copy<float, double><<<grid_for(nc_), kBlock, 0, st_>>>(nc_, qf_.p, gW_.p + a * n);
+          pdl_launch(k::cast_copy<float, double>, grid_for(nc_), kBlock, 0, st_, nc_, qf_.p, gW_.p + a * n);
           NDS_LAUNCH();
         }
       }
     }
-    k::guess_dots<K><<<g, kBlock, 0, st_>>>(nc_, gY_.p, gW_.p, rhs, fgpart_.p);
+    pdl_launch(k::guess_dots<K>, g, kBlock, 0, st_, nc_, gY_.p, gW_.p, rhs, fgpart_.p);
     NDS_LAUNCH();
-    k::reduce_partials<NG><<<1, kBlock, 0, st_>>>(fgpart_.p, g, sc_.p + S_GUESS);
+    pdl_launch(k::reduce_partials<NG>, 1, kBlock, 0, st_, fgpart_.p, g, sc_.p + S_GUESS);
     NDS_LAUNCH();
     fetch(S_GUESS, NG);
     // G c = f by Cholesky (no guess when G is not numerically positive
@@ -2342,7 +2346,7 @@ class Solver final : public ISolver {
       hsc_[S_COEF + a] = c[a];
     }
     NDS_CUDA(cudaMemcpyAsync(sc_.p + S_COEF, hsc_ + S_COEF, K * sizeof(double), cudaMemcpyHostToDevice, st_));
-    k::guess_combine<K><<<grid_for(nc_), kBlock, 0, st_>>>(nc_, gY_.p, sc_.p + S_COEF, x_.p);
+    pdl_launch(k::guess_combine<K>, grid_for(nc_), kBlock, 0, st_, nc_, gY_.p, sc_.p + S_COEF, x_.p);
     NDS_LAUNCH();
     op_resid(fine_op(), (const double*)x_.p, rhs, r_.p);
     return std::sqrt(dot_fetch((const double*)r_.p, (const double*)r_.p, nc_, S_TMP));
@@ -2365,10 +2369,10 @@ class Solver final : public ISolver {
   void store_guess(const double* rhs) {
     if (o_.p_guess <= 0) return;
     const size_t o = (size_t)guess_head_ * nc_;
-    k::guess_store<<<grid_for(nc_), kBlock, 0, st_>>>(nc_, x_.p, rhs, r_.p, gY_.p + o, gW_.p + o);
+    pdl_launch(k::guess_store, grid_for(nc_), kBlock, 0, st_, nc_, x_.p, rhs, r_.p, gY_.p + o, gW_.p + o);
     NDS_LAUNCH();
     if (gYf_.p) {
-      k::cast_copy<double, float><<<grid_for(nc_), kBlock, 0, st_>>>(nc_, x_.p, gYf_.p + o);
+      pdl_launch(k::cast_copy<double, float>, grid_for(nc_), kBlock, 0, st_, nc_, x_.p, gYf_.p + o);
       NDS_LAUNCH();
     }
     guess_head_ = (guess_head_ + 1) % o_.p_guess;
@@ -2413,14 +2417,15 @@ class Solver final : public ISolver {
         } else {
           if (pre_fused()) {
             const PolyPlan pl = fine_plan();
-            k::scale_to_float<<<grid_for(nc_), kBlock, 0, st_>>>(nc_, r_.p, 1.0 / rn, rf_.p, pl.den0, float(pl.w0),
-                                                                 poly_first(pl, zf_.p, fpong_.p));
+            pdl_launch(k::scale_to_float, grid_for(nc_), kBlock, 0, st_, nc_, r_.p, 1.0 / rn, rf_.p, pl.den0,
+                       float(pl.w0), fine_first(zf_.p), (float*)nullptr);
           } else {
-            k::scale_to_float<<<grid_for(nc_), kBlock, 0, st_>>>(nc_, r_.p, 1.0 / rn, rf_.p);
+            pdl_launch(k::scale_to_float, grid_for(nc_), kBlock, 0, st_, nc_, r_.p, 1.0 / rn, rf_.p,
+                       (const float*)nullptr, 0.f, (float*)nullptr, (float*)nullptr);
           }
           NDS_LAUNCH();
           R.its += inner_pcg(tol, cap);
-          k::axpy_from_float<<<grid_for(nc_), kBlock, 0, st_>>>(nc_, rn, xf_.p, x_.p);
+          pdl_launch(k::axpy_from_float, grid_for(nc_), kBlock, 0, st_, nc_, rn, xf_.p, x_.p);
           NDS_LAUNCH();
         }
         ++passes;
@@ -2477,7 +2482,7 @@ class Solver final : public ISolver {
     ProfScope ps(prof, st_, P_ASSEMBLE);
     if (fused_assembly_) {
       // one pass: each incidence's convection row is evaluated in place
-      k::mom_assemble<T, 1><<<grid_for(nv_, kBlock / 8), kBlock, mom_smem_ + 1536 * sizeof(T), st_>>>(a);
+      pdl_launch(k::mom_assemble<T, 1>, grid_for(nv_, kBlock / 8), kBlock, mom_smem_ + 1536 * sizeof(T), st_, a);
       NDS_LAUNCH();
       return;
     }
@@ -2493,7 +2498,7 @@ class Solver final : public ISolver {
                                                         det_.p, centT_.p, zpos_.p, cconv_.p, p_.p, pz_.p, nullptr,
                                                         nullptr, sa);
     NDS_LAUNCH();
-    k::mom_assemble<T><<<grid_for(nv_, kBlock / 8), kBlock, mom_smem_, st_>>>(a);
+    pdl_launch(k::mom_assemble<T>, grid_for(nv_, kBlock / 8), kBlock, mom_smem_, st_, a);
     NDS_LAUNCH();
   }
   void gs_pass(bool reverse) {
@@ -2503,9 +2508,8 @@ class Solver final : public ISolver {
       const int s = color_off_[(size_t)c], n = color_off_[(size_t)c + 1] - s;
       if (!n) continue;
       ProfScope ps(prof, st_, P_GS);
-      k::mom_gs_color<T><<<grid_for((long long)n * 8), kBlock, 0, st_>>>(
-          n, color_rows_.p + s, gspan_.p + s, mcol_.p, A_.p, diag_.p, b_[0].p, b_[1].p, b_[2].p, uc(0), uc(1), uc(2),
-          T(o_.mom_omega));
+      pdl_launch(k::mom_gs_color<T>, grid_for((long long)n * 8), kBlock, 0, st_, n, color_rows_.p + s, gspan_.p + s,
+                 mcol_.p, A_.p, diag_.p, b_[0].p, b_[1].p, b_[2].p, uc(0), uc(1), uc(2), T(o_.mom_omega));
       NDS_LAUNCH();
     }
   }
@@ -2583,8 +2587,8 @@ class Solver final : public ISolver {
     {
       const int g = red_grid(nc_);
       ProfScope ps(prof, st_, P_CONTINUITY);
-      k::continuity<T><<<g, kBlock, 0, st_>>>(nc_, ref_.p, bco_.p, fixed_div_.p, uc(0), uc(1), uc(2), rhs_.p,
-                                             part_.p);
+      pdl_launch(k::continuity<T>, g, kBlock, 0, st_, nc_, ref_.p, bco_.p, fixed_div_.p, uc(0), uc(1), uc(2), rhs_.p,
+                 part_.p);
       NDS_LAUNCH();
       reduce_to<1>(g, S_CONT2);
       fetch(S_CONT2, 1);
@@ -2870,6 +2874,7 @@ class Solver final : public ISolver {
   DBuf<__half> fvalH_;  // FP16 copy of the fine operator for the V-cycle (amg_half)
   double hscale_ = 1.0;
   DBuf<double> fg_, fgpart_, gY_, gW_;
+  DBuf<unsigned> fgtick_;  // of the FGMRES dots, one per basis vector
   LoopGraph g_loopf_, g_fgmres_;
   // learned stage: network state, face graph (neighbours, SELL offsets of
   // the edges, edge weights, Jacobi scaling), work vectors, counters
@@ -2878,7 +2883,8 @@ class Solver final : public ISolver {
   DBuf<uint8_t> sg_face_;
   DBuf<float> sg_ew_, sg_dscale_, st_z1_, st_t_;
   DBuf<unsigned long long> st_cnt_;
-  DBuf<double> part_, sc_;
+  DBuf<double> part_, sc_, tailpart_;
+  DBuf<unsigned> ticket_;  // of the reduction tails (stream st_, one launch at a time)
   DBuf<int> flags_;
   double* hsc_ = nullptr;
   int* hflags_ = nullptr;  // [0] flags, [4..7] device-loop control words

@@ -64,6 +64,7 @@ constexpr int kSplitAhead = 4;
 template <class V, int REC>
 __global__ void __launch_bounds__(kBlock) split_vertex(SplitVerts a, const V* __restrict__ rau,
                                                        const V* __restrict__ x, V* __restrict__ w, V scale) {
+  pdl_begin();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int g = t >> 3, lane = t & 7;
   if (g >= a.n) return;
@@ -252,45 +253,63 @@ __device__ __forceinline__ V split_row(const SplitCells& a, const V* __restrict_
   return s;
 }
 
-// The modes of sell_spmv on the split form (w from split_vertex on the same
-// x); MODE SELL_DOT walks the cells grid-stride and leaves partials of x.y.
-template <class V, int MODE, bool D16, class MT = V>
+// The modes Y, RESID and SMOOTH of sell_spmv on the split form (w from
+// split_vertex on the same x).  Y with y2: also x into vector at[0] of y2.
+// STEP PCG_RHO (SMOOTH with y2, the last step
+// of the V-cycle): also r.z of the new z = y2 with the reduction tail.
+template <class V, int MODE, bool D16, class MT, int STEP = 0, class R = V>
 __global__ void __launch_bounds__(kBlock) split_cell(SplitCells a, const V* __restrict__ w, const V* __restrict__ x,
                                                      const V* __restrict__ b, const V* __restrict__ den, V wt,
-                                                     V* __restrict__ y, V* __restrict__ y2, double* __restrict__ part,
-                                                     V tinv) {
-  if (MODE == SELL_DOT) {
-    double acc[1] = {0.0};
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < a.n; c += gridDim.x * blockDim.x) {
-      const V xc = x[c];
-      const V s = split_row<V, MT, D16>(a, x, w, c, xc, tinv);
-      y[c] = s;
-      acc[0] += (double)xc * (double)s;
-    }
-    write_partials<1>(acc, part);
-    return;
-  }
+                                                     V* __restrict__ y, V* __restrict__ y2, V tinv,
+                                                     const R* __restrict__ rr, ReduceTail tail,
+                                                     const int* __restrict__ at) {
+  pdl_begin();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= a.n) return;
-  const V xc = x[c];
-  V bc = 0, dc = 1;
-  if (MODE != SELL_Y) {
-    bc = b[c];
-    if (MODE == SELL_SMOOTH || den) dc = den[c];
+  double acc = 0.0;
+  if (c < a.n) {
+    const V xc = x[c];
+    V bc = 0, dc = 1;
+    if (MODE != SELL_Y) {
+      bc = b[c];
+      if (MODE == SELL_SMOOTH || den) dc = den[c];
+    }
+    const V s = split_row<V, MT, D16>(a, x, w, c, xc, tinv);
+    if (MODE == SELL_Y) {
+      y[c] = s;
+      if (y2) y2[(size_t)at[0] * a.n + c] = xc;
+    } else if (MODE == SELL_RESID) {
+      const V q = bc - s;
+      y[c] = q;
+      if (den) y2[c] = wt * q / dc;
+      else if (y2) y2[c] = q;
+    } else {
+      V val = xc + wt * (bc - s) / dc;
+      if (y2) {
+        val += y2[c];
+        y2[c] = val;
+      } else {
+        y[c] = val;
+      }
+      if (STEP != 0) acc = (double)rr[c] * (double)val;
+    }
   }
-  const V s = split_row<V, MT, D16>(a, x, w, c, xc, tinv);
-  if (MODE == SELL_Y) {
-    y[c] = s;
-  } else if (MODE == SELL_RESID) {
-    const V q = bc - s;
-    y[c] = q;
-    if (den) y2[c] = wt * q / dc;
-    else if (y2) y2[c] = q;
-  } else {
-    const V val = xc + wt * (bc - s) / dc;
-    if (y2) y2[c] += val;
-    else y[c] = val;
+  if (STEP != 0) reduce_tail<STEP>(acc, tail);
+}
+// q = A p with p.q and the step alpha of PCG (grid-stride; the data type of
+// the operator is that of the vectors)
+template <class V, bool D16>
+__global__ void __launch_bounds__(kBlock) split_cell_dot(SplitCells a, const V* __restrict__ w,
+                                                         const V* __restrict__ p, V* __restrict__ q, V tinv,
+                                                         ReduceTail tail) {
+  pdl_begin();
+  double acc = 0.0;
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < a.n; c += gridDim.x * blockDim.x) {
+    const V pc = p[c];
+    const V s = split_row<V, V, D16>(a, p, w, c, pc, tinv);
+    q[c] = s;
+    acc += (double)pc * (double)s;
   }
+  reduce_tail<PCG_ALPHA>(acc, tail);
 }
 
 // Refresh of the split form from rAU: thread c writes cell c's face couplings

@@ -18,13 +18,17 @@
 // t_i = x_i sqrt(a_ii) / sigma_s for pairs (v, x) of pressure-correction
 // right-hand sides and solutions: the diagonal-weighted error of z against x.
 //
-// Layer kernel (forward): persistent CTAs of 128 threads, one 128-row tile at
-// a time: each thread gathers its row's own features and its neighbours'
-// (L2-resident under the mesh numbering), writes the row [h_i ; m_i] as BF16
-// into the A tile (canonical no-swizzle layout), one thread issues 8 MMAs
-// (M = 128, N = 64, K = 16) against the weight tile kept in shared memory,
-// the accumulator (128 lanes x 64 columns of TMEM) is read back with
-// tcgen05.ld for the bias + ReLU epilogue.  Backward uses the same tiles:
+// Layer kernel (forward): persistent CTAs of 512 threads, one 128-row tile at
+// a time, bound by memory: four threads gather a row, 16 features each (its
+// own and its neighbours', L2-resident under the mesh numbering; a warp reads
+// whole 128-byte rows and each thread has all its loads in flight), and write
+// [h_i ; m_i] as BF16 into the A tile (canonical no-swizzle layout); one
+// thread issues 8 MMAs (M = 128, N = 64, K = 16) against the weight tile kept
+// in shared memory, and the accumulator (128 lanes x 64 columns of TMEM) is
+// read back with tcgen05.ld for the bias + ReLU epilogue, warp w taking lanes
+// 32 (w mod 4) and columns 16 (w / 4).  403,680 nodes: 127 us a layer with one thread per
+// row (two waves of 128-byte rows per warp load), 70 us so (0.25 TB/s of
+// neighbours' rows from L2 beside the 103 MB read and written).  Backward uses the same tiles:
 // dX = delta W (M 128, N 128, K 64) and dW^T += X^T delta (M 128, N 64,
 // K = the 128 nodes of the tile, both operands read MN-major from the same
 // shared-memory tiles), accumulated in TMEM over all tiles of a CTA.
@@ -49,7 +53,9 @@ namespace mp {
 
 constexpr int kH = 64;         // hidden width
 constexpr int kX = 2 * kH;     // dense-layer input width [h ; m]
-constexpr int kTile = 128;     // rows per tile (= threads per CTA)
+constexpr int kTile = 128;     // rows per tile
+constexpr int kThreads = 512;  // threads per CTA: four per row
+constexpr int kPart = kH / 4;  // features of a row that one thread handles
 constexpr uint64_t kWaitNs = 2000000000ull;  // bound of every mbarrier wait: 2 s of wall time
 
 // parameter layout (FP32 master copy; gradients use the same layout)
@@ -176,65 +182,80 @@ struct LayerIn {
   const float2* f;                 // layer 1
   const __nv_bfloat16* hin;        // layers 2, 3
 };
-template <bool ENC>
-__device__ __forceinline__ void encoder_row(float2 fi, const float* __restrict__ s_we, const float* __restrict__ s_be,
-                                            float (&h)[kH]) {
+// features k0 .. k0 + 15 of the encoder's output, rounded as a stored activation
+__device__ __forceinline__ void encoder_part(float2 fi, const float* __restrict__ s_we, const float* __restrict__ s_be,
+                                             int k0, float (&h)[kPart]) {
 #pragma unroll
-  for (int k = 0; k < kH; ++k) {
-    const float v = fmaf(s_we[2 * k], fi.x, fmaf(s_we[2 * k + 1], fi.y, s_be[k]));
+  for (int k = 0; k < kPart; ++k) {
+    const float v = fmaf(s_we[2 * (k0 + k)], fi.x, fmaf(s_we[2 * (k0 + k) + 1], fi.y, s_be[k0 + k]));
     h[k] = __bfloat162float(__float2bfloat16_rn(fmaxf(v, 0.f)));
   }
 }
+// thread's part (features 16 part ..) of row r of the tile, graph node `row`
 template <bool ENC>
-__device__ void build_row(const LayerIn& in, int row, uint8_t* __restrict__ X, int r, const float* __restrict__ s_we,
-                          const float* __restrict__ s_be) {
-  float m[kH];
-#pragma unroll
-  for (int k = 0; k < kH; ++k) m[k] = 0.f;
+__device__ __forceinline__ void build_part(const LayerIn& in, int row, uint8_t* __restrict__ X, int r, int part,
+                                           const float* __restrict__ s_we, const float* __restrict__ s_be) {
+  const int c0 = 2 * part;  // 16-byte chunks c0, c0 + 1 of the row's 8
   if (row >= in.n) {
     const uint4 z = make_uint4(0, 0, 0, 0);
 #pragma unroll
-    for (int c = 0; c < 16; ++c) *reinterpret_cast<uint4*>(X + tile_off(r, c, 2048)) = z;
+    for (int c = 0; c < 2; ++c) {
+      *reinterpret_cast<uint4*>(X + tile_off(r, c0 + c, 2048)) = z;
+      *reinterpret_cast<uint4*>(X + tile_off(r, 8 + c0 + c, 2048)) = z;
+    }
     return;
   }
-  if (ENC) {
-    float h[kH];
-    encoder_row<true>(in.f[row], s_we, s_be, h);
+  float m[kPart];
 #pragma unroll
-    for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(X + tile_off(r, c, 2048)) = pack8(h + 8 * c);
+  for (int k = 0; k < kPart; ++k) m[k] = 0.f;
+  // (the graph's arrays are the caller's: no alignment beyond their type's)
+  if (ENC) {
+    float h[kPart];
+    encoder_part(in.f[row], s_we, s_be, kPart * part, h);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) *reinterpret_cast<uint4*>(X + tile_off(r, c0 + c, 2048)) = pack8(h + 8 * c);
 #pragma unroll 1
     for (int k = 0; k < 4; ++k) {
       const int j = in.nbr[4 * (size_t)row + k];
       if (j < 0 || j >= in.n) continue;
       const float w = in.ew[4 * (size_t)row + k];
-      encoder_row<true>(in.f[j], s_we, s_be, h);
+      encoder_part(in.f[j], s_we, s_be, kPart * part, h);
 #pragma unroll
-      for (int q = 0; q < kH; ++q) m[q] = fmaf(w, h[q], m[q]);
+      for (int q = 0; q < kPart; ++q) m[q] = fmaf(w, h[q], m[q]);
     }
   } else {
-    const uint4* self = reinterpret_cast<const uint4*>(in.hin + (size_t)row * kH);
+    int jj[4];
+    float ww[4];
 #pragma unroll
-    for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(X + tile_off(r, c, 2048)) = self[c];
-#pragma unroll 1
     for (int k = 0; k < 4; ++k) {
-      const int j = in.nbr[4 * (size_t)row + k];
-      if (j < 0 || j >= in.n) continue;
-      const float w = in.ew[4 * (size_t)row + k];
-      const uint4* hj = reinterpret_cast<const uint4*>(in.hin + (size_t)j * kH);
-      uint4 u[8];
+      jj[k] = in.nbr[4 * (size_t)row + k];
+      ww[k] = in.ew[4 * (size_t)row + k];
+    }
+    const uint4* self = reinterpret_cast<const uint4*>(in.hin + (size_t)row * kH) + c0;
+    uint4 u[4][2];
 #pragma unroll
-      for (int c = 0; c < 8; ++c) u[c] = hj[c];
+    for (int k = 0; k < 4; ++k) {
+      const bool ok = jj[k] >= 0 && jj[k] < in.n;
+      const uint4* hj = reinterpret_cast<const uint4*>(in.hin + (size_t)(ok ? jj[k] : row) * kH) + c0;
+      u[k][0] = hj[0];
+      u[k][1] = hj[1];
+    }
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
+    for (int c = 0; c < 2; ++c) *reinterpret_cast<uint4*>(X + tile_off(r, c0 + c, 2048)) = self[c];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (jj[k] < 0 || jj[k] >= in.n) continue;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
         float t[8];
-        unpack8(u[c], t);
+        unpack8(u[k][c], t);
 #pragma unroll
-        for (int q = 0; q < 8; ++q) m[8 * c + q] = fmaf(w, t[q], m[8 * c + q]);
+        for (int q = 0; q < 8; ++q) m[8 * c + q] = fmaf(ww[k], t[q], m[8 * c + q]);
       }
     }
   }
 #pragma unroll
-  for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(X + tile_off(r, 8 + c, 2048)) = pack8(m + 8 * c);
+  for (int c = 0; c < 2; ++c) *reinterpret_cast<uint4*>(X + tile_off(r, 8 + c0 + c, 2048)) = pack8(m + 8 * c);
 }
 
 // ---------------------------------------------------------------------------
@@ -258,7 +279,7 @@ struct FwdArgs {
 constexpr int kFwdSmem = 16384 + 32768 + 1024;  // W tile, X tile, alignment slack
 
 template <bool ENC, bool DEC>
-__global__ void __launch_bounds__(kTile) layer_fwd(FwdArgs a) {
+__global__ void __launch_bounds__(kThreads, 2) layer_fwd(FwdArgs a) {
   extern __shared__ uint8_t dsm[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dsm) + 1023) & ~uintptr_t(1023));
   uint8_t* Wsm = base;
@@ -266,19 +287,21 @@ __global__ void __launch_bounds__(kTile) layer_fwd(FwdArgs a) {
   __shared__ uint64_t mbar;
   __shared__ uint32_t tbase_s;
   __shared__ float s_we[2 * kH], s_be[kH], s_b[kH], s_wd[kH];
+  __shared__ float s_dec[4][kTile];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int er = 32 * (warp & 3) + lane, eg = warp >> 2;  // epilogue: row of the tile, group of 16 columns
 
   // weight tile: W[o][i] as B (N = 64 rows o, K = 128), K-major
-  for (int e = tid; e < kH * 16; e += kTile) {
+  for (int e = tid; e < kH * 16; e += kThreads) {
     const int o = e >> 4, c = e & 15;
     *reinterpret_cast<uint4*>(Wsm + tile_off(o, c, 2048)) = reinterpret_cast<const uint4*>(a.W)[e];
   }
-  for (int q = tid; q < kH; q += kTile) {
+  for (int q = tid; q < kH; q += kThreads) {
     s_b[q] = a.params[off_b(a.layer) + q];
     s_be[q] = a.params[OFF_BE + q];
     s_wd[q] = a.params[OFF_WD + q];
   }
-  for (int q = tid; q < 2 * kH; q += kTile) s_we[q] = a.params[OFF_WE + q];
+  for (int q = tid; q < 2 * kH; q += kThreads) s_we[q] = a.params[OFF_WE + q];
   if (warp == 0) {
     tc::tmem_alloc(&tbase_s, 64);
     tc::tmem_relinquish();
@@ -295,8 +318,7 @@ __global__ void __launch_bounds__(kTile) layer_fwd(FwdArgs a) {
   uint32_t phase = 0;
   const int ntiles = (a.in.n + kTile - 1) / kTile;
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int row = tile * kTile + tid;
-    build_row<ENC>(a.in, row, Xsm, tid, s_we, s_be);
+    build_part<ENC>(a.in, tile * kTile + (tid >> 2), Xsm, tid >> 2, tid & 3, s_we, s_be);
     tc::fence_async_smem();
     tc::fence_before_sync();
     __syncthreads();
@@ -315,33 +337,34 @@ __global__ void __launch_bounds__(kTile) layer_fwd(FwdArgs a) {
       break;
     }
     tc::fence_after_sync();
-    float acc[kH];
-    {
-      float t[32];
-      tc::tmem_ld32(tbase + ((uint32_t)(32 * warp) << 16), t);
-#pragma unroll
-      for (int q = 0; q < 32; ++q) acc[q] = t[q];
-      tc::tmem_ld32(tbase + ((uint32_t)(32 * warp) << 16) + 32, t);
-#pragma unroll
-      for (int q = 0; q < 32; ++q) acc[32 + q] = t[q];
-    }
+    float acc[kPart];
+    tc::tmem_ld16(tbase + ((uint32_t)(32 * (warp & 3)) << 16) + kPart * eg, acc);
+    const int row = tile * kTile + er;
     if (row < a.in.n) {
-      float h[kH];
+      float h[kPart];
 #pragma unroll
-      for (int q = 0; q < kH; ++q) h[q] = __bfloat162float(__float2bfloat16_rn(fmaxf(acc[q] + s_b[q], 0.f)));
+      for (int q = 0; q < kPart; ++q)
+        h[q] = __bfloat162float(__float2bfloat16_rn(fmaxf(acc[q] + s_b[kPart * eg + q], 0.f)));
       if (a.hout) {
-        uint4* dst = reinterpret_cast<uint4*>(a.hout + (size_t)row * kH);
-#pragma unroll
-        for (int c = 0; c < 8; ++c) dst[c] = pack8(h + 8 * c);
+        uint4* dst = reinterpret_cast<uint4*>(a.hout + (size_t)row * kH) + 2 * eg;
+        dst[0] = pack8(h);
+        dst[1] = pack8(h + 8);
       }
       if (DEC) {
-        float o = bd;
+        float o = 0.f;
 #pragma unroll
-        for (int q = 0; q < kH; ++q) o = fmaf(s_wd[q], h[q], o);
-        const float si = a.in.f[row].x;
-        o = fmaf(cs, si, o);
-        if (a.out) a.out[row] = o;
-        if (a.z) a.z[row] = o * a.sigma[seg_of(row, a.seg_off, a.nseg)] * a.dscale[row];
+        for (int q = 0; q < kPart; ++q) o = fmaf(s_wd[kPart * eg + q], h[q], o);
+        s_dec[eg][er] = o;
+      }
+    }
+    if (DEC) {
+      __syncthreads();
+      const int orow = tile * kTile + tid;
+      if (tid < kTile && orow < a.in.n) {
+        float o = bd + ((s_dec[0][tid] + s_dec[1][tid]) + (s_dec[2][tid] + s_dec[3][tid]));
+        o = fmaf(cs, a.in.f[orow].x, o);
+        if (a.out) a.out[orow] = o;
+        if (a.z) a.z[orow] = o * a.sigma[seg_of(orow, a.seg_off, a.nseg)] * a.dscale[orow];
       }
     }
     tc::fence_before_sync();
@@ -351,7 +374,6 @@ __global__ void __launch_bounds__(kTile) layer_fwd(FwdArgs a) {
   tc::fence_before_sync();
   __syncthreads();
   if (warp == 0) tc::tmem_dealloc(tbase, 64);
-  (void)lane;
 }
 
 // ---------------------------------------------------------------------------
@@ -374,7 +396,7 @@ struct BwdArgs {
 constexpr int kBwdSmem = 16384 + 32768 + 16384 + 1024 + 40000;  // W^T, X, delta tiles; slack limits 2 CTAs / SM
 
 template <bool ENC>
-__global__ void __launch_bounds__(kTile) layer_bwd(BwdArgs a) {
+__global__ void __launch_bounds__(kThreads, 2) layer_bwd(BwdArgs a) {
   extern __shared__ uint8_t dsm[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dsm) + 1023) & ~uintptr_t(1023));
   uint8_t* WTsm = base;            // B of dX: N = 128 (i), K = 64 (o), K-major, 8-row groups at 1024 B
@@ -383,9 +405,11 @@ __global__ void __launch_bounds__(kTile) layer_bwd(BwdArgs a) {
   __shared__ uint64_t mbar;
   __shared__ uint32_t tbase_s;
   __shared__ float s_we[2 * kH], s_be[kH];
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int br = tid >> 2, part = tid & 3;                // building: row of the tile, 16 features
+  const int er = 32 * (warp & 3) + lane, eg = warp >> 2;  // epilogue: row, group of columns
 
-  for (int e = tid; e < kX * 8; e += kTile) {
+  for (int e = tid; e < kX * 8; e += kThreads) {
     // W^T[i][o]: row i, 16-byte chunk c covers o = 8c..8c+7
     const int i = e >> 3, c = e & 7;
     float t[8];
@@ -393,8 +417,8 @@ __global__ void __launch_bounds__(kTile) layer_bwd(BwdArgs a) {
     for (int q = 0; q < 8; ++q) t[q] = __bfloat162float(a.W[(size_t)(8 * c + q) * kX + i]);
     *reinterpret_cast<uint4*>(WTsm + tile_off(i, c, 1024)) = pack8(t);
   }
-  for (int q = tid; q < kH; q += kTile) s_be[q] = a.params[OFF_BE + q];
-  for (int q = tid; q < 2 * kH; q += kTile) s_we[q] = a.params[OFF_WE + q];
+  for (int q = tid; q < kH; q += kThreads) s_be[q] = a.params[OFF_BE + q];
+  for (int q = tid; q < 2 * kH; q += kThreads) s_we[q] = a.params[OFF_WE + q];
   if (warp == 0) {
     tc::tmem_alloc(&tbase_s, 256);
     tc::tmem_relinquish();
@@ -408,21 +432,21 @@ __global__ void __launch_bounds__(kTile) layer_bwd(BwdArgs a) {
   constexpr uint32_t idx_dx = tc::idesc_bf16_f32(128, 128, 0, 0);
   constexpr uint32_t idx_dw = tc::idesc_bf16_f32(128, 64, 1, 1);
   const uint32_t xs = tc::smem_addr(Xsm), ds = tc::smem_addr(Dsm), wts = tc::smem_addr(WTsm);
-  float dbacc[kH];
+  float dbacc[kPart];
 #pragma unroll
-  for (int q = 0; q < kH; ++q) dbacc[q] = 0.f;
+  for (int q = 0; q < kPart; ++q) dbacc[q] = 0.f;
   uint32_t phase = 0;
   bool first = true, aborted = false;
   const int ntiles = (a.in.n + kTile - 1) / kTile;
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int row = tile * kTile + tid;
     {
-      float d[kH];
+      const int row = tile * kTile + br;
+      float d[kPart];
       if (row < a.in.n) {
-        const float4* g = reinterpret_cast<const float4*>(a.dh + (size_t)row * kH);
-        const uint4* hh = reinterpret_cast<const uint4*>(a.h + (size_t)row * kH);
+        const float4* g = reinterpret_cast<const float4*>(a.dh + (size_t)row * kH) + 4 * part;
+        const uint4* hh = reinterpret_cast<const uint4*>(a.h + (size_t)row * kH) + 2 * part;
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
+        for (int c = 0; c < 2; ++c) {
           float hv[8];
           unpack8(hh[c], hv);
           const float4 g0 = g[2 * c], g1 = g[2 * c + 1];
@@ -432,17 +456,17 @@ __global__ void __launch_bounds__(kTile) layer_bwd(BwdArgs a) {
         }
       } else {
 #pragma unroll
-        for (int q = 0; q < kH; ++q) d[q] = 0.f;
+        for (int q = 0; q < kPart; ++q) d[q] = 0.f;
       }
 #pragma unroll
-      for (int q = 0; q < kH; ++q) {
+      for (int q = 0; q < kPart; ++q) {
         d[q] = __bfloat162float(__float2bfloat16_rn(d[q]));
         dbacc[q] += d[q];
       }
 #pragma unroll
-      for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(Dsm + tile_off(tid, c, 1024)) = pack8(d + 8 * c);
+      for (int c = 0; c < 2; ++c) *reinterpret_cast<uint4*>(Dsm + tile_off(br, 2 * part + c, 1024)) = pack8(d + 8 * c);
+      build_part<ENC>(a.in, row, Xsm, br, part, s_we, s_be);
     }
-    build_row<ENC>(a.in, row, Xsm, tid, s_we, s_be);
     tc::fence_async_smem();
     tc::fence_before_sync();
     __syncthreads();
@@ -469,13 +493,14 @@ __global__ void __launch_bounds__(kTile) layer_bwd(BwdArgs a) {
     }
     tc::fence_after_sync();
     // tcgen05.ld is a warp-collective (.sync.aligned): every lane of the warp
-    // executes the same loads, rows past n only skip the stores
-#pragma unroll
-    for (int part = 0; part < 4; ++part) {
+    // executes the same loads, rows past n only skip the stores.  Columns 32
+    // eg .. of dX: groups 0, 1 the own part, 2, 3 the neighbours' part.
+    {
+      const int row = tile * kTile + er;
       float t[32];
-      tc::tmem_ld32(tbase + ((uint32_t)(32 * warp) << 16) + 32 * part, t);
+      tc::tmem_ld32(tbase + ((uint32_t)(32 * (warp & 3)) << 16) + 32 * eg, t);
       if (row < a.in.n) {
-        float* dst = part < 2 ? a.dself + (size_t)row * kH + 32 * part : a.dm + (size_t)row * kH + 32 * (part - 2);
+        float* dst = (eg < 2 ? a.dself : a.dm) + (size_t)row * kH + 32 * (eg & 1);
 #pragma unroll
         for (int q = 0; q < 32; q += 4) *reinterpret_cast<float4*>(dst + q) = make_float4(t[q], t[q + 1], t[q + 2], t[q + 3]);
       }
@@ -484,32 +509,33 @@ __global__ void __launch_bounds__(kTile) layer_bwd(BwdArgs a) {
     __syncthreads();
     tc::fence_after_sync();
   }
-  // dW^T partial of this CTA: thread (warp, lane) holds row i = 32 warp + lane
+  // dW^T partial of this CTA: lane er of TMEM holds row i = er, columns 16 eg ..
   float* wp = a.wpart + (size_t)blockIdx.x * kX * kH;
   if (first || aborted) {
-    for (int q = tid; q < kX * kH; q += kTile) wp[q] = 0.f;
+    for (int q = tid; q < kX * kH; q += kThreads) wp[q] = 0.f;
   } else {
-    float t[32];
-    const int i = 32 * warp + (tid & 31);
+    float t[kPart];
+    tc::tmem_ld16(tbase + ((uint32_t)(32 * (warp & 3)) << 16) + 128 + kPart * eg, t);
 #pragma unroll
-    for (int part = 0; part < 2; ++part) {
-      tc::tmem_ld32(tbase + ((uint32_t)(32 * warp) << 16) + 128 + 32 * part, t);
-#pragma unroll
-      for (int q = 0; q < 32; ++q) wp[(size_t)i * kH + 32 * part + q] = t[q];
-    }
+    for (int q = 0; q < kPart; ++q) wp[(size_t)er * kH + kPart * eg + q] = t[q];
   }
-  // db partial: block sum of the per-thread sums, fixed order
+  // db partial: the sums of the four threads of a row over the rows, in a
+  // fixed order (eight rows of a warp by shuffles, then the warps)
   {
-    __shared__ float red[kTile];
-    for (int q = 0; q < kH; ++q) {
-      red[tid] = dbacc[q];
-      __syncthreads();
-      if (tid == 0) {
-        float s = 0.f;
-        for (int r = 0; r < kTile; ++r) s += red[r];
-        a.bpart[(size_t)blockIdx.x * kH + q] = s;
-      }
-      __syncthreads();
+    __shared__ float red[kThreads / 32][kH];
+#pragma unroll
+    for (int q = 0; q < kPart; ++q) {
+      float v = dbacc[q];
+      v += __shfl_xor_sync(0xffffffffu, v, 4);
+      v += __shfl_xor_sync(0xffffffffu, v, 8);
+      v += __shfl_xor_sync(0xffffffffu, v, 16);
+      if (lane < 4) red[warp][kPart * lane + q] = v;
+    }
+    __syncthreads();
+    if (tid < kH) {
+      float s = 0.f;
+      for (int w = 0; w < kThreads / 32; ++w) s += red[w][tid];
+      a.bpart[(size_t)blockIdx.x * kH + tid] = s;
     }
   }
   tc::fence_before_sync();
@@ -538,29 +564,37 @@ __global__ void scatter_bwd(int n, const int32_t* __restrict__ nbr, const float*
   reinterpret_cast<float4*>(dh + (size_t)i * kH)[c] = s;
 }
 
-// encoder backward: delta0 = dh0 (.) [h0 > 0]; partials of dWe (64 x 2), dbe (64)
+// encoder backward: delta0 = dh0 (.) [h0 > 0]; partials of dWe (64 x 2), dbe
+// (64), FP64.  A thread keeps one unit and walks the rows, four rows of a
+// block at a time, so that a warp reads 32 consecutive gradients and the sums
+// stay in registers.  Bound by reading dh0 (103 MB at 403,680
+// nodes: 80 us; 782 us with 192 sums per thread, which spilled).
 __global__ void __launch_bounds__(kBlock) encoder_bwd(int n, const float2* __restrict__ f, const float* __restrict__ dh0,
                                                       const float* __restrict__ params, double* __restrict__ part) {
-  __shared__ float s_we[2 * kH], s_be[kH];
-  for (int q = threadIdx.x; q < 2 * kH; q += blockDim.x) s_we[q] = params[OFF_WE + q];
-  for (int q = threadIdx.x; q < kH; q += blockDim.x) s_be[q] = params[OFF_BE + q];
-  __syncthreads();
-  double acc[3 * kH];
-#pragma unroll
-  for (int q = 0; q < 3 * kH; ++q) acc[q] = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  constexpr int kRows = kBlock / kH;
+  __shared__ double red[kRows][3 * kH];
+  const int k = threadIdx.x % kH, rg = threadIdx.x / kH;
+  const float w0 = params[OFF_WE + 2 * k], w1 = params[OFF_WE + 2 * k + 1], be = params[OFF_BE + k];
+  double a0 = 0.0, a1 = 0.0, a2 = 0.0;
+#pragma unroll 4
+  for (int i = blockIdx.x * kRows + rg; i < n; i += gridDim.x * kRows) {
     const float2 fi = f[i];
-    for (int k = 0; k < kH; ++k) {
-      const float v = fmaf(s_we[2 * k], fi.x, fmaf(s_we[2 * k + 1], fi.y, s_be[k]));
-      if (v > 0.f) {
-        const double d = dh0[(size_t)i * kH + k];
-        acc[2 * k] += d * fi.x;
-        acc[2 * k + 1] += d * fi.y;
-        acc[2 * kH + k] += d;
-      }
+    const double d = dh0[(size_t)i * kH + k];
+    if (fmaf(w0, fi.x, fmaf(w1, fi.y, be)) > 0.f) {
+      a0 += d * fi.x;
+      a1 += d * fi.y;
+      a2 += d;
     }
   }
-  write_partials<3 * kH>(acc, part);
+  red[rg][2 * k] = a0;
+  red[rg][2 * k + 1] = a1;
+  red[rg][2 * kH + k] = a2;
+  __syncthreads();
+  if (threadIdx.x < 3 * kH) {
+    double s = 0.0;
+    for (int q = 0; q < kRows; ++q) s += red[q][threadIdx.x];
+    part[(size_t)blockIdx.x * (3 * kH) + threadIdx.x] = s;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -581,41 +615,64 @@ __global__ void __launch_bounds__(kBlock) seg_loss(int lo, int hi, const float* 
   }
   write_partials<2>(acc, part);
 }
-// dout = coef_s (out - t); partials of dwd (64), dbd, dcs; dh3 = dout wd
+// The decoder's backward from g_i = dL/d out_i (functor): dh3 = g wd, and
+// partials of dwd (64), dbd, dcs in FP64.  Sixteen threads a row, four units
+// each: rows are read and written whole by half-warps and a thread keeps four
+// sums.  Bound by writing dh3 (128 us before at
+// 403,680 nodes, 64 us so).
+template <class G>
+__device__ __forceinline__ void decoder_rows(int n, const G& grad, const __nv_bfloat16* __restrict__ h3,
+                                             const float2* __restrict__ f, const float* __restrict__ params,
+                                             float* __restrict__ dh3, double* __restrict__ part) {
+  constexpr int kRows = kBlock / 16;
+  __shared__ double red[kRows][kH + 2];
+  const int c = threadIdx.x & 15, rg = threadIdx.x >> 4;
+  float wd[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) wd[q] = params[OFF_WD + 4 * c + q];
+  double acc[4] = {0.0, 0.0, 0.0, 0.0}, ab = 0.0, as = 0.0;
+  for (int i = blockIdx.x * kRows + rg; i < n; i += gridDim.x * kRows) {
+    const float g = grad(i);
+    const uint2 u = reinterpret_cast<const uint2*>(h3 + (size_t)i * kH)[c];
+    const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
+    const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+    acc[0] += (double)g * lo.x;
+    acc[1] += (double)g * lo.y;
+    acc[2] += (double)g * hi.x;
+    acc[3] += (double)g * hi.y;
+    reinterpret_cast<float4*>(dh3 + (size_t)i * kH)[c] = make_float4(g * wd[0], g * wd[1], g * wd[2], g * wd[3]);
+    if (c == 0) {
+      ab += g;
+      as += (double)g * f[i].x;
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) red[rg][4 * c + q] = acc[q];
+  if (c == 0) {
+    red[rg][kH] = ab;
+    red[rg][kH + 1] = as;
+  }
+  __syncthreads();
+  if (threadIdx.x < kH + 2) {
+    double s = 0.0;
+    for (int q = 0; q < kRows; ++q) s += red[q][threadIdx.x];
+    part[(size_t)blockIdx.x * (kH + 2) + threadIdx.x] = s;
+  }
+}
+// from the loss: g = coef_s (out - t)
 __global__ void __launch_bounds__(kBlock) decoder_bwd(int n, const float* __restrict__ out, const float* __restrict__ x,
                                                       const float* __restrict__ dscale, const float* __restrict__ sigma,
                                                       const int32_t* __restrict__ seg_off, int nseg,
                                                       const double* __restrict__ coef, const __nv_bfloat16* __restrict__ h3,
                                                       const float2* __restrict__ f, const float* __restrict__ params,
                                                       float* __restrict__ dh3, double* __restrict__ part) {
-  double acc[kH + 2];
-#pragma unroll
-  for (int q = 0; q < kH + 2; ++q) acc[q] = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  decoder_rows(n, [&](int i) {
     const int s = seg_of(i, seg_off, nseg);
     const double t = (double)x[i] / ((double)dscale[i] * (double)sigma[s]);
-    const float g = (float)(coef[s] * ((double)out[i] - t));
-    const uint4* hh = reinterpret_cast<const uint4*>(h3 + (size_t)i * kH);
-    float4* d = reinterpret_cast<float4*>(dh3 + (size_t)i * kH);
-    for (int c = 0; c < 8; ++c) {
-      float hv[8];
-      unpack8(hh[c], hv);
-      float o[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        acc[8 * c + q] += (double)g * hv[q];
-        o[q] = g * params[OFF_WD + 8 * c + q];
-      }
-      d[2 * c] = make_float4(o[0], o[1], o[2], o[3]);
-      d[2 * c + 1] = make_float4(o[4], o[5], o[6], o[7]);
-    }
-    acc[kH] += g;
-    acc[kH + 1] += (double)g * f[i].x;
-  }
-  write_partials<kH + 2>(acc, part);
+    return (float)(coef[s] * ((double)out[i] - t));
+  }, h3, f, params, dh3, part);
 }
-// the same from a gradient dz with respect to z = out sigma dscale:
-// dout = dz sigma dscale
+// from a gradient dz with respect to z = out sigma dscale: g = dz sigma dscale
 __global__ void __launch_bounds__(kBlock) decoder_bwd_dz(int n, const float* __restrict__ dz,
                                                          const float* __restrict__ dscale,
                                                          const float* __restrict__ sigma,
@@ -623,51 +680,28 @@ __global__ void __launch_bounds__(kBlock) decoder_bwd_dz(int n, const float* __r
                                                          const __nv_bfloat16* __restrict__ h3,
                                                          const float2* __restrict__ f, const float* __restrict__ params,
                                                          float* __restrict__ dh3, double* __restrict__ part) {
-  double acc[kH + 2];
+  decoder_rows(n, [&](int i) { return dz[i] * sigma[seg_of(i, seg_off, nseg)] * dscale[i]; }, h3, f, params, dh3, part);
+}
+// out[c] = sum_r part[r][c], FP64 sums in a fixed order, into FP32: a block
+// takes 32 columns, its eight warps every eighth row each.  transpose: column
+// c = i kH + o of dW^T goes to W's entry o kX + i.
+template <class P>
+__global__ void __launch_bounds__(kBlock) reduce_rows(const P* __restrict__ part, int rows, int cols,
+                                                      float* __restrict__ out, int transpose) {
+  __shared__ double red[kWarps][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
+  double s = 0.0;
+  if (c < cols)
+#pragma unroll 4
+    for (int r = w; r < rows; r += kWarps) s += (double)part[(size_t)r * cols + c];
+  red[w][lane] = s;
+  __syncthreads();
+  if (w == 0 && c < cols) {
+    double t = 0.0;
 #pragma unroll
-  for (int q = 0; q < kH + 2; ++q) acc[q] = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const float g = dz[i] * sigma[seg_of(i, seg_off, nseg)] * dscale[i];
-    const uint4* hh = reinterpret_cast<const uint4*>(h3 + (size_t)i * kH);
-    float4* d = reinterpret_cast<float4*>(dh3 + (size_t)i * kH);
-    for (int c = 0; c < 8; ++c) {
-      float hv[8];
-      unpack8(hh[c], hv);
-      float o[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        acc[8 * c + q] += (double)g * hv[q];
-        o[q] = g * params[OFF_WD + 8 * c + q];
-      }
-      d[2 * c] = make_float4(o[0], o[1], o[2], o[3]);
-      d[2 * c + 1] = make_float4(o[4], o[5], o[6], o[7]);
-    }
-    acc[kH] += g;
-    acc[kH + 1] += (double)g * f[i].x;
+    for (int q = 0; q < kWarps; ++q) t += red[q][lane];
+    out[transpose ? (c % kH) * kX + c / kH : c] = (float)t;
   }
-  write_partials<kH + 2>(acc, part);
-}
-// out[c] = sum_r part[r][c] (fixed order), into grad at offset (FP32)
-__global__ void reduce_rows_f(const float* __restrict__ part, int rows, int cols, float* __restrict__ out) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cols) return;
-  double s = 0.0;
-  for (int r = 0; r < rows; ++r) s += part[(size_t)r * cols + c];
-  out[c] = (float)s;
-}
-__global__ void reduce_rows_d(const double* __restrict__ part, int rows, int cols, float* __restrict__ out) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cols) return;
-  double s = 0.0;
-  for (int r = 0; r < rows; ++r) s += part[(size_t)r * cols + c];
-  out[c] = (float)s;
-}
-// dW[o][i] = dW^T[i][o]
-__global__ void transpose_into(const float* __restrict__ wt, float* __restrict__ w) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= kH * kX) return;
-  const int o = e / kX, i = e % kX;
-  w[e] = wt[(size_t)i * kH + o];
 }
 
 // Adam (bias-corrected), then the BF16 weight copies
@@ -727,7 +761,7 @@ struct MpnnImpl {
   cudaStream_t st = nullptr;
   Dev<float> params, grads, m1, m2;
   Dev<__nv_bfloat16> wbf;              // 3 x [64][128]
-  Dev<float> s, out, sigma, dh, dself, dm, wpart, bpart, wtmp;
+  Dev<float> s, out, sigma, dh, dself, dm, wpart, bpart;
   Dev<float2> f;
   Dev<__nv_bfloat16> h1, h2, h3;
   Dev<double> dpart, segd;
@@ -751,7 +785,7 @@ struct MpnnImpl {
     dpart.alloc((size_t)kMaxBlocks * (3 * mp::kH));
     err.alloc(1);
     NDS_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), st));
-    fwd_grid = 4 * sm_count();
+    fwd_grid = 2 * sm_count();
     bwd_grid = 2 * sm_count();
     if (train) {
       grads.alloc(mp::kNParam);
@@ -765,7 +799,6 @@ struct MpnnImpl {
       dm.alloc(n * mp::kH);
       wpart.alloc((size_t)bwd_grid * mp::kX * mp::kH);
       bpart.alloc((size_t)bwd_grid * mp::kH);
-      wtmp.alloc((size_t)mp::kX * mp::kH);
     }
     NDS_CUDA(cudaFuncSetAttribute(mp::layer_fwd<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, mp::kFwdSmem));
     NDS_CUDA(cudaFuncSetAttribute(mp::layer_fwd<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, mp::kFwdSmem));
@@ -843,19 +876,19 @@ struct MpnnImpl {
     const int grid = std::max(1, std::min(fwd_grid, tiles(g.n)));
     mp::FwdArgs a1 = fwd_args(g, 1, nseg);
     a1.hout = h1.p;
-    mp::layer_fwd<true, false><<<grid, mp::kTile, mp::kFwdSmem, st>>>(a1);
+    mp::layer_fwd<true, false><<<grid, mp::kThreads, mp::kFwdSmem, st>>>(a1);
     NDS_LAUNCH();
     mp::FwdArgs a2 = fwd_args(g, 2, nseg);
     a2.in.hin = h1.p;
     a2.hout = h2.p;
-    mp::layer_fwd<false, false><<<grid, mp::kTile, mp::kFwdSmem, st>>>(a2);
+    mp::layer_fwd<false, false><<<grid, mp::kThreads, mp::kFwdSmem, st>>>(a2);
     NDS_LAUNCH();
     mp::FwdArgs a3 = fwd_args(g, 3, nseg);
     a3.in.hin = h2.p;
     a3.hout = training ? h3.p : nullptr;
     a3.out = out.p;
     a3.z = z;
-    mp::layer_fwd<false, true><<<grid, mp::kTile, mp::kFwdSmem, st>>>(a3);
+    mp::layer_fwd<false, true><<<grid, mp::kThreads, mp::kFwdSmem, st>>>(a3);
     NDS_LAUNCH();
   }
   // forward, loss, backward: gradients in grads; returns the mean segment loss
@@ -902,7 +935,7 @@ struct MpnnImpl {
   }
   // decoder partials in dpart and dh3 in dh -> every parameter gradient
   void layers_backward(const nds_mpnn_graph& g, int rg) {
-    mp::reduce_rows_d<<<1, 128, 0, st>>>(dpart.p, rg, mp::kH + 2, grads.p + mp::OFF_WD);
+    mp::reduce_rows<double><<<(mp::kH + 2 + 31) / 32, kBlock, 0, st>>>(dpart.p, rg, mp::kH + 2, grads.p + mp::OFF_WD, 0);
     NDS_LAUNCH();
     const int bgrid = std::max(1, std::min(bwd_grid, tiles(g.n)));
     const __nv_bfloat16* hs[4] = {nullptr, h1.p, h2.p, h3.p};
@@ -919,14 +952,13 @@ struct MpnnImpl {
       b.wpart = wpart.p;
       b.bpart = bpart.p;
       b.err = err.p;
-      if (l == 1) mp::layer_bwd<true><<<bgrid, mp::kTile, mp::kBwdSmem, st>>>(b);
-      else mp::layer_bwd<false><<<bgrid, mp::kTile, mp::kBwdSmem, st>>>(b);
+      if (l == 1) mp::layer_bwd<true><<<bgrid, mp::kThreads, mp::kBwdSmem, st>>>(b);
+      else mp::layer_bwd<false><<<bgrid, mp::kThreads, mp::kBwdSmem, st>>>(b);
       NDS_LAUNCH();
-      mp::reduce_rows_f<<<grid_for(mp::kX * mp::kH), kBlock, 0, st>>>(wpart.p, bgrid, mp::kX * mp::kH, wtmp.p);
+      mp::reduce_rows<float><<<mp::kX * mp::kH / 32, kBlock, 0, st>>>(wpart.p, bgrid, mp::kX * mp::kH,
+                                                                      grads.p + mp::off_w(l), 1);
       NDS_LAUNCH();
-      mp::transpose_into<<<grid_for(mp::kX * mp::kH), kBlock, 0, st>>>(wtmp.p, grads.p + mp::off_w(l));
-      NDS_LAUNCH();
-      mp::reduce_rows_f<<<1, mp::kH, 0, st>>>(bpart.p, bgrid, mp::kH, grads.p + mp::off_b(l));
+      mp::reduce_rows<float><<<mp::kH / 32, kBlock, 0, st>>>(bpart.p, bgrid, mp::kH, grads.p + mp::off_b(l), 0);
       NDS_LAUNCH();
       // gradient into h^{l-1} (h0 for l = 1)
       mp::scatter_bwd<<<grid_for((long long)g.n * 16), kBlock, 0, st>>>(g.n, g.nbr, g.ew, dself.p, dm.p, dh.p);
@@ -934,12 +966,9 @@ struct MpnnImpl {
     }
     mp::encoder_bwd<<<rg, kBlock, 0, st>>>(g.n, f.p, dh.p, params.p, dpart.p);
     NDS_LAUNCH();
-    {
-      // partial rows: [dWe (2 per unit, unit-major) ; dbe]
-      mp::reduce_rows_d<<<1, 3 * mp::kH, 0, st>>>(dpart.p, rg, 3 * mp::kH, wtmp.p);
-      NDS_LAUNCH();
-      NDS_CUDA(cudaMemcpyAsync(grads.p + mp::OFF_WE, wtmp.p, sizeof(float) * 3 * mp::kH, cudaMemcpyDeviceToDevice, st));
-    }
+    // partial rows: [dWe (2 per unit, unit-major) ; dbe], as in the parameter vector
+    mp::reduce_rows<double><<<3 * mp::kH / 32, kBlock, 0, st>>>(dpart.p, rg, 3 * mp::kH, grads.p + mp::OFF_WE, 0);
+    NDS_LAUNCH();
     check_err();
   }
   void adam_step(float lr, float b1, float b2, float eps, int step) {

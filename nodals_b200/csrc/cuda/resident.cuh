@@ -1,22 +1,27 @@
-// PCG with its V-cycle as one kernel, for meshes that leave the chip idle.
+// PCG with its V-cycle as one kernel of one cluster, for small meshes.
 //
-// A PCG iteration of the split operator with a dense coarse level is fifteen
-// kernels of one to three microseconds of work each; below about a hundred
-// thousand cells their launches and their cold first loads are most of the
-// time.  Here one block per SM (or one cluster of eight blocks on the
-// smallest meshes) stays resident for the whole solve: the steps are
-// separated by barriers, the operator's constant data stays in the L1 caches
-// (a cell is always visited by the same thread), and only the vectors that
-// other blocks read go through L2 (loads that bypass L1).
+// A PCG iteration of the split operator with a dense coarse level is fourteen
+// dependent steps.  On a few thousand cells each has well under a microsecond
+// of work, and as kernels (or as phases of a grid that meets at barriers in
+// global memory) a step costs two to three microseconds of launch, cold loads
+// and round trips to L2.  Here one cluster of eight blocks keeps every vector
+// of the solve in its shared memory: block k owns the cells, free vertices
+// and coarse rows of the k-th eighth, neighbours are read through distributed
+// shared memory, and the steps are separated by the cluster's hardware
+// barrier.  The barrier's acquire empties L1, so constant data read from
+// global memory costs an L2 round trip in every step: the operators' data is
+// copied to shared memory too, as far as it fits (the V-cycle's first: four
+// of five products).  Bound by the chain of latencies in a step (shared
+// memory, FP64 arithmetic and shuffles, barrier), about 1.5 us each.
+// Microseconds of an iteration, loop of kernels / this: 720 cells FP64 42 /
+// 21, FP32 44 / 22; 2,400 cells FP64 43 / 25, mixed FP16 53 / 37; 4,608 cells
+// FP32 41 / 37.  One block instead of eight was tried: 34 at 720 cells, 93 at
+// 2,400 (FP64); one block per SM meeting at barriers in global memory: 44 at
+// 720 cells, 57 to 65 at 48,000, no better than the kernels.
 //
-// The scalars are formed by every block from the same per-block partial sums
-// in the same order, so all blocks take the same decisions and a run is
-// reproducible.  Barriers between the blocks of a grid wait on a counter for
-// at most kResidentSpins polls; when one runs out the kernel sets flag 32,
-// and every block leaves.  The launch is cooperative (or one cluster), so all
-// blocks run at the same time.
+// Every block forms the scalars from the same eight partial sums in the same
+// order, so all take the same decisions and a run is reproducible.
 #pragma once
-#include <cooperative_groups.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -30,83 +35,141 @@
 namespace nds {
 namespace k {
 
-constexpr int kResidentBlock = 512;
-constexpr int kResidentWarps = kResidentBlock / 32;
-constexpr int kResidentCluster = 8;
-constexpr int kResidentSteps = 16;        // smoother degrees up to 16
-constexpr unsigned kResidentSpins = 1u << 22;  // about a second
-constexpr int kResidentRows = 64;         // rows of the dense level a block takes at a time
-constexpr int kResidentParts = 4;         // warps that share such a row
+constexpr int kResBlock = 512;
+constexpr int kResWarps = kResBlock / 32;
+constexpr int kResCluster = 8;
+constexpr int kResSteps = 16;  // smoother degrees up to 16
+constexpr int kResParts = 4;   // warps that share a row of the dense level
 
 template <class S, class TA>
 struct Resident {
-  int nc;
+  int nc, chunk;             // cells, cells per block
+  unsigned inv_chunk;        // cell / chunk = umulhi(cell, inv_chunk)
+  int vchunk;                // vertices per block
+  unsigned inv_vchunk;
   // operator of the Krylov method (precision S) and of the V-cycle (TA)
   SplitVerts vs, va;
   SplitCells cs, ca;
   const S* rvs;
   const TA* rva;
-  S* ws;
-  TA* wa;
   TA wscale, tinv;
   const TA* den;
   int m;                     // smoothing steps after the diagonal one
-  TA w[kResidentSteps];      // weights: diagonal step, then the steps
+  TA w[kResSteps];           // weights: diagonal step, then the steps
   // coarse level: R in CSR, its V-cycle matrix (row stride ld), P in ELL
-  int nk, ld, pw;
+  int nk, kchunk, ld, pw;
   const int32_t* rr;
   const int32_t* rc;
   const TA* rv;
   const TA* dense;
   const int32_t* pc;
   const TA* pv;
-  // vectors
-  S *x, *r, *q, *p0, *p1;
-  TA *z, *rA;                // rA: r in TA (r itself when S = TA)
-  TA *b0, *b1, *g0, *g1, *res, *rhs2;
-  TA *cb, *cx;               // coarse right-hand side (padded to ld) and result
-  double* part;              // 3 x gridDim.x
-  unsigned* bar;             // zero at launch
+  // largest number of vertex incidences of a block, and whether the V-cycle's
+  // and the Krylov method's operator are copied to shared memory (with the
+  // same data, both are when the first is)
+  int zmax, copy_a, copy_s;
+  const S* r;                // in: the residual
+  S* x;                      // out: the solution (from zero)
   double* sc;                // [3] ||r||^2 out
   int r0_slot, target_slot;
   int* flags;
   int* ctl;                  // [0] iterations, [1] converged out; [3] cap in
 };
-
-template <class T>
-__device__ __forceinline__ T ld_l2(const T* p) {
-  return __ldcg(p);
+// floor(2^32 / chunk) + 1: umulhi(i, .) = i / chunk for i chunk < 2^32
+inline unsigned res_inverse(int chunk) { return (unsigned)(0x100000000ull / (unsigned)chunk + 1); }
+// bytes of dynamic shared memory per block
+template <class S, class TA>
+inline size_t res_smem(int chunk, int vchunk, int ld) {
+  const bool same = std::is_same<S, TA>::value;
+  return (size_t)chunk * (5 * sizeof(S) + (same ? 5 : 6) * sizeof(TA)) + 4 * (size_t)vchunk * sizeof(S) +
+         2 * (size_t)ld * sizeof(TA) + 16 * 16;
+}
+// bytes of an operator's copy (V: arithmetic type; MT: its data)
+template <class V, class MT>
+inline size_t res_copy_bytes(int chunk, int vchunk, int zmax, bool d16, bool rec8) {
+  const bool half = std::is_same<MT, __half>::value;
+  const size_t cell = 16 + (d16 ? 8 : 16) + (half ? 32 : 13 * sizeof(V)) + sizeof(V);  // with den
+  const size_t inc = std::is_same<V, double>::value ? 28 : rec8 ? 8 : 16;
+  return (size_t)chunk * cell + (size_t)zmax * inc + (size_t)(vchunk + 1) * (4 + 4 + sizeof(V)) + 16 * 16;
 }
 
-// a barrier of all blocks; false when it ran out
-template <bool CLUSTER>
-__device__ __forceinline__ bool resident_sync(unsigned* bar, unsigned& seq, int* flags) {
-  if constexpr (CLUSTER) {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    return true;
-  } else {
-    __shared__ int ok;
-    ++seq;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      const unsigned goal = seq * gridDim.x;
-      unsigned now;
-      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
-      unsigned n = 0;
-      do {
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(bar) : "memory");
-      } while ((int)(now - goal) < 0 && ++n < kResidentSpins);
-      ok = (int)(now - goal) >= 0;
-      if (!ok) atomicOr(flags, 32);
-    }
-    __syncthreads();
-    return ok != 0;
+__device__ __forceinline__ uint32_t dsm_addr(const void* p, unsigned cta) {
+  uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(p)), o;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(o) : "r"(a), "r"(cta));
+  return o;
+}
+__device__ __forceinline__ void dsm_load(uint32_t a, float& v) {
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void dsm_load(uint32_t a, double& v) {
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void dsm_load3(uint32_t a, float (&v)[3]) {
+  float pad;
+  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(pad)
+               : "r"(a)
+               : "memory");
+}
+__device__ __forceinline__ void dsm_load3(uint32_t a, double (&v)[3]) {
+  asm volatile("ld.shared::cluster.v2.f64 {%0,%1}, [%2];" : "=d"(v[0]), "=d"(v[1]) : "r"(a) : "memory");
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v[2]) : "r"(a + 16) : "memory");
+}
+__device__ __forceinline__ void dsm_store(uint32_t a, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+__device__ __forceinline__ void dsm_store(uint32_t a, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// a distributed vector (its part in every block at the same place)
+template <class V>
+struct DsmVector {
+  const V* x;
+  int chunk;
+  unsigned inv;
+  __device__ __forceinline__ V operator()(int c) const {
+    const unsigned k = __umulhi((unsigned)c, inv);
+    V v;
+    dsm_load(dsm_addr(x + (c - (int)k * chunk), k), v);
+    return v;
   }
-}
+};
+// the search direction p = z + beta p_old (p = z at the first iteration),
+// formed where it is read
+template <class S, class TA>
+struct DsmDirection {
+  DsmVector<TA> z;
+  DsmVector<S> old;
+  S beta;
+  bool first;
+  __device__ __forceinline__ S operator()(int c) const {
+    const S zc = S(z(c));
+    return first ? zc : zc + beta * old(c);
+  }
+};
+// the vertex sums (four values a vertex)
+template <class V>
+struct DsmVertices {
+  const V* w;
+  int n, chunk;
+  unsigned inv;
+  __device__ __forceinline__ void operator()(int v, V (&o)[3]) const {
+    if (v >= n) {  // fixed
+      o[0] = o[1] = o[2] = V(0);
+      return;
+    }
+    const unsigned k = __umulhi((unsigned)v, inv);
+    dsm_load3(dsm_addr(w + 4 * (v - (int)k * chunk), k), o);
+  }
+};
 
-// products of one vertex's incidences with x (read through L2), group of
-// eight lanes; the sums are valid in every lane
+// products of one vertex's incidences with x, by a group of eight lanes; the
+// sums are valid in every lane
 template <class V, class X>
 __device__ __forceinline__ void resident_vertex(const SplitVerts& a, int g, int lane, unsigned mask, const X& x,
                                                 V (&s)[3]) {
@@ -156,131 +219,214 @@ __device__ __forceinline__ void resident_vertex(const SplitVerts& a, int g, int 
   s[2] = group_sum<8>(s2, mask);
 }
 
-template <class V>
-struct L2Vector {
-  const V* x;
-  __device__ __forceinline__ V operator()(int c) const { return ld_l2(x + c); }
-};
-// the search direction p = z + beta p_old, formed where it is read (p = z at
-// the first iteration): two gathers, but one step between barriers less
-template <class S, class TA>
-struct L2Direction {
-  const TA* z;
-  const S* old;
-  S beta;
-  bool first;
-  __device__ __forceinline__ S operator()(int c) const {
-    const S zc = S(ld_l2(z + c));
-    return first ? zc : zc + beta * ld_l2(old + c);
-  }
-};
-
-template <class S, class TA, class MT, bool CLUSTER>
-__global__ void __launch_bounds__(kResidentBlock, 1) pcg_resident(const Resident<S, TA> a) {
+template <class S, class TA, class MT>
+__global__ void __launch_bounds__(kResBlock, 1) __cluster_dims__(kResCluster, 1, 1)
+    pcg_resident(const Resident<S, TA> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  TA* sv = reinterpret_cast<TA*>(smem_raw);  // a coarse vector (ld values)
-  __shared__ TA srow[kResidentRows][kResidentParts];
-  __shared__ double sred[kResidentWarps];
-  __shared__ double stot;
-  const int tid = threadIdx.x, nt = gridDim.x * kResidentBlock, gt = blockIdx.x * kResidentBlock + tid;
-  const int lane = tid & 31, warp = tid >> 5;
-  unsigned seq = 0;
-  bool alive = true;
+  __shared__ TA srow[kResWarps];
+  __shared__ double sred[kResWarps];
+  __shared__ double spart[3][kResCluster];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned me = blockIdx.x;  // one cluster: the block's rank
+  const int n = a.chunk, lo = (int)me * n, cnt = max(0, min(n, a.nc - lo));
+  const int vlo = (int)me * a.vchunk, vcnt = max(0, min(a.vchunk, a.vs.n - vlo));
+  const int klo = (int)me * a.kchunk, kcnt = max(0, min(a.kchunk, a.nk - klo));
+  // shared arrays, 16-byte aligned, at the same place in every block
+  unsigned char* top = smem_raw;
+  auto take = [&](auto tag, size_t len) {
+    using V = decltype(tag);
+    V* p = reinterpret_cast<V*>(top);
+    top += (len * sizeof(V) + 15) / 16 * 16;
+    return p;
+  };
+  S* const w = take(S{}, 4 * (size_t)a.vchunk);
+  TA* const wa = reinterpret_cast<TA*>(w);
+  TA* const cb = take(TA{}, (size_t)a.ld);
+  TA* const cx = take(TA{}, (size_t)a.ld);
+  S* const x = take(S{}, (size_t)n);
+  S* const r = take(S{}, (size_t)n);
+  S* const q = take(S{}, (size_t)n);
+  S* const p0 = take(S{}, (size_t)n);
+  S* const p1 = take(S{}, (size_t)n);
+  TA* const z = take(TA{}, (size_t)n);
+  TA* const v0 = take(TA{}, (size_t)n);
+  TA* const v1 = take(TA{}, (size_t)n);
+  TA* const res = take(TA{}, (size_t)n);
+  TA* const ex = take(TA{}, (size_t)n);
+  TA* rA;
+  if constexpr (std::is_same<S, TA>::value) rA = r;
+  else rA = take(TA{}, (size_t)n);
 
-  auto sync = [&] { alive = alive && resident_sync<CLUSTER>(a.bar, seq, a.flags); };
-  // sum over all threads of all blocks, the same value everywhere; also a barrier
+  // the operators, from shared memory where copied (their pointers shifted so
+  // that global indices address the block's part)
+  SplitCells ca = a.ca, cs = a.cs;
+  SplitVerts va = a.va, vs = a.vs;
+  const TA* rva = a.rva;
+  const S* rvs = a.rvs;
+  const TA* den = a.den + lo;
+  auto fetch = [&](auto*& src, ptrdiff_t from, ptrdiff_t len, size_t room) {
+    using V = std::remove_const_t<std::remove_pointer_t<std::remove_reference_t<decltype(src)>>>;
+    V* d = take(V{}, room);
+    for (ptrdiff_t k = tid; k < len; k += kResBlock) d[k] = src[from + k];
+    src = d - from;
+  };
+  auto copy_op = [&](auto tag, auto mt, SplitCells& cc, SplitVerts& vv, auto*& rau) {
+    using V = decltype(tag);
+    using M = decltype(mt);
+    const int zlo = vcnt > 0 ? vv.off[vlo] : 0, zn = vcnt > 0 ? vv.off[vlo + vcnt] - zlo : 0;
+    fetch(cc.vid, lo, cnt, n);
+    if (cc.nd16) fetch(cc.nd16, lo, cnt, n);
+    else fetch(cc.nid, lo, cnt, n);
+    auto part = [&](const void*& p, auto t, ptrdiff_t per) {
+      using U = decltype(t);
+      const U* q = static_cast<const U*>(p);
+      fetch(q, per * lo, per * cnt, (size_t)per * n);
+      p = q;
+    };
+    if constexpr (std::is_same<M, __half>::value) {
+      part(cc.g0, uint4{}, 1);
+      part(cc.g1, uint2{}, 1);
+      part(cc.tau, uint2{}, 1);
+    } else if constexpr (std::is_same<V, float>::value) {
+      part(cc.g0, float4{}, 1);
+      part(cc.g1, float4{}, 1);
+      part(cc.g2, float{}, 1);
+      part(cc.tau, float4{}, 1);
+    } else {
+      double2* d = take(double2{}, 4 * (size_t)n);
+      const double2* g = static_cast<const double2*>(cc.g0);
+      for (int k = tid; k < 4 * cnt; k += kResBlock) {
+        const int q4 = k / cnt, l = k - q4 * cnt;
+        d[q4 * n + l] = g[(size_t)q4 * cc.n + lo + l];
+      }
+      cc.g0 = d - lo;
+      cc.n = n;  // stride of the four parts
+      part(cc.g2, double{}, 1);
+      part(cc.tau, double2{}, 2);
+    }
+    if constexpr (std::is_same<V, double>::value) {
+      fetch(vv.bx, zlo, zn, a.zmax);
+      fetch(vv.by, zlo, zn, a.zmax);
+      fetch(vv.bz, zlo, zn, a.zmax);
+      fetch(vv.cell, zlo, zn, a.zmax);
+    } else if (vv.rec8) {
+      fetch(vv.rec8, zlo, zn, a.zmax);
+      fetch(vv.base, vlo, vcnt, a.vchunk);
+    } else {
+      fetch(vv.rec16, zlo, zn, a.zmax);
+    }
+    fetch(vv.off, vlo, vcnt > 0 ? vcnt + 1 : 0, a.vchunk + 1);
+    fetch(rau, vlo, vcnt, a.vchunk);
+  };
+  if (a.copy_a) {
+    copy_op(TA{}, MT{}, ca, va, rva);
+    const TA* d = a.den;
+    fetch(d, lo, cnt, n);
+    den = d + lo;
+    if constexpr (std::is_same<S, TA>::value && std::is_same<MT, TA>::value) {
+      cs = ca;
+      vs = va;
+      rvs = rva;
+    }
+  }
+  if constexpr (!(std::is_same<S, TA>::value && std::is_same<MT, TA>::value)) {
+    if (a.copy_s) copy_op(S{}, S{}, cs, vs, rvs);
+  }
+  __syncthreads();
+
+  auto vec = [&](const auto* y) {
+    using V = std::remove_const_t<std::remove_pointer_t<decltype(y)>>;
+    return DsmVector<V>{y, n, a.inv_chunk};
+  };
+  const unsigned mask8 = group8_mask();
+  auto vertices = [&](auto* ww, const SplitVerts& v, const auto* rau, const auto& xx, auto scale) {
+    using V = std::remove_pointer_t<decltype(ww)>;
+    for (int l = tid >> 3; l < vcnt; l += kResBlock / 8) {
+      V s[3];
+      const V rr = scale * rau[vlo + l];
+      resident_vertex<V>(v, vlo + l, tid & 7, mask8, xx, s);
+      if ((tid & 7) == 0) {
+        ww[4 * l] = rr * s[0];
+        ww[4 * l + 1] = rr * s[1];
+        ww[4 * l + 2] = rr * s[2];
+      }
+    }
+  };
+  auto vert_a = [&](const TA* y) { vertices(wa, va, rva, vec(y), a.wscale); };
+  const DsmVertices<TA> wva{wa, a.va.n, a.vchunk, a.inv_vchunk};
+  const DsmVertices<S> wvs{w, a.vs.n, a.vchunk, a.inv_vchunk};
+  auto row_a = [&](const TA* y, int l, TA yc) {
+    return ca.nd16 ? split_row<TA, MT, true>(ca, vec(y), wva, lo + l, yc, a.tinv)
+                     : split_row<TA, MT, false>(ca, vec(y), wva, lo + l, yc, a.tinv);
+  };
+  // sum over all threads of the cluster, the same value everywhere; a barrier
   auto reduce = [&](double v, int slot) {
     v = warp_sum(v);
     if (lane == 0) sred[warp] = v;
     __syncthreads();
-    if (tid == 0) {
-      double s = 0;
-      for (int q = 0; q < kResidentWarps; ++q) s += sred[q];
-      a.part[slot * gridDim.x + blockIdx.x] = s;
-      __threadfence();
-    }
-    sync();
     if (warp == 0) {
-      double s = 0;
-      for (int b = lane; b < (int)gridDim.x; b += 32) s += ld_l2(a.part + slot * gridDim.x + b);
+      double s = lane < kResWarps ? sred[lane] : 0.0;
       s = warp_sum(s);
-      if (lane == 0) stot = s;
+      if (lane < kResCluster) dsm_store(dsm_addr(&spart[slot][me], (unsigned)lane), s);
     }
-    __syncthreads();
-    return stot;
+    cluster_sync();
+    double s = 0;
+#pragma unroll
+    for (int k = 0; k < kResCluster; ++k) s += spart[slot][k];
+    return s;
   };
-  const unsigned mask8 = group8_mask();
-  auto vertices = [&](auto tag, const SplitVerts& v, const auto* rau, const auto& x, auto* w, auto scale) {
-    using V = decltype(tag);
-    for (int g = gt >> 3; g < v.n; g += nt >> 3) {
-      V s[3];
-      const V r = scale * rau[g];
-      resident_vertex<V>(v, g, tid & 7, mask8, x, s);
-      if ((tid & 7) == 0) {
-        if constexpr (std::is_same<V, float>::value) {
-          reinterpret_cast<float4*>(w)[g] = make_float4(r * s[0], r * s[1], r * s[2], 0.f);
-        } else {
-          reinterpret_cast<double2*>(w)[2 * (size_t)g] = make_double2(r * s[0], r * s[1]);
-          w[4 * (size_t)g + 2] = r * s[2];
-        }
-      }
-    }
-  };
-  auto row_a = [&](const TA* x, int c, TA xc) {
-    return a.ca.nd16 ? split_row<TA, MT, true, true>(a.ca, L2Vector<TA>{x}, a.wa, c, xc, a.tinv)
-                     : split_row<TA, MT, false, true>(a.ca, L2Vector<TA>{x}, a.wa, c, xc, a.tinv);
-  };
-  auto vert_a = [&](const TA* x) { vertices(TA{}, a.va, a.rva, L2Vector<TA>{x}, a.wa, a.wscale); };
-
   // r in the V-cycle's precision and the first smoothing step
-  auto first_step = [&](int c, S r) {
-    TA ra;
-    if constexpr (std::is_same<S, TA>::value) {
-      ra = r;
-    } else {
-      ra = TA(r);
-      a.rA[c] = ra;
-    }
-    a.b0[c] = a.w[0] * ra / a.den[c];
+  auto first_step = [&](int l, S rr) {
+    const TA ra = TA(rr);
+    if constexpr (!std::is_same<S, TA>::value) rA[l] = ra;
+    v0[l] = a.w[0] * ra / den[l];
   };
-  for (int c = gt; c < a.nc; c += nt) first_step(c, a.r[c]);
+
+  for (int l = tid; l < cnt; l += kResBlock) {
+    const S rr = a.r[lo + l];
+    r[l] = rr;
+    x[l] = S(0);
+    first_step(l, rr);
+  }
+  for (int k = tid; k < a.ld; k += kResBlock) cb[k] = cx[k] = TA(0);
   const double target = a.sc[a.target_slot], r0 = a.sc[a.r0_slot];
   const int cap = a.ctl[3];
   double rho = 0, rn2 = 0;
   int its = 0, flags = 0, conv = 0;
   bool first = true;
-  sync();
+  cluster_sync();
 
-  while (alive) {
+  for (;;) {
     // ---- z = M r
-    TA* cur = a.b0;
-    TA* nxt = a.b1;
+    TA* cur = v0;
+    TA* nxt = v1;
     for (int st = 1; st <= a.m; ++st) {
       vert_a(cur);
-      sync();
-      for (int c = gt; c < a.nc; c += nt) {
-        const TA xc = cur[c];
-        nxt[c] = xc + a.w[st] * (a.rA[c] - row_a(cur, c, xc)) / a.den[c];
+      cluster_sync();
+      for (int l = tid; l < cnt; l += kResBlock) {
+        const TA xc = cur[l];
+        nxt[l] = xc + a.w[st] * (rA[l] - row_a(cur, l, xc)) / den[l];
       }
-      sync();
+      cluster_sync();
       TA* t = cur;
       cur = nxt;
       nxt = t;
     }
     vert_a(cur);
-    sync();
-    for (int c = gt; c < a.nc; c += nt) a.res[c] = a.rA[c] - row_a(cur, c, cur[c]);
-    sync();
-    // restriction: 16 lanes a coarse row
+    cluster_sync();
+    for (int l = tid; l < cnt; l += kResBlock) res[l] = rA[l] - row_a(cur, l, cur[l]);
+    cluster_sync();
+    // restriction, 16 lanes a coarse row; the result goes to every block
     {
       const int l16 = tid & 15;
       const unsigned m16 = group_mask<16>();
-      for (int i = gt >> 4; i < a.nk; i += nt >> 4) {
+      const auto f = vec(res);
+      for (int l = tid >> 4; l < kcnt; l += kResBlock / 16) {
+        const int i = klo + l, re = a.rr[i + 1];
         TA s = 0;
-        const int re = a.rr[i + 1];
         for (int k0 = a.rr[i] + l16; k0 < re; k0 += 128) {
           int j[8];
-          TA v[8], f[8];
+          TA v[8], fv[8];
 #pragma unroll
           for (int u = 0; u < 8; ++u) {
             const int k = k0 + 16 * u;
@@ -288,97 +434,90 @@ __global__ void __launch_bounds__(kResidentBlock, 1) pcg_resident(const Resident
             v[u] = k < re ? a.rv[k] : TA(0);
           }
 #pragma unroll
-          for (int u = 0; u < 8; ++u) f[u] = j[u] >= 0 ? ld_l2(a.res + j[u]) : TA(0);
+          for (int u = 0; u < 8; ++u) fv[u] = j[u] >= 0 ? f(j[u]) : TA(0);
 #pragma unroll
-          for (int u = 0; u < 8; ++u) s += v[u] * f[u];
+          for (int u = 0; u < 8; ++u) s += v[u] * fv[u];
         }
         s = group_sum<16>(s, m16);
-        if (l16 == 0) a.cb[i] = s;
+        if (l16 < kResCluster) dsm_store(dsm_addr(cb + i, (unsigned)l16), s);
       }
     }
-    sync();
-    // dense coarse level: each block takes the rows blockIdx.x + k gridDim.x,
-    // four warps a row (a few dozen rows of 10 to 40 KB per block)
+    cluster_sync();
+    // dense coarse level, four warps a row
     {
       constexpr int W = 16 / sizeof(TA);
       using V4 = typename std::conditional<std::is_same<TA, float>::value, float4, double2>::type;
-      V4* s4 = reinterpret_cast<V4*>(sv);
-      const int nv = a.ld / W;
-      for (int k = tid; k < nv; k += kResidentBlock) s4[k] = ld_l2(reinterpret_cast<const V4*>(a.cb) + k);
-      __syncthreads();
-      const int per = (nv + kResidentParts - 1) / kResidentParts;
-      const int rows = blockIdx.x < (unsigned)a.nk ? (a.nk - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-      for (int base = 0; base < rows; base += kResidentRows) {
-        const int cnt = rows - base < kResidentRows ? rows - base : kResidentRows;
-        for (int t = warp; t < cnt * kResidentParts; t += kResidentWarps) {
-          const int rI = t / kResidentParts, pt = t % kResidentParts;
-          const size_t i = blockIdx.x + (size_t)(base + rI) * gridDim.x;
-          const V4* A4 = reinterpret_cast<const V4*>(a.dense + i * a.ld);
+      const V4* s4 = reinterpret_cast<const V4*>(cb);
+      const int nv = a.ld / W, per = (nv + kResParts - 1) / kResParts;
+      const int pt = warp % kResParts, row0 = warp / kResParts;
+      constexpr int rows = kResWarps / kResParts;  // at a time
+      for (int base = 0; base < kcnt; base += rows) {
+        const int l = base + row0;
+        if (l < kcnt) {
+          const V4* A4 = reinterpret_cast<const V4*>(a.dense + (size_t)(klo + l) * a.ld);
           const int e = min(nv, (pt + 1) * per);
           TA s = 0;
 #pragma unroll 4
           for (int k = pt * per + lane; k < e; k += 32) {
-            const V4 p = __ldcs(A4 + k), q = s4[k];
-            if constexpr (W == 4) s += p.x * q.x + p.y * q.y + p.z * q.z + p.w * q.w;
-            else s += p.x * q.x + p.y * q.y;
+            const V4 p = A4[k], y = s4[k];
+            if constexpr (W == 4) s += p.x * y.x + p.y * y.y + p.z * y.z + p.w * y.w;
+            else s += p.x * y.x + p.y * y.y;
           }
           s = warp_sum(s);
-          if (lane == 0) srow[rI][pt] = s;
+          if (lane == 0) srow[warp] = s;
         }
         __syncthreads();
-        if (tid < cnt) {
-          TA s = srow[tid][0];
+        if (l < kcnt && pt == 0 && lane < kResCluster) {
+          TA s = srow[warp];
 #pragma unroll
-          for (int q = 1; q < kResidentParts; ++q) s += srow[tid][q];
-          a.cx[blockIdx.x + (size_t)(base + tid) * gridDim.x] = s;
+          for (int k = 1; k < kResParts; ++k) s += srow[warp + k];
+          dsm_store(dsm_addr(cx + klo + l, (unsigned)lane), s);
         }
         __syncthreads();
       }
     }
-    sync();
-    // x += P x_c
-    for (int k = tid; k < a.nk; k += kResidentBlock) sv[k] = ld_l2(a.cx + k);
-    __syncthreads();
-    for (int c = gt; c < a.nc; c += nt) {
+    cluster_sync();
+    // cur += P x_c
+    for (int l = tid; l < cnt; l += kResBlock) {
       TA s = 0;
       for (int k = 0; k < a.pw; ++k) {
-        const size_t o = (size_t)k * a.nc + c;
-        s += a.pv[o] * sv[a.pc[o]];
+        const size_t o = (size_t)k * a.nc + lo + l;
+        s += a.pv[o] * cx[a.pc[o]];
       }
-      cur[c] += s;
+      cur[l] += s;
     }
-    sync();
-    // post-smoothing; the last step forms z and r.z
+    cluster_sync();
+    // post-smoothing (res now its right-hand side); the last step forms z and r.z
     vert_a(cur);
-    sync();
+    cluster_sync();
     double acc = 0;
-    TA* g = a.g0;
-    TA* gn = a.g1;
-    for (int c = gt; c < a.nc; c += nt) {
-      const TA xc = cur[c];
-      const TA q = a.rA[c] - row_a(cur, c, xc);
+    TA* g = nxt;
+    TA* gn = ex;
+    for (int l = tid; l < cnt; l += kResBlock) {
+      const TA xc = cur[l];
+      const TA e = rA[l] - row_a(cur, l, xc);
       if (a.m == 0) {
-        const TA zc = xc + a.w[0] * q / a.den[c];
-        a.z[c] = zc;
-        acc += (double)a.r[c] * (double)zc;
+        const TA zc = xc + a.w[0] * e / den[l];
+        z[l] = zc;
+        acc += (double)r[l] * (double)zc;
       } else {
-        a.rhs2[c] = q;
-        g[c] = a.w[0] * q / a.den[c];
+        res[l] = e;
+        g[l] = a.w[0] * e / den[l];
       }
     }
     for (int st = 1; st <= a.m; ++st) {
-      sync();
+      cluster_sync();
       vert_a(g);
-      sync();
-      for (int c = gt; c < a.nc; c += nt) {
-        const TA xc = g[c];
-        const TA val = xc + a.w[st] * (a.rhs2[c] - row_a(g, c, xc)) / a.den[c];
+      cluster_sync();
+      for (int l = tid; l < cnt; l += kResBlock) {
+        const TA xc = g[l];
+        const TA val = xc + a.w[st] * (res[l] - row_a(g, l, xc)) / den[l];
         if (st < a.m) {
-          gn[c] = val;
+          gn[l] = val;
         } else {
-          const TA zc = val + cur[c];
-          a.z[c] = zc;
-          acc += (double)a.r[c] * (double)zc;
+          const TA zc = val + cur[l];
+          z[l] = zc;
+          acc += (double)r[l] * (double)zc;
         }
       }
       TA* t = g;
@@ -389,23 +528,24 @@ __global__ void __launch_bounds__(kResidentBlock, 1) pcg_resident(const Resident
     const double rhon = reduce(acc, 0);
     double beta = 0;
     if (!(rhon > 0.0) || !isfinite(rhon)) flags |= first ? 8 : 2;
-    if (first) rho = rhon;
-    else if (!(flags & 2)) {
+    if (first) {
+      rho = rhon;
+    } else if (!(flags & 2)) {
       beta = rhon / rho;
       rho = rhon;
     }
     // ---- q = A p, p.q
-    const L2Direction<S, TA> dir{a.z, (its & 1) ? a.p1 : a.p0, S(beta), first};
-    S* pn = (its & 1) ? a.p0 : a.p1;
-    vertices(S{}, a.vs, a.rvs, dir, a.ws, S(1));
-    sync();
+    const DsmDirection<S, TA> dir{vec(z), vec((its & 1) ? p1 : p0), S(beta), first};
+    S* const pn = (its & 1) ? p0 : p1;
+    vertices(w, vs, rvs, dir, S(1));
+    cluster_sync();
     acc = 0;
-    for (int c = gt; c < a.nc; c += nt) {
-      const S pc = dir(c);
-      const S s = a.cs.nd16 ? split_row<S, S, true, true>(a.cs, dir, a.ws, c, pc, S(1))
-                            : split_row<S, S, false, true>(a.cs, dir, a.ws, c, pc, S(1));
-      pn[c] = pc;
-      a.q[c] = s;
+    for (int l = tid; l < cnt; l += kResBlock) {
+      const S pc = dir(lo + l);
+      const S s = cs.nd16 ? split_row<S, S, true>(cs, dir, wvs, lo + l, pc, S(1))
+                            : split_row<S, S, false>(cs, dir, wvs, lo + l, pc, S(1));
+      pn[l] = pc;
+      q[l] = s;
       acc += (double)pc * (double)s;
     }
     const double pq = reduce(acc, 1);
@@ -415,11 +555,11 @@ __global__ void __launch_bounds__(kResidentBlock, 1) pcg_resident(const Resident
     // ---- x, r, ||r||^2, the next first step
     const S al = S(alpha);
     acc = 0;
-    for (int c = gt; c < a.nc; c += nt) {
-      a.x[c] += al * pn[c];
-      const S rr = a.r[c] - al * a.q[c];
-      a.r[c] = rr;
-      first_step(c, rr);
+    for (int l = tid; l < cnt; l += kResBlock) {
+      x[l] += al * pn[l];
+      const S rr = r[l] - al * q[l];
+      r[l] = rr;
+      first_step(l, rr);
       acc += (double)rr * (double)rr;
     }
     rn2 = reduce(acc, 2);
@@ -430,13 +570,15 @@ __global__ void __launch_bounds__(kResidentBlock, 1) pcg_resident(const Resident
     conv = rn <= target;
     if (conv || flags != 0 || its >= cap) break;
   }
-  if (gt == 0) {
+  for (int l = tid; l < cnt; l += kResBlock) a.x[lo + l] = x[l];
+  if (me == 0 && tid == 0) {
     a.sc[3] = rn2;
     a.ctl[0] = its;
     a.ctl[1] = conv;
     a.ctl[2] = 0;
-    if (flags) atomicOr(a.flags, flags);
+    *a.flags = flags;
   }
+  cluster_sync();  // no block leaves while another may still read its memory
 }
 
 }  // namespace k

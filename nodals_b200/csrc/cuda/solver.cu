@@ -29,6 +29,7 @@
 #include "kernels.cuh"
 #include "krylov.cuh"
 #include "mpnn.hpp"
+#include "resident.cuh"
 #include "split.cuh"
 
 namespace nds {
@@ -90,10 +91,10 @@ struct DBuf {
 // fine_spmv_amg: the fine-level operator inside the V-cycle
 // fine_spmv_half: the V-cycle's fine-level operator in FP16 (amg_half)
 enum ProfCat { P_FINE_SPMV = 0, P_COARSE_SPMV, P_REFRESH, P_ASSEMBLE, P_GS, P_CONTINUITY, P_TRANSFER, P_TERMINAL,
-               P_VECTOR, P_FINE_AMG, P_FINE_HALF, P_NCAT };
+               P_VECTOR, P_FINE_AMG, P_FINE_HALF, P_RESIDENT, P_NCAT };
 static const char* const kProfNames[P_NCAT] = {"fine_spmv", "coarse_spmv", "fine_refresh", "mom_assemble", "mom_gs",
                                                "continuity", "transfer", "terminal_dense", "vector_reduce",
-                                               "fine_spmv_amg", "fine_spmv_half"};
+                                               "fine_spmv_amg", "fine_spmv_half", "pcg_resident"};
 struct Profiler {
   bool on = false;
   std::vector<cudaEvent_t> ev;
@@ -603,6 +604,7 @@ class Solver final : public ISolver {
       for (auto& v : level_lambda_) v = 1.0;
     }
     build_dense_level();
+    plan_resident();
     if (o_.pressure_solver == NDS_P_CHEB) p_cheb_lambda_ = precond_power(o_.p_power_its, o_.p_power_safety);
     NDS_CUDA(cudaStreamSynchronize(st_));
     tm.mark("refresh_and_spectrum");
@@ -1901,6 +1903,126 @@ class Solver final : public ISolver {
     if constexpr (kSame) return {x_.p, r_.p, q_.p, pp_.p, z_.p, nullptr};
     else return {x_.p, r_.p, q_.p, pp_.p, zA_.p, rA_.p};
   }
+  // The whole PCG loop as one kernel of one cluster (resident.cuh): the split
+  // operator with a coarse level applied as a dense matrix, on meshes of up to
+  // kResidentCells cells whose vectors fit the cluster's shared memory: half
+  // the time of the loop of kernels on 720 to 2,400 cells, a tenth less (FP32
+  // and mixed) or the same (FP64) on 4,608, slower from about 6,000 on, where
+  // eight SMs no longer keep up.  NDS_RESIDENT overrides it (0: none).
+  static constexpr int kResidentCells = 5000;
+  static constexpr size_t kResidentDense = (size_t)4 << 20;
+  // entries of n per block (at least 2: res_inverse)
+  static int res_part(int n) { return std::max(2, (n + k::kResCluster - 1) / k::kResCluster); }
+  void plan_resident() {
+    resident_ = false;
+    const bool dense0 = dense_level_ == 0 || L_.size() == 1;
+    if (!split_ || !use_graphs_ || !dense0 || o_.learned || (mixed_ && fg_m_ > 0)) return;
+    if (o_.pressure_solver != NDS_P_PCG || fine_plan().m >= k::kResSteps) return;
+    int cells = kResidentCells;
+    if (const char* e = std::getenv("NDS_RESIDENT")) cells = std::atoi(e);
+    const size_t ld = dense_ld(L_[0].n);
+    if (nc_ > cells || ld * (size_t)L_[0].n * sizeof(TA) > kResidentDense) return;
+    const int chunk = res_part(nc_), vchunk = res_part(svert_.n);
+    res_smem_ = mixed_ ? k::res_smem<float, TA>(chunk, vchunk, (int)ld) : k::res_smem<T, TA>(chunk, vchunk, (int)ld);
+    int most = 0;
+    NDS_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, o_.device));
+    most -= 2048;  // the kernel's static arrays
+    if ((long long)res_smem_ > (long long)most) return;
+    // the operators' copies, as far as they fit
+    res_zmax_ = 0;
+    for (int v = 0; v < svert_.n; v += vchunk)
+      res_zmax_ = std::max(res_zmax_, P_.setup.fine.inc_off[(size_t)std::min(v + vchunk, svert_.n)] -
+                                          P_.setup.fine.inc_off[(size_t)v]);
+    const bool d16 = scell_.nd16 != nullptr;
+    const size_t ca = mixed_ && o_.amg_half ? k::res_copy_bytes<TA, __half>(chunk, vchunk, res_zmax_, d16, sp_rec8_.p)
+                                            : k::res_copy_bytes<TA, TA>(chunk, vchunk, res_zmax_, d16, false);
+    const size_t cs = mixed_ ? k::res_copy_bytes<float, float>(chunk, vchunk, res_zmax_, d16, false)
+                             : k::res_copy_bytes<T, T>(chunk, vchunk, res_zmax_, d16, false);
+    const bool shared = (kSame || mixed_) && !(mixed_ && o_.amg_half);  // one operator for both
+    res_copy_a_ = res_smem_ + ca <= (size_t)most;
+    if (res_copy_a_) res_smem_ += ca;
+    res_copy_s_ = !shared && res_copy_a_ && res_smem_ + cs <= (size_t)most;
+    if (res_copy_s_) res_smem_ += cs;
+    // one limit for every solver of the process: the attribute is the kernel's
+    auto allow = [&](auto* kernel) {
+      NDS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    };
+    if constexpr (kSame) {
+      allow(k::pcg_resident<T, TA, TA>);
+    } else if (mixed_) {
+      if (o_.amg_half) allow(k::pcg_resident<float, float, __half>);
+      else allow(k::pcg_resident<float, float, float>);
+    } else {
+      allow(k::pcg_resident<T, TA, TA>);
+    }
+    resident_ = true;
+  }
+  template <class S>
+  void pcg_on_chip(const PcgVecs<S>& v, const OpView<S>& A) {
+    k::Resident<S, TA> a{};
+    const OpView<TA> V = fine_opV();
+    a.nc = nc_;
+    a.chunk = res_part(nc_);
+    a.inv_chunk = k::res_inverse(a.chunk);
+    a.vchunk = res_part(svert_.n);
+    a.inv_vchunk = k::res_inverse(a.vchunk);
+    a.vs = A.sv;
+    a.cs = A.sc;
+    a.rvs = A.rv;
+    a.va = V.sv;
+    a.ca = V.sc;
+    a.rva = V.rv;
+    a.wscale = TA(V.wscale);
+    a.tinv = TA(V.tinv);
+    const PolyPlan pl = fine_plan();
+    const bool cheb = o_.amg_smoother == NDS_SM_CHEB2;
+    const double lo = cheb ? o_.amg_lambda_low_fraction * fine_lambda_ : 0.0;
+    a.den = pl.den0;
+    a.m = pl.m;
+    a.w[0] = TA(pl.w0);
+    for (int q = 1; q <= pl.m; ++q)
+      a.w[q] = TA(cheb ? 1.0 / cheb_root(fine_lambda_, lo, q, o_.amg_cheb_degree) : o_.amg_jacobi_omega);
+    const Xfer& X = X_[0];
+    a.nk = L_[0].n;
+    a.kchunk = (a.nk + k::kResCluster - 1) / k::kResCluster;
+    a.ld = (int)dense_ld(a.nk);
+    a.dense = dense_level_ == 0 ? dense_.p : tinv_.p;
+    a.rr = X.rrow.p;
+    a.rc = X.rcol.p;
+    a.rv = X.rval.p;
+    a.pw = X.pw;
+    a.pc = X.pcol.p;
+    a.pv = X.pval.p;
+    a.zmax = res_zmax_;
+    a.copy_a = res_copy_a_;
+    a.copy_s = res_copy_s_;
+    a.r = v.r;
+    a.x = v.x;
+    a.sc = sc_.p;
+    a.r0_slot = S_R0;
+    a.target_slot = S_TARGET;
+    a.flags = flags_.p;
+    a.ctl = ctl_.p;
+    static_assert(S_RN2 == 3, "result slot of the kernel");
+    {
+      ProfScope ps(prof, st_, P_RESIDENT);
+      if constexpr (std::is_same<S, float>::value && std::is_same<TA, float>::value && !kSame) {
+        if (V.half) k::pcg_resident<S, TA, __half><<<k::kResCluster, k::kResBlock, res_smem_, st_>>>(a);
+        else k::pcg_resident<S, TA, TA><<<k::kResCluster, k::kResBlock, res_smem_, st_>>>(a);
+      } else {
+        k::pcg_resident<S, TA, TA><<<k::kResCluster, k::kResBlock, res_smem_, st_>>>(a);
+      }
+      NDS_LAUNCH();
+    }
+    read_loop_state();
+  }
+  // control words, flags and ||r||^2 of a loop that ran on the device
+  void read_loop_state() {
+    NDS_CUDA(cudaMemcpyAsync(hflags_ + 4, ctl_.p, 4 * sizeof(int), cudaMemcpyDeviceToHost, st_));
+    NDS_CUDA(cudaMemcpyAsync(hflags_, flags_.p, sizeof(int), cudaMemcpyDeviceToHost, st_));
+    NDS_CUDA(cudaMemcpyAsync(hsc_ + S_RN2, sc_.p + S_RN2, sizeof(double), cudaMemcpyDeviceToHost, st_));
+    NDS_CUDA(cudaStreamSynchronize(st_));
+  }
   // PCG with the iteration loop on the device: two host synchronisations per
   // solve (initial norm, final state) instead of one per iteration.  With
   // graphs off or the profiler on the same body runs launch by launch.
@@ -1908,10 +2030,14 @@ class Solver final : public ISolver {
     const double r0 = p_start(rhs);
     start_readback();
     if (r0 <= o_.p_atol) return {0, 0.0, true};
-    pcg_first(pcg_vecs());
     set_target(std::max(o_.p_atol, o_.p_rtol * r0), r0);
     set_ctl(0, 0, 1, o_.p_max);
-    run_loop(g_loop_, [&](cudaGraphConditionalHandle h) { pcg_body(pcg_vecs(), fine_op(), h); });
+    if (resident_) {
+      pcg_on_chip(pcg_vecs(), fine_op());
+    } else {
+      pcg_first(pcg_vecs());
+      run_loop(g_loop_, [&](cudaGraphConditionalHandle h) { pcg_body(pcg_vecs(), fine_op(), h); });
+    }
     const int f = hflags_[0];
     if (f & 8) throw SolveFailure(NDS_E_BREAKDOWN, "pressure PCG initial rho nonpositive");
     if (f & 1) throw SolveFailure(NDS_E_BREAKDOWN, "pressure PCG pAp nonpositive");
@@ -2217,10 +2343,7 @@ class Solver final : public ISolver {
   void run_loop(LoopGraph& G, Body&& body) {
     if (use_graphs_ && !prof.on && !G.failed && (G.exec || build_loop(G, body))) {
       NDS_CUDA(cudaGraphLaunch(G.exec, st_));
-      NDS_CUDA(cudaMemcpyAsync(hflags_ + 4, ctl_.p, 4 * sizeof(int), cudaMemcpyDeviceToHost, st_));
-      NDS_CUDA(cudaMemcpyAsync(hflags_, flags_.p, sizeof(int), cudaMemcpyDeviceToHost, st_));
-      NDS_CUDA(cudaMemcpyAsync(hsc_ + S_RN2, sc_.p + S_RN2, sizeof(double), cudaMemcpyDeviceToHost, st_));
-      NDS_CUDA(cudaStreamSynchronize(st_));
+      read_loop_state();
       g_launches += (unsigned long long)hflags_[4] * G.body_kernels;
       return;
     }
@@ -2228,10 +2351,7 @@ class Solver final : public ISolver {
     // leaves the decision to this loop, which reads ctl and the flags
     for (;;) {
       body(cudaGraphConditionalHandle{});
-      NDS_CUDA(cudaMemcpyAsync(hflags_ + 4, ctl_.p, 4 * sizeof(int), cudaMemcpyDeviceToHost, st_));
-      NDS_CUDA(cudaMemcpyAsync(hflags_, flags_.p, sizeof(int), cudaMemcpyDeviceToHost, st_));
-      NDS_CUDA(cudaMemcpyAsync(hsc_ + S_RN2, sc_.p + S_RN2, sizeof(double), cudaMemcpyDeviceToHost, st_));
-      NDS_CUDA(cudaStreamSynchronize(st_));
+      read_loop_state();
       prof.collect();
       const int its = hflags_[4], conv = hflags_[5], cap = hflags_[7];
       if (conv || hflags_[0] != 0 || its >= cap) break;
@@ -2256,7 +2376,8 @@ class Solver final : public ISolver {
     set_ctl(0, 0, 1, cap);
     if constexpr (!kSame) {
       const PcgVecs<float> v{xf_.p, rf_.p, qf_.p, pf_.p, zf_.p, nullptr};
-      run_loop(g_loopf_, [&](cudaGraphConditionalHandle h) { pcg_body(v, fine_opA(), h); });
+      if (resident_) pcg_on_chip(v, fine_opA());
+      else run_loop(g_loopf_, [&](cudaGraphConditionalHandle h) { pcg_body(v, fine_opA(), h); });
     }
     const int f = hflags_[0];
     if (f & 8) throw SolveFailure(NDS_E_BREAKDOWN, "inner FP32 PCG initial rho nonpositive");
@@ -2415,7 +2536,7 @@ class Solver final : public ISolver {
         if (fg_m_ > 0) {
           R.its += inner_fgmres(rn, tol, std::min(cap, fg_m_));
         } else {
-          if (pre_fused()) {
+          if (pre_fused() && !resident_) {
             const PolyPlan pl = fine_plan();
             pdl_launch(k::scale_to_float, grid_for(nc_), kBlock, 0, st_, nc_, r_.p, 1.0 / rn, rf_.p, pl.den0,
                        float(pl.w0), fine_first(zf_.p), (float*)nullptr);
@@ -2883,6 +3004,10 @@ class Solver final : public ISolver {
   DBuf<uint8_t> sg_face_;
   DBuf<float> sg_ew_, sg_dscale_, st_z1_, st_t_;
   DBuf<unsigned long long> st_cnt_;
+  bool resident_ = false;  // PCG as one kernel
+  size_t res_smem_ = 0;
+  int res_zmax_ = 0;
+  bool res_copy_a_ = false, res_copy_s_ = false;
   DBuf<double> part_, sc_, tailpart_;
   DBuf<unsigned> ticket_;  // of the reduction tails (stream st_, one launch at a time)
   DBuf<int> flags_;

@@ -151,10 +151,32 @@ struct SplitCells {
   const void* tau = nullptr;
 };
 
-// sum of cell c's row products: vertices from w, faces from x (xc = x[c])
-template <class V, class MT, bool D16>
-__device__ __forceinline__ V split_row(const SplitCells& a, const V* __restrict__ x, const V* __restrict__ w, int c,
-                                       V xc, V tinv) {
+// a vector read as it is
+template <class V>
+struct PlainVector {
+  const V* __restrict__ x;
+  __device__ __forceinline__ V operator()(int c) const { return x[c]; }
+};
+
+// the vertex sums of split_vertex
+template <class V>
+struct PlainVertices {
+  const V* __restrict__ w;
+  __device__ __forceinline__ void operator()(int v, V (&o)[3]) const {
+    if constexpr (std::is_same<V, float>::value) {
+      const float4 u = reinterpret_cast<const float4*>(w)[v];
+      o[0] = u.x; o[1] = u.y; o[2] = u.z;
+    } else {
+      const double2 u = reinterpret_cast<const double2*>(w)[2 * (size_t)v];
+      o[0] = u.x; o[1] = u.y;
+      o[2] = w[4 * (size_t)v + 2];
+    }
+  }
+};
+
+// sum of cell c's row products: vertices from w, faces from x (xc = x(c))
+template <class V, class MT, bool D16, class X, class W>
+__device__ __forceinline__ V split_row(const SplitCells& a, const X& x, const W& w, int c, V xc, V tinv) {
   const int4 vi = a.vid[c];
   int nb[4];
   if (D16) {
@@ -176,21 +198,20 @@ __device__ __forceinline__ V split_row(const SplitCells& a, const V* __restrict_
     const uint2 th = static_cast<const uint2*>(a.tau)[c];
     const uint4 p = static_cast<const uint4*>(a.g0)[c];
     const uint2 q = static_cast<const uint2*>(a.g1)[c];
-    float4 wv[4];
-    const float4* w4 = reinterpret_cast<const float4*>(w);
-    wv[0] = w4[vi.x];
-    wv[1] = w4[vi.y];
-    wv[2] = w4[vi.z];
-    wv[3] = w4[vi.w];
+    V wv[4][3];
+    w(vi.x, wv[0]);
+    w(vi.y, wv[1]);
+    w(vi.z, wv[2]);
+    w(vi.w, wv[3]);
     V xn[4];
 #pragma unroll
-    for (int f = 0; f < 4; ++f) xn[f] = nb[f] >= 0 ? x[nb[f]] : V(0);
+    for (int f = 0; f < 4; ++f) xn[f] = nb[f] >= 0 ? x(nb[f]) : V(0);
     auto h2 = [](unsigned u) { return __half22float2(*reinterpret_cast<const __half2*>(&u)); };
     const float2 b01 = h2(p.x), b23 = h2(p.y), b45 = h2(p.z), b67 = h2(p.w), b89 = h2(q.x), bab = h2(q.y);
-    s = b01.x * wv[0].x + b01.y * wv[0].y + b23.x * wv[0].z;
-    s += b23.y * wv[1].x + b45.x * wv[1].y + b45.y * wv[1].z;
-    s += b67.x * wv[2].x + b67.y * wv[2].y + b89.x * wv[2].z;
-    s += b89.y * wv[3].x + bab.x * wv[3].y + bab.y * wv[3].z;
+    s = b01.x * wv[0][0] + b01.y * wv[0][1] + b23.x * wv[0][2];
+    s += b23.y * wv[1][0] + b45.x * wv[1][1] + b45.y * wv[1][2];
+    s += b67.x * wv[2][0] + b67.y * wv[2][1] + b89.x * wv[2][2];
+    s += b89.y * wv[3][0] + bab.x * wv[3][1] + bab.y * wv[3][2];
     const float2 t01 = h2(th.x), t23 = h2(th.y);
     t[0] = t01.x;
     t[1] = t01.y;
@@ -209,16 +230,9 @@ __device__ __forceinline__ V split_row(const SplitCells& a, const V* __restrict_
       b[8] = static_cast<const float*>(a.g2)[c];
       const float4 tt = static_cast<const float4*>(a.tau)[c];
       t[0] = tt.x; t[1] = tt.y; t[2] = tt.z; t[3] = tt.w;
-      const float4* w4 = reinterpret_cast<const float4*>(w);
-      const int vv[4] = {vi.x, vi.y, vi.z, vi.w};
-#pragma unroll
-      for (int q4 = 0; q4 < 4; ++q4) {
-        const float4 u = w4[vv[q4]];
-        wv[q4][0] = u.x; wv[q4][1] = u.y; wv[q4][2] = u.z;
-      }
     } else {
       const double2* g = static_cast<const double2*>(a.g0);
-      const size_t n = (size_t)a.n;
+      const ptrdiff_t n = a.n;
 #pragma unroll
       for (int q4 = 0; q4 < 4; ++q4) {
         const double2 p = g[q4 * n + c];
@@ -226,21 +240,17 @@ __device__ __forceinline__ V split_row(const SplitCells& a, const V* __restrict_
         b[2 * q4 + 1] = p.y;
       }
       b[8] = static_cast<const double*>(a.g2)[c];
-      const double2* tp = static_cast<const double2*>(a.tau) + 2 * (size_t)c;
+      const double2* tp = static_cast<const double2*>(a.tau) + 2 * (ptrdiff_t)c;
       const double2 ta = tp[0], tb = tp[1];
       t[0] = ta.x; t[1] = ta.y; t[2] = tb.x; t[3] = tb.y;
-      const double2* w2 = reinterpret_cast<const double2*>(w);
-      const int vv[4] = {vi.x, vi.y, vi.z, vi.w};
-#pragma unroll
-      for (int q4 = 0; q4 < 4; ++q4) {
-        const double2 u = w2[2 * (size_t)vv[q4]];
-        wv[q4][0] = u.x; wv[q4][1] = u.y;
-        wv[q4][2] = w[4 * (size_t)vv[q4] + 2];
-      }
     }
+    w(vi.x, wv[0]);
+    w(vi.y, wv[1]);
+    w(vi.z, wv[2]);
+    w(vi.w, wv[3]);
     V xn[4];
 #pragma unroll
-    for (int f = 0; f < 4; ++f) xn[f] = nb[f] >= 0 ? x[nb[f]] : V(0);
+    for (int f = 0; f < 4; ++f) xn[f] = nb[f] >= 0 ? x(nb[f]) : V(0);
 #pragma unroll
     for (int j = 0; j < 3; ++j)
 #pragma unroll
@@ -273,7 +283,7 @@ __global__ void __launch_bounds__(kBlock) split_cell(SplitCells a, const V* __re
       bc = b[c];
       if (MODE == SELL_SMOOTH || den) dc = den[c];
     }
-    const V s = split_row<V, MT, D16>(a, x, w, c, xc, tinv);
+    const V s = split_row<V, MT, D16>(a, PlainVector<V>{x}, PlainVertices<V>{w}, c, xc, tinv);
     if (MODE == SELL_Y) {
       y[c] = s;
       if (y2) y2[(size_t)at[0] * a.n + c] = xc;
@@ -305,7 +315,7 @@ __global__ void __launch_bounds__(kBlock) split_cell_dot(SplitCells a, const V* 
   double acc = 0.0;
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < a.n; c += gridDim.x * blockDim.x) {
     const V pc = p[c];
-    const V s = split_row<V, V, D16>(a, p, w, c, pc, tinv);
+    const V s = split_row<V, V, D16>(a, PlainVector<V>{p}, PlainVertices<V>{w}, c, pc, tinv);
     q[c] = s;
     acc += (double)pc * (double)s;
   }

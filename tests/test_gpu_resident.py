@@ -1,0 +1,55 @@
+"""PCG as one kernel of one cluster against the loop of kernels
+(NDS_RESIDENT=0) on small meshes: the same method in another order of sums.
+FP64: equal iteration counts, iterates to 1e-9 relative (rounding amplified by
+the solves); FP32 state as the FP32 path against FP64; mixed and FP32 V-cycle:
+every solve meets its own target p_rtol = 1e-6, as do the fields.  Sizes: not
+multiples of the cluster's eight parts, fewer coarse rows than blocks, several
+cells per thread; the smoother's degrees 1 (Jacobi), 2, 3 and 4.
+"""
+from __future__ import annotations
+
+import pytest
+
+from conftest import rel_l2
+
+CFG = dict(re=20.0, alpha_u=0.7, alpha_p=0.3, p_rtol=1e-6, p_max=400, amg_terminal=60, max_outer=10,
+           pressure_solver="pcg")
+SA = dict(amg_hierarchy="sa", amg_smoother="cheb2")
+CASES = {
+    "fp64": (dict(SA), 1e-9, 1e-9),
+    "fp64_terminal": (dict(SA, amg_terminal=1000), 1e-9, 1e-9),
+    "degree3": (dict(SA, amg_cheb_degree=3), 1e-9, 1e-9),
+    "degree4": (dict(SA, amg_cheb_degree=4), 1e-9, 1e-9),
+    "jacobi": (dict(amg_hierarchy="cf", cf_interp="exti", cf_pmax=8, amg_smoother="jacobi", amg_jacobi_omega=0.5), 1e-9,
+               1e-9),
+    "fp32": (dict(SA, precision="fp32", p_rtol=1e-4), 1e-3, 1e-3),
+    "amg_fp32": (dict(SA, precision="amg_fp32"), 1e-5, 1e-6),
+    "mixed": (dict(SA, precision="mixed", p_guess=2), 1e-5, 1e-6),
+    "mixed_half": (dict(SA, precision="mixed", amg_half=1), 1e-5, 1e-6),
+    "mixed_half_wide": (dict(SA, precision="mixed", amg_half=1), 1e-5, 1e-6),
+}
+MESHES = [(2, 8, 6), (2, 8, 7), (3, 16, 12), (4, 24, 13)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mesh", MESHES, ids=["%d_%d_%d" % m for m in MESHES])
+@pytest.mark.parametrize("case", sorted(CASES))
+def test_resident_pcg_matches_the_loop(native, monkeypatch, case, mesh):
+    from nodals_b200 import meshgen
+    kw, tol_cont, tol_field = CASES[case]
+    nr, nt, nz = mesh
+    m = native.Mesh.from_tetmesh(meshgen.pipe_mesh(nr=nr, ntheta=nt, nz=nz, length=0.5 * nz, jitter=0.05, seed=nz))
+    P = native.Problem(m, **dict(CFG, **kw))
+    if case.endswith("wide"):
+        monkeypatch.setenv("NDS_SELL_COL32", "1")
+    A, A2 = native.Solver(P), native.Solver(P)
+    monkeypatch.setenv("NDS_RESIDENT", "0")
+    B = native.Solver(P)
+    for _ in range(4):
+        a, a2, b = A.step(), A2.step(), B.step()
+        assert (a.p_its, a.rel_cont, a.p_rel) == (a2.p_its, a2.rel_cont, a2.p_rel)  # reproducible
+        assert abs(a.rel_cont - b.rel_cont) <= tol_cont * abs(b.rel_cont), (a.it, a.rel_cont, b.rel_cont)
+        if tol_field == 1e-9:
+            assert a.p_its == b.p_its
+    for x, y in zip(A.fields(), B.fields()):
+        assert rel_l2(x, y) <= tol_field

@@ -692,6 +692,89 @@ __global__ void __launch_bounds__(kBlock) spmv_smooth(int n, const int32_t* __re
   }
 }
 
+// The same three products on FP64 levels of many rows, with x staged in shared
+// memory: a level's numbering keeps a row's columns near the row (at most
+// 4,544 away on the 74,540-row level of the 1.23M-cell pipe), so the rows of a
+// block read one window of x, which the block copies once, and gather from
+// shared memory.  Persistent blocks, 16 lanes a row, ten entries in flight per
+// lane, row bounds one row ahead.  win: first and one-past-last column of each
+// block's rows.  The explicit levels of that mesh's FP64 V-cycle take 20 us a
+// product on average, 25 with the kernel of a lane group per row, which waits
+// for the scattered reads of x.  FP16 levels keep that one: windows of packed entries
+// gained 1 us a product by themselves but nothing to 26 us were lost an
+// iteration, as their shared memory keeps the next launch from starting early.
+enum { LEV_Y = 0, LEV_RESID = 1, LEV_SMOOTH = 2 };
+constexpr int kWinBlock = 512, kWinPerSm = 2, kWinAhead = 10;
+template <int MODE, class CT>
+__global__ void __launch_bounds__(kWinBlock, kWinPerSm)
+    level_window(int n, int rows, const int2* __restrict__ win, const int32_t* __restrict__ rp,
+                 const CT* __restrict__ ci, const double* __restrict__ v, const double* __restrict__ x,
+                 const double* __restrict__ b, const double* __restrict__ den, double w, double* __restrict__ y,
+                 double* __restrict__ y2) {
+  using T = double;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T* sx = reinterpret_cast<T*>(smem_raw);
+  pdl_begin();
+  const int r0 = blockIdx.x * rows, r1 = min(n, r0 + rows);
+  if (r0 >= n) return;
+  constexpr int groups = kWinBlock / 16;
+  const int lane = threadIdx.x & 15;
+  const unsigned mask = group_mask<16>();
+  int r = r0 + (threadIdx.x >> 4);
+  int rb = 0, re = 0;
+  if (r < r1) {
+    rb = rp[r];
+    re = rp[r + 1];
+  }
+  const int2 wn = win[blockIdx.x];
+  for (int i = wn.x + threadIdx.x; i < wn.y; i += kWinBlock) sx[i - wn.x] = x[i];
+  __syncthreads();
+  const T* xs = sx - wn.x;
+  for (; r < r1; r += groups) {
+    int nb = 0, ne = 0;
+    if (r + groups < r1) {
+      nb = rp[r + groups];
+      ne = rp[r + groups + 1];
+    }
+    T bi = 0, di = 1;
+    if (MODE != LEV_Y && lane == 0) {
+      bi = b[r];
+      if (MODE == LEV_SMOOTH || den) di = den[r];
+    }
+    T s = 0;
+    for (int k0 = rb + lane; k0 < re; k0 += 16 * kWinAhead) {
+      int c[kWinAhead];
+      T a[kWinAhead];
+#pragma unroll
+      for (int u = 0; u < kWinAhead; ++u) {
+        const int k = k0 + 16 * u;
+        c[u] = k < re ? col_at(ci, k, r) : -1;
+        a[u] = k < re ? v[k] : T(0);
+      }
+#pragma unroll
+      for (int u = 0; u < kWinAhead; ++u)
+        if (c[u] >= 0) s += a[u] * xs[c[u]];
+    }
+    s = group_sum<16>(s, mask);
+    if (lane == 0) {
+      if (MODE == LEV_Y) {
+        y[r] = s;
+      } else if (MODE == LEV_RESID) {
+        const T q = bi - s;
+        y[r] = q;
+        if (den) y2[r] = w * q / di;
+        else if (y2) y2[r] = q;
+      } else {
+        const T val = xs[r] + w * (bi - s) / di;
+        if (y2) y2[r] += val;
+        else y[r] = val;
+      }
+    }
+    rb = nb;
+    re = ne;
+  }
+}
+
 // ---------------------------------------------------------------------------
 // vector kernels (g5e_fp32_kernels.cuh:132-150, vector_kernels.cuh)
 // ---------------------------------------------------------------------------
@@ -869,6 +952,17 @@ __device__ __forceinline__ void reduce_tail(double value, const ReduceTail& t) {
   }
 }
 
+// x.y with the reduction tail STEP
+template <class T, class U, int STEP>
+__global__ void __launch_bounds__(kBlock) dot_step(int n, const T* __restrict__ x, const U* __restrict__ y,
+                                                   ReduceTail tail) {
+  pdl_begin();
+  double acc = 0.0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    acc += (double)x[i] * (double)y[i];
+  reduce_tail<STEP>(acc, tail);
+}
+
 // x += a p; r -= a q; partial r.r.  a = alpha_dev ? *alpha_dev : alpha.
 // With x1: also the first (diagonal) step of the next preconditioner
 // application's fine pre-smoother on the new r, x1 = w0 r / den0 (the
@@ -904,32 +998,35 @@ __global__ void __launch_bounds__(kBlock) xr_update(int n, double alpha, const d
 // ---------------------------------------------------------------------------
 // f += P c (one thread per fine row; P in ELL with entry k of row i at
 // k nf + i, so a warp's loads of P are coalesced).  Sequential sum over k
-// with the loads of four entries issued ahead; padding adds 0 c[0].
+// with the loads of eight entries issued ahead (a row of the SA transfers has
+// about eight); padding adds 0 c[0].  18.6 us at 1.23M cells in FP32, 22.4
+// with four entries ahead.
 template <class T>
 __global__ void prolong_add(int nf, int pw, const int32_t* __restrict__ pc, const T* __restrict__ pv,
                             const T* __restrict__ c, T* __restrict__ f) {
   pdl_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nf) return;
+  const T fi = f[i];
   T s = 0;
-  int k = 0;
   const size_t n = (size_t)nf;
-  for (; k + 3 < pw; k += 4) {
-    const size_t o = (size_t)k * n + i;
-    const int c0 = pc[o], c1 = pc[o + n], c2 = pc[o + 2 * n], c3 = pc[o + 3 * n];
-    const T a0 = pv[o], a1 = pv[o + n], a2 = pv[o + 2 * n], a3 = pv[o + 3 * n];
-    const T x0 = c[c0], x1 = c[c1], x2 = c[c2], x3 = c[c3];
-    s += a0 * x0;
-    s += a1 * x1;
-    s += a2 * x2;
-    s += a3 * x3;
+  for (int k0 = 0; k0 < pw; k0 += 8) {
+    int j[8];
+    T a[8], x[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const size_t o = (size_t)(k0 + u) * n + i;
+      j[u] = k0 + u < pw ? pc[o] : 0;
+      a[u] = k0 + u < pw ? pv[o] : T(0);
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) x[u] = k0 + u < pw ? c[j[u]] : T(0);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) s += a[u] * x[u];
   }
-  for (; k < pw; ++k) {
-    const size_t o = (size_t)k * n + i;
-    s += pv[o] * c[pc[o]];
-  }
-  f[i] += s;
+  f[i] = fi + s;
 }
+
 // ---------------------------------------------------------------------------
 // Dense form of the V-cycle from a level down: the explicit levels never
 // change after setup, so the cycle from level l on is one constant matrix
@@ -1420,6 +1517,62 @@ __global__ void sell_gs_color(int count, const int32_t* __restrict__ rows, Sell 
   x[i] = old + omega * (gs - old);
 }
 
+// The restriction to a level of many rows: a warp a row, persistent, the next
+// row's entries (160 in one round; a row of the SA transfers has about 130)
+// loaded before the current row's gathers and sum.  At 1.23M cells in FP32 the
+// transfers of a V-cycle average 16.8 us, 17.8 with a lane group per row and
+// four entries of the prolongation ahead.
+constexpr int kRestAhead = 5;
+template <class T>
+__global__ void __launch_bounds__(kBlock, 4) restrict_stream(int nc, const int32_t* __restrict__ rr,
+                                                             const int32_t* __restrict__ rc, const T* __restrict__ rv,
+                                                             const T* __restrict__ f, T* __restrict__ c,
+                                                             const T* __restrict__ den0, T w0, T* __restrict__ x1) {
+  pdl_begin();
+  const int lane = threadIdx.x & 31, stride = gridDim.x * kWarps;
+  int I = blockIdx.x * kWarps + (threadIdx.x >> 5);
+  auto bounds = [&](int i) { return i < nc ? make_int2(rr[i], rr[i + 1]) : make_int2(0, 0); };
+  auto entries = [&](int (&j)[kRestAhead], T (&v)[kRestAhead], int2 o) {
+#pragma unroll
+    for (int u = 0; u < kRestAhead; ++u) {
+      const int k = o.x + lane + 32 * u;
+      j[u] = k < o.y ? rc[k] : -1;
+      v[u] = k < o.y ? rv[k] : T(0);
+    }
+  };
+  int2 cur = bounds(I), nxt = bounds(I + stride);
+  int j[kRestAhead];
+  T v[kRestAhead];
+  entries(j, v, cur);
+  for (; I < nc; I += stride) {
+    const int2 nn = bounds(I + 2 * stride);
+    T x[kRestAhead];
+#pragma unroll
+    for (int u = 0; u < kRestAhead; ++u) x[u] = j[u] >= 0 ? f[j[u]] : T(0);
+    int jn[kRestAhead];
+    T vn[kRestAhead];
+    entries(jn, vn, nxt);
+    T di = 1;
+    if (x1 && lane == 0) di = den0[I];
+    T s = 0;
+#pragma unroll
+    for (int u = 0; u < kRestAhead; ++u) s += v[u] * x[u];
+    for (int k = cur.x + lane + 32 * kRestAhead; k < cur.y; k += 32) s += rv[k] * f[rc[k]];
+    s = warp_sum(s);
+    if (lane == 0) {
+      c[I] = s;
+      // with x1: the coarse pre-smoother's diagonal step w0 c / den0
+      if (x1) x1[I] = w0 * s / di;
+    }
+    cur = nxt;
+    nxt = nn;
+#pragma unroll
+    for (int u = 0; u < kRestAhead; ++u) {
+      j[u] = jn[u];
+      v[u] = vn[u];
+    }
+  }
+}
 // c = P^T f, a kRowLanes group per coarse row over R = P^T (deterministic
 // tree per row)
 template <class T, int GL = kRowLanes>

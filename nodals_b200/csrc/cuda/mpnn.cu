@@ -26,9 +26,10 @@
 // thread issues 8 MMAs (M = 128, N = 64, K = 16) against the weight tile kept
 // in shared memory, and the accumulator (128 lanes x 64 columns of TMEM) is
 // read back with tcgen05.ld for the bias + ReLU epilogue, warp w taking lanes
-// 32 (w mod 4) and columns 16 (w / 4).  403,680 nodes: 127 us a layer with one thread per
-// row (two waves of 128-byte rows per warp load), 70 us so (0.25 TB/s of
-// neighbours' rows from L2 beside the 103 MB read and written).  Backward uses the same tiles:
+// 32 (w mod 4) and columns 16 (w / 4).  A layer on 403,680 nodes takes 70 us
+// (133 us with one thread a row); the 103 MB read and written would take 16
+// us, the rest is the latency of the gathers at 1,024 threads an SM.  Backward
+// uses the same tiles:
 // dX = delta W (M 128, N 128, K 64) and dW^T += X^T delta (M 128, N 64,
 // K = the 128 nodes of the tile, both operands read MN-major from the same
 // shared-memory tiles), accumulated in TMEM over all tiles of a CTA.

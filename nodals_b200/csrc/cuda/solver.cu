@@ -297,6 +297,11 @@ class Solver final : public ISolver {
     DBuf<__half> hval;
     DBuf<int16_t> hcol;
     double hinv = 1.0;
+    // windows of x of the level's persistent SpMV (empty: not used)
+    DBuf<int2> win;
+    DBuf<int16_t> dcol;  // FP64 levels with windows: columns as 16-bit deltas to the row, when they fit
+    int wrows = 0, wblocks = 0;
+    size_t wsmem = 0;
   };
   struct Xfer {  // P (fine rows, ELL k-major) and R = P^T (coarse rows, CSR)
     int nf = 0, nc = 0, pw = 0;
@@ -507,6 +512,7 @@ class Solver final : public ISolver {
       // the mixed path's V-cycle reads FP16 copies of the explicit levels
       // (the terminal level goes through its dense inverse)
       if (!kSame && o_.precision == NDS_MIXED && o_.amg_half && l + 1 < H.A.size()) level_to_half(Lv, A);
+      if (l + 1 < H.A.size()) level_windows(Lv, A);
       if (o_.amg_smoother == NDS_SM_MCGS && l + 1 < H.A.size()) {
         std::vector<int32_t> rows;
         std::vector<int32_t> r32 = to_i32(A.row, "AMG level CSR");
@@ -963,6 +969,7 @@ class Solver final : public ISolver {
   }
 
   // ------------------------------------------------------------------ helpers
+  static constexpr int kSms = 148;
   static constexpr int kMaxPartBlocks = 1184;  // 8 x 148 SMs
   static constexpr int kScalars = 128;
   enum { S_RHO = 0, S_PQ = 1, S_ALPHA = 2, S_RN2 = 3, S_RHON = 4, S_BETA = 5, S_R0 = 6, S_TARGET = 7, S_TMP = 8,
@@ -1096,6 +1103,10 @@ class Solver final : public ISolver {
     const __half* vh = nullptr;  // FP16 copy of the values, scaled by 1 / vinv
     double vinv = 1.0;
     const int16_t* ch = nullptr;  // CSR levels with vh: columns as deltas to the row
+    const int2* win = nullptr;    // CSR levels: windows of x (level_window)
+    int wrows = 0, wblocks = 0;
+    size_t wsmem = 0;
+    const int16_t* dc = nullptr;  // with win: columns as deltas to the row
     // fine operator in split form (sell is set too)
     bool split = false, half = false;
     k::SplitVerts sv{};
@@ -1117,16 +1128,16 @@ class Solver final : public ISolver {
   }
   template <class V>
   void split_vertices(const OpView<V>& A, const V* x) {
-    const int gv = grid_for(8LL * A.sv.n);
-    if (A.sv.n > 0) {
-      if constexpr (std::is_same<V, double>::value)
-        pdl_launch(k::split_vertex<V, k::REC_SOA>, gv, kBlock, 0, st_, A.sv, A.rv, x, A.w, V(A.wscale));
-      else if (A.sv.rec8)
-        pdl_launch(k::split_vertex<V, k::REC_8>, gv, kBlock, 0, st_, A.sv, A.rv, x, A.w, V(A.wscale));
-      else
-        pdl_launch(k::split_vertex<V, k::REC_16>, gv, kBlock, 0, st_, A.sv, A.rv, x, A.w, V(A.wscale));
-      NDS_LAUNCH();
-    }
+    if (A.sv.n <= 0) return;
+    auto go = [&](auto rec) {
+      constexpr int REC = decltype(rec)::value;
+      const int gv = std::min(grid_for(8LL * A.sv.n), kSms * k::split_vertex_blocks<REC>());
+      pdl_launch(k::split_vertex<V, REC>, gv, kBlock, 0, st_, A.sv, A.rv, x, A.w, V(A.wscale));
+    };
+    if constexpr (std::is_same<V, double>::value) go(std::integral_constant<int, k::REC_SOA>{});
+    else if (A.sv.rec8) go(std::integral_constant<int, k::REC_8>{});
+    else go(std::integral_constant<int, k::REC_16>{});
+    NDS_LAUNCH();
   }
   // f(value type of the cells' data, 16-bit neighbour deltas)
   template <class V, class F>
@@ -1265,7 +1276,75 @@ class Solver final : public ISolver {
       V.vinv = A.hinv;
       V.ch = A.hcol.p;
     }
+    V.win = A.win.p;
+    V.wrows = A.wrows;
+    V.wblocks = A.wblocks;
+    V.wsmem = A.wsmem;
+    V.dc = A.dcol.p;
     return V;
+  }
+  // windows of a level's rows (FP64 levels): from kWinRows rows on, when a
+  // window fits the block's share of shared memory.  The line: with fewer rows
+  // than about two per lane group of the 296 blocks there is no next row to
+  // look ahead to and the copy of the window is not paid back.  At 74,540 rows
+  // a product takes 20 us on average over the explicit levels instead of 25.
+  static constexpr int kWinRows = 16384;
+  static constexpr size_t kWinBytes = 72 * 1024;
+  void level_windows(Level& Lv, const CsrHost& A) {
+    if (A.n < stream_rows(kWinRows) || !std::is_same<TA, double>::value) return;
+    int sms = 0;
+    NDS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, o_.device));
+    const int blocks = sms * k::kWinPerSm, rows = (A.n + blocks - 1) / blocks;
+    std::vector<int2> win((size_t)blocks, make_int2(0, 0));
+    int most = 0;
+#pragma omp parallel for schedule(static) reduction(max : most)
+    for (int q = 0; q < blocks; ++q) {
+      const int r0 = std::min(A.n, q * rows), r1 = std::min(A.n, r0 + rows);
+      int lo = A.n, hi = 0;
+      for (int i = r0; i < r1; ++i) {
+        lo = std::min(lo, i);
+        hi = std::max(hi, i + 1);
+        for (int64_t k = A.row[(size_t)i]; k < A.row[(size_t)i + 1]; ++k) {
+          lo = std::min(lo, (int)A.col[(size_t)k]);
+          hi = std::max(hi, (int)A.col[(size_t)k] + 1);
+        }
+      }
+      if (lo < hi) win[(size_t)q] = make_int2(lo, hi);
+      most = std::max(most, hi - lo);
+    }
+    if ((size_t)most * sizeof(double) > kWinBytes) return;
+    std::vector<int16_t> dc(A.col.size());
+    int too_far = 0;
+#pragma omp parallel for schedule(static) reduction(| : too_far)
+    for (int i = 0; i < A.n; ++i)
+      for (int64_t k = A.row[(size_t)i]; k < A.row[(size_t)i + 1]; ++k) {
+        const int d = A.col[(size_t)k] - i;
+        if (d < -32767 || d > 32767) too_far = 1;
+        else dc[(size_t)k] = (int16_t)d;
+      }
+    if (!too_far && !std::getenv("NDS_SELL_COL32")) Lv.dcol.upload(dc);
+    Lv.win.upload(win);
+    Lv.wrows = rows;
+    Lv.wblocks = blocks;
+    Lv.wsmem = (size_t)most * sizeof(double);
+  }
+  // a product of a level with windows; false when it has none
+  template <int MODE, class V>
+  bool window_launch(const OpView<V>& A, const V* x, const V* b, const V* den, double w, V* y, V* y2) {
+    if (!A.win) return false;
+    if constexpr (std::is_same<V, double>::value) {
+      auto go = [&](auto* ci) {
+        using CT = std::remove_const_t<std::remove_pointer_t<decltype(ci)>>;
+        auto* kernel = k::level_window<MODE, CT>;
+        NDS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWinBytes));
+        pdl_launch(kernel, A.wblocks, k::kWinBlock, A.wsmem, st_, A.n, A.wrows, A.win, A.rp, ci, A.v, x, b, den, w, y,
+                   y2);
+      };
+      if (A.dc) go(A.dc);
+      else go(A.ci);
+      return true;
+    }
+    return false;
   }
   // FP16 copy of an explicit level's CSR values (a setup snapshot), scaled by
   // the power of two that puts its largest diagonal at 2^11
@@ -1304,7 +1383,8 @@ class Solver final : public ISolver {
   void op_spmv(const OpView<V>& A, const V* x, V* y) {
     ProfScope ps(prof, st_, A.cat);
     if (A.sell) sell_launch<k::SELL_Y, V>(A, grid_for(A.n), x, nullptr, nullptr, 0.0, y, nullptr);
-    else if (A.vh && A.ch && std::is_same<V, float>::value)
+    else if (window_launch<k::LEV_Y, V>(A, x, nullptr, nullptr, 0.0, y, nullptr)) {
+    } else if (A.vh && A.ch && std::is_same<V, float>::value)
       level_half_launch(A, [&](auto gl) {
         constexpr int GL = decltype(gl)::value;
         pdl_launch(k::spmv<V, __half, int16_t, GL>, grid_for((long long)A.n * GL), kBlock, 0, st_, A.n, A.rp, A.ch,
@@ -1326,7 +1406,8 @@ class Solver final : public ISolver {
                 double w = 0.0) {
     ProfScope ps(prof, st_, A.cat);
     if (A.sell) sell_launch<k::SELL_RESID, V>(A, grid_for(A.n), x, b, den, w, r, r2);
-    else if (A.vh && A.ch && std::is_same<V, float>::value)
+    else if (window_launch<k::LEV_RESID, V>(A, x, b, den, w, r, r2)) {
+    } else if (A.vh && A.ch && std::is_same<V, float>::value)
       level_half_launch(A, [&](auto gl) {
         constexpr int GL = decltype(gl)::value;
         pdl_launch(k::spmv_resid<V, __half, int16_t, GL>, grid_for((long long)A.n * GL), kBlock, 0, st_, A.n, A.rp,
@@ -1348,7 +1429,8 @@ class Solver final : public ISolver {
   void op_smooth(const OpView<V>& A, const V* xin, const V* b, const V* den, double w, V* xout, V* add_to = nullptr) {
     ProfScope ps(prof, st_, A.cat);
     if (A.sell) sell_launch<k::SELL_SMOOTH, V>(A, grid_for(A.n), xin, b, den, w, xout, add_to);
-    else if (A.vh && A.ch && std::is_same<V, float>::value)
+    else if (window_launch<k::LEV_SMOOTH, V>(A, xin, b, den, w, xout, add_to)) {
+    } else if (A.vh && A.ch && std::is_same<V, float>::value)
       level_half_launch(A, [&](auto gl) {
         constexpr int GL = decltype(gl)::value;
         pdl_launch(k::spmv_smooth<V, __half, int16_t, GL>, grid_for((long long)A.n * GL), kBlock, 0, st_, A.n, A.rp,
@@ -1502,6 +1584,16 @@ class Solver final : public ISolver {
   // whether the pre-smoother of level l can take its diagonal step in the
   // restriction that feeds it (a polynomial smoother, not the terminal level)
   bool fuse_pre(int l) const { return o_.amg_smoother != NDS_SM_MCGS && l < (int)L_.size() - 1 && l != dense_level_; }
+  // coarse rows from which the restriction streams: more than a wave of warps, so
+  // that there is a next row to load ahead (fewer rows: a lane group a row)
+  static constexpr int kStreamRows = 8192;
+  // NDS_STREAM_ROWS overrides the row counts from which the streaming kernels
+  // of the levels and the restriction are used
+  static int stream_rows(int rows) {
+    const char* e = std::getenv("NDS_STREAM_ROWS");
+    return e ? std::atoi(e) : rows;
+  }
+  int rest_rows_ = stream_rows(kStreamRows);
   // lanes per coarse row of the restriction (the FP16 levels' count on the
   // mixed FP16 path, a warp otherwise)
   int restrict_lanes() const { return mixed_ && o_.amg_half ? level_lanes_ : 32; }
@@ -1519,7 +1611,10 @@ class Solver final : public ISolver {
       w0 = pl.w0;
       x1 = poly_first(pl, C.x.p, C.pong.p);
     }
-    if (restrict_lanes() != 32) {
+    if (X.nc >= rest_rows_) {
+      const int g = std::min(grid_for(X.nc, kBlock / 32), 4 * kSms);
+      pdl_launch(k::restrict_stream<TA>, g, kBlock, 0, st_, X.nc, X.rrow.p, X.rcol.p, X.rval.p, f, c, den0, TA(w0), x1);
+    } else if (restrict_lanes() != 32) {
       auto run = [&](auto gl) {
         constexpr int GL = decltype(gl)::value;
         pdl_launch(k::restrict_rows<TA, GL>, grid_for((long long)X.nc * GL), kBlock, 0, st_, X.nc, X.rrow.p,
@@ -1828,6 +1923,11 @@ class Solver final : public ISolver {
     if (!std::isfinite(r0)) throw SolveFailure(NDS_E_BREAKDOWN, "pressure initial norm nonfinite");
     return r0;
   }
+  // r.z taken by the V-cycle's last kernel up to this many cells: it saves a
+  // launch there, but each of that kernel's blocks waits for its stores before
+  // it leaves its partial sum, which costs 12 us at 1.23M cells against 6 us
+  // for a pass of its own.
+  static constexpr int kRhoCells = 200000;
   // Vectors of a PCG solve in precision S (the preconditioner runs in TA):
   // rA the residual in TA when the precisions differ.
   template <class S>
@@ -1863,13 +1963,12 @@ class Solver final : public ISolver {
     const bool fused = pre_fused();
     const TA* r = v.rA;
     if constexpr (std::is_same<S, TA>::value) r = v.r;
-    if (split_) {
+    if (split_ && nc_ <= kRhoCells) {
       amg_apply<S>(r, v.z, fused, v.r);
     } else {
       amg_apply(r, v.z, fused);
-      pdl_launch(k::dot<S, TA>, g, kBlock, 0, st_, nc_, v.r, v.z, part_.p);
+      pdl_launch(k::dot_step<S, TA, k::PCG_RHO>, g, kBlock, 0, st_, nc_, v.r, v.z, tail(S_RHON));
       NDS_LAUNCH();
-      reduce_pcg<k::PCG_RHO>(g, S_RHON);
     }
     pdl_launch(k::p_update_dev<S, TA>, grid_for(nc_), kBlock, 0, st_, nc_, sc_.p + S_BETA, ctl_.p, v.z, v.p);
     NDS_LAUNCH();

@@ -57,78 +57,128 @@ struct SplitVerts {
 };
 enum SplitRec { REC_SOA = 0, REC_16 = 1, REC_8 = 2 };
 
+// one incidence as stored
+template <int REC>
+struct SplitRaw;
+template <>
+struct SplitRaw<REC_SOA> {
+  double x, y, z;
+  int c;
+  __device__ __forceinline__ void load(const SplitVerts& a, int k) {
+    x = a.bx[k];
+    y = a.by[k];
+    z = a.bz[k];
+    c = a.cell[k];
+  }
+  __device__ __forceinline__ int cell(int) const { return c; }
+  __device__ __forceinline__ void vec(double (&b)[3]) const { b[0] = x; b[1] = y; b[2] = z; }
+};
+template <>
+struct SplitRaw<REC_16> {
+  float4 q;
+  __device__ __forceinline__ void load(const SplitVerts& a, int k) { q = a.rec16[k]; }
+  __device__ __forceinline__ int cell(int) const { return __float_as_int(q.w); }
+  __device__ __forceinline__ void vec(float (&b)[3]) const { b[0] = q.x; b[1] = q.y; b[2] = q.z; }
+};
+template <>
+struct SplitRaw<REC_8> {
+  uint2 q;
+  __device__ __forceinline__ void load(const SplitVerts& a, int k) { q = a.rec8[k]; }
+  __device__ __forceinline__ int cell(int base) const { return base + (int)(q.y >> 16); }
+  __device__ __forceinline__ void vec(float (&b)[3]) const {
+    const float2 xy = __half22float2(*reinterpret_cast<const __half2*>(&q.x));
+    b[0] = xy.x;
+    b[1] = xy.y;
+    b[2] = __half2float(__ushort_as_half((unsigned short)(q.y & 0xFFFFu)));
+  }
+};
+
 // w_v = scale rAU_v sum B x over the vertex's cells, eight lanes a vertex
-// (24 incidences on average: four records in flight per lane cover 32 in one
-// round).  w holds 4 values a vertex; entry n stays zero (fixed vertices).
+// (24 incidences on average: four records per lane cover 32 in one round).  w
+// holds 4 values a vertex; entry n stays zero (fixed vertices).
+//
+// Three dependent loads a vertex (offsets, records, x) and little else: bound
+// by their latency when each group does one vertex (21 us at 1.23M cells in
+// FP16, 46 MB).  So the groups are persistent and pipelined: the offsets are
+// loaded two vertices ahead and the records one ahead, and a vertex waits
+// only for its gathers: 13.3 us so.
 constexpr int kSplitAhead = 4;
+template <int REC>
+constexpr int split_vertex_blocks() { return REC == REC_SOA ? 2 : REC == REC_16 ? 4 : 5; }  // per SM
 template <class V, int REC>
-__global__ void __launch_bounds__(kBlock) split_vertex(SplitVerts a, const V* __restrict__ rau,
-                                                       const V* __restrict__ x, V* __restrict__ w, V scale) {
+__global__ void __launch_bounds__(kBlock, split_vertex_blocks<REC>())
+    split_vertex(SplitVerts a, const V* __restrict__ rau, const V* __restrict__ x, V* __restrict__ w, V scale) {
   pdl_begin();
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int g = t >> 3, lane = t & 7;
-  if (g >= a.n) return;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, stride = (gridDim.x * blockDim.x) >> 3;
+  const int lane = t & 7;
   const unsigned mask = group8_mask();
-  const int zb = a.off[g], ze = a.off[g + 1];
-  int c0 = 0;
-  if (REC == REC_8) c0 = a.base[g];
-  V r = 0;
-  if (lane == 0) r = scale * rau[g];
-  V s0 = 0, s1 = 0, s2 = 0;
-  for (int z0 = zb + lane; z0 < ze; z0 += 8 * kSplitAhead) {
-    V b0[kSplitAhead], b1[kSplitAhead], b2[kSplitAhead], xv[kSplitAhead];
-    int c[kSplitAhead];
+  int g = t >> 3;
+  struct Off {
+    int b, e, base;
+  };
+  auto offsets = [&](int v) {
+    Off o{0, 0, 0};
+    if (v < a.n) {
+      o.b = a.off[v];
+      o.e = a.off[v + 1];
+      if (REC == REC_8) o.base = a.base[v];
+    }
+    return o;
+  };
+  auto records = [&](SplitRaw<REC> (&raw)[kSplitAhead], const Off& o) {
 #pragma unroll
     for (int u = 0; u < kSplitAhead; ++u) {
-      const int z = z0 + 8 * u;
-      const bool ok = z < ze;
-      c[u] = -1;
-      b0[u] = b1[u] = b2[u] = V(0);
-      if constexpr (REC == REC_SOA) {
-        if (ok) {
-          b0[u] = V(a.bx[z]);
-          b1[u] = V(a.by[z]);
-          b2[u] = V(a.bz[z]);
-          c[u] = a.cell[z];
-        }
-      } else if constexpr (REC == REC_16) {
-        if (ok) {
-          const float4 q = a.rec16[z];
-          b0[u] = q.x;
-          b1[u] = q.y;
-          b2[u] = q.z;
-          c[u] = __float_as_int(q.w);
-        }
+      const int z = o.b + lane + 8 * u;
+      if (z < o.e) raw[u].load(a, z);
+    }
+  };
+  Off cur = offsets(g), nxt = offsets(g + stride);
+  SplitRaw<REC> raw[kSplitAhead] = {};
+  records(raw, cur);
+  for (; g < a.n; g += stride) {
+    const Off nn = offsets(g + 2 * stride);
+    SplitRaw<REC> rawn[kSplitAhead] = {};
+    V xv[kSplitAhead];
+#pragma unroll
+    for (int u = 0; u < kSplitAhead; ++u)
+      xv[u] = cur.b + lane + 8 * u < cur.e ? x[raw[u].cell(cur.base)] : V(0);
+    records(rawn, nxt);
+    V r = 0;
+    if (lane == 0) r = scale * rau[g];
+    V s0 = 0, s1 = 0, s2 = 0;
+#pragma unroll
+    for (int u = 0; u < kSplitAhead; ++u) {
+      V b[3];
+      raw[u].vec(b);
+      s0 += b[0] * xv[u];
+      s1 += b[1] * xv[u];
+      s2 += b[2] * xv[u];
+    }
+    for (int z = cur.b + lane + 8 * kSplitAhead; z < cur.e; z += 8) {
+      SplitRaw<REC> q;
+      q.load(a, z);
+      V b[3];
+      q.vec(b);
+      const V xz = x[q.cell(cur.base)];
+      s0 += b[0] * xz;
+      s1 += b[1] * xz;
+      s2 += b[2] * xz;
+    }
+    s0 = group_sum<8>(s0, mask);
+    s1 = group_sum<8>(s1, mask);
+    s2 = group_sum<8>(s2, mask);
+    if (lane == 0) {
+      if constexpr (std::is_same<V, float>::value) {
+        reinterpret_cast<float4*>(w)[g] = make_float4(r * s0, r * s1, r * s2, 0.f);
       } else {
-        if (ok) {
-          const uint2 q = a.rec8[z];
-          const float2 xy = __half22float2(*reinterpret_cast<const __half2*>(&q.x));
-          b0[u] = xy.x;
-          b1[u] = xy.y;
-          b2[u] = __half2float(__ushort_as_half((unsigned short)(q.y & 0xFFFFu)));
-          c[u] = c0 + (int)(q.y >> 16);
-        }
+        reinterpret_cast<double2*>(w)[2 * (size_t)g] = make_double2(r * s0, r * s1);
+        w[4 * (size_t)g + 2] = r * s2;
       }
     }
+    cur = nxt;
+    nxt = nn;
 #pragma unroll
-    for (int u = 0; u < kSplitAhead; ++u) xv[u] = c[u] >= 0 ? x[c[u]] : V(0);
-#pragma unroll
-    for (int u = 0; u < kSplitAhead; ++u) {
-      s0 += b0[u] * xv[u];
-      s1 += b1[u] * xv[u];
-      s2 += b2[u] * xv[u];
-    }
-  }
-  s0 = group_sum<8>(s0, mask);
-  s1 = group_sum<8>(s1, mask);
-  s2 = group_sum<8>(s2, mask);
-  if (lane == 0) {
-    if constexpr (std::is_same<V, float>::value) {
-      reinterpret_cast<float4*>(w)[g] = make_float4(r * s0, r * s1, r * s2, 0.f);
-    } else {
-      reinterpret_cast<double2*>(w)[2 * (size_t)g] = make_double2(r * s0, r * s1);
-      w[4 * (size_t)g + 2] = r * s2;
-    }
+    for (int u = 0; u < kSplitAhead; ++u) raw[u] = rawn[u];
   }
 }
 

@@ -26,12 +26,18 @@ extern unsigned long long g_launches;
 // Launch of a kernel that begins with pdl_begin(): the grid may be set up
 // while the kernel before it in the stream still runs (programmatic dependent
 // launch), which takes about a microsecond off every step of a chain of short
-// kernels.  pdl_begin() lets the next kernel be set up and then waits for the
-// whole of the previous one, so nothing is read or written early; every kernel
-// launched this way must call it before it touches memory.
+// kernels.  pdl_trigger() lets the next kernel be set up, pdl_wait() waits for
+// the whole of the previous one (and so for all before it).  Every kernel
+// launched this way calls both; before pdl_wait() it may read only what no
+// kernel of the stream writes between a full dependency (host
+// synchronisation, event wait, graph boundary) and itself: the kernels of the
+// pressure solve load their matrix entries there, constant during a solve, so
+// that these round trips overlap the previous kernel's end.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_begin() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_trigger();
+  pdl_wait();
 }
 template <class... P, class... A>
 inline void pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {

@@ -606,34 +606,44 @@ __device__ __forceinline__ T load_val(const MT* __restrict__ v, int k) {
 // column of entry k of row i: absolute (int32) or a 16-bit delta to the row
 __device__ __forceinline__ int col_at(const int32_t* __restrict__ ci, int k, int) { return ci[k]; }
 __device__ __forceinline__ int col_at(const int16_t* __restrict__ ci, int k, int i) { return i + ci[k]; }
-template <int G, class T, class MT = T, class CT = int32_t>
+// The entries are constant during a solve: WAIT loads the first round of them
+// before pdl_wait().
+template <int G, class T, class MT = T, class CT = int32_t, bool WAIT = false>
 __device__ __forceinline__ T lane_batched_dot(int rb, int re, const CT* __restrict__ ci, const MT* __restrict__ v,
                                               const T* __restrict__ x, int lane, int i = 0) {
   T s = 0;
-  for (int k0 = rb + lane; k0 < re; k0 += 8 * G) {
-    int c[8];
-    T a[8];
+  int c[8];
+  T a[8];
+  auto entries = [&](int k0) {
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       const int k = k0 + u * G;
       c[u] = k < re ? col_at(ci, k, i) : -1;
       a[u] = k < re ? load_val<T, MT>(v, k) : T(0);
     }
+  };
+  entries(rb + lane);
+  if (WAIT) pdl_wait();
+  for (int k0 = rb + lane; k0 < re; k0 += 8 * G) {
     T xv[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u) xv[u] = c[u] >= 0 ? x[c[u]] : T(0);
 #pragma unroll
     for (int u = 0; u < 8; ++u)
       if (c[u] >= 0) s += a[u] * xv[u];
+    entries(k0 + 8 * G);
   }
   return s;
 }
 constexpr int kRowLanes = 32;
+// live: the group has a row; every thread of the block calls it (it waits for
+// the previous kernel after loading the first entries)
 template <class T, class MT = T, class CT = int32_t, int GL = kRowLanes>
 __device__ __forceinline__ T group_row_dot(const int32_t* __restrict__ rp, const CT* __restrict__ ci,
                                            const MT* __restrict__ v, const T* __restrict__ x, int i, int lane,
-                                           unsigned mask, T vinv = T(1)) {
-  T s = group_sum<GL>(lane_batched_dot<GL, T, MT, CT>(rp[i], rp[i + 1], ci, v, x, lane, i), mask);
+                                           unsigned mask, bool live, T vinv = T(1)) {
+  const int rb = live ? rp[i] : 0, re = live ? rp[i + 1] : 0;
+  T s = group_sum<GL>(lane_batched_dot<GL, T, MT, CT, true>(rb, re, ci, v, x, lane, i), mask);
   if constexpr (!std::is_same<MT, T>::value) s *= vinv;
   return s;
 }
@@ -643,12 +653,11 @@ template <class T, class MT = T, class CT = int32_t, int GL = kRowLanes>
 __global__ void __launch_bounds__(kBlock) spmv(int n, const int32_t* __restrict__ rp, const CT* __restrict__ ci,
                                                const MT* __restrict__ v, const T* __restrict__ x, T* __restrict__ y,
                                                T vinv = T(1)) {
-  pdl_begin();
+  pdl_trigger();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int i = t / GL, lane = t % GL;
-  if (i >= n) return;
-  const T s = group_row_dot<T, MT, CT, GL>(rp, ci, v, x, i, lane, group_mask<GL>(), vinv);
-  if (lane == 0) y[i] = s;
+  const T s = group_row_dot<T, MT, CT, GL>(rp, ci, v, x, i, lane, group_mask<GL>(), i < n, vinv);
+  if (i < n && lane == 0) y[i] = s;
 }
 
 // r = b - A x  (optionally also r2 = r)
@@ -657,12 +666,11 @@ __global__ void __launch_bounds__(kBlock) spmv_resid(int n, const int32_t* __res
                                                      const MT* __restrict__ v, const T* __restrict__ x,
                                                      const T* __restrict__ b, T* __restrict__ r, T* __restrict__ r2,
                                                      const T* __restrict__ den, T w, T vinv = T(1)) {
-  pdl_begin();
+  pdl_trigger();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int i = t / GL, lane = t % GL;
-  if (i >= n) return;
-  const T s = group_row_dot<T, MT, CT, GL>(rp, ci, v, x, i, lane, group_mask<GL>(), vinv);
-  if (lane == 0) {
+  const T s = group_row_dot<T, MT, CT, GL>(rp, ci, v, x, i, lane, group_mask<GL>(), i < n, vinv);
+  if (i < n && lane == 0) {
     // r; r2 = r (den null) or the first Jacobi step w r / den
     const T q = b[i] - s;
     r[i] = q;
@@ -678,12 +686,11 @@ __global__ void __launch_bounds__(kBlock) spmv_smooth(int n, const int32_t* __re
                                                       const T* __restrict__ xin, const T* __restrict__ b,
                                                       const T* __restrict__ den, T w, T* __restrict__ xout,
                                                       T* __restrict__ add_to, T vinv = T(1)) {
-  pdl_begin();
+  pdl_trigger();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int i = t / GL, lane = t % GL;
-  if (i >= n) return;
-  const T s = group_row_dot<T, MT, CT, GL>(rp, ci, v, xin, i, lane, group_mask<GL>(), vinv);
-  if (lane == 0) {
+  const T s = group_row_dot<T, MT, CT, GL>(rp, ci, v, xin, i, lane, group_mask<GL>(), i < n, vinv);
+  if (i < n && lane == 0) {
     // with add_to the step is added to add_to instead of stored in xout
     const T r = b[i] - s;
     const T val = xin[i] + w * r / den[i];
@@ -704,6 +711,20 @@ __global__ void __launch_bounds__(kBlock) spmv_smooth(int n, const int32_t* __re
 // gained 1 us a product by themselves but nothing to 26 us were lost an
 // iteration, as their shared memory keeps the next launch from starting early.
 enum { LEV_Y = 0, LEV_RESID = 1, LEV_SMOOTH = 2 };
+// x[lo, hi) into shared memory at the offset lo - lo4, lo4 = lo rounded down to
+// a 16-byte boundary: vector loads, eight in flight (x from cudaMalloc, padded
+// reads stay inside [lo4, hi))
+template <int BLOCK, class T>
+__device__ __forceinline__ void stage_window(T* __restrict__ sx, const T* __restrict__ x, int lo4, int hi) {
+  constexpr int W = 16 / sizeof(T);
+  using V = typename std::conditional<std::is_same<T, float>::value, float4, double2>::type;
+  const int nv = (hi - lo4) / W;
+  const V* src = reinterpret_cast<const V*>(x + lo4);
+  V* dst = reinterpret_cast<V*>(sx);
+#pragma unroll 8
+  for (int i = threadIdx.x; i < nv; i += BLOCK) dst[i] = src[i];
+  for (int i = lo4 + nv * W + threadIdx.x; i < hi; i += BLOCK) sx[i - lo4] = x[i];
+}
 constexpr int kWinBlock = 512, kWinPerSm = 2, kWinAhead = 10;
 template <int MODE, class CT>
 __global__ void __launch_bounds__(kWinBlock, kWinPerSm)
@@ -714,9 +735,8 @@ __global__ void __launch_bounds__(kWinBlock, kWinPerSm)
   using T = double;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* sx = reinterpret_cast<T*>(smem_raw);
-  pdl_begin();
+  pdl_trigger();
   const int r0 = blockIdx.x * rows, r1 = min(n, r0 + rows);
-  if (r0 >= n) return;
   constexpr int groups = kWinBlock / 16;
   const int lane = threadIdx.x & 15;
   const unsigned mask = group_mask<16>();
@@ -727,9 +747,11 @@ __global__ void __launch_bounds__(kWinBlock, kWinPerSm)
     re = rp[r + 1];
   }
   const int2 wn = win[blockIdx.x];
-  for (int i = wn.x + threadIdx.x; i < wn.y; i += kWinBlock) sx[i - wn.x] = x[i];
+  pdl_wait();
+  const int lo4 = wn.x & ~(16 / (int)sizeof(T) - 1);
+  stage_window<kWinBlock>(sx, x, lo4, wn.y);
   __syncthreads();
-  const T* xs = sx - wn.x;
+  const T* xs = sx - lo4;
   for (; r < r1; r += groups) {
     int nb = 0, ne = 0;
     if (r + groups < r1) {
@@ -1004,23 +1026,30 @@ __global__ void __launch_bounds__(kBlock) xr_update(int n, double alpha, const d
 template <class T>
 __global__ void prolong_add(int nf, int pw, const int32_t* __restrict__ pc, const T* __restrict__ pv,
                             const T* __restrict__ c, T* __restrict__ f) {
-  pdl_begin();
+  pdl_trigger();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t n = (size_t)nf;
+  int j[8];
+  T a[8];
+  auto entries = [&](int k0) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const bool ok = i < nf && k0 + u < pw;
+      const size_t o = (size_t)(k0 + u) * n + i;
+      j[u] = ok ? pc[o] : -1;
+      a[u] = ok ? pv[o] : T(0);
+    }
+  };
+  entries(0);
+  pdl_wait();
   if (i >= nf) return;
   const T fi = f[i];
   T s = 0;
-  const size_t n = (size_t)nf;
   for (int k0 = 0; k0 < pw; k0 += 8) {
-    int j[8];
-    T a[8], x[8];
+    if (k0) entries(k0);
+    T x[8];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const size_t o = (size_t)(k0 + u) * n + i;
-      j[u] = k0 + u < pw ? pc[o] : 0;
-      a[u] = k0 + u < pw ? pv[o] : T(0);
-    }
-#pragma unroll
-    for (int u = 0; u < 8; ++u) x[u] = k0 + u < pw ? c[j[u]] : T(0);
+    for (int u = 0; u < 8; ++u) x[u] = j[u] >= 0 ? c[j[u]] : T(0);
 #pragma unroll
     for (int u = 0; u < 8; ++u) s += a[u] * x[u];
   }
@@ -1103,12 +1132,14 @@ __global__ void block_add(size_t total, const T* __restrict__ x, T* __restrict__
 // with zeros, x readable up to ld): a block of kDenseWarps warps per row, so
 // that a few thousand rows of 10 to 40 KB keep every SM's loads in flight;
 // 16-byte loads.  Fixed order: lanes, then warps.
+// The first entries of a row are loaded before the previous kernel is waited
+// for.
 constexpr int kDenseWarps = 4;
 template <class T>
 __global__ void __launch_bounds__(32 * kDenseWarps) dense_rows(int n, int ld, const T* __restrict__ A,
                                                                const T* __restrict__ b, T* __restrict__ x) {
-  pdl_begin();
-  constexpr int W = 16 / sizeof(T);
+  pdl_trigger();
+  constexpr int W = 16 / sizeof(T), step = 32 * kDenseWarps, ahead = 4;
   using V = typename std::conditional<std::is_same<T, float>::value, float4, double2>::type;
   __shared__ T part[kDenseWarps];
   const int i = blockIdx.x;
@@ -1116,11 +1147,23 @@ __global__ void __launch_bounds__(32 * kDenseWarps) dense_rows(int n, int ld, co
   const V* bb = reinterpret_cast<const V*>(b);
   T s = 0;
   const int nv = ld / W;
-#pragma unroll 4
-  for (int k = threadIdx.x; k < nv; k += 32 * kDenseWarps) {
-    const V p = a[k], q = bb[k];
-    if constexpr (W == 4) s += p.x * q.x + p.y * q.y + p.z * q.z + p.w * q.w;
-    else s += p.x * q.x + p.y * q.y;
+  V p[ahead];
+  auto entries = [&](int k0) {
+#pragma unroll
+    for (int u = 0; u < ahead; ++u) p[u] = k0 + u * step < nv ? a[k0 + u * step] : V{};
+  };
+  entries(threadIdx.x);
+  pdl_wait();
+  for (int k0 = threadIdx.x; k0 < nv; k0 += ahead * step) {
+    V q[ahead];
+#pragma unroll
+    for (int u = 0; u < ahead; ++u) q[u] = k0 + u * step < nv ? bb[k0 + u * step] : V{};
+#pragma unroll
+    for (int u = 0; u < ahead; ++u) {
+      if constexpr (W == 4) s += p[u].x * q[u].x + p[u].y * q[u].y + p[u].z * q[u].z + p[u].w * q[u].w;
+      else s += p[u].x * q[u].x + p[u].y * q[u].y;
+    }
+    entries(k0 + ahead * step);
   }
   s = warp_sum(s);
   if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
@@ -1520,15 +1563,17 @@ __global__ void sell_gs_color(int count, const int32_t* __restrict__ rows, Sell 
 // The restriction to a level of many rows: a warp a row, persistent, the next
 // row's entries (160 in one round; a row of the SA transfers has about 130)
 // loaded before the current row's gathers and sum.  At 1.23M cells in FP32 the
-// transfers of a V-cycle average 16.8 us, 17.8 with a lane group per row and
+// transfers of a V-cycle average 15.7 us, 17.8 with a lane group per row and
 // four entries of the prolongation ahead.
 constexpr int kRestAhead = 5;
 template <class T>
-__global__ void __launch_bounds__(kBlock, 4) restrict_stream(int nc, const int32_t* __restrict__ rr,
+constexpr int rest_blocks() { return sizeof(T) == 8 ? 4 : 6; }  // per SM
+template <class T>
+__global__ void __launch_bounds__(kBlock, rest_blocks<T>()) restrict_stream(int nc, const int32_t* __restrict__ rr,
                                                              const int32_t* __restrict__ rc, const T* __restrict__ rv,
                                                              const T* __restrict__ f, T* __restrict__ c,
                                                              const T* __restrict__ den0, T w0, T* __restrict__ x1) {
-  pdl_begin();
+  pdl_trigger();
   const int lane = threadIdx.x & 31, stride = gridDim.x * kWarps;
   int I = blockIdx.x * kWarps + (threadIdx.x >> 5);
   auto bounds = [&](int i) { return i < nc ? make_int2(rr[i], rr[i + 1]) : make_int2(0, 0); };
@@ -1544,6 +1589,7 @@ __global__ void __launch_bounds__(kBlock, 4) restrict_stream(int nc, const int32
   int j[kRestAhead];
   T v[kRestAhead];
   entries(j, v, cur);
+  pdl_wait();
   for (; I < nc; I += stride) {
     const int2 nn = bounds(I + 2 * stride);
     T x[kRestAhead];
@@ -1580,12 +1626,11 @@ __global__ void __launch_bounds__(kBlock) restrict_rows(int nc, const int32_t* _
                                                         const int32_t* __restrict__ rc, const T* __restrict__ rv,
                                                         const T* __restrict__ f, T* __restrict__ c,
                                                         const T* __restrict__ den0, T w0, T* __restrict__ x1) {
-  pdl_begin();
+  pdl_trigger();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int I = t / GL, lane = t % GL;
-  if (I >= nc) return;
-  const T s = group_row_dot<T, T, int32_t, GL>(rr, rc, rv, f, I, lane, group_mask<GL>());
-  if (lane == 0) {
+  const T s = group_row_dot<T, T, int32_t, GL>(rr, rc, rv, f, I, lane, group_mask<GL>(), I < nc);
+  if (I < nc && lane == 0) {
     c[I] = s;
     // with x1: the coarse pre-smoother's diagonal step w0 c / den0
     if (x1) x1[I] = w0 * s / den0[I];

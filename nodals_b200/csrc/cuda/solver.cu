@@ -1310,7 +1310,7 @@ class Solver final : public ISolver {
         }
       }
       if (lo < hi) win[(size_t)q] = make_int2(lo, hi);
-      most = std::max(most, hi - lo);
+      most = std::max(most, hi - lo + 4);  // staged from a 16-byte boundary
     }
     if ((size_t)most * sizeof(double) > kWinBytes) return;
     std::vector<int16_t> dc(A.col.size());
@@ -1612,7 +1612,7 @@ class Solver final : public ISolver {
       x1 = poly_first(pl, C.x.p, C.pong.p);
     }
     if (X.nc >= rest_rows_) {
-      const int g = std::min(grid_for(X.nc, kBlock / 32), 4 * kSms);
+      const int g = std::min(grid_for(X.nc, kBlock / 32), kSms * k::rest_blocks<TA>());
       pdl_launch(k::restrict_stream<TA>, g, kBlock, 0, st_, X.nc, X.rrow.p, X.rcol.p, X.rval.p, f, c, den0, TA(w0), x1);
     } else if (restrict_lanes() != 32) {
       auto run = [&](auto gl) {

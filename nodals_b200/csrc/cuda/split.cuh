@@ -101,14 +101,19 @@ struct SplitRaw<REC_8> {
 // by their latency when each group does one vertex (21 us at 1.23M cells in
 // FP16, 46 MB).  So the groups are persistent and pipelined: the offsets are
 // loaded two vertices ahead and the records one ahead, and a vertex waits
-// only for its gathers: 13.3 us so.
+// only for its gathers: 13.3 us so.  FP64 records keep one vertex's in
+// registers: with the next one's only two blocks fit an SM and the next kernel
+// cannot start early (40k cells: 62 us an iteration of the pressure loop
+// instead of 56).  The first records, constant during a solve, are loaded
+// before the wait for the kernel that writes x.
 constexpr int kSplitAhead = 4;
 template <int REC>
-constexpr int split_vertex_blocks() { return REC == REC_SOA ? 2 : REC == REC_16 ? 4 : 5; }  // per SM
+constexpr int split_vertex_blocks() { return REC == REC_SOA ? 3 : REC == REC_16 ? 4 : 5; }  // per SM
 template <class V, int REC>
 __global__ void __launch_bounds__(kBlock, split_vertex_blocks<REC>())
     split_vertex(SplitVerts a, const V* __restrict__ rau, const V* __restrict__ x, V* __restrict__ w, V scale) {
-  pdl_begin();
+  pdl_trigger();
+  constexpr bool PIPE = REC != REC_SOA;  // the next vertex's records in registers
   const int t = blockIdx.x * blockDim.x + threadIdx.x, stride = (gridDim.x * blockDim.x) >> 3;
   const int lane = t & 7;
   const unsigned mask = group8_mask();
@@ -135,14 +140,15 @@ __global__ void __launch_bounds__(kBlock, split_vertex_blocks<REC>())
   Off cur = offsets(g), nxt = offsets(g + stride);
   SplitRaw<REC> raw[kSplitAhead] = {};
   records(raw, cur);
-  for (; g < a.n; g += stride) {
+  pdl_wait();
+  while (g < a.n) {
     const Off nn = offsets(g + 2 * stride);
     SplitRaw<REC> rawn[kSplitAhead] = {};
     V xv[kSplitAhead];
 #pragma unroll
     for (int u = 0; u < kSplitAhead; ++u)
       xv[u] = cur.b + lane + 8 * u < cur.e ? x[raw[u].cell(cur.base)] : V(0);
-    records(rawn, nxt);
+    if (PIPE) records(rawn, nxt);
     V r = 0;
     if (lane == 0) r = scale * rau[g];
     V s0 = 0, s1 = 0, s2 = 0;
@@ -175,10 +181,15 @@ __global__ void __launch_bounds__(kBlock, split_vertex_blocks<REC>())
         w[4 * (size_t)g + 2] = r * s2;
       }
     }
+    g += stride;
     cur = nxt;
     nxt = nn;
+    if (PIPE) {
 #pragma unroll
-    for (int u = 0; u < kSplitAhead; ++u) raw[u] = rawn[u];
+      for (int u = 0; u < kSplitAhead; ++u) raw[u] = rawn[u];
+    } else if (g < a.n) {
+      records(raw, cur);
+    }
   }
 }
 
@@ -224,93 +235,125 @@ struct PlainVertices {
   }
 };
 
-// sum of cell c's row products: vertices from w, faces from x (xc = x(c))
-template <class V, class MT, bool D16, class X, class W>
-__device__ __forceinline__ V split_row(const SplitCells& a, const X& x, const W& w, int c, V xc, V tinv) {
-  const int4 vi = a.vid[c];
-  int nb[4];
-  if (D16) {
-    const short4 d = a.nd16[c];
-    nb[0] = d.x ? c + d.x : -1;
-    nb[1] = d.y ? c + d.y : -1;
-    nb[2] = d.z ? c + d.z : -1;
-    nb[3] = d.w ? c + d.w : -1;
-  } else {
-    const int4 d = a.nid[c];
-    nb[0] = d.x;
-    nb[1] = d.y;
-    nb[2] = d.z;
-    nb[3] = d.w;
+// A cell's data (constant during a solve) and its row's product
+template <class V, class MT>
+struct SplitGeo;
+template <class V>
+struct SplitGeo<V, __half> {
+  uint4 p;
+  uint2 q, th;
+  __device__ __forceinline__ void load(const SplitCells& a, int c) {
+    p = static_cast<const uint4*>(a.g0)[c];
+    q = static_cast<const uint2*>(a.g1)[c];
+    th = static_cast<const uint2*>(a.tau)[c];
   }
-  V t[4];
-  V s = 0;
-  if constexpr (std::is_same<MT, __half>::value) {
-    const uint2 th = static_cast<const uint2*>(a.tau)[c];
-    const uint4 p = static_cast<const uint4*>(a.g0)[c];
-    const uint2 q = static_cast<const uint2*>(a.g1)[c];
-    V wv[4][3];
-    w(vi.x, wv[0]);
-    w(vi.y, wv[1]);
-    w(vi.z, wv[2]);
-    w(vi.w, wv[3]);
-    V xn[4];
-#pragma unroll
-    for (int f = 0; f < 4; ++f) xn[f] = nb[f] >= 0 ? x(nb[f]) : V(0);
-    auto h2 = [](unsigned u) { return __half22float2(*reinterpret_cast<const __half2*>(&u)); };
+  static __device__ __forceinline__ float2 h2(unsigned u) { return __half22float2(*reinterpret_cast<const __half2*>(&u)); }
+  __device__ __forceinline__ void tau(V (&t)[4]) const {
+    const float2 t01 = h2(th.x), t23 = h2(th.y);
+    t[0] = t01.x; t[1] = t01.y; t[2] = t23.x; t[3] = t23.y;
+  }
+  __device__ __forceinline__ V vertices(const V (&wv)[4][3]) const {
     const float2 b01 = h2(p.x), b23 = h2(p.y), b45 = h2(p.z), b67 = h2(p.w), b89 = h2(q.x), bab = h2(q.y);
-    s = b01.x * wv[0][0] + b01.y * wv[0][1] + b23.x * wv[0][2];
+    V s = b01.x * wv[0][0] + b01.y * wv[0][1] + b23.x * wv[0][2];
     s += b23.y * wv[1][0] + b45.x * wv[1][1] + b45.y * wv[1][2];
     s += b67.x * wv[2][0] + b67.y * wv[2][1] + b89.x * wv[2][2];
     s += b89.y * wv[3][0] + bab.x * wv[3][1] + bab.y * wv[3][2];
-    const float2 t01 = h2(th.x), t23 = h2(th.y);
-    t[0] = t01.x;
-    t[1] = t01.y;
-    t[2] = t23.x;
-    t[3] = t23.y;
-    V f = 0;
+    return s;
+  }
+};
+// the vertices enter by the gradients of 1, 2, 3: sum_j S_j . (w_j - w_0)
+template <class V>
+__device__ __forceinline__ V split_gradients(const V (&b)[9], const V (&wv)[4][3]) {
+  V s = 0;
 #pragma unroll
-    for (int q4 = 0; q4 < 4; ++q4) f += t[q4] * (xc - xn[q4]);
-    s += tinv * f;
-  } else {
-    V b[9], wv[4][3];
-    if constexpr (std::is_same<V, float>::value) {
-      const float4 p = static_cast<const float4*>(a.g0)[c], q = static_cast<const float4*>(a.g1)[c];
-      b[0] = p.x; b[1] = p.y; b[2] = p.z; b[3] = p.w;
-      b[4] = q.x; b[5] = q.y; b[6] = q.z; b[7] = q.w;
-      b[8] = static_cast<const float*>(a.g2)[c];
-      const float4 tt = static_cast<const float4*>(a.tau)[c];
-      t[0] = tt.x; t[1] = tt.y; t[2] = tt.z; t[3] = tt.w;
+  for (int j = 0; j < 3; ++j)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) s += b[3 * j + d] * (wv[j + 1][d] - wv[0][d]);
+  return s;
+}
+template <>
+struct SplitGeo<float, float> {
+  float4 p, q, tt;
+  float l;
+  __device__ __forceinline__ void load(const SplitCells& a, int c) {
+    p = static_cast<const float4*>(a.g0)[c];
+    q = static_cast<const float4*>(a.g1)[c];
+    l = static_cast<const float*>(a.g2)[c];
+    tt = static_cast<const float4*>(a.tau)[c];
+  }
+  __device__ __forceinline__ void tau(float (&t)[4]) const {
+    t[0] = tt.x; t[1] = tt.y; t[2] = tt.z; t[3] = tt.w;
+  }
+  __device__ __forceinline__ float vertices(const float (&wv)[4][3]) const {
+    const float b[9] = {p.x, p.y, p.z, p.w, q.x, q.y, q.z, q.w, l};
+    return split_gradients(b, wv);
+  }
+};
+template <>
+struct SplitGeo<double, double> {
+  double2 g[4], ta, tb;
+  double l;
+  __device__ __forceinline__ void load(const SplitCells& a, int c) {
+    const double2* gp = static_cast<const double2*>(a.g0);
+    const ptrdiff_t n = a.n;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) g[k] = gp[k * n + c];
+    l = static_cast<const double*>(a.g2)[c];
+    const double2* tp = static_cast<const double2*>(a.tau) + 2 * (ptrdiff_t)c;
+    ta = tp[0];
+    tb = tp[1];
+  }
+  __device__ __forceinline__ void tau(double (&t)[4]) const {
+    t[0] = ta.x; t[1] = ta.y; t[2] = tb.x; t[3] = tb.y;
+  }
+  __device__ __forceinline__ double vertices(const double (&wv)[4][3]) const {
+    const double b[9] = {g[0].x, g[0].y, g[1].x, g[1].y, g[2].x, g[2].y, g[3].x, g[3].y, l};
+    return split_gradients(b, wv);
+  }
+};
+template <class V, class MT, bool D16>
+struct SplitRow {
+  int4 vi;
+  int nb[4];
+  SplitGeo<V, MT> geo;
+  __device__ __forceinline__ void load(const SplitCells& a, int c) {
+    vi = a.vid[c];
+    if (D16) {
+      const short4 d = a.nd16[c];
+      nb[0] = d.x ? c + d.x : -1;
+      nb[1] = d.y ? c + d.y : -1;
+      nb[2] = d.z ? c + d.z : -1;
+      nb[3] = d.w ? c + d.w : -1;
     } else {
-      const double2* g = static_cast<const double2*>(a.g0);
-      const ptrdiff_t n = a.n;
-#pragma unroll
-      for (int q4 = 0; q4 < 4; ++q4) {
-        const double2 p = g[q4 * n + c];
-        b[2 * q4] = p.x;
-        b[2 * q4 + 1] = p.y;
-      }
-      b[8] = static_cast<const double*>(a.g2)[c];
-      const double2* tp = static_cast<const double2*>(a.tau) + 2 * (ptrdiff_t)c;
-      const double2 ta = tp[0], tb = tp[1];
-      t[0] = ta.x; t[1] = ta.y; t[2] = tb.x; t[3] = tb.y;
+      const int4 d = a.nid[c];
+      nb[0] = d.x; nb[1] = d.y; nb[2] = d.z; nb[3] = d.w;
     }
+    geo.load(a, c);
+  }
+  // vertices from w, faces from x (xc = x(c))
+  template <class X, class W>
+  __device__ __forceinline__ V product(const X& x, const W& w, V xc, V tinv) const {
+    V wv[4][3], xn[4], t[4];
     w(vi.x, wv[0]);
     w(vi.y, wv[1]);
     w(vi.z, wv[2]);
     w(vi.w, wv[3]);
-    V xn[4];
 #pragma unroll
     for (int f = 0; f < 4; ++f) xn[f] = nb[f] >= 0 ? x(nb[f]) : V(0);
-#pragma unroll
-    for (int j = 0; j < 3; ++j)
-#pragma unroll
-      for (int d = 0; d < 3; ++d) s += b[3 * j + d] * (wv[j + 1][d] - wv[0][d]);
+    const V s = geo.vertices(wv);
+    geo.tau(t);
     V f = 0;
 #pragma unroll
-    for (int q4 = 0; q4 < 4; ++q4) f += t[q4] * (xc - xn[q4]);
-    s += f;
+    for (int k = 0; k < 4; ++k) f += t[k] * (xc - xn[k]);
+    if constexpr (std::is_same<MT, __half>::value) return s + tinv * f;
+    else return s + f;
   }
-  return s;
+};
+template <class V, class MT, bool D16, class X, class W>
+__device__ __forceinline__ V split_row(const SplitCells& a, const X& x, const W& w, int c, V xc, V tinv) {
+  SplitRow<V, MT, D16> r;
+  r.load(a, c);
+  return r.product(x, w, xc, tinv);
 }
 
 // The modes Y, RESID and SMOOTH of sell_spmv on the split form (w from
@@ -323,17 +366,20 @@ __global__ void __launch_bounds__(kBlock) split_cell(SplitCells a, const V* __re
                                                      V* __restrict__ y, V* __restrict__ y2, V tinv,
                                                      const R* __restrict__ rr, ReduceTail tail,
                                                      const int* __restrict__ at) {
-  pdl_begin();
+  pdl_trigger();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   double acc = 0.0;
+  SplitRow<V, MT, D16> row;
+  V dc = 1;
+  if (c < a.n) {
+    row.load(a, c);
+    if (MODE == SELL_SMOOTH || (MODE == SELL_RESID && den)) dc = den[c];
+  }
+  pdl_wait();
   if (c < a.n) {
     const V xc = x[c];
-    V bc = 0, dc = 1;
-    if (MODE != SELL_Y) {
-      bc = b[c];
-      if (MODE == SELL_SMOOTH || den) dc = den[c];
-    }
-    const V s = split_row<V, MT, D16>(a, PlainVector<V>{x}, PlainVertices<V>{w}, c, xc, tinv);
+    const V bc = MODE != SELL_Y ? b[c] : V(0);
+    const V s = row.product(PlainVector<V>{x}, PlainVertices<V>{w}, xc, tinv);
     if (MODE == SELL_Y) {
       y[c] = s;
       if (y2) y2[(size_t)at[0] * a.n + c] = xc;
@@ -361,13 +407,19 @@ template <class V, bool D16>
 __global__ void __launch_bounds__(kBlock) split_cell_dot(SplitCells a, const V* __restrict__ w,
                                                          const V* __restrict__ p, V* __restrict__ q, V tinv,
                                                          ReduceTail tail) {
-  pdl_begin();
+  pdl_trigger();
   double acc = 0.0;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < a.n; c += gridDim.x * blockDim.x) {
+  int c = blockIdx.x * blockDim.x + threadIdx.x;
+  SplitRow<V, V, D16> row;
+  if (c < a.n) row.load(a, c);
+  pdl_wait();
+  while (c < a.n) {
     const V pc = p[c];
-    const V s = split_row<V, V, D16>(a, PlainVector<V>{p}, PlainVertices<V>{w}, c, pc, tinv);
+    const V s = row.product(PlainVector<V>{p}, PlainVertices<V>{w}, pc, tinv);
     q[c] = s;
     acc += (double)pc * (double)s;
+    c += gridDim.x * blockDim.x;
+    if (c < a.n) row.load(a, c);
   }
   reduce_tail<PCG_ALPHA>(acc, tail);
 }

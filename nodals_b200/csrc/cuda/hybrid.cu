@@ -1079,6 +1079,78 @@ __global__ void amg_cheb_add(int n, double w, const double* bs, const double* Hy
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) y[i] += w * (bs[i] - Hy[i]);
 }
+// Products of a level fused with the vector steps around them (the V-cycle of
+// a few ten thousand rows is launches: a smoother call of degree 2 took seven
+// kernels of 3 us, a residual two).  L lanes a row, eight entries in flight
+// per lane.
+template <int L>
+__device__ __forceinline__ double amg_row(int i, int lane, const int32_t* __restrict__ row,
+                                          const int32_t* __restrict__ col, const double* __restrict__ val,
+                                          const double* __restrict__ x) {
+  double s = 0;
+  const int e = row[i + 1];
+  for (int k0 = row[i] + lane; k0 < e; k0 += 8 * L) {
+    int c[8];
+    double a[8], v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int k = k0 + u * L;
+      c[u] = k < e ? col[k] : -1;
+      a[u] = k < e ? val[k] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = c[u] >= 0 ? x[c[u]] : 0.0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) s += a[u] * v[u];
+  }
+  return s;
+}
+// symmetric Chebyshev on D^-1/2 A D^-1/2, first step: bs = b / sqrt(d),
+// y = w bs, x = y / sqrt(d)
+__global__ void amg_cheb_first(int n, double w, const double* __restrict__ b, const double* __restrict__ d,
+                               double* __restrict__ bs, double* __restrict__ y, double* __restrict__ x) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double q = sqrt(d[i]), s = b[i] / q, yi = w * s;
+  bs[i] = s;
+  y[i] = yi;
+  x[i] = yi / q;
+}
+// a further step: y += w (bs - (A x) / sqrt(d)), xo = y / sqrt(d); with
+// add_to the result is added to add_to instead of stored in xo
+template <int L>
+__global__ void __launch_bounds__(kTPB) amg_cheb_step(int n, const int32_t* __restrict__ row,
+                                                      const int32_t* __restrict__ col, const double* __restrict__ val,
+                                                      double w, const double* __restrict__ x,
+                                                      const double* __restrict__ bs, const double* __restrict__ d,
+                                                      double* __restrict__ y, double* __restrict__ xo,
+                                                      double* __restrict__ add_to) {
+  const long long gt = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const int i = (int)(gt / L), lane = (int)(gt % L);
+  const bool live = i < n;
+  double s = live ? amg_row<L>(i, lane, row, col, val, x) : 0.0;
+  s = group_sum<L>(s);
+  if (live && lane == 0) {
+    const double q = sqrt(d[i]), yi = y[i] + w * (bs[i] - s / q);
+    y[i] = yi;
+    if (add_to) add_to[i] += yi / q;
+    else xo[i] = yi / q;
+  }
+}
+// r = b - A x
+template <int L>
+__global__ void __launch_bounds__(kTPB) amg_residual(int n, const int32_t* __restrict__ row,
+                                                     const int32_t* __restrict__ col, const double* __restrict__ val,
+                                                     const double* __restrict__ x, const double* __restrict__ b,
+                                                     double* __restrict__ r) {
+  const long long gt = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const int i = (int)(gt / L), lane = (int)(gt % L);
+  const bool live = i < n;
+  double s = live ? amg_row<L>(i, lane, row, col, val, x) : 0.0;
+  s = group_sum<L>(s);
+  if (live && lane == 0) r[i] = b[i] - s;
+}
+
 // one colour of a Gauss-Seidel sweep, one warp per row
 __global__ void amg_gs_colour(int count, const int32_t* __restrict__ rows, const int32_t* __restrict__ row,
                               const int32_t* __restrict__ col, const double* __restrict__ val,
@@ -1106,9 +1178,7 @@ __global__ void amg_csr_add(int n, const int32_t* __restrict__ row, const int32_
   const long long gt = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const int i = (int)(gt / L), lane = (int)(gt % L);
   const bool live = i < n;
-  double s = 0;
-  if (live)
-    for (int k = row[i] + lane; k < row[i + 1]; k += L) s += val[k] * x[col[k]];
+  double s = live ? amg_row<L>(i, lane, row, col, val, x) : 0.0;
   s = group_sum<L>(s);
   if (live && lane == 0) y[i] = accumulate ? y[i] + s : s;
 }
@@ -1191,6 +1261,11 @@ struct AmgLevel {
     amg_csr_add<32><<<grid((long long)n * 32), kTPB>>>(n, row.p, col.p, val.p, in, out, 0);
     NDS_LAUNCH();
   }
+  // out = b - A in
+  void residual_to(const double* in, const double* rhs, double* out) const {
+    amg_residual<32><<<grid((long long)n * 32), kTPB>>>(n, row.p, col.p, val.p, in, rhs, out);
+    NDS_LAUNCH();
+  }
 };
 struct AmgTransfer {
   int nf, nc;
@@ -1255,6 +1330,30 @@ struct HybridAmgDevice {
     const double centre = 0.5 * (hi + lo), radius = 0.5 * (hi - lo), pi = 3.141592653589793238462643383279502884;
     return centre - radius * std::cos(pi * (2.0 * k + 1.0) / (2.0 * degree));
   }
+  // the Chebyshev smoother with work vectors that do not alias: x = S b, or
+  // add_to += S b.  y and bs hold the scaled iterate and right-hand side, t
+  // the second buffer of the unscaled iterate.
+  void cheb_fused(AmgLevel& A, const double* b, double* x, double* t, double* bs, double* y, double lambda,
+                  double* add_to) {
+    const int n = A.n, deg = o.amg_cheb_degree;
+    const double lo = o.amg_lambda_low_fraction * lambda;
+    if (!(lambda > lo && lo > 0)) throw std::runtime_error("AMG Chebyshev interval invalid");
+    double* cur = deg % 2 == 1 ? x : t;  // the last step writes x
+    double* nxt = cur == x ? t : x;
+    amg_cheb_first<<<grid(n), kTPB>>>(n, 1.0 / cheb_root(lambda, lo, 0, deg), b, A.diag.p, bs, y, cur);
+    for (int k = 1; k < deg; ++k) {
+      amg_cheb_step<32><<<grid((long long)n * 32), kTPB>>>(n, A.row.p, A.col.p, A.val.p,
+                                                           1.0 / cheb_root(lambda, lo, k, deg), cur, bs, A.diag.p, y,
+                                                           nxt, k + 1 == deg ? add_to : nullptr);
+      std::swap(cur, nxt);
+    }
+    if (deg == 1 && add_to) amg_axpy<<<grid(n), kTPB>>>(n, x, add_to);
+    NDS_LAUNCH();
+  }
+  // the calls whose work vectors are distinct: every pre-smoothing, and the
+  // post-smoothing with amg_separate_post
+  bool fused(bool post) const { return o.amg_smoother == NDS_SM_CHEB2 && (!post || o.amg_separate_post); }
+
   // zero initial guess: x = S b.  The work vectors are passed as the
   // reference passes them (hybrid_amg.cuh:445-506): its post-smoothing calls
   // hand the same vector as x and corr (and, on the fine level, as b and r),
@@ -1311,15 +1410,24 @@ struct HybridAmgDevice {
   }
   // post = true: the post-smoothing call; with amg_separate_post it gets work
   // vectors of its own, which makes the V-cycle symmetric
-  void smooth_fine(const double* b, double* x, bool post = false) {
+  void smooth_fine(const double* b, double* x, bool post = false, double* add_to = nullptr) {
     AmgLevel& F = *fine;
     const bool sep = post && o.amg_separate_post;
+    if (fused(post)) {
+      cheb_fused(F, b, x, F.tmp.p, sep ? F.r2.p : F.r.p, sep ? F.corr2.p : F.corr.p, fine_lambda, add_to);
+      return;
+    }
     smooth(F, b, x, F.tmp.p, sep ? F.r2.p : F.r.p, sep ? F.corr2.p : F.corr.p,
            o.amg_smoother == NDS_SM_MCGS ? o.amg_mcgs_fine_sweeps : o.amg_jacobi_fine_sweeps, fine_lambda);
   }
-  void smooth_coarse(size_t l, const double* b, double* x, bool post = false) {
+  void smooth_coarse(size_t l, const double* b, double* x, bool post = false, double* add_to = nullptr) {
     AmgLevel& A = *L[l];
     const bool sep = post && o.amg_separate_post;
+    if (fused(post)) {
+      cheb_fused(A, b, x, A.tmp.p, sep ? A.r2.p : A.r.p, sep ? A.corr2.p : A.corr.p,
+                 l < level_lambda.size() ? level_lambda[l] : 0.0, add_to);
+      return;
+    }
     smooth(A, b, x, A.tmp.p, sep ? A.r2.p : A.r.p, sep ? A.corr2.p : A.corr.p,
            o.amg_smoother == NDS_SM_MCGS ? o.amg_mcgs_coarse_sweeps : o.amg_jacobi_coarse_sweeps,
            l < level_lambda.size() ? level_lambda[l] : 0.0);
@@ -1332,14 +1440,16 @@ struct HybridAmgDevice {
       return;
     }
     smooth_coarse(l, b, x);
-    A.apply(x, A.tmp.p);
-    residual<<<grid(A.n), kTPB>>>(A.n, b, A.tmp.p, A.r.p);
+    A.residual_to(x, b, A.r.p);
     AmgLevel& Cn = *L[l + 1];
     P[l + 1]->restrict_to(A.r.p, Cn.b.p);
     vcycle(l + 1, Cn.b.p, Cn.x.p);
     P[l + 1]->prolong_add(Cn.x.p, x);
-    A.apply(x, A.tmp.p);
-    residual<<<grid(A.n), kTPB>>>(A.n, b, A.tmp.p, A.r.p);
+    A.residual_to(x, b, A.r.p);
+    if (fused(true)) {
+      smooth_coarse(l, A.r.p, A.corr.p, true, x);
+      return;
+    }
     NDS_CUDA(cudaMemcpyAsync(A.b.p, A.r.p, (size_t)A.n * sizeof(double), cudaMemcpyDeviceToDevice));
     smooth_coarse(l, A.b.p, A.corr.p, true);
     amg_axpy<<<grid(A.n), kTPB>>>(A.n, A.corr.p, x);
@@ -1349,14 +1459,16 @@ struct HybridAmgDevice {
   void apply(const double* b, double* z) {
     AmgLevel& F = *fine;
     smooth_fine(b, z);
-    F.apply(z, F.tmp.p);
-    residual<<<grid(F.n), kTPB>>>(F.n, b, F.tmp.p, F.r.p);
+    F.residual_to(z, b, F.r.p);
     AmgLevel& C0 = *L[0];
     P[0]->restrict_to(F.r.p, C0.b.p);
     vcycle(0, C0.b.p, C0.x.p);
     P[0]->prolong_add(C0.x.p, z);
-    F.apply(z, F.tmp.p);
-    residual<<<grid(F.n), kTPB>>>(F.n, b, F.tmp.p, F.r.p);
+    F.residual_to(z, b, F.r.p);
+    if (fused(true)) {
+      smooth_fine(F.r.p, F.corr.p, true, z);
+      return;
+    }
     smooth_fine(F.r.p, F.corr.p, true);
     amg_axpy<<<grid(F.n), kTPB>>>(F.n, F.corr.p, z);
     NDS_LAUNCH();

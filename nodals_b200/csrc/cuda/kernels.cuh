@@ -889,6 +889,38 @@ __global__ void p_update_dev(int n, const double* __restrict__ beta_dev, const i
   if (i >= n) return;
   p[i] = ctl[2] ? T(z[i]) : T(z[i]) + T(*beta_dev) * p[i];
 }
+// A loop's end state written straight to page-locked host memory (the host
+// reads it after it has waited for the stream), instead of three copies of a
+// few bytes behind the loop.
+struct HostWords {
+  double* rn2;  // ||r||^2
+  int* words;   // [0] flags, [4] iterations, [5] converged, [7] cap
+  __device__ __forceinline__ void put(int it, int conv, int cap, int flags, double v) const {
+    words[0] = flags;
+    words[4] = it;
+    words[5] = conv;
+    words[7] = cap;
+    *rn2 = v;
+    __threadfence_system();
+  }
+};
+// the scalars a solve starts from, set by its first kernel
+struct SolveInit {
+  double* sc;
+  int* ctl;
+  int* flags;
+  int r0_slot, target_slot, first, cap;
+  double r0, target;
+  __device__ __forceinline__ void set() const {
+    sc[r0_slot] = r0;
+    sc[target_slot] = target;
+    ctl[0] = 0;
+    ctl[1] = 0;
+    ctl[2] = first;
+    ctl[3] = cap;
+    *flags = 0;
+  }
+};
 // End of the loop body: count the iteration and test ||r|| <= target the way
 // the host loop does (sqrt, then compare); stop on convergence, on any flag
 // or at max_its.  The loop always ends: every body pass runs this kernel and
@@ -897,7 +929,8 @@ __global__ void p_update_dev(int n, const double* __restrict__ beta_dev, const i
 // launched outside a graph (host-driven loop), no condition to set.
 __device__ __forceinline__ void pcg_check_step(const double* __restrict__ sc, int rn2_slot, int r0_slot,
                                                int target_slot, int* __restrict__ flags, int* __restrict__ ctl,
-                                               int max_its, cudaGraphConditionalHandle loop, int in_graph) {
+                                               int max_its, cudaGraphConditionalHandle loop, int in_graph,
+                                               const HostWords& host) {
   if (max_its < 0) max_its = ctl[3];
   const int it = ++ctl[0];
   ctl[2] = 0;
@@ -907,12 +940,13 @@ __device__ __forceinline__ void pcg_check_step(const double* __restrict__ sc, in
   ctl[1] = conv;
   const bool stop = conv || *flags != 0 || it >= max_its;
   if (in_graph) cudaGraphSetConditional(loop, stop ? 0u : 1u);
+  if (stop || !in_graph) host.put(it, conv, ctl[3], *flags, sc[rn2_slot]);
 }
 // A reduction of one value's block partials (as reduce_partials<1>) whose
 // thread 0 then takes the next scalar step of the device PCG: rho and beta
 // (PCG_RHO), alpha (PCG_ALPHA) or the stopping test (PCG_CHECK).  One launch
 // instead of two; the same sums and the same scalar arithmetic.
-enum { PCG_RHO = 1, PCG_ALPHA = 2, PCG_CHECK = 3 };
+enum { PCG_RHO = 1, PCG_ALPHA = 2, PCG_CHECK = 3, SUM_ONLY = 4 };
 struct PcgScalars {
   double* sc;
   int* flags;
@@ -920,6 +954,7 @@ struct PcgScalars {
   int rn2_slot, r0_slot, target_slot, max_its;
   cudaGraphConditionalHandle loop;
   int in_graph;
+  HostWords host;
 };
 template <int STEP>
 __global__ void reduce_pcg(const double* __restrict__ part, int nblocks, double* __restrict__ out, PcgScalars s) {
@@ -931,7 +966,7 @@ __global__ void reduce_pcg(const double* __restrict__ part, int nblocks, double*
     out[0] = v[0];
     if (STEP == PCG_RHO) pcg_rho_step(s.sc, s.flags, s.ctl);
     else if (STEP == PCG_ALPHA) pcg_alpha_step(s.sc, s.flags);
-    else pcg_check_step(s.sc, s.rn2_slot, s.r0_slot, s.target_slot, s.flags, s.ctl, s.max_its, s.loop, s.in_graph);
+    else pcg_check_step(s.sc, s.rn2_slot, s.r0_slot, s.target_slot, s.flags, s.ctl, s.max_its, s.loop, s.in_graph, s.host);
   }
 }
 
@@ -968,9 +1003,9 @@ __device__ __forceinline__ void reduce_tail(double value, const ReduceTail& t) {
     t.out[0] = v[0];
     if (STEP == PCG_RHO) pcg_rho_step(t.ps.sc, t.ps.flags, t.ps.ctl);
     else if (STEP == PCG_ALPHA) pcg_alpha_step(t.ps.sc, t.ps.flags);
-    else
+    else if (STEP == PCG_CHECK)
       pcg_check_step(t.ps.sc, t.ps.rn2_slot, t.ps.r0_slot, t.ps.target_slot, t.ps.flags, t.ps.ctl, t.ps.max_its,
-                     t.ps.loop, t.ps.in_graph);
+                     t.ps.loop, t.ps.in_graph, t.ps.host);
   }
 }
 
@@ -983,6 +1018,41 @@ __global__ void __launch_bounds__(kBlock) dot_step(int n, const T* __restrict__ 
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     acc += (double)x[i] * (double)y[i];
   reduce_tail<STEP>(acc, tail);
+}
+
+// Start of a pressure solve: r = b, x = 0, and ||b||^2 (SUM_ONLY tail)
+template <class T>
+__global__ void __launch_bounds__(kBlock) solve_start(int n, const T* __restrict__ b, T* __restrict__ r,
+                                                      T* __restrict__ x, ReduceTail tail) {
+  pdl_begin();
+  double acc = 0.0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const T v = b[i];
+    r[i] = v;
+    x[i] = T(0);
+    acc += (double)v * (double)v;
+  }
+  reduce_tail<SUM_ONLY>(acc, tail);
+}
+// Start of a Krylov loop from the residual r: the loop's scalars; with rs the
+// scaled residual rs = s r in precision S (and rs2 = rs), with x zero = 0;
+// with rA the residual in the preconditioner's precision, and with x1 the
+// first (diagonal) step of its fine pre-smoother on it, x1 = w0 r / den0.
+template <class R, class S, class TA>
+__global__ void loop_start(int n, const R* __restrict__ r, double s, S* __restrict__ rs, S* __restrict__ rs2,
+                           S* __restrict__ x, TA* __restrict__ rA, const TA* __restrict__ den0, TA w0,
+                           TA* __restrict__ x1, SolveInit init) {
+  pdl_begin();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) init.set();
+  if (i >= n) return;
+  const S v = rs ? (S)(s * (double)r[i]) : (S)r[i];
+  if (rs) rs[i] = v;
+  if (rs2) rs2[i] = v;
+  if (x) x[i] = S(0);
+  const TA a = TA(v);
+  if (rA) rA[i] = a;
+  if (x1) x1[i] = w0 * a / den0[i];
 }
 
 // x += a p; r -= a q; partial r.r.  a = alpha_dev ? *alpha_dev : alpha.

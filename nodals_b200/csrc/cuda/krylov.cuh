@@ -24,21 +24,6 @@
 namespace nds {
 namespace k {
 
-// y = float(s x)
-// y = s x in FP32; with x1 also the first (diagonal) step of the fine
-// pre-smoother on y, x1 = w0 y / den0 (the expression of jacobi_zero)
-// and with y2 also y2 = y
-__global__ void scale_to_float(int n, const double* __restrict__ x, double s, float* __restrict__ y,
-                               const float* __restrict__ den0 = nullptr, float w0 = 0.f, float* __restrict__ x1 = nullptr,
-                               float* __restrict__ y2 = nullptr) {
-  pdl_begin();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float v = (float)(s * x[i]);
-  y[i] = v;
-  if (y2) y2[i] = v;
-  if (x1) x1[i] = w0 * v / den0[i];
-}
 // x += s y (y in FP32, x in FP64)
 __global__ void axpy_from_float(int n, double s, const float* __restrict__ y, double* __restrict__ x) {
   pdl_begin();
@@ -82,6 +67,7 @@ struct FgScalars {
   int* flags;
   cudaGraphConditionalHandle loop;
   int in_graph;
+  HostWords host;
 };
 __device__ __forceinline__ void fg_givens(double* __restrict__ fg, const FgLayout& L, const FgScalars& p) {
   double* const sc = p.sc;
@@ -125,6 +111,7 @@ __device__ __forceinline__ void fg_givens(double* __restrict__ fg, const FgLayou
   ctl[1] = conv;
   const bool stop = conv || bad || j + 1 >= ctl[3];
   if (in_graph) cudaGraphSetConditional(loop, stop ? 0u : 1u);
+  if (stop || !in_graph) p.host.put(j + 1, conv, ctl[3], *flags, sc[wn2_slot]);
 }
 // H[i][j] = V_i . w for i <= j = ctl[0]: blockIdx.y takes the vectors y, y +
 // gridDim.y, ...; each vector's block partials (part[i gridDim.x + block]) are
@@ -210,13 +197,9 @@ __global__ void fg_normalize(int n, const float* __restrict__ w, const double* _
   in[i] = v;
   if (x1) x1[i] = w0 * v / den0[i];
 }
-// start of a pass: g = (1, 0, ...), j = 0
-__global__ void fg_start(double* __restrict__ fg, FgLayout L, int* __restrict__ ctl, int cap) {
-  for (int q = 0; q <= L.m; ++q) fg[L.g(q)] = 0.0;
-  fg[L.g(0)] = 1.0;
-  ctl[0] = 0;
-  ctl[1] = 0;
-  ctl[3] = cap;
+// start of a pass: g = (1, 0, ...) (the loop's scalars: loop_start)
+__global__ void fg_start(double* __restrict__ fg, FgLayout L) {
+  for (int q = 0; q <= L.m; ++q) fg[L.g(q)] = q == 0 ? 1.0 : 0.0;
 }
 // y = R^-1 g over the k = ctl[0] columns built (back substitution, FP64)
 __global__ void fg_backsolve(double* __restrict__ fg, FgLayout L, const int* __restrict__ ctl) {
@@ -277,16 +260,19 @@ __global__ void __launch_bounds__(kBlock) guess_dots(int n, const double* __rest
   }
   write_partials<NG>(acc, part);
 }
-// x = sum c_a y_a (c in coef[0..K))
+// x = sum c_a y_a
 template <int K>
-__global__ void guess_combine(int n, const double* __restrict__ Y, const double* __restrict__ coef,
-                              double* __restrict__ x) {
+struct GuessCoef {
+  double c[K];
+};
+template <int K>
+__global__ void guess_combine(int n, const double* __restrict__ Y, GuessCoef<K> coef, double* __restrict__ x) {
   pdl_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double xs = 0.0;
 #pragma unroll
-  for (int a = 0; a < K; ++a) xs += coef[a] * Y[(size_t)a * n + i];
+  for (int a = 0; a < K; ++a) xs += coef.c[a] * Y[(size_t)a * n + i];
   x[i] = xs;
 }
 // the stored product of a new correction: w = b - r (= A x for r = b - A x)

@@ -74,6 +74,7 @@ struct Resident {
   int r0_slot, target_slot;
   int* flags;
   int* ctl;                  // [0] iterations, [1] converged out; [3] cap in
+  HostWords host;
 };
 // floor(2^32 / chunk) + 1: umulhi(i, .) = i / chunk for i chunk < 2^32
 inline unsigned res_inverse(int chunk) { return (unsigned)(0x100000000ull / (unsigned)chunk + 1); }
@@ -577,6 +578,7 @@ __global__ void __launch_bounds__(kResBlock, 1) __cluster_dims__(kResCluster, 1,
     a.ctl[1] = conv;
     a.ctl[2] = 0;
     *a.flags = flags;
+    a.host.put(its, conv, cap, flags, rn2);
   }
   cluster_sync();  // no block leaves while another may still read its memory
 }

@@ -1065,22 +1065,33 @@ class Solver final : public ISolver {
   // reduction of one value into sc[slot], then the PCG scalar step STEP
   template <int STEP>
   void reduce_pcg(int nblocks, int slot, int max_its = 0, cudaGraphConditionalHandle h = {}, int in_graph = 1) {
-    const k::PcgScalars ps{sc_.p, flags_.p, ctl_.p, S_RN2, S_R0, S_TARGET, max_its, h, in_graph};
+    const k::PcgScalars ps{sc_.p, flags_.p, ctl_.p, S_RN2, S_R0, S_TARGET, max_its, h, in_graph, host_words()};
     pdl_launch(k::reduce_pcg<STEP>, 1, kBlock, 0, st_, part_.p, nblocks, sc_.p + slot, ps);
     NDS_LAUNCH();
   }
-  void fetch(int first, int count) {
-    NDS_CUDA(cudaMemcpyAsync(hsc_ + first, sc_.p + first, sizeof(double) * count, cudaMemcpyDeviceToHost, st_));
-    NDS_CUDA(cudaStreamSynchronize(st_));
+  // a sum that the host needs: the reduction writes it to page-locked memory
+  k::ReduceTail host_tail(int slot) {
+    k::ReduceTail t = tail(slot);
+    t.out = hsc_ + slot;
+    return t;
   }
   template <class V>
   double dot_fetch(const V* x, const V* y, int n, int slot) {
-    const int g = red_grid(n);
-    pdl_launch(k::dot<V>, g, kBlock, 0, st_, n, x, y, part_.p);
+    pdl_launch(k::dot_step<V, V, k::SUM_ONLY>, red_grid(n), kBlock, 0, st_, n, x, y, host_tail(slot));
     NDS_LAUNCH();
-    reduce_to<1>(g, slot);
-    fetch(slot, 1);
+    NDS_CUDA(cudaStreamSynchronize(st_));
     return hsc_[slot];
+  }
+  // block partials in part summed straight into hsc_[slot ..]
+  template <int NV>
+  void reduce_host(const double* part, int nblocks, int slot) {
+    pdl_launch(k::reduce_partials<NV>, 1, kBlock, 0, st_, part, nblocks, hsc_ + slot);
+    NDS_LAUNCH();
+    NDS_CUDA(cudaStreamSynchronize(st_));
+  }
+  k::HostWords host_words() const { return k::HostWords{hsc_ + S_RN2, hflags_}; }
+  k::SolveInit solve_init(double target, double r0, int first, int cap) const {
+    return k::SolveInit{sc_.p, ctl_.p, flags_.p, S_R0, S_TARGET, first, cap, r0, target};
   }
   template <class V>
   void dot_dev(const V* x, const V* y, int n, int slot) {
@@ -1182,7 +1193,7 @@ class Solver final : public ISolver {
   // a reduction into sc[slot] taken by the producing kernel's last block
   k::ReduceTail tail(int slot, cudaGraphConditionalHandle h = {}) {
     return k::ReduceTail{tailpart_.p, ticket_.p, sc_.p + slot,
-                         k::PcgScalars{sc_.p, flags_.p, ctl_.p, S_RN2, S_R0, S_TARGET, -1, h, in_graph_}};
+                         k::PcgScalars{sc_.p, flags_.p, ctl_.p, S_RN2, S_R0, S_TARGET, -1, h, in_graph_, host_words()}};
   }
   template <int MODE, class V>
   void sell_launch(const OpView<V>& A, int grid, const V* x, const V* b, const V* den, double w, V* y, V* y2) {
@@ -1917,9 +1928,10 @@ class Solver final : public ISolver {
   };
   // ||r0|| and the zero solution
   double p_start(const T* rhs) {
-    x_.zero(st_);
-    vcopy(nc_, rhs, r_.p);
-    const double r0 = std::sqrt(dot_fetch(r_.p, r_.p, nc_, S_TMP));
+    pdl_launch(k::solve_start<T>, red_grid(nc_), kBlock, 0, st_, nc_, rhs, r_.p, x_.p, host_tail(S_TMP));
+    NDS_LAUNCH();
+    NDS_CUDA(cudaStreamSynchronize(st_));
+    const double r0 = std::sqrt(hsc_[S_TMP]);
     if (!std::isfinite(r0)) throw SolveFailure(NDS_E_BREAKDOWN, "pressure initial norm nonfinite");
     return r0;
   }
@@ -1938,20 +1950,28 @@ class Solver final : public ISolver {
   // the PCG loops take the fine pre-smoother's first step in the kernels that
   // produce r (plain V-cycle with a polynomial smoother only)
   bool pre_fused() const { return !stage_ && o_.amg_smoother != NDS_SM_MCGS; }
-  // the pre-smoother's first step on the initial residual
+  // start of a PCG loop from the residual in v.r, or (from given) from s times
+  // the FP64 residual `from`, scaled into v.r with v.x zeroed
   template <class S>
-  void pcg_first(const PcgVecs<S>& v) {
-    if constexpr (std::is_same<S, TA>::value) {
-      if (!pre_fused()) return;
-      const PolyPlan pl = fine_plan();
-      pdl_launch(k::jacobi_zero<TA>, grid_for(nc_), kBlock, 0, st_, nc_, TA(pl.w0), v.r, pl.den0, fine_first(v.z));
-    } else if (pre_fused()) {
-      const PolyPlan pl = fine_plan();
-      pdl_launch(k::cast_jacobi<S, TA>, grid_for(nc_), kBlock, 0, st_, nc_, v.r, v.rA, TA(pl.w0), pl.den0,
-                 fine_first(v.z));
-    } else {
-      pdl_launch(k::cast_copy<S, TA>, grid_for(nc_), kBlock, 0, st_, nc_, v.r, v.rA);
+  void pcg_first(const PcgVecs<S>& v, double target, double r0, int cap, const double* from = nullptr, double s = 1.0) {
+    const TA* den0 = nullptr;
+    TA w0 = 0, *x1 = nullptr, *rA = nullptr;
+    if (!resident_) {
+      if (pre_fused()) {
+        const PolyPlan pl = fine_plan();
+        den0 = pl.den0;
+        w0 = TA(pl.w0);
+        x1 = fine_first(v.z);
+      }
+      rA = v.rA;
     }
+    const k::SolveInit init = solve_init(target, r0, 1, cap);
+    if (from)
+      pdl_launch(k::loop_start<double, S, TA>, grid_for(nc_), kBlock, 0, st_, nc_, from, s, v.r, (S*)nullptr, v.x, rA,
+                 den0, w0, x1, init);
+    else
+      pdl_launch(k::loop_start<S, S, TA>, rA || x1 ? grid_for(nc_) : 1, kBlock, 0, st_, rA || x1 ? nc_ : 0, v.r, 1.0,
+                 (S*)nullptr, (S*)nullptr, (S*)nullptr, rA, den0, w0, x1, init);
     NDS_LAUNCH();
   }
   // One pass of a PCG loop: z = M r; rho (first pass: p = z) and beta; q = A p;
@@ -2102,6 +2122,7 @@ class Solver final : public ISolver {
     a.target_slot = S_TARGET;
     a.flags = flags_.p;
     a.ctl = ctl_.p;
+    a.host = host_words();
     static_assert(S_RN2 == 3, "result slot of the kernel");
     {
       ProfScope ps(prof, st_, P_RESIDENT);
@@ -2113,13 +2134,6 @@ class Solver final : public ISolver {
       }
       NDS_LAUNCH();
     }
-    read_loop_state();
-  }
-  // control words, flags and ||r||^2 of a loop that ran on the device
-  void read_loop_state() {
-    NDS_CUDA(cudaMemcpyAsync(hflags_ + 4, ctl_.p, 4 * sizeof(int), cudaMemcpyDeviceToHost, st_));
-    NDS_CUDA(cudaMemcpyAsync(hflags_, flags_.p, sizeof(int), cudaMemcpyDeviceToHost, st_));
-    NDS_CUDA(cudaMemcpyAsync(hsc_ + S_RN2, sc_.p + S_RN2, sizeof(double), cudaMemcpyDeviceToHost, st_));
     NDS_CUDA(cudaStreamSynchronize(st_));
   }
   // PCG with the iteration loop on the device: two host synchronisations per
@@ -2129,14 +2143,9 @@ class Solver final : public ISolver {
     const double r0 = p_start(rhs);
     start_readback();
     if (r0 <= o_.p_atol) return {0, 0.0, true};
-    set_target(std::max(o_.p_atol, o_.p_rtol * r0), r0);
-    set_ctl(0, 0, 1, o_.p_max);
-    if (resident_) {
-      pcg_on_chip(pcg_vecs(), fine_op());
-    } else {
-      pcg_first(pcg_vecs());
-      run_loop(g_loop_, [&](cudaGraphConditionalHandle h) { pcg_body(pcg_vecs(), fine_op(), h); });
-    }
+    pcg_first(pcg_vecs(), std::max(o_.p_atol, o_.p_rtol * r0), r0, o_.p_max);
+    if (resident_) pcg_on_chip(pcg_vecs(), fine_op());
+    else run_loop(g_loop_, [&](cudaGraphConditionalHandle h) { pcg_body(pcg_vecs(), fine_op(), h); });
     const int f = hflags_[0];
     if (f & 8) throw SolveFailure(NDS_E_BREAKDOWN, "pressure PCG initial rho nonpositive");
     if (f & 1) throw SolveFailure(NDS_E_BREAKDOWN, "pressure PCG pAp nonpositive");
@@ -2177,8 +2186,7 @@ class Solver final : public ISolver {
                  T(0),
                  nullptr, nullptr);
       NDS_LAUNCH();
-      reduce_to<1>(g, S_RN2);
-      fetch(S_RN2, 1);
+      reduce_host<1>(part_.p, g, S_RN2);
       const double rn = std::sqrt(hsc_[S_RN2]);
       R.its = kk + 1;
       R.rel = rn / std::max(r0, 1e-300);
@@ -2383,7 +2391,7 @@ class Solver final : public ISolver {
                  fgpart_.p, fgtick_.p, L, fg_.p);
       NDS_LAUNCH();
       pdl_launch(k::fg_orth, g, kBlock, 0, st_, nc_, fgV_.p, fg_.p, L, qf_.p, part_.p, ticket_.p, k::FgScalars{sc_.p,
-                 S_RN2, S_WN, S_TARGET, ctl_.p, flags_.p, h, in_graph_});
+                 S_RN2, S_WN, S_TARGET, ctl_.p, flags_.p, h, in_graph_, host_words()});
       NDS_LAUNCH();
       const PolyPlan pl = pre_fused() ? fine_plan() : PolyPlan{};
       pdl_launch(k::fg_normalize, grid_for(nc_), kBlock, 0, st_, nc_, qf_.p, sc_.p, S_WN, ctl_.p, fgV_.p, rf_.p,
@@ -2442,7 +2450,7 @@ class Solver final : public ISolver {
   void run_loop(LoopGraph& G, Body&& body) {
     if (use_graphs_ && !prof.on && !G.failed && (G.exec || build_loop(G, body))) {
       NDS_CUDA(cudaGraphLaunch(G.exec, st_));
-      read_loop_state();
+      NDS_CUDA(cudaStreamSynchronize(st_));
       g_launches += (unsigned long long)hflags_[4] * G.body_kernels;
       return;
     }
@@ -2450,31 +2458,18 @@ class Solver final : public ISolver {
     // leaves the decision to this loop, which reads ctl and the flags
     for (;;) {
       body(cudaGraphConditionalHandle{});
-      read_loop_state();
+      NDS_CUDA(cudaStreamSynchronize(st_));
       prof.collect();
       const int its = hflags_[4], conv = hflags_[5], cap = hflags_[7];
       if (conv || hflags_[0] != 0 || its >= cap) break;
     }
   }
-  void set_target(double tol, double r0) {
-    hsc_[S_R0] = r0;
-    hsc_[S_TARGET] = tol;
-    NDS_CUDA(cudaMemcpyAsync(sc_.p + S_R0, hsc_ + S_R0, 2 * sizeof(double), cudaMemcpyHostToDevice, st_));
-  }
-  void set_ctl(int a, int b, int c, int d) {
-    const int init[4] = {a, b, c, d};
-    std::memcpy(hflags_ + 4, init, sizeof(init));
-    NDS_CUDA(cudaMemcpyAsync(ctl_.p, hflags_ + 4, 4 * sizeof(int), cudaMemcpyHostToDevice, st_));
-    NDS_CUDA(cudaMemsetAsync(flags_.p, 0, sizeof(int), st_));
-  }
-  // inner FP32 PCG on rf_ (unit norm) from xf_ = 0 to ||r|| <= tol within
-  // cap iterations; returns the iterations
-  int inner_pcg(double tol, int cap) {
-    xf_.zero(st_);
-    set_target(tol, 1.0);
-    set_ctl(0, 0, 1, cap);
+  // inner FP32 PCG on r_ / rn from zero to ||r|| <= tol within cap iterations;
+  // returns the iterations
+  int inner_pcg(double rn, double tol, int cap) {
     if constexpr (!kSame) {
       const PcgVecs<float> v{xf_.p, rf_.p, qf_.p, pf_.p, zf_.p, nullptr};
+      pcg_first(v, tol, 1.0, cap, r_.p, 1.0 / rn);
       if (resident_) pcg_on_chip(v, fine_opA());
       else run_loop(g_loopf_, [&](cudaGraphConditionalHandle h) { pcg_body(v, fine_opA(), h); });
     }
@@ -2491,13 +2486,12 @@ class Solver final : public ISolver {
     const k::FgLayout L{fg_m_};
     if constexpr (!kSame) {
       const PolyPlan pl = pre_fused() ? fine_plan() : PolyPlan{};
-      pdl_launch(k::scale_to_float, grid_for(nc_), kBlock, 0, st_, nc_, r_.p, 1.0 / rn, fgV_.p, pl.den0,
-                 float(pl.w0), pre_fused() ? fine_first(zf_.p) : nullptr, rf_.p);
+      pdl_launch(k::loop_start<double, float, float>, grid_for(nc_), kBlock, 0, st_, nc_, r_.p, 1.0 / rn, fgV_.p,
+                 rf_.p, (float*)nullptr, (float*)nullptr, pl.den0, float(pl.w0),
+                 pre_fused() ? fine_first(zf_.p) : nullptr, solve_init(tol, 1.0, 0, cap));
+      NDS_LAUNCH();
     }
-    NDS_LAUNCH();
-    set_target(tol, 1.0);
-    set_ctl(0, 0, 0, cap);
-    k::fg_start<<<1, 1, 0, st_>>>(fg_.p, L, ctl_.p, cap);
+    k::fg_start<<<1, 1, 0, st_>>>(fg_.p, L);
     NDS_LAUNCH();
     run_loop(g_fgmres_, [&](cudaGraphConditionalHandle h) { fg_body(h); });
     if (hflags_[0] & 16) throw SolveFailure(NDS_E_BREAKDOWN, "inner FGMRES breakdown or nonfinite value");
@@ -2528,9 +2522,7 @@ class Solver final : public ISolver {
     }
     pdl_launch(k::guess_dots<K>, g, kBlock, 0, st_, nc_, gY_.p, gW_.p, rhs, fgpart_.p);
     NDS_LAUNCH();
-    pdl_launch(k::reduce_partials<NG>, 1, kBlock, 0, st_, fgpart_.p, g, sc_.p + S_GUESS);
-    NDS_LAUNCH();
-    fetch(S_GUESS, NG);
+    reduce_host<NG>(fgpart_.p, g, S_GUESS);
     // G c = f by Cholesky (no guess when G is not numerically positive
     // definite, e.g. for dependent corrections)
     double G[K][K], f[K], c[K];
@@ -2561,15 +2553,34 @@ class Solver final : public ISolver {
       for (int e = a + 1; e < K; ++e) sum -= Lc[e][a] * c[e];
       c[a] = sum / Lc[a][a];
     }
+    k::GuessCoef<K> coef;
     for (int a = 0; a < K; ++a) {
       if (!std::isfinite(c[a])) return -1.0;
-      hsc_[S_COEF + a] = c[a];
+      coef.c[a] = c[a];
     }
-    NDS_CUDA(cudaMemcpyAsync(sc_.p + S_COEF, hsc_ + S_COEF, K * sizeof(double), cudaMemcpyHostToDevice, st_));
-    pdl_launch(k::guess_combine<K>, grid_for(nc_), kBlock, 0, st_, nc_, gY_.p, sc_.p + S_COEF, x_.p);
+    pdl_launch(k::guess_combine<K>, grid_for(nc_), kBlock, 0, st_, nc_, gY_.p, coef, x_.p);
     NDS_LAUNCH();
-    op_resid(fine_op(), (const double*)x_.p, rhs, r_.p);
-    return std::sqrt(dot_fetch((const double*)r_.p, (const double*)r_.p, nc_, S_TMP));
+    return defect_norm(rhs);
+  }
+  // r_ = b - A x_ on the FP64 operator; returns ||r||
+  double defect_norm(const double* rhs) {
+    if constexpr (std::is_same<T, double>::value) {
+      if (split_ && nc_ <= kRhoCells) {
+        const OpView<double> A = fine_op();
+        ProfScope ps(prof, st_, A.cat);
+        split_vertices(A, (const double*)x_.p);
+        split_types(A, [&](auto mt, auto d16) {
+          pdl_launch(k::split_cell<double, k::SELL_RESID, decltype(d16)::value, decltype(mt), k::SUM_ONLY>,
+                     grid_for(A.n), kBlock, 0, st_, A.sc, A.w, x_.p, rhs, (const double*)nullptr, 0.0, r_.p,
+                     (double*)nullptr, A.tinv, (const double*)nullptr, host_tail(S_TMP), (const int*)nullptr);
+        });
+        NDS_LAUNCH();
+        NDS_CUDA(cudaStreamSynchronize(st_));
+        return std::sqrt(hsc_[S_TMP]);
+      }
+    }
+    op_resid(fine_op(), (const T*)x_.p, (const T*)rhs, r_.p);
+    return std::sqrt(dot_fetch((const T*)r_.p, (const T*)r_.p, nc_, S_TMP));
   }
   double apply_guess(const double* rhs) {
     switch (std::min(o_.p_guess, nguess_)) {
@@ -2635,22 +2646,12 @@ class Solver final : public ISolver {
         if (fg_m_ > 0) {
           R.its += inner_fgmres(rn, tol, std::min(cap, fg_m_));
         } else {
-          if (pre_fused() && !resident_) {
-            const PolyPlan pl = fine_plan();
-            pdl_launch(k::scale_to_float, grid_for(nc_), kBlock, 0, st_, nc_, r_.p, 1.0 / rn, rf_.p, pl.den0,
-                       float(pl.w0), fine_first(zf_.p), (float*)nullptr);
-          } else {
-            pdl_launch(k::scale_to_float, grid_for(nc_), kBlock, 0, st_, nc_, r_.p, 1.0 / rn, rf_.p,
-                       (const float*)nullptr, 0.f, (float*)nullptr, (float*)nullptr);
-          }
-          NDS_LAUNCH();
-          R.its += inner_pcg(tol, cap);
+          R.its += inner_pcg(rn, tol, cap);
           pdl_launch(k::axpy_from_float, grid_for(nc_), kBlock, 0, st_, nc_, rn, xf_.p, x_.p);
           NDS_LAUNCH();
         }
         ++passes;
-        op_resid(fine_op(), (const double*)x_.p, rhs, r_.p);
-        rn = std::sqrt(dot_fetch((const double*)r_.p, (const double*)r_.p, nc_, S_TMP));
+        rn = defect_norm(rhs);
         if (!std::isfinite(rn)) throw SolveFailure(NDS_E_BREAKDOWN, "pressure defect nonfinite");
       }
       R.rel = rn / std::max(bn, 1e-300);
@@ -2738,8 +2739,7 @@ class Solver final : public ISolver {
     k::mom_audit<T><<<g, kBlock, 0, st_>>>(nv_, mspan_.p, mcol_.p, A_.p, b_[0].p, b_[1].p, b_[2].p, uc(0), uc(1),
                                            uc(2), part_.p);
     NDS_LAUNCH();
-    reduce_to<6>(g, S_AUDIT);
-    fetch(S_AUDIT, 6);
+    reduce_host<6>(part_.p, g, S_AUDIT);
     std::array<double, 3> q{};
     for (int d = 0; d < 3; ++d) {
       double bn = std::sqrt(std::max(0.0, hsc_[S_AUDIT + d]));
@@ -2810,8 +2810,7 @@ class Solver final : public ISolver {
       pdl_launch(k::continuity<T>, g, kBlock, 0, st_, nc_, ref_.p, bco_.p, fixed_div_.p, uc(0), uc(1), uc(2), rhs_.p,
                  part_.p);
       NDS_LAUNCH();
-      reduce_to<1>(g, S_CONT2);
-      fetch(S_CONT2, 1);
+      reduce_host<1>(part_.p, g, S_CONT2);
     }
     const double cn = std::sqrt(hsc_[S_CONT2]);
     if (it == 1) cont0_ = cn;

@@ -357,7 +357,7 @@ __device__ __forceinline__ V split_row(const SplitCells& a, const X& x, const W&
 }
 
 // The modes Y, RESID and SMOOTH of sell_spmv on the split form (w from
-// split_vertex on the same x).  Y with y2: also x into vector at[0] of y2.
+// split_vertex on the same x).  STEP SUM_ONLY (RESID): also ||r||^2.  Y with y2: also x into vector at[0] of y2.
 // STEP PCG_RHO (SMOOTH with y2, the last step
 // of the V-cycle): also r.z of the new z = y2 with the reduction tail.
 template <class V, int MODE, bool D16, class MT, int STEP = 0, class R = V>
@@ -388,6 +388,7 @@ __global__ void __launch_bounds__(kBlock) split_cell(SplitCells a, const V* __re
       y[c] = q;
       if (den) y2[c] = wt * q / dc;
       else if (y2) y2[c] = q;
+      if (STEP != 0) acc = (double)q * (double)q;
     } else {
       V val = xc + wt * (bc - s) / dc;
       if (y2) {

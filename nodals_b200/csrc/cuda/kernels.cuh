@@ -90,139 +90,271 @@ __global__ void deinterleave3(int n, const T* __restrict__ u, T* __restrict__ a0
 // the same pass.
 // ---------------------------------------------------------------------------
 
+// Cell pass: each cell's 8x8 convection block, row a of it written to C[8 z + b],
+// z the incidence (c, a) in the velocity rows' incidence lists, so that a
+// row's blocks lie contiguous; the cell's pressure goes to pz[z] for the B^T p
+// terms of the row pass.
+//
+// Four lanes a cell, lane i with the columns of
+// vertex i and of the bubble opposite to it.  With the velocity in
+// barycentric components s_k(m) = u_m . grad lambda_k (s_0 = -(s_1 + s_2 +
+// s_3)), a vertex column needs one mass matrix, C[a][i] = det sum_m M[a][m]
+// s_i(m), and a bubble column three tensors, C[a][4+i] = det sum_(k != i)
+// sum_m N_ik[a][m] s_k(m) with N_ik[a][m] = int phi_a phi_m dphi_(4+i)/dlambda_k;
+// M and N are symmetric in (a, m).  So a cell takes 1024 multiply-adds instead
+// of 1536, and a lane reads each of the 36 symmetric table records (its three
+// N and M, two 16-byte loads) once for both (a, m) and (m, a): 9 loads of a
+// warp per cell where the 8-lane form takes 48, which bound it (shared-memory
+// stalls).  Assembly at 1.23M cells 1.55 -> 1.31 ms, at 404k 0.50 -> 0.43, at
+// 40k 0.079 -> 0.070.
+template <class T>
+__device__ __forceinline__ void conv_record(const T* __restrict__ t, T& n0, T& n1, T& n2, T& mm) {
+  if constexpr (sizeof(T) == 8) {
+    const double2 a = reinterpret_cast<const double2*>(t)[0], b = reinterpret_cast<const double2*>(t)[1];
+    n0 = a.x; n1 = a.y; n2 = b.x; mm = b.y;
+  } else {
+    const float4 a = reinterpret_cast<const float4*>(t)[0];
+    n0 = a.x; n1 = a.y; n2 = a.z; mm = a.w;
+  }
+}
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+// the records (three N and M of column pair i) of the pairs a <= m in shared
+// memory, from the reference tensor T[a][m][b][j] = int phi_a phi_m dphi_b/dxi_j
+constexpr int kConvTable = 36 * 16;
+template <class T>
+__device__ __forceinline__ void conv_table(T* __restrict__ sN, const T* __restrict__ centT) {
+  for (int e = threadIdx.x; e < kConvTable; e += blockDim.x) {
+    const int i = (e >> 2) & 3, q = e & 3;
+    int a = 0, m = e >> 4;  // pair index -> a <= m
+    while (m >= 8 - a) {
+      m -= 8 - a;
+      ++a;
+    }
+    m += a;
+    const T* t = centT + ((a * 8 + m) * 8 + 4 + i) * 3;  // T[a][m][4+i][.] = N_ij - N_i0
+    T v;
+    if (q == 3) {
+      v = centT[((a * 8 + m) * 8 + 1) * 3];  // M: phi_1 = lambda_1
+    } else {
+      const int k = q + (q >= i);  // the q-th k != i
+      const T n0 = i == 0 ? T(0) : -t[i - 1];
+      v = k == 0 ? n0 : t[k - 1] + n0;
+    }
+    sN[e] = v;
+  }
+}
+template <class T>
+__global__ void __launch_bounds__(kBlock, 2) mom_cell_conv(int nc, const int32_t* __restrict__ ref,
+                                                            const T* __restrict__ fixed, const T* __restrict__ u0,
+                                                            const T* __restrict__ u1, const T* __restrict__ u2,
+                                                            const T* __restrict__ invJ, const T* __restrict__ det,
+                                                            const T* __restrict__ centT,
+                                                            const int32_t* __restrict__ zpos, T* __restrict__ C,
+                                                            const T* __restrict__ p, T* __restrict__ pz) {
+  __shared__ __align__(16) T sN[kConvTable];
+  conv_table(sN, centT);
+  __syncthreads();
+  const int i = threadIdx.x & 3;
+  const unsigned mask = 0xFu << (threadIdx.x & 28);
+  const int groups = blockDim.x >> 2;
+  for (int c = blockIdx.x * groups + (threadIdx.x >> 2); c < nc; c += gridDim.x * groups) {
+    int g[2];
+    T r[2][3];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) g[h] = ref[8 * (size_t)c + 4 * h + i];
+    T I[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) I[k] = invJ[9 * (size_t)c + k];
+    const T dc = det[c], pc = p[c];
+    int zl[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) zl[h] = zpos[8 * (size_t)c + 4 * h + i];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      T q0, q1, q2;
+      if (g[h] >= 0) {
+        q0 = u0[kVel * (size_t)g[h]];
+        q1 = u1[kVel * (size_t)g[h]];
+        q2 = u2[kVel * (size_t)g[h]];
+      } else {
+        const T* f = fixed + 3 * (size_t)(-g[h] - 1);
+        q0 = f[0];
+        q1 = f[1];
+        q2 = f[2];
+      }
+#pragma unroll
+      for (int j = 0; j < 3; ++j) r[h][j] = fma(q2, I[3 * j + 2], fma(q1, I[3 * j + 1], q0 * I[3 * j]));
+      if (zl[h] >= 0) pz[zl[h]] = pc;
+    }
+    // A0..A2: s_k of the three k != i (ascending), D: s_i
+    T A0[8], A1[8], A2[8], D[8];
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+      const T s1 = __shfl_sync(mask, r[m >> 2][0], m & 3, 4), s2 = __shfl_sync(mask, r[m >> 2][1], m & 3, 4),
+              s3 = __shfl_sync(mask, r[m >> 2][2], m & 3, 4);
+      const T s0 = -(s1 + s2 + s3);
+      A0[m] = i == 0 ? s1 : s0;
+      A1[m] = i <= 1 ? s2 : s1;
+      A2[m] = i <= 2 ? s3 : s2;
+      D[m] = i == 0 ? s0 : i == 1 ? s1 : i == 2 ? s2 : s3;
+    }
+    T cb[8], cv[8];
+#pragma unroll
+    for (int a = 0; a < 8; ++a) cb[a] = cv[a] = T(0);
+    int e = 0;
+#pragma unroll
+    for (int a = 0; a < 8; ++a) {
+#pragma unroll
+      for (int m = a; m < 8; ++m, ++e) {
+        T n0, n1, n2, mm;
+        conv_record(sN + 16 * e + 4 * i, n0, n1, n2, mm);
+        cb[a] = fma(n2, A2[m], fma(n1, A1[m], fma(n0, A0[m], cb[a])));
+        cv[a] = fma(mm, D[m], cv[a]);
+        if (m > a) {
+          cb[m] = fma(n2, A2[a], fma(n1, A1[a], fma(n0, A0[a], cb[m])));
+          cv[m] = fma(mm, D[a], cv[m]);
+        }
+      }
+    }
+#pragma unroll
+    for (int a = 0; a < 8; ++a) {
+      const int za = __shfl_sync(mask, zl[a >> 2], a & 3, 4);
+      if (za >= 0) {
+        C[8 * (size_t)za + i] = cv[a] * dc;
+        C[8 * (size_t)za + 4 + i] = cb[a] * dc;
+      }
+    }
+  }
+}
+
 // Laminar SUPG terms, implicit form (h7_momentum_assembly.cuh:100-226; host
-// twin g4_host.hpp:324-419): column b of the cell block
+// twin g4_host.hpp:324-419), added to the rows the cell pass wrote:
 //   S[a][b] = sum_q tau_q w_q det (adv_q . grad phi_a) strong_b(q),
 //   strong_b = adv . grad phi_b (- nu lap phi_b for the bubbles),
 //   tau_q = tau_scale / sqrt(max(4 |adv_q|^2 / h^2 + magic (4 nu / h^2)^2, 1e-30)),
 // over the 64-point collapsed rule (rule: 64 x (lambda0..3, weight)).
-// Lane m of the 8-lane group holds the velocity q of basis m; lane b returns
-// S[0..7][b].
+// With sigma_k = adv . grad lambda_k every adv . grad phi_a is a few products
+// of sigma and lambda, so a point is given by sigma_1..3 and its weight: of
+// the four lanes of a cell each prepares every fourth point (velocity from
+// shared memory, square root and division), the lanes exchange the four
+// values, and lane i adds the columns of vertex i and of the bubble opposite
+// to it.  Bound by FP64 arithmetic: assembly with these terms at 35k
+// cells takes 0.132 ms, 0.288 when every lane of eight evaluated the basis
+// gradients at every point.
 struct SupgArgs {
   double nu, tau_scale, magic;
 };
 template <class T>
-__device__ __forceinline__ void supg_column(const T* __restrict__ I, T h2, T dc, T q0, T q1, T q2,
-                                            const T* __restrict__ rule, const SupgArgs& sa, int lane8,
-                                            unsigned gmask, T S[8]) {
-  T gl[4][3], gd[4][4];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    gl[0][d] = -(I[d] + I[3 + d] + I[6 + d]);
-    gl[1][d] = I[d];
-    gl[2][d] = I[3 + d];
-    gl[3][d] = I[6 + d];
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = i; j < 4; ++j) {
-      T v = 0;
-#pragma unroll
-      for (int d = 0; d < 3; ++d) v += gl[i][d] * gl[j][d];
-      gd[i][j] = gd[j][i] = v;
+__global__ void __launch_bounds__(kBlock, 2) mom_cell_supg(int nc, const int32_t* __restrict__ ref,
+                                                           const T* __restrict__ fixed, const T* __restrict__ u0,
+                                                           const T* __restrict__ u1, const T* __restrict__ u2,
+                                                           const T* __restrict__ invJ, const T* __restrict__ det,
+                                                           const int32_t* __restrict__ zpos, T* __restrict__ C,
+                                                           const T* __restrict__ rule, const T* __restrict__ h2,
+                                                           SupgArgs sa) {
+  constexpr int kCells = kBlock / 4;
+  __shared__ T sr[64][13];          // lambda0..3, weight, phi_0..7
+  __shared__ T su[kCells][8][3];    // velocities of the block's cells
+  for (int q = threadIdx.x; q < 64; q += blockDim.x) {
+    T l[4];
+    for (int k = 0; k < 4; ++k) sr[q][k] = l[k] = rule[5 * q + k];
+    sr[q][4] = rule[5 * q + 4];
+    for (int k = 0; k < 4; ++k) {
+      sr[q][5 + k] = l[k];
+      const T a = k == 0 ? l[1] : l[0], b = k <= 1 ? l[2] : l[1], c = k <= 2 ? l[3] : l[2];
+      sr[q][9 + k] = T(27) * a * b * c;
     }
-  // this lane's basis function: vertex i = lane8 (< 4) or the bubble on the
-  // face opposite vertex i = lane8 - 4, with the other vertices j0 < j1 < j2
-  const int i = lane8 & 3;
-  const int j0 = i == 0 ? 1 : 0, j1 = i <= 1 ? 2 : 1, j2 = i <= 2 ? 3 : 2;
-  const bool bubble = lane8 >= 4;
-  const T nu = T(sa.nu), diff = T(4) * nu / h2;
-#pragma unroll
-  for (int a = 0; a < 8; ++a) S[a] = 0;
-  for (int qp = 0; qp < 64; ++qp) {
-    const T* lam = rule + 5 * qp;
-    const T l0 = lam[j0], l1 = lam[j1], l2 = lam[j2];
-    const T phi = bubble ? T(27) * l0 * l1 * l2 : lam[i];
-    const T a0 = group_sum<8>(q0 * phi, gmask), a1 = group_sum<8>(q1 * phi, gmask), a2 = group_sum<8>(q2 * phi, gmask);
-    T g0, g1, g2, lap = 0;
-    if (!bubble) {
-      g0 = gl[i][0];
-      g1 = gl[i][1];
-      g2 = gl[i][2];
-    } else {
-      g0 = T(27) * (l1 * l2 * gl[j0][0] + l0 * l2 * gl[j1][0] + l0 * l1 * gl[j2][0]);
-      g1 = T(27) * (l1 * l2 * gl[j0][1] + l0 * l2 * gl[j1][1] + l0 * l1 * gl[j2][1]);
-      g2 = T(27) * (l1 * l2 * gl[j0][2] + l0 * l2 * gl[j1][2] + l0 * l1 * gl[j2][2]);
-      lap = T(54) * (l2 * gd[j0][j1] + l1 * gd[j0][j2] + l0 * gd[j1][j2]);
-    }
-    const T stream = a0 * g0 + a1 * g1 + a2 * g2;
-    const T strong = bubble ? -nu * lap + stream : stream;
-    const T speed2 = a0 * a0 + a1 * a1 + a2 * a2;
-    const T den = fmax(T(4) * speed2 / h2 + T(sa.magic) * diff * diff, T(1e-30));
-    const T w = T(sa.tau_scale) / sqrt(den) * lam[4] * dc;
-    const T ta = w * stream;
-#pragma unroll
-    for (int a = 0; a < 8; ++a) S[a] += __shfl_sync(gmask, ta, a, 8) * strong;
   }
-}
-
-// 8 lanes per cell; lane b computes column b of the cell's block (convection,
-// plus the SUPG terms when SUPG; supg_rule and h2 are read only then).  Row a
-// of the block is written to C[8 z + b], z the incidence (c, a) in the
-// velocity rows' incidence lists, so that a row's blocks lie contiguous; the
-// cell's pressure goes to pz[z] for the B^T p terms of the row pass.
-template <class T, bool SUPG>
-__global__ void __launch_bounds__(kBlock, SUPG ? 2 : 4) mom_cell_conv(int nc, const int32_t* __restrict__ ref,
-                                                        const T* __restrict__ fixed, const T* __restrict__ u0,
-                                                        const T* __restrict__ u1, const T* __restrict__ u2,
-                                                        const T* __restrict__ invJ, const T* __restrict__ det,
-                                                        const T* __restrict__ centT, const int32_t* __restrict__ zpos,
-                                                        T* __restrict__ C, const T* __restrict__ p, T* __restrict__ pz,
-                                                        const T* __restrict__ supg_rule, const T* __restrict__ h2,
-                                                        SupgArgs sa) {
-  __shared__ T sT[1536];
-  __shared__ T sQ[SUPG ? 320 : 1];
-  for (int k = threadIdx.x; k < 1536; k += blockDim.x) sT[k] = centT[k];
-  if (SUPG)
-    for (int k = threadIdx.x; k < 320; k += blockDim.x) sQ[k] = supg_rule[k];
   __syncthreads();
-  const int lane8 = threadIdx.x & 7;
-  const int groups = blockDim.x >> 3;
-  const unsigned gmask = group8_mask();
-  for (int c = blockIdx.x * groups + (threadIdx.x >> 3); c < nc; c += gridDim.x * groups) {
-    // lane m: velocity of basis function m of cell c, mapped by J^-1
-    const int gm = ref[8 * (size_t)c + lane8];
-    T q0, q1, q2;
-    if (gm >= 0) {
-      q0 = u0[kVel * (size_t)gm];
-      q1 = u1[kVel * (size_t)gm];
-      q2 = u2[kVel * (size_t)gm];
-    } else {
-      const T* f = fixed + 3 * (size_t)(-gm - 1);
-      q0 = f[0];
-      q1 = f[1];
-      q2 = f[2];
-    }
-    const T* I = invJ + 9 * (size_t)c;
-    const T r0 = q0 * I[0] + q1 * I[1] + q2 * I[2];
-    const T r1 = q0 * I[3] + q1 * I[4] + q2 * I[5];
-    const T r2 = q0 * I[6] + q1 * I[7] + q2 * I[8];
-    T w[8][3];
+  const int i = threadIdx.x & 3, slot = threadIdx.x >> 2;
+  const unsigned mask = 0xFu << (threadIdx.x & 28);
+  const int j0 = i == 0 ? 1 : 0, j1 = i <= 1 ? 2 : 1, j2 = i <= 2 ? 3 : 2;  // the vertices of face i
+  const T nu = T(sa.nu);
+  for (int c = blockIdx.x * kCells + slot; c < nc; c += gridDim.x * kCells) {
+    int zl[2];
 #pragma unroll
-    for (int m = 0; m < 8; ++m) {
-      w[m][0] = __shfl_sync(gmask, r0, m, 8);
-      w[m][1] = __shfl_sync(gmask, r1, m, 8);
-      w[m][2] = __shfl_sync(gmask, r2, m, 8);
+    for (int h = 0; h < 2; ++h) {
+      const int m = 4 * h + i, g = ref[8 * (size_t)c + m];
+      zl[h] = zpos[8 * (size_t)c + m];
+      if (g >= 0) {
+        su[slot][m][0] = u0[kVel * (size_t)g];
+        su[slot][m][1] = u1[kVel * (size_t)g];
+        su[slot][m][2] = u2[kVel * (size_t)g];
+      } else {
+        const T* f = fixed + 3 * (size_t)(-g - 1);
+        su[slot][m][0] = f[0];
+        su[slot][m][1] = f[1];
+        su[slot][m][2] = f[2];
+      }
     }
-    const T dc = det[c];
-    // row a of the block goes to the incidence slot zpos[8c + a] (-1: the
-    // dof of basis a is fixed and has no momentum row)
-    const int zl = zpos[8 * (size_t)c + lane8];
-    if (zl >= 0) pz[zl] = p[c];  // the cell's pressure, by the incidences of its bases
-    T S[8];
-    if (SUPG) supg_column<T>(I, h2[c], dc, q0, q1, q2, sQ, sa, lane8, gmask, S);
-#pragma unroll 2
-    for (int a = 0; a < 8; ++a) {
-      T cv = 0;
+    T I[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) I[k] = invJ[9 * (size_t)c + k];
+    const T dc = det[c], h = h2[c], diff = T(4) * nu / h, base = T(sa.magic) * diff * diff;
+    // products of the gradients of face i's vertices (grad lambda_0 = -(sum of the others))
+    auto grad = [&](int k, int d) { return k == 0 ? -(I[d] + I[3 + d] + I[6 + d]) : I[3 * (k - 1) + d]; };
+    T g01 = 0, g02 = 0, g12 = 0;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const T a = grad(j0, d), b = grad(j1, d), e = grad(j2, d);
+      g01 += a * b;
+      g02 += a * e;
+      g12 += b * e;
+    }
+    __syncwarp(mask);
+    T cv[8], cb[8];
+#pragma unroll
+    for (int a = 0; a < 8; ++a) cv[a] = cb[a] = T(0);
+    for (int q4 = 0; q4 < 64; q4 += 4) {
+      // this lane's point
+      T a0 = 0, a1 = 0, a2 = 0;
 #pragma unroll
       for (int m = 0; m < 8; ++m) {
-        const T* t = sT + ((a * 8 + m) * 8 + lane8) * 3;
-        cv += w[m][0] * t[0] + w[m][1] * t[1] + w[m][2] * t[2];
+        const T ph = sr[q4 + i][5 + m];
+        a0 += su[slot][m][0] * ph;
+        a1 += su[slot][m][1] * ph;
+        a2 += su[slot][m][2] * ph;
       }
-      const int za = __shfl_sync(gmask, zl, a, 8);
-      if (za >= 0) C[8 * (size_t)za + lane8] = SUPG ? cv * dc + S[a] : cv * dc;
+      const T den = fmax(T(4) * (a0 * a0 + a1 * a1 + a2 * a2) / h + base, T(1e-30));
+      const T wq = T(sa.tau_scale) / sqrt(den) * sr[q4 + i][4] * dc;
+      const T p1 = a0 * I[0] + a1 * I[1] + a2 * I[2], p2 = a0 * I[3] + a1 * I[4] + a2 * I[5],
+              p3 = a0 * I[6] + a1 * I[7] + a2 * I[8];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const T w = __shfl_sync(mask, wq, t, 4), s1 = __shfl_sync(mask, p1, t, 4), s2 = __shfl_sync(mask, p2, t, 4),
+                s3 = __shfl_sync(mask, p3, t, 4), s0 = -(s1 + s2 + s3);
+        const T* l = sr[q4 + t];
+        const T l0 = l[0], l1 = l[1], l2 = l[2], l3 = l[3];
+        T st[8];
+        st[0] = s0;
+        st[1] = s1;
+        st[2] = s2;
+        st[3] = s3;
+        st[4] = T(27) * (l2 * l3 * s1 + l1 * l3 * s2 + l1 * l2 * s3);
+        st[5] = T(27) * (l2 * l3 * s0 + l0 * l3 * s2 + l0 * l2 * s3);
+        st[6] = T(27) * (l1 * l3 * s0 + l0 * l3 * s1 + l0 * l1 * s3);
+        st[7] = T(27) * (l1 * l2 * s0 + l0 * l2 * s1 + l0 * l1 * s2);
+        const T lap = T(54) * (l[j2] * g01 + l[j1] * g02 + l[j0] * g12);
+        const T sv = i == 0 ? st[0] : i == 1 ? st[1] : i == 2 ? st[2] : st[3];
+        const T sb = (i == 0 ? st[4] : i == 1 ? st[5] : i == 2 ? st[6] : st[7]) - nu * lap;
+#pragma unroll
+        for (int a = 0; a < 8; ++a) {
+          const T ta = w * st[a];
+          cv[a] += ta * sv;
+          cb[a] += ta * sb;
+        }
+      }
     }
+#pragma unroll
+    for (int a = 0; a < 8; ++a) {
+      const int za = __shfl_sync(mask, zl[a >> 2], a & 3, 4);
+      if (za >= 0) {
+        C[8 * (size_t)za + i] += cv[a];
+        C[8 * (size_t)za + 4 + i] += cb[a];
+      }
+    }
+    __syncwarp(mask);  // the slot's velocities are read no more
   }
 }
 
@@ -267,11 +399,11 @@ struct MomArgs {
 
 // 8 lanes per velocity row; lane b adds column b of each incident block.
 // Convection entries C_c[a][lane8] of one incidence (cell c, basis a), the
-// same expression and order as mom_cell_conv: lane m maps the velocity of
+// same expressions and order as mom_cell_conv: lane m maps the velocity of
 // basis m by J^-1, the group shares the eight mapped velocities, lane b sums
 // over m.  ga: this lane's DOF of cell c (ref[8 c + lane8]).
 template <class T>
-__device__ __forceinline__ T conv_entry(const MomArgs<T>& g, const T* __restrict__ sT, int c, int a, int ga,
+__device__ __forceinline__ T conv_entry(const MomArgs<T>& g, const T* __restrict__ sN, int c, int a, int ga,
                                         int lane8, unsigned gmask) {
   T q0, q1, q2;
   if (ga >= 0) {
@@ -285,17 +417,25 @@ __device__ __forceinline__ T conv_entry(const MomArgs<T>& g, const T* __restrict
     q2 = f[2];
   }
   const T* I = g.invJ + 9 * (size_t)c;
-  const T r0 = q0 * I[0] + q1 * I[1] + q2 * I[2];
-  const T r1 = q0 * I[3] + q1 * I[4] + q2 * I[5];
-  const T r2 = q0 * I[6] + q1 * I[7] + q2 * I[8];
-  T cv = 0;
+  T r[3];
+#pragma unroll
+  for (int j = 0; j < 3; ++j) r[j] = fma(q2, I[3 * j + 2], fma(q1, I[3 * j + 1], q0 * I[3 * j]));
+  const int i = lane8 & 3;
+  T cb = 0, cv = 0;
 #pragma unroll
   for (int m = 0; m < 8; ++m) {
-    const T w0 = __shfl_sync(gmask, r0, m, 8), w1 = __shfl_sync(gmask, r1, m, 8), w2 = __shfl_sync(gmask, r2, m, 8);
-    const T* t = sT + ((a * 8 + m) * 8 + lane8) * 3;
-    cv += w0 * t[0] + w1 * t[1] + w2 * t[2];
+    const T s1 = __shfl_sync(gmask, r[0], m, 8), s2 = __shfl_sync(gmask, r[1], m, 8), s3 = __shfl_sync(gmask, r[2], m, 8);
+    const T s0 = -(s1 + s2 + s3);
+    const T A0 = i == 0 ? s1 : s0, A1 = i <= 1 ? s2 : s1, A2 = i <= 2 ? s3 : s2;
+    const T D = i == 0 ? s0 : i == 1 ? s1 : i == 2 ? s2 : s3;
+    const int lo = a < m ? a : m, hi = a < m ? m : a;
+    T n0, n1, n2, mm;
+    conv_record(sN + 16 * (lo * 8 - lo * (lo - 1) / 2 + hi - lo) + 4 * i, n0, n1, n2, mm);
+    cb = fma(n2, A2, fma(n1, A1, fma(n0, A0, cb)));
+    cv = fma(mm, D, cv);
   }
-  return cv * g.det[c];
+  const T dc = g.det[c];
+  return mul_rn(lane8 < 4 ? cv : cb, dc);  // rounded here: the cell pass stores the product
 }
 
 // FUSED 0: the row pass of the two-pass assembly; each velocity row reads
@@ -317,7 +457,7 @@ __global__ void __launch_bounds__(kBlock) mom_assemble(MomArgs<T> g) {
   T* buf = sRow + (size_t)grp * g.row_cap;
   T* sT = sRow + (size_t)groups * g.row_cap;
   if (FUSED) {
-    for (int k = tid; k < 1536; k += blockDim.x) sT[k] = g.centT[k];
+    conv_table(sT, g.centT);
     __syncthreads();
   }
   const unsigned gmask = group8_mask();

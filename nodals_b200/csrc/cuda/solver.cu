@@ -421,7 +421,7 @@ class Solver final : public ISolver {
     if (mom_smem_ > 200 * 1024) throw std::runtime_error("momentum row too long for the shared-memory assembly buffer");
     NDS_CUDA(cudaFuncSetAttribute(k::mom_assemble<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mom_smem_));
     NDS_CUDA(cudaFuncSetAttribute(k::mom_assemble<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)(mom_smem_ + 1536 * sizeof(T))));
+                                  (int)(mom_smem_ + k::kConvTable * sizeof(T))));
     // The two-pass assembly by default: the cell pass writes each cell's
     // convection block row by row into the incidence slots of the velocity
     // rows (8 values per incidence, contiguous per row), the row pass
@@ -2703,21 +2703,20 @@ class Solver final : public ISolver {
     ProfScope ps(prof, st_, P_ASSEMBLE);
     if (fused_assembly_) {
       // one pass: each incidence's convection row is evaluated in place
-      pdl_launch(k::mom_assemble<T, 1>, grid_for(nv_, kBlock / 8), kBlock, mom_smem_ + 1536 * sizeof(T), st_, a);
+      pdl_launch(k::mom_assemble<T, 1>, grid_for(nv_, kBlock / 8), kBlock, mom_smem_ + k::kConvTable * sizeof(T), st_, a);
       NDS_LAUNCH();
       return;
     }
     // cell blocks: a grid of 8 blocks per SM amortises the shared tensor load
     k::SupgArgs sa{P_.setup.pipe.nu, o_.supg_tau_scale, o_.supg_magic};
-    const int gc = std::min(grid_for(nc_, kBlock / 8), 8 * 148);
-    if (o_.supg)
-      k::mom_cell_conv<T, true><<<gc, kBlock, 0, st_>>>(nc_, ref_.p, fixed_.p, uc(0), uc(1), uc(2), invJ_.p,
-                                                       det_.p, centT_.p, zpos_.p, cconv_.p, p_.p, pz_.p, supg_rule_.p,
-                                                       h2_.p, sa);
-    else
-      k::mom_cell_conv<T, false><<<gc, kBlock, 0, st_>>>(nc_, ref_.p, fixed_.p, uc(0), uc(1), uc(2), invJ_.p,
-                                                        det_.p, centT_.p, zpos_.p, cconv_.p, p_.p, pz_.p, nullptr,
-                                                        nullptr, sa);
+    const int gc = std::min(grid_for(nc_, kBlock / 4), 4 * kSms);
+    k::mom_cell_conv<T><<<gc, kBlock, 0, st_>>>(nc_, ref_.p, fixed_.p, uc(0), uc(1), uc(2), invJ_.p, det_.p, centT_.p,
+                                                 zpos_.p, cconv_.p, p_.p, pz_.p);
+    if (o_.supg) {
+      NDS_LAUNCH();
+      k::mom_cell_supg<T><<<gc, kBlock, 0, st_>>>(nc_, ref_.p, fixed_.p, uc(0), uc(1), uc(2), invJ_.p, det_.p, zpos_.p,
+                                                  cconv_.p, supg_rule_.p, h2_.p, sa);
+    }
     NDS_LAUNCH();
     pdl_launch(k::mom_assemble<T>, grid_for(nv_, kBlock / 8), kBlock, mom_smem_, st_, a);
     NDS_LAUNCH();

@@ -24,7 +24,7 @@ Steps: W warm-up and K timed SIMPLE iterations of the fast configuration on
 a separate solver give ``ms_per_step`` (barrier + synchronize around the K
 steps, max over ranks); a profiled pass of further iterations (per-kernel
 CUDA events, launch-by-launch loops) times the roofline kernel live.  The
-per-iteration working set (fine operator ~1 GB) is larger than the 126 MB
+per-iteration working set (momentum matrix ~1 GB) is larger than the 126 MB
 L2, so no flush is inserted.
 
 Modes:
@@ -166,15 +166,21 @@ def _barrier_max(x: float, ws: int, device: int) -> float:
     return float(t.item())
 
 
-def fine_spmv_bytes(problem, s: int, sx: int | None = None) -> float:
-    """Compulsory bytes of one fine Schur SpMV in CSR terms: values (s B) and
-    column indices (4 B) of every entry, row offsets, x and y once (sx B
-    each; default s)."""
+def split_bytes(problem, s: int, sx: int | None = None) -> float:
+    """Bytes of one product with the pressure operator A = B diag(rAU) B^T in
+    its split form (values s B, vectors sx B, default s), every array once: per
+    cell the ids of its vertices (16 B) and face neighbours (8 B), the vectors
+    of its vertices (12 halves, 9 floats or doubles), its 4 face couplings, x,
+    y and the two further vectors of a smoothing step; per vertex incidence a
+    record of vector and cell (8, 16 or 28 B); per vertex its offset, rAU and
+    sum."""
     sx = s if sx is None else sx
-    row = problem.array("fine.row")
-    n = len(row) - 1
-    nnz = int(row[-1])
-    return nnz * (s + 4) + 4 * (n + 1) + 2 * sx * n
+    ref = problem.array("cell.ref").reshape(-1, 8)[:, :4]
+    free = ref[ref >= 0]
+    nc, inc, nvert = len(ref), free.size, int(free.max()) + 1
+    geo = 12 if s == 2 else 9
+    rec = {2: 8, 4: 16, 8: 28}[s]
+    return nc * (16 + 8 + (geo + 4) * s + 4 * sx) + inc * rec + nvert * (8 + 9 * sx)
 
 
 def outer_kernel_bytes(problem) -> dict:
@@ -188,13 +194,12 @@ def outer_kernel_bytes(problem) -> dict:
     c = problem.counts()
     nc, nv = c["nc"], c["nv"]
     zm = int(problem.array("mom.row")[-1])
-    zp = int(problem.array("fine.row")[-1])
-    zd = int(problem.array("fine.contribOff")[-1])
+    nvert = int(problem.array("cell.ref").reshape(-1, 8)[:, :4].max()) + 1
     return {
         "mom_assemble": 5 * s * zm + (172 + 48 * s) * nc + (12 + 25 * s) * nv,
         "mom_gs": (4 + s) * zm + (16 + 8 * s) * nv,
         "continuity": (48 * s + 36) * nc,
-        "fine_refresh": (s + 4 + 2) * zp + 5 * zd + (24 * s + 8) * nc + s * nv,
+        "fine_refresh": (32 + 4 * s + 4 * (s + 4 + 2) + 4) * nc + s * nv + (s + 4) * nvert,
     }
 
 
@@ -218,24 +223,9 @@ def outer_kernels(prof, kbytes, steps) -> dict | None:
     out["peak_gbs"] = peak
     out["peak_kind"] = kind
     out["note"] = ("mom_gs and fine_refresh run concurrently on two streams; mom_assemble covers the cell and row "
-                   "passes; bytes per the survey's per-kernel formulas with FP64 values")
+                   "passes; fine_refresh writes the split form's couplings in FP64, FP32 and FP16; FP64 values, "
+                   "4-byte indices")
     return out
-
-
-def sell_format_bytes(problem, s: int, sx: int | None = None) -> float:
-    """Bytes the SELL-32x4 fine operator actually streams per SpMV: padded
-    values (s B) and 16-bit column deltas (slice width rounded up to a
-    multiple of 4), slice offsets/widths, x and y (sx B each)."""
-    sx = s if sx is None else sx
-    row = problem.array("fine.row")
-    n = len(row) - 1
-    lens = np.diff(row)
-    ns = (n + 31) // 32
-    w = np.zeros(ns * 32, dtype=np.int64)
-    w[:n] = lens
-    widths = (w.reshape(ns, 32).max(axis=1) + 3) // 4 * 4
-    padded = int(widths.sum()) * 32
-    return padded * (s + 2) + 8 * ns + 2 * sx * n
 
 
 def _rel(a, b):
@@ -305,7 +295,7 @@ def run_nodals(args):
         raise RuntimeError(f"the fast solve did not converge ({rep.outer_its} iterations)")
     del S
 
-    # --- roofline: the dominant kernel, the V-cycle's fine-level SELL SpMV --
+    # --- roofline: the dominant product, the V-cycle's fine-level operator --
     # (FP16 values, FP32 vectors: 4 per inner iteration); the inner Krylov
     # product (FP32 values) and the FP64 defect product are reported beside it
     roof = None
@@ -319,24 +309,22 @@ def run_nodals(args):
         if c == 0:
             return None
         return {"avg_launch_ms": round(t / c, 5), "launches": c,
-                "achieved": round(fine_spmv_bytes(P, s_val, s_vec) / (t / c * 1e-3) / 1e9, 1)}
+                "achieved": round(split_bytes(P, s_val, s_vec) / (t / c * 1e-3) / 1e9, 1)}
     if args.profile_steps > 0 and calls > 0:
         avg_ms = tot / calls
         sv = 2 if half else 4
-        alg = fine_spmv_bytes(P, sv, 4)
-        fmt = sell_format_bytes(P, sv, 4)
+        alg = split_bytes(P, sv, 4)
         achieved = alg / (avg_ms * 1e-3) / 1e9
         roof = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                 "frac": round(achieved / peak, 4),
                 "traffic": _traffic("bytes_per_launch_pipe1m_half" if half else "bytes_per_launch_pipe1m_fp32"),
                 "peak_kind": peak_kind,
-                "kernel": ("fine Schur SELL-32x4 SpMV of the V-cycle (sell_spmv<float,*,*,__half>: FP16 values, "
-                           "16-bit column deltas, FP32 vectors): fine-level smoothing and residual steps") if half else
-                          "fine Schur SELL-32x4 SpMV in FP32 (sell_spmv<float,*>)",
+                "kernel": ("pressure operator in split form in the V-cycle (split_vertex, then split_cell<float,*,*,"
+                           "__half>: FP16 geometry and couplings, FP32 vectors): fine-level smoothing and residual "
+                           "steps, two launches a product") if half else
+                          "pressure operator in split form in FP32 (split_vertex, then split_cell<float,*,*,float>)",
                 "algorithmic_bytes_per_launch": int(alg),
-                "algorithmic_bytes_rule": f"nnz*({sv}+4) + 4(n+1) + 2*4*n (CSR index 4 B, value {sv} B, x and y once)",
-                "format_bytes_per_launch": int(fmt),
-                "format_frac": round(fmt / (avg_ms * 1e-3) / 1e9 / peak, 4),
+                "algorithmic_bytes_rule": "every array of the split form once (see split_bytes)",
                 "avg_launch_ms": round(avg_ms, 5), "launches": calls,
                 "timed_in": f"profiled pass of {args.profile_steps} steps after the timed steps",
                 "inner_krylov_spmv_fp32": side("fine_spmv_amg", 4, 4),
@@ -377,7 +365,7 @@ def run_nodals(args):
                        "pressure_s": round(rep.pressure_ms / 1e3, 3),
                        "step": "one SIMPLE outer iteration (ms_per_step: K timed iterations after W warm-up)",
                        "timed_steps_pressure_iterations": round(float(np.mean(p_its)), 2),
-                       "l2": "working set per step > 126 MB L2 (fine operator ~1 GB); no flush",
+                       "l2": "working set per step > 126 MB L2 (momentum matrix ~1 GB); no flush",
                        "parallelism": "replicas" if ws > 1 else "single GPU", "host_setup_s": round(setup_s, 3)},
             "field_rel_l2_vs_fp64": errors,
             "roofline": roof, "cpu_baseline": cpu,

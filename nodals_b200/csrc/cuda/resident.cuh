@@ -13,9 +13,9 @@
 // copied to shared memory too, as far as it fits (the V-cycle's first: four
 // of five products).  Bound by the chain of latencies in a step (shared
 // memory, FP64 arithmetic and shuffles, barrier), about 1.5 us each.
-// Microseconds of an iteration, loop of kernels / this: 720 cells FP64 42 /
-// 21, FP32 44 / 22; 2,400 cells FP64 43 / 25, mixed FP16 53 / 37; 4,608 cells
-// FP32 41 / 37.  One block instead of eight was tried: 34 at 720 cells, 93 at
+// Microseconds of an iteration, loop of kernels / this: 720 cells FP64 35.5 /
+// 20, FP32 37 / 20; 2,400 cells FP64 38 / 24, mixed FP16 45 / 30; 4,608 cells
+// FP32 35 / 35.  One block instead of eight was tried: 34 at 720 cells, 93 at
 // 2,400 (FP64); one block per SM meeting at barriers in global memory: 44 at
 // 720 cells, 57 to 65 at 48,000, no better than the kernels.
 //

@@ -2024,11 +2024,13 @@ class Solver final : public ISolver {
   }
   // The whole PCG loop as one kernel of one cluster (resident.cuh): the split
   // operator with a coarse level applied as a dense matrix, on meshes of up to
-  // kResidentCells cells whose vectors fit the cluster's shared memory: half
-  // the time of the loop of kernels on 720 to 2,400 cells, a tenth less (FP32
-  // and mixed) or the same (FP64) on 4,608, slower from about 6,000 on, where
-  // eight SMs no longer keep up.  NDS_RESIDENT overrides it (0: none).
-  static constexpr int kResidentCells = 5000;
+  // kResidentCells cells whose vectors fit the cluster's shared memory.
+  // Microseconds of an iteration, loop of kernels / this: 720 cells FP64 35.5 /
+  // 19.9, FP32 37 / 20, mixed FP16 46 / 30; 2,688 cells 37 / 29, 35.5 / 25.5,
+  // 41 / 30.5; 4,608 cells 38 / 42, 35 / 35, 42 / 40; at 9,600 cells half as
+  // fast, as eight SMs no longer keep up.  NDS_RESIDENT overrides the line (0:
+  // none).
+  static constexpr int kResidentCells = 4000;
   static constexpr size_t kResidentDense = (size_t)4 << 20;
   // entries of n per block (at least 2: res_inverse)
   static int res_part(int n) { return std::max(2, (n + k::kResCluster - 1) / k::kResCluster); }

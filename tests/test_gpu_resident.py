@@ -42,6 +42,7 @@ def test_resident_pcg_matches_the_loop(native, monkeypatch, case, mesh):
     P = native.Problem(m, **dict(CFG, **kw))
     if case.endswith("wide"):
         monkeypatch.setenv("NDS_SELL_COL32", "1")
+    monkeypatch.setenv("NDS_RESIDENT", "5000")  # also just above the size rule
     A, A2 = native.Solver(P), native.Solver(P)
     monkeypatch.setenv("NDS_RESIDENT", "0")
     B = native.Solver(P)

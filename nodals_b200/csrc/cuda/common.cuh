@@ -32,7 +32,12 @@ extern unsigned long long g_launches;
 // kernel of the stream writes between a full dependency (host
 // synchronisation, event wait, graph boundary) and itself: the kernels of the
 // pressure solve load their matrix entries there, constant during a solve, so
-// that these round trips overlap the previous kernel's end.
+// that these round trips overlap the previous kernel's end.  For the same
+// reason a pointer to memory that a kernel of such a chain writes is no
+// __restrict__ parameter where it is read: const __restrict__ lets the compiler
+// take its loads as invariant for the whole kernel, which begins before the
+// writer has ended, and move them above pdl_wait().  Constant data and outputs
+// that are only stored to keep the qualifier.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_begin() {

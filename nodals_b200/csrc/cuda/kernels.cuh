@@ -21,7 +21,7 @@ namespace k {
 // block partial reductions -> out[NV] (single block, fixed order)
 // ---------------------------------------------------------------------------
 template <int NV>
-__global__ void reduce_partials(const double* __restrict__ part, int nblocks, double* __restrict__ out) {
+__global__ void reduce_partials(const double* part, int nblocks, double* __restrict__ out) {
   pdl_begin();
   double v[NV];
 #pragma unroll
@@ -368,10 +368,10 @@ struct MomArgs {
   const uint32_t* __restrict__ inc;     // (cell << 3) | a
   const int32_t* __restrict__ ref;      // 8 per cell
   const uint8_t* __restrict__ slot;     // 64 per cell
-  const T* __restrict__ C;              // 8 per incidence: convection rows from mom_cell_conv
+  const T* C;              // 8 per incidence: convection rows from mom_cell_conv
   const uint8_t* __restrict__ slotz;    // 8 per incidence: slot[c][a][b] of incidence (c, a)
   const T* __restrict__ Bz;             // 3 per incidence: B[c][a]
-  const T* __restrict__ pz;             // per incidence: p_c (written by the cell pass)
+  const T* pz;             // per incidence: p_c (written by the cell pass)
   const uint8_t* __restrict__ fixz;     // per incidence: bit b set when dof b of the cell is fixed
   const T* __restrict__ bco;            // 24 per cell
   const T* __restrict__ fixed;          // 3 per fixed slot
@@ -581,10 +581,8 @@ constexpr int kGsAhead = 2;
 template <class T>
 __global__ void __launch_bounds__(kBlock, 6) mom_gs_color(int count, const int32_t* __restrict__ rows,
                                                        const int2* __restrict__ span, const int32_t* __restrict__ ci,
-                                                       const T* __restrict__ av, const T* __restrict__ diag,
-                                                       const T* __restrict__ b0, const T* __restrict__ b1,
-                                                       const T* __restrict__ b2, T* __restrict__ x0, T* __restrict__ x1,
-                                                       T* __restrict__ x2, T omega) {
+                                                       const T* av, const T* diag, const T* b0, const T* b1,
+                                                       const T* b2, T* x0, T* x1, T* x2, T omega) {
   pdl_begin();
   const int lane8 = threadIdx.x & 7;
   const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
@@ -680,8 +678,8 @@ __global__ void __launch_bounds__(kBlock) mom_audit(int n, const int2* __restric
 // ---------------------------------------------------------------------------
 template <class T, int VS = kVel>
 __global__ void __launch_bounds__(kBlock) continuity(int nc, const int32_t* __restrict__ ref, const T* __restrict__ bco,
-                                                     const T* __restrict__ fixed_div, const T* __restrict__ u0,
-                                                     const T* __restrict__ u1, const T* __restrict__ u2,
+                                                     const T* __restrict__ fixed_div, const T* u0,
+                                                     const T* u1, const T* u2,
                                                      T* __restrict__ rhs, double* __restrict__ part) {
   pdl_begin();
   double acc[1] = {0.0};
@@ -750,7 +748,7 @@ __device__ __forceinline__ int col_at(const int16_t* __restrict__ ci, int k, int
 // before pdl_wait().
 template <int G, class T, class MT = T, class CT = int32_t, bool WAIT = false>
 __device__ __forceinline__ T lane_batched_dot(int rb, int re, const CT* __restrict__ ci, const MT* __restrict__ v,
-                                              const T* __restrict__ x, int lane, int i = 0) {
+                                              const T* x, int lane, int i = 0) {
   T s = 0;
   int c[8];
   T a[8];
@@ -780,7 +778,7 @@ constexpr int kRowLanes = 32;
 // the previous kernel after loading the first entries)
 template <class T, class MT = T, class CT = int32_t, int GL = kRowLanes>
 __device__ __forceinline__ T group_row_dot(const int32_t* __restrict__ rp, const CT* __restrict__ ci,
-                                           const MT* __restrict__ v, const T* __restrict__ x, int i, int lane,
+                                           const MT* __restrict__ v, const T* x, int i, int lane,
                                            unsigned mask, bool live, T vinv = T(1)) {
   const int rb = live ? rp[i] : 0, re = live ? rp[i + 1] : 0;
   T s = group_sum<GL>(lane_batched_dot<GL, T, MT, CT, true>(rb, re, ci, v, x, lane, i), mask);
@@ -791,7 +789,7 @@ __device__ __forceinline__ T group_row_dot(const int32_t* __restrict__ rp, const
 // y = A x (GL lanes per row)
 template <class T, class MT = T, class CT = int32_t, int GL = kRowLanes>
 __global__ void __launch_bounds__(kBlock) spmv(int n, const int32_t* __restrict__ rp, const CT* __restrict__ ci,
-                                               const MT* __restrict__ v, const T* __restrict__ x, T* __restrict__ y,
+                                               const MT* __restrict__ v, const T* x, T* __restrict__ y,
                                                T vinv = T(1)) {
   pdl_trigger();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -803,8 +801,8 @@ __global__ void __launch_bounds__(kBlock) spmv(int n, const int32_t* __restrict_
 // r = b - A x  (optionally also r2 = r)
 template <class T, class MT = T, class CT = int32_t, int GL = kRowLanes>
 __global__ void __launch_bounds__(kBlock) spmv_resid(int n, const int32_t* __restrict__ rp, const CT* __restrict__ ci,
-                                                     const MT* __restrict__ v, const T* __restrict__ x,
-                                                     const T* __restrict__ b, T* __restrict__ r, T* __restrict__ r2,
+                                                     const MT* __restrict__ v, const T* x,
+                                                     const T* b, T* __restrict__ r, T* __restrict__ r2,
                                                      const T* __restrict__ den, T w, T vinv = T(1)) {
   pdl_trigger();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -823,9 +821,9 @@ __global__ void __launch_bounds__(kBlock) spmv_resid(int n, const int32_t* __res
 template <class T, class MT = T, class CT = int32_t, int GL = kRowLanes>
 __global__ void __launch_bounds__(kBlock) spmv_smooth(int n, const int32_t* __restrict__ rp,
                                                       const CT* __restrict__ ci, const MT* __restrict__ v,
-                                                      const T* __restrict__ xin, const T* __restrict__ b,
+                                                      const T* xin, const T* b,
                                                       const T* __restrict__ den, T w, T* __restrict__ xout,
-                                                      T* __restrict__ add_to, T vinv = T(1)) {
+                                                      T* add_to, T vinv = T(1)) {
   pdl_trigger();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int i = t / GL, lane = t % GL;
@@ -855,7 +853,7 @@ enum { LEV_Y = 0, LEV_RESID = 1, LEV_SMOOTH = 2 };
 // a 16-byte boundary: vector loads, eight in flight (x from cudaMalloc, padded
 // reads stay inside [lo4, hi))
 template <int BLOCK, class T>
-__device__ __forceinline__ void stage_window(T* __restrict__ sx, const T* __restrict__ x, int lo4, int hi) {
+__device__ __forceinline__ void stage_window(T* __restrict__ sx, const T* x, int lo4, int hi) {
   constexpr int W = 16 / sizeof(T);
   using V = typename std::conditional<std::is_same<T, float>::value, float4, double2>::type;
   const int nv = (hi - lo4) / W;
@@ -869,9 +867,9 @@ constexpr int kWinBlock = 512, kWinPerSm = 2, kWinAhead = 10;
 template <int MODE, class CT>
 __global__ void __launch_bounds__(kWinBlock, kWinPerSm)
     level_window(int n, int rows, const int2* __restrict__ win, const int32_t* __restrict__ rp,
-                 const CT* __restrict__ ci, const double* __restrict__ v, const double* __restrict__ x,
-                 const double* __restrict__ b, const double* __restrict__ den, double w, double* __restrict__ y,
-                 double* __restrict__ y2) {
+                 const CT* __restrict__ ci, const double* __restrict__ v, const double* x,
+                 const double* b, const double* __restrict__ den, double w, double* __restrict__ y,
+                 double* y2) {
   using T = double;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* sx = reinterpret_cast<T*>(smem_raw);
@@ -941,13 +939,13 @@ __global__ void __launch_bounds__(kWinBlock, kWinPerSm)
 // vector kernels (g5e_fp32_kernels.cuh:132-150, vector_kernels.cuh)
 // ---------------------------------------------------------------------------
 template <class T>
-__global__ void jacobi_zero(int n, T w, const T* __restrict__ b, const T* __restrict__ d, T* __restrict__ x) {
+__global__ void jacobi_zero(int n, T w, const T* b, const T* __restrict__ d, T* __restrict__ x) {
   pdl_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) x[i] = w * b[i] / d[i];
 }
 template <class T>
-__global__ void axpy(int n, T a, const T* __restrict__ x, T* __restrict__ y) {
+__global__ void axpy(int n, T a, const T* x, T* y) {
   pdl_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) y[i] += a * x[i];
@@ -978,7 +976,7 @@ __global__ void power_init(int n, T* __restrict__ v) {
 
 // partial sums of x.y
 template <class T, class U = T>
-__global__ void __launch_bounds__(kBlock) dot(int n, const T* __restrict__ x, const U* __restrict__ y,
+__global__ void __launch_bounds__(kBlock) dot(int n, const T* x, const U* y,
                                               double* __restrict__ part) {
   pdl_begin();
   double acc[1] = {0.0};
@@ -1022,8 +1020,8 @@ __device__ __forceinline__ void pcg_rho_step(double* __restrict__ sc, int* __res
 }
 // p = z on the first iteration, else p = z + beta p
 template <class T, class Z = T>
-__global__ void p_update_dev(int n, const double* __restrict__ beta_dev, const int* __restrict__ ctl,
-                             const Z* __restrict__ z, T* __restrict__ p) {
+__global__ void p_update_dev(int n, const double* beta_dev, const int* ctl,
+                             const Z* z, T* p) {
   pdl_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -1097,7 +1095,7 @@ struct PcgScalars {
   HostWords host;
 };
 template <int STEP>
-__global__ void reduce_pcg(const double* __restrict__ part, int nblocks, double* __restrict__ out, PcgScalars s) {
+__global__ void reduce_pcg(const double* part, int nblocks, double* __restrict__ out, PcgScalars s) {
   pdl_begin();
   double v[1] = {0.0};
   for (int b = threadIdx.x; b < nblocks; b += blockDim.x) v[0] += part[b];
@@ -1151,7 +1149,7 @@ __device__ __forceinline__ void reduce_tail(double value, const ReduceTail& t) {
 
 // x.y with the reduction tail STEP
 template <class T, class U, int STEP>
-__global__ void __launch_bounds__(kBlock) dot_step(int n, const T* __restrict__ x, const U* __restrict__ y,
+__global__ void __launch_bounds__(kBlock) dot_step(int n, const T* x, const U* y,
                                                    ReduceTail tail) {
   pdl_begin();
   double acc = 0.0;
@@ -1162,7 +1160,7 @@ __global__ void __launch_bounds__(kBlock) dot_step(int n, const T* __restrict__ 
 
 // Start of a pressure solve: r = b, x = 0, and ||b||^2 (SUM_ONLY tail)
 template <class T>
-__global__ void __launch_bounds__(kBlock) solve_start(int n, const T* __restrict__ b, T* __restrict__ r,
+__global__ void __launch_bounds__(kBlock) solve_start(int n, const T* b, T* __restrict__ r,
                                                       T* __restrict__ x, ReduceTail tail) {
   pdl_begin();
   double acc = 0.0;
@@ -1179,7 +1177,7 @@ __global__ void __launch_bounds__(kBlock) solve_start(int n, const T* __restrict
 // with rA the residual in the preconditioner's precision, and with x1 the
 // first (diagonal) step of its fine pre-smoother on it, x1 = w0 r / den0.
 template <class R, class S, class TA>
-__global__ void loop_start(int n, const R* __restrict__ r, double s, S* __restrict__ rs, S* __restrict__ rs2,
+__global__ void loop_start(int n, const R* r, double s, S* __restrict__ rs, S* __restrict__ rs2,
                            S* __restrict__ x, TA* __restrict__ rA, const TA* __restrict__ den0, TA w0,
                            TA* __restrict__ x1, SolveInit init) {
   pdl_begin();
@@ -1202,17 +1200,18 @@ __global__ void loop_start(int n, const R* __restrict__ r, double s, S* __restri
 // precision (x1 from it).  STEP PCG_CHECK: the reduction and the stopping
 // test by the last block; 0: partials only (to tail.part).
 template <class T, class TA, int STEP>
-__global__ void __launch_bounds__(kBlock) xr_update(int n, double alpha, const double* __restrict__ alpha_dev,
-                                                    const T* __restrict__ p, const T* __restrict__ q,
-                                                    T* __restrict__ x, T* __restrict__ r,
+__global__ void __launch_bounds__(kBlock) xr_update(int n, double alpha, const double* alpha_dev,
+                                                    const T* p, const T* q,
+                                                    T* x, T* r,
                                                     ReduceTail tail, const TA* __restrict__ den0, TA w0,
                                                     TA* __restrict__ x1, TA* __restrict__ rA) {
   pdl_begin();
   const T a = T(alpha_dev ? *alpha_dev : alpha);
   double acc[1] = {0.0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    x[i] += a * p[i];
-    const T rr = r[i] - a * q[i];
+    const T pi = p[i], qi = q[i], xi = x[i], ri = r[i];
+    x[i] = xi + a * pi;
+    const T rr = ri - a * qi;
     r[i] = rr;
     if (x1) {
       const TA ra = TA(rr);
@@ -1235,7 +1234,7 @@ __global__ void __launch_bounds__(kBlock) xr_update(int n, double alpha, const d
 // with four entries ahead.
 template <class T>
 __global__ void prolong_add(int nf, int pw, const int32_t* __restrict__ pc, const T* __restrict__ pv,
-                            const T* __restrict__ c, T* __restrict__ f) {
+                            const T* c, T* f) {
   pdl_trigger();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const size_t n = (size_t)nf;
@@ -1347,7 +1346,7 @@ __global__ void block_add(size_t total, const T* __restrict__ x, T* __restrict__
 constexpr int kDenseWarps = 4;
 template <class T>
 __global__ void __launch_bounds__(32 * kDenseWarps) dense_rows(int n, int ld, const T* __restrict__ A,
-                                                               const T* __restrict__ b, T* __restrict__ x) {
+                                                               const T* b, T* __restrict__ x) {
   pdl_trigger();
   constexpr int W = 16 / sizeof(T), step = 32 * kDenseWarps, ahead = 4;
   using V = typename std::conditional<std::is_same<T, float>::value, float4, double2>::type;
@@ -1498,7 +1497,7 @@ enum SellMode { SELL_Y = 0, SELL_RESID = 1, SELL_SMOOTH = 2, SELL_DOT = 3 };
 // s1; the last w mod 8 entries (and the zero padding) go to s0 in order.
 // Fixed order -> deterministic.
 template <class T, bool D16, class MT = T>
-__device__ __forceinline__ T sell_row(const Sell& A, const MT* __restrict__ v, const T* __restrict__ x, int i) {
+__device__ __forceinline__ T sell_row(const Sell& A, const MT* __restrict__ v, const T* x, int i) {
   const int s = i >> 5, lane = i & 31;
   const int b = A.base[s];
   const int w = A.width[s];
@@ -1564,9 +1563,9 @@ __device__ __forceinline__ T sell_row(const Sell& A, const MT* __restrict__ v, c
 // MT: the operator's value type (T, or __half for the FP16 copy whose values
 // are a s, with vinv = 1 / s: a power of two, so the product is exact)
 template <class T, int MODE, bool D16, class MT = T>
-__global__ void __launch_bounds__(kBlock, 8) sell_spmv(Sell A, const MT* __restrict__ v, const T* __restrict__ x,
-                                                    const T* __restrict__ b, const T* __restrict__ den, T w,
-                                                    T* __restrict__ y, T* __restrict__ y2, double* __restrict__ part,
+__global__ void __launch_bounds__(kBlock, 8) sell_spmv(Sell A, const MT* __restrict__ v, const T* x,
+                                                    const T* b, const T* __restrict__ den, T w,
+                                                    T* __restrict__ y, T* y2, double* __restrict__ part,
                                                     T vinv = T(1)) {
   pdl_begin();
   if (MODE == SELL_DOT) {
@@ -1732,7 +1731,7 @@ __global__ void __launch_bounds__(kRefreshBlock) sell_refresh(int nc, const int3
 }
 
 template <class Tin, class Tout>
-__global__ void cast_copy(int n, const Tin* __restrict__ a, Tout* __restrict__ b) {
+__global__ void cast_copy(int n, const Tin* a, Tout* __restrict__ b) {
   pdl_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) b[i] = Tout(a[i]);
@@ -1740,7 +1739,7 @@ __global__ void cast_copy(int n, const Tin* __restrict__ a, Tout* __restrict__ b
 // b = a in the other precision, and the fine pre-smoother's diagonal step
 // x1 = w0 b / den0
 template <class Tin, class Tout>
-__global__ void cast_jacobi(int n, const Tin* __restrict__ a, Tout* __restrict__ b, Tout w0,
+__global__ void cast_jacobi(int n, const Tin* a, Tout* __restrict__ b, Tout w0,
                             const Tout* __restrict__ den0, Tout* __restrict__ x1) {
   pdl_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1781,7 +1780,7 @@ constexpr int rest_blocks() { return sizeof(T) == 8 ? 4 : 6; }  // per SM
 template <class T>
 __global__ void __launch_bounds__(kBlock, rest_blocks<T>()) restrict_stream(int nc, const int32_t* __restrict__ rr,
                                                              const int32_t* __restrict__ rc, const T* __restrict__ rv,
-                                                             const T* __restrict__ f, T* __restrict__ c,
+                                                             const T* f, T* __restrict__ c,
                                                              const T* __restrict__ den0, T w0, T* __restrict__ x1) {
   pdl_trigger();
   const int lane = threadIdx.x & 31, stride = gridDim.x * kWarps;
@@ -1834,7 +1833,7 @@ __global__ void __launch_bounds__(kBlock, rest_blocks<T>()) restrict_stream(int 
 template <class T, int GL = kRowLanes>
 __global__ void __launch_bounds__(kBlock) restrict_rows(int nc, const int32_t* __restrict__ rr,
                                                         const int32_t* __restrict__ rc, const T* __restrict__ rv,
-                                                        const T* __restrict__ f, T* __restrict__ c,
+                                                        const T* f, T* __restrict__ c,
                                                         const T* __restrict__ den0, T w0, T* __restrict__ x1) {
   pdl_trigger();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;

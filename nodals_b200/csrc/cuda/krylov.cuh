@@ -25,7 +25,7 @@ namespace nds {
 namespace k {
 
 // x += s y (y in FP32, x in FP64)
-__global__ void axpy_from_float(int n, double s, const float* __restrict__ y, double* __restrict__ x) {
+__global__ void axpy_from_float(int n, double s, const float* y, double* x) {
   pdl_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) x[i] += s * (double)y[i];
@@ -50,7 +50,7 @@ struct FgLayout {
 };
 
 // Z[ctl[0]] = z
-__global__ void fg_store(int n, const float* __restrict__ z, const int* __restrict__ ctl, float* __restrict__ Z) {
+__global__ void fg_store(int n, const float* z, const int* ctl, float* __restrict__ Z) {
   pdl_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) Z[(size_t)ctl[0] * n + i] = z[i];
@@ -117,9 +117,9 @@ __device__ __forceinline__ void fg_givens(double* __restrict__ fg, const FgLayou
 // gridDim.y, ...; each vector's block partials (part[i gridDim.x + block]) are
 // added in order by the vector's last block (tickets, zero between launches)
 constexpr int kDotRows = 8;
-__global__ void __launch_bounds__(kBlock) fg_dots(int n, const float* __restrict__ V, const float* __restrict__ w,
-                                                  const int* __restrict__ ctl, double* __restrict__ part,
-                                                  unsigned* __restrict__ tickets, FgLayout L, double* __restrict__ fg) {
+__global__ void __launch_bounds__(kBlock) fg_dots(int n, const float* V, const float* w,
+                                                  const int* ctl, double* part,
+                                                  unsigned* tickets, FgLayout L, double* __restrict__ fg) {
   pdl_begin();
   __shared__ bool last;
   const int j = ctl[0];
@@ -150,9 +150,9 @@ __global__ void __launch_bounds__(kBlock) fg_dots(int n, const float* __restrict
 }
 // w -= sum_{i <= j} H[i][j] V_i (FP64 sums, FP32 storage) and ||w||^2, whose
 // last block then takes the Givens step
-__global__ void __launch_bounds__(kBlock) fg_orth(int n, const float* __restrict__ V, double* __restrict__ fg,
-                                                  FgLayout L, float* __restrict__ w, double* __restrict__ part,
-                                                  unsigned* __restrict__ ticket, FgScalars a) {
+__global__ void __launch_bounds__(kBlock) fg_orth(int n, const float* V, double* fg,
+                                                  FgLayout L, float* w, double* part,
+                                                  unsigned* ticket, FgScalars a) {
   pdl_begin();
   __shared__ bool last;
   const int j = a.ctl[0];
@@ -185,8 +185,8 @@ __global__ void __launch_bounds__(kBlock) fg_orth(int n, const float* __restrict
 }
 // v = w / ||w|| (zero when ||w|| = 0) into V[ctl[0]] and into the next
 // preconditioner input; with x1 also the first step of its fine pre-smoother
-__global__ void fg_normalize(int n, const float* __restrict__ w, const double* __restrict__ sc, int wn_slot,
-                             const int* __restrict__ ctl, float* __restrict__ V, float* __restrict__ in,
+__global__ void fg_normalize(int n, const float* w, const double* sc, int wn_slot,
+                             const int* ctl, float* __restrict__ V, float* __restrict__ in,
                              const float* __restrict__ den0, float w0, float* __restrict__ x1) {
   pdl_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -235,8 +235,8 @@ __global__ void fg_combine(int n, const float* __restrict__ Z, const double* __r
 constexpr int kMaxGuess = 8;
 // partials, per block: G (upper triangle, row-major a <= b) then f
 template <int K>
-__global__ void __launch_bounds__(kBlock) guess_dots(int n, const double* __restrict__ Y, const double* __restrict__ W,
-                                                     const double* __restrict__ b, double* __restrict__ part) {
+__global__ void __launch_bounds__(kBlock) guess_dots(int n, const double* Y, const double* W,
+                                                     const double* b, double* __restrict__ part) {
   pdl_begin();
   constexpr int NG = K * (K + 1) / 2 + K;
   double acc[NG];
@@ -266,7 +266,7 @@ struct GuessCoef {
   double c[K];
 };
 template <int K>
-__global__ void guess_combine(int n, const double* __restrict__ Y, GuessCoef<K> coef, double* __restrict__ x) {
+__global__ void guess_combine(int n, const double* Y, GuessCoef<K> coef, double* __restrict__ x) {
   pdl_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -276,8 +276,8 @@ __global__ void guess_combine(int n, const double* __restrict__ Y, GuessCoef<K> 
   x[i] = xs;
 }
 // the stored product of a new correction: w = b - r (= A x for r = b - A x)
-__global__ void guess_store(int n, const double* __restrict__ x, const double* __restrict__ b,
-                            const double* __restrict__ r, double* __restrict__ y, double* __restrict__ w) {
+__global__ void guess_store(int n, const double* x, const double* b,
+                            const double* r, double* __restrict__ y, double* __restrict__ w) {
   pdl_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;

@@ -111,7 +111,7 @@ template <int REC>
 constexpr int split_vertex_blocks() { return REC == REC_SOA ? 3 : REC == REC_16 ? 4 : 5; }  // per SM
 template <class V, int REC>
 __global__ void __launch_bounds__(kBlock, split_vertex_blocks<REC>())
-    split_vertex(SplitVerts a, const V* __restrict__ rau, const V* __restrict__ x, V* __restrict__ w, V scale) {
+    split_vertex(SplitVerts a, const V* __restrict__ rau, const V* x, V* __restrict__ w, V scale) {
   pdl_trigger();
   constexpr bool PIPE = REC != REC_SOA;  // the next vertex's records in registers
   const int t = blockIdx.x * blockDim.x + threadIdx.x, stride = (gridDim.x * blockDim.x) >> 3;
@@ -215,14 +215,14 @@ struct SplitCells {
 // a vector read as it is
 template <class V>
 struct PlainVector {
-  const V* __restrict__ x;
+  const V* x;
   __device__ __forceinline__ V operator()(int c) const { return x[c]; }
 };
 
 // the vertex sums of split_vertex
 template <class V>
 struct PlainVertices {
-  const V* __restrict__ w;
+  const V* w;
   __device__ __forceinline__ void operator()(int v, V (&o)[3]) const {
     if constexpr (std::is_same<V, float>::value) {
       const float4 u = reinterpret_cast<const float4*>(w)[v];
@@ -361,11 +361,11 @@ __device__ __forceinline__ V split_row(const SplitCells& a, const X& x, const W&
 // STEP PCG_RHO (SMOOTH with y2, the last step
 // of the V-cycle): also r.z of the new z = y2 with the reduction tail.
 template <class V, int MODE, bool D16, class MT, int STEP = 0, class R = V>
-__global__ void __launch_bounds__(kBlock) split_cell(SplitCells a, const V* __restrict__ w, const V* __restrict__ x,
-                                                     const V* __restrict__ b, const V* __restrict__ den, V wt,
-                                                     V* __restrict__ y, V* __restrict__ y2, V tinv,
-                                                     const R* __restrict__ rr, ReduceTail tail,
-                                                     const int* __restrict__ at) {
+__global__ void __launch_bounds__(kBlock) split_cell(SplitCells a, const V* w, const V* x,
+                                                     const V* b, const V* __restrict__ den, V wt,
+                                                     V* __restrict__ y, V* y2, V tinv,
+                                                     const R* rr, ReduceTail tail,
+                                                     const int* at) {
   pdl_trigger();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   double acc = 0.0;
@@ -405,8 +405,8 @@ __global__ void __launch_bounds__(kBlock) split_cell(SplitCells a, const V* __re
 // q = A p with p.q and the step alpha of PCG (grid-stride; the data type of
 // the operator is that of the vectors)
 template <class V, bool D16>
-__global__ void __launch_bounds__(kBlock) split_cell_dot(SplitCells a, const V* __restrict__ w,
-                                                         const V* __restrict__ p, V* __restrict__ q, V tinv,
+__global__ void __launch_bounds__(kBlock) split_cell_dot(SplitCells a, const V* w,
+                                                         const V* p, V* __restrict__ q, V tinv,
                                                          ReduceTail tail) {
   pdl_trigger();
   double acc = 0.0;

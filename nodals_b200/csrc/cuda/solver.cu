@@ -914,8 +914,10 @@ class Solver final : public ISolver {
       NDS_CUDA(cudaMemset(sp_wA_.p, 0, sp_wA_.bytes()));
     }
     if (half) {
-      // B scaled by the power of two that puts its largest component at
-      // 2^14 .. 2^15 (the smallest normal half is 2^29 below)
+      // B of the free vertices scaled by the power of two that puts its largest
+      // component at 2^14 .. 2^15 (the smallest normal half is 2^29 below).  A
+      // fixed vertex's vector may be larger than a half holds; its w is zero,
+      // so a cell keeps zero for it.
       double bmax = 0.0;
 #pragma omp parallel for schedule(static) reduction(max : bmax)
       for (size_t z = 0; z < nz; ++z)
@@ -957,8 +959,10 @@ class Solver final : public ISolver {
 #pragma omp parallel for schedule(static)
       for (int c = 0; c < nc_; ++c) {
         unsigned w[6];
-        for (int k = 0; k < 6; ++k)
-          w[k] = bits(h(vert(c, 2 * k / 3, 2 * k % 3))) | bits(h(vert(c, (2 * k + 1) / 3, (2 * k + 1) % 3))) << 16;
+        auto value = [&](int q) {
+          return S.ref[8 * (size_t)c + (size_t)(q / 3)] >= 0 ? bits(h(vert(c, q / 3, q % 3))) : 0u;
+        };
+        for (int k = 0; k < 6; ++k) w[k] = value(2 * k) | value(2 * k + 1) << 16;
         p[(size_t)c] = make_uint4(w[0], w[1], w[2], w[3]);
         q[(size_t)c] = make_uint2(w[4], w[5]);
       }

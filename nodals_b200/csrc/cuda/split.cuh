@@ -199,7 +199,8 @@ __global__ void __launch_bounds__(kBlock, split_vertex_blocks<REC>())
 //  none) when they all fit; tau: the four face couplings (0 on a fixed face).
 //  geo: B of the vertices 1, 2, 3 (the four sum to zero): float 4 + 4 + 1,
 //  double 2 + 2 + 2 + 2 + 1; __half: all four, scaled, in 8 + 4 values, each
-//  rounded as in the vertex records, so that the FP16 operator is symmetric.
+//  rounded as in the vertex records, so that the FP16 operator is symmetric
+//  (zero for a fixed vertex).
 //  A free face without a neighbour (outlet) couples as tau x_c.
 struct SplitCells {
   int n = 0;

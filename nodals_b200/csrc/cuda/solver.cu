@@ -2033,7 +2033,8 @@ class Solver final : public ISolver {
   // 19.9, FP32 37 / 20, mixed FP16 46 / 30; 2,688 cells 37 / 29, 35.5 / 25.5,
   // 41 / 30.5; 4,608 cells 38 / 42, 35 / 35, 42 / 40; at 9,600 cells half as
   // fast, as eight SMs no longer keep up.  NDS_RESIDENT overrides the line (0:
-  // none).
+  // none).  It is an ordinary launch, taken with graphs off and under the
+  // profiler too, so that those runs have the same sums.
   static constexpr int kResidentCells = 4000;
   static constexpr size_t kResidentDense = (size_t)4 << 20;
   // entries of n per block (at least 2: res_inverse)
@@ -2041,7 +2042,7 @@ class Solver final : public ISolver {
   void plan_resident() {
     resident_ = false;
     const bool dense0 = dense_level_ == 0 || L_.size() == 1;
-    if (!split_ || !use_graphs_ || !dense0 || o_.learned || (mixed_ && fg_m_ > 0)) return;
+    if (!split_ || !dense0 || o_.learned || (mixed_ && fg_m_ > 0)) return;
     if (o_.pressure_solver != NDS_P_PCG || fine_plan().m >= k::kResSteps) return;
     int cells = kResidentCells;
     if (const char* e = std::getenv("NDS_RESIDENT")) cells = std::atoi(e);

@@ -10,7 +10,9 @@ V-cycle); ``fp64`` and ``amg_fp32`` are the plain FP64 path and the FP32
 V-cycle inside FP64 PCG.  The physical and solver controls are those of the
 benchmark (Re 100, alpha_u 0.7, alpha_p 0.3, SA + Chebyshev(2), pressure
 rtol 1e-6).  ``NDS_NO_GRAPHS=1`` in the environment makes the pressure loops
-launch kernel by kernel, which profilers need to see them one by one.
+launch kernel by kernel, which profilers need to see them one by one
+(``NDS_RESIDENT=0`` as well on meshes up to 4,000 cells, whose PCG is one
+kernel otherwise).
 """
 from __future__ import annotations
 

@@ -8,6 +8,7 @@ cells per thread; the smoother's degrees 1 (Jacobi), 2, 3 and 4.
 """
 from __future__ import annotations
 
+import numpy as np
 import pytest
 
 from conftest import rel_l2
@@ -54,3 +55,25 @@ def test_resident_pcg_matches_the_loop(native, monkeypatch, case, mesh):
             assert a.p_its == b.p_its
     for x, y in zip(A.fields(), B.fields()):
         assert rel_l2(x, y) <= tol_field
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mesh", [(2, 8, 7), (3, 16, 12)], ids=["one_kernel", "loop"])
+@pytest.mark.parametrize("case", ["fp64", "mixed_half"])
+def test_graphs_off_runs_the_same_solves(native, monkeypatch, case, mesh):
+    """NDS_NO_GRAPHS=1 and the profiler keep the form a solver takes by its
+    size: bitwise-equal runs (840 cells: one kernel; 4,608: the loop)."""
+    from nodals_b200 import meshgen
+    nr, nt, nz = mesh
+    m = native.Mesh.from_tetmesh(meshgen.pipe_mesh(nr=nr, ntheta=nt, nz=nz, length=0.5 * nz, jitter=0.05, seed=nz))
+    P = native.Problem(m, **dict(CFG, **CASES[case][0]))
+    A, C = native.Solver(P), native.Solver(P)
+    C.profile(True)
+    monkeypatch.setenv("NDS_NO_GRAPHS", "1")
+    B = native.Solver(P)
+    for _ in range(4):
+        a, b, c = A.step(), B.step(), C.step()
+        assert (a.p_its, a.rel_cont, a.p_rel) == (b.p_its, b.rel_cont, b.p_rel) == (c.p_its, c.rel_cont, c.p_rel)
+    assert (C.profile_read()["pcg_resident"][0] > 0) == (mesh[0] == 2)
+    for x, y, z in zip(A.fields(), B.fields(), C.fields()):
+        assert np.array_equal(x, y) and np.array_equal(x, z)

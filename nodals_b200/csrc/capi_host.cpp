@@ -814,6 +814,8 @@ void Problem::index_arrays() {
     auto& t = scalars["centT"];
     t.assign(&RT.T[0][0][0][0], &RT.T[0][0][0][0] + 8 * 8 * 8 * 3);
     A["centT"] = view(t, 0);
+    scalars["convTable"] = conv_table();
+    A["convTable"] = view(scalars["convTable"], 0);
     auto& dd = scalars["diffT"];
     dd.assign(&RT.D[0][0][0][0], &RT.D[0][0][0][0] + 8 * 8 * 3 * 3);
     A["diffT"] = view(dd, 0);

@@ -12,6 +12,7 @@
 #include <cstdint>
 #include <type_traits>
 
+#include "../host/fem.hpp"
 #include "common.cuh"
 
 namespace nds {
@@ -119,41 +120,21 @@ __device__ __forceinline__ void conv_record(const T* __restrict__ t, T& n0, T& n
 }
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-// the records (three N and M of column pair i) of the pairs a <= m in shared
-// memory, from the reference tensor T[a][m][b][j] = int phi_a phi_m dphi_b/dxi_j
-constexpr int kConvTable = 36 * 16;
+// the records (three N and M of column pair i) of the pairs a <= m in shared memory
 template <class T>
-__device__ __forceinline__ void conv_table(T* __restrict__ sN, const T* __restrict__ centT) {
-  for (int e = threadIdx.x; e < kConvTable; e += blockDim.x) {
-    const int i = (e >> 2) & 3, q = e & 3;
-    int a = 0, m = e >> 4;  // pair index -> a <= m
-    while (m >= 8 - a) {
-      m -= 8 - a;
-      ++a;
-    }
-    m += a;
-    const T* t = centT + ((a * 8 + m) * 8 + 4 + i) * 3;  // T[a][m][4+i][.] = N_ij - N_i0
-    T v;
-    if (q == 3) {
-      v = centT[((a * 8 + m) * 8 + 1) * 3];  // M: phi_1 = lambda_1
-    } else {
-      const int k = q + (q >= i);  // the q-th k != i
-      const T n0 = i == 0 ? T(0) : -t[i - 1];
-      v = k == 0 ? n0 : t[k - 1] + n0;
-    }
-    sN[e] = v;
-  }
+__device__ __forceinline__ void conv_load(T* __restrict__ sN, const T* __restrict__ table) {
+  for (int e = threadIdx.x; e < kConvTable; e += blockDim.x) sN[e] = table[e];
 }
 template <class T>
 __global__ void __launch_bounds__(kBlock, 2) mom_cell_conv(int nc, const int32_t* __restrict__ ref,
                                                             const T* __restrict__ fixed, const T* __restrict__ u0,
                                                             const T* __restrict__ u1, const T* __restrict__ u2,
                                                             const T* __restrict__ invJ, const T* __restrict__ det,
-                                                            const T* __restrict__ centT,
+                                                            const T* __restrict__ table,
                                                             const int32_t* __restrict__ zpos, T* __restrict__ C,
                                                             const T* __restrict__ p, T* __restrict__ pz) {
   __shared__ __align__(16) T sN[kConvTable];
-  conv_table(sN, centT);
+  conv_load(sN, table);
   __syncthreads();
   const int i = threadIdx.x & 3;
   const unsigned mask = 0xFu << (threadIdx.x & 28);
@@ -385,7 +366,7 @@ struct MomArgs {
   // fused form (no cell pass): C rows are evaluated per incidence
   const T* __restrict__ invJ;           // 9 per cell
   const T* __restrict__ det;            // 1 per cell
-  const T* __restrict__ centT;          // reference tensor T[8][8][8][3]
+  const T* __restrict__ table;          // convection records (conv_table)
   T alpha_u, rau_scale;
   int row_cap;                          // shared row buffer length per group
   T* __restrict__ A;
@@ -457,7 +438,7 @@ __global__ void __launch_bounds__(kBlock) mom_assemble(MomArgs<T> g) {
   T* buf = sRow + (size_t)grp * g.row_cap;
   T* sT = sRow + (size_t)groups * g.row_cap;
   if (FUSED) {
-    conv_table(sT, g.centT);
+    conv_load(sT, g.table);
     __syncthreads();
   }
   const unsigned gmask = group8_mask();

@@ -408,12 +408,7 @@ class Solver final : public ISolver {
     p_.alloc((size_t)nc_);
     color_rows_.upload(S.color_rows);
     color_off_ = S.color_off;
-    {
-      const RefTensors& RT = ref_tensors();
-      std::vector<double> t(1536);
-      std::memcpy(t.data(), &RT.T[0][0][0][0], sizeof(double) * 1536);
-      centT_.upload(t);
-    }
+    conv_table_.upload(conv_table());
     row_cap_ = 8;
     for (int i = 0; i < nv_; ++i) row_cap_ = std::max<int>(row_cap_, (int)(S.mom.row[(size_t)i + 1] - S.mom.row[(size_t)i]));
     row_cap_ = (row_cap_ + 7) / 8 * 8;
@@ -421,7 +416,7 @@ class Solver final : public ISolver {
     if (mom_smem_ > 200 * 1024) throw std::runtime_error("momentum row too long for the shared-memory assembly buffer");
     NDS_CUDA(cudaFuncSetAttribute(k::mom_assemble<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mom_smem_));
     NDS_CUDA(cudaFuncSetAttribute(k::mom_assemble<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)(mom_smem_ + k::kConvTable * sizeof(T))));
+                                  (int)(mom_smem_ + kConvTable * sizeof(T))));
     // The two-pass assembly by default: the cell pass writes each cell's
     // convection block row by row into the incidence slots of the velocity
     // rows (8 values per incidence, contiguous per row), the row pass
@@ -2706,19 +2701,19 @@ class Solver final : public ISolver {
     a.b2 = b_[2].p;
     a.invJ = invJ_.p;
     a.det = det_.p;
-    a.centT = centT_.p;
+    a.table = conv_table_.p;
     ProfScope ps(prof, st_, P_ASSEMBLE);
     if (fused_assembly_) {
       // one pass: each incidence's convection row is evaluated in place
-      pdl_launch(k::mom_assemble<T, 1>, grid_for(nv_, kBlock / 8), kBlock, mom_smem_ + k::kConvTable * sizeof(T), st_, a);
+      pdl_launch(k::mom_assemble<T, 1>, grid_for(nv_, kBlock / 8), kBlock, mom_smem_ + kConvTable * sizeof(T), st_, a);
       NDS_LAUNCH();
       return;
     }
     // cell blocks: a grid of 8 blocks per SM amortises the shared tensor load
     k::SupgArgs sa{P_.setup.pipe.nu, o_.supg_tau_scale, o_.supg_magic};
     const int gc = std::min(grid_for(nc_, kBlock / 4), 4 * kSms);
-    k::mom_cell_conv<T><<<gc, kBlock, 0, st_>>>(nc_, ref_.p, fixed_.p, uc(0), uc(1), uc(2), invJ_.p, det_.p, centT_.p,
-                                                 zpos_.p, cconv_.p, p_.p, pz_.p);
+    k::mom_cell_conv<T><<<gc, kBlock, 0, st_>>>(nc_, ref_.p, fixed_.p, uc(0), uc(1), uc(2), invJ_.p, det_.p,
+                                                 conv_table_.p, zpos_.p, cconv_.p, p_.p, pz_.p);
     if (o_.supg) {
       NDS_LAUNCH();
       k::mom_cell_supg<T><<<gc, kBlock, 0, st_>>>(nc_, ref_.p, fixed_.p, uc(0), uc(1), uc(2), invJ_.p, det_.p, zpos_.p,
@@ -3050,7 +3045,7 @@ class Solver final : public ISolver {
   DBuf<uint32_t> inc_;
   DBuf<int32_t> zpos_;  // incidence of (cell, basis), -1 for a fixed dof
   DBuf<uint8_t> slot_, slotz_, fixz_;  // slots per (cell, basis) and per incidence; fixed-dof masks
-  DBuf<T> K_, A_, diag_, delta_, rau_, rau_pc_, det_, invJ_, bco_, fixed_, fixed_div_, centT_, cconv_, fgeo_, p_, bz_, pz_;
+  DBuf<T> K_, A_, diag_, delta_, rau_, rau_pc_, det_, invJ_, bco_, fixed_, fixed_div_, conv_table_, cconv_, fgeo_, p_, bz_, pz_;
   DBuf<T> h2_, supg_rule_;
   DBuf<T> u3_, b_[3], s_[3], v_[3];  // u3_: interleaved velocity; v_: staging of get/set fields
   static constexpr int kVelComponents = k::kVel;

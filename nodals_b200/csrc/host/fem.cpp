@@ -137,4 +137,21 @@ const RefTensors& ref_tensors() {
   return T;
 }
 
+std::vector<double> conv_table() {
+  const RefTensors& R = ref_tensors();
+  std::vector<double> out;
+  out.reserve(kConvTable);
+  for (int a = 0; a < 8; ++a)
+    for (int m = a; m < 8; ++m)
+      for (int i = 0; i < 4; ++i) {
+        // T[a][m][4+i][j] = N_i(j+1) - N_i0 with N_ii = 0
+        const double* t = R.T[a][m][4 + i];
+        const double n0 = i == 0 ? 0.0 : -t[i - 1];
+        for (int k = 0; k < 4; ++k)
+          if (k != i) out.push_back(k == 0 ? n0 : t[k - 1] + n0);
+        out.push_back(R.T[a][m][1][0]);  // phi_1 = lambda_1, so dphi_1/dxi_0 = 1
+      }
+  return out;
+}
+
 }  // namespace nds

@@ -40,6 +40,14 @@ struct RefTensors {
 };
 const RefTensors& ref_tensors();
 
+// The convection table of the device assembly, from T: for every pair a <= m of
+// the 36 (row by row) and every i < 4 the record
+//   N_ik[a][m] = int phi_a phi_m dphi_(4+i)/dlambda_k  (the three k != i, ascending),
+//   M[a][m]    = int phi_a phi_m,
+// 16 values a pair.  Formed here in FP64, so that a table in FP32 is rounded once.
+constexpr int kConvTable = 36 * 16;
+std::vector<double> conv_table();
+
 // values and reference gradients of the 8 basis functions at lam
 void basis_eval(const std::array<double, 4>& lam, double phi[8], double grad[8][3]);
 

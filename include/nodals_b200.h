@@ -310,6 +310,12 @@ int nds_solver_pressure_pair(nds_solver* s, float* rhs, float* x);
 /* y = A x with the solver's current pressure operator in FP32 (device
  * arrays of nc values; precision mixed) */
 int nds_solver_apply_operator(nds_solver* s, const float* x, float* y);
+/* y = A x in one of the forms a solver keeps of it (device arrays of nc
+ * values): the Krylov method's or defect's in the state's precision (float with
+ * precision fp32, else double), or the V-cycle's on the fine level (double
+ * with precision fp64, else float; FP16 data with amg_half) */
+enum nds_operator_form { NDS_OP_STATE = 0, NDS_OP_VCYCLE = 1 };
+int nds_solver_apply_operator_form(nds_solver* s, int form, const void* x, void* y);
 /* counters of the learned stage since the solver was created: applications
  * and fallbacks to the plain V-cycle */
 int nds_solver_stage_counts(nds_solver* s, long long* applied, long long* fallbacks);

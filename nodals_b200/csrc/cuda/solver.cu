@@ -165,6 +165,7 @@ struct ISolver {
   virtual void pressure_pair(float* rhs, float* x) = 0;
   virtual void stage_counts(long long* applied, long long* fallbacks) = 0;
   virtual void apply_operator(const float* x, float* y) = 0;
+  virtual void apply_operator_form(int form, const void* x, void* y) = 0;
   Profiler prof;
 };
 
@@ -2356,6 +2357,12 @@ class Solver final : public ISolver {
       NDS_CUDA(cudaStreamSynchronize(st_));
     }
   }
+  void apply_operator_form(int form, const void* x, void* y) override {
+    if (form == NDS_OP_STATE) op_spmv(fine_op(), static_cast<const T*>(x), static_cast<T*>(y));
+    else if (form == NDS_OP_VCYCLE) op_spmv(fine_opV(), static_cast<const TA*>(x), static_cast<TA*>(y));
+    else throw SolveFailure(NDS_E_INVALID, "unknown operator form");
+    NDS_CUDA(cudaStreamSynchronize(st_));
+  }
   void stage_counts(long long* applied, long long* fallbacks) override {
     unsigned long long c[2] = {0, 0};
     if (st_cnt_.p) {
@@ -3204,6 +3211,10 @@ int nds_solver_pressure_pair(nds_solver* s, float* rhs, float* x) {
 int nds_solver_apply_operator(nds_solver* s, const float* x, float* y) {
   if (!s || !x || !y) return fail(NDS_E_INVALID, "null argument");
   return guarded([&] { s->impl->apply_operator(x, y); });
+}
+int nds_solver_apply_operator_form(nds_solver* s, int form, const void* x, void* y) {
+  if (!s || !x || !y) return fail(NDS_E_INVALID, "null argument");
+  return guarded([&] { s->impl->apply_operator_form(form, x, y); });
 }
 int nds_solver_stage_counts(nds_solver* s, long long* applied, long long* fallbacks) {
   if (!s) return fail(NDS_E_INVALID, "null solver");

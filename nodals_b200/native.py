@@ -220,6 +220,7 @@ def lib():
             L.nds_mpnn_adam_step.argtypes = [vp, C.c_float, C.c_float, C.c_float, C.c_float, C.c_int]
             L.nds_mpnn_backward.argtypes = [vp, C.c_void_p, vp]
             L.nds_solver_apply_operator.argtypes = [vp, vp, vp]
+            L.nds_solver_apply_operator_form.argtypes = [vp, C.c_int, vp, vp]
             L.nds_mpnn_activations.argtypes = [vp, C.c_int, vp]
             L.nds_mpnn_destroy.argtypes = [vp]
             L.nds_solver_load_stage.argtypes = [vp, vp, C.c_int]
@@ -564,6 +565,11 @@ def solver_pressure_pair(solver: "Solver", rhs, x):
 def solver_apply_operator(solver: "Solver", x, y):
     """y = A x with the solver's current FP32 pressure operator (device arrays)."""
     _check(lib().nds_solver_apply_operator(solver._h, Mpnn._addr(x), Mpnn._addr(y)))
+
+
+def solver_apply_operator_form(solver: "Solver", form: str, x, y):
+    """y = A x in the form "state" or "vcycle" (device arrays in that form's vector type)."""
+    _check(lib().nds_solver_apply_operator_form(solver._h, ("state", "vcycle").index(form), Mpnn._addr(x), Mpnn._addr(y)))
 
 
 def solver_stage_counts(solver: "Solver"):

@@ -174,14 +174,16 @@ def check_hp(got: dict, want, tol: float):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("variant", ["amg_fp32", "mixed_half"])
-def test_sell_column_formats_agree(native, meshes, monkeypatch, variant):
-    """The fine operator (and, with the FP16 V-cycle, the explicit levels'
+@pytest.mark.parametrize("variant,smoother", [("amg_fp32", "cheb2"), ("amg_fp32", "l1jacobi"), ("amg_fp32", "mcgs"),
+                                              ("mixed_half", "cheb2"), ("mixed_half", "l1jacobi")])
+def test_sell_column_formats_agree(native, meshes, monkeypatch, variant, smoother):
+    """The fine operator (in split form with cheb2, as assembled rows with the
+    other smoothers; and, with the FP16 V-cycle, the explicit levels'
     FP16 copies) keep 16-bit column deltas when the ordering allows and
     absolute 32-bit columns otherwise (NDS_SELL_COL32 forces the latter):
     both formats give bitwise-equal solves."""
     kw = dict(precision="amg_fp32") if variant == "amg_fp32" else dict(precision="mixed", p_guess=4, amg_half=1)
-    P = _make(native, meshes, "pipe_small", **kw, **ORACLE_CASES["sa_pcg"])
+    P = _make(native, meshes, "pipe_small", **kw, **dict(ORACLE_CASES["sa_pcg"], amg_smoother=smoother))
     A = native.Solver(P)
     monkeypatch.setenv("NDS_SELL_COL32", "1")
     B = native.Solver(P)

@@ -3,7 +3,8 @@ V-cycle (NDS_DENSE_MB=0): the same operator up to rounding, for every
 polynomial smoother, hierarchy depth and precision.  FP64: the iterates agree
 to rounding amplified by the solves (1e-9 relative, equal iteration counts);
 FP32 state: 1e-3 on relCont as for the FP32 path against FP64; mixed: every
-solve meets its own target p_rtol = 1e-6, as do the fields.
+solve meets its own target p_rtol = 1e-6, as do the fields, in as many
+iterations give or take two (a cycle that is wrong but converges takes more).
 """
 from __future__ import annotations
 
@@ -38,7 +39,6 @@ def test_dense_levels_match(native, meshes, monkeypatch, case, mesh):
     for _ in range(4):
         a, b = A.step(), B.step()
         assert abs(a.rel_cont - b.rel_cont) <= tol_cont * abs(b.rel_cont), (a.it, a.rel_cont, b.rel_cont)
-        if tol_field == 1e-9:
-            assert a.p_its == b.p_its
+        assert abs(a.p_its - b.p_its) <= (0 if tol_field == 1e-9 else 2), (a.it, a.p_its, b.p_its)
     for x, y in zip(A.fields(), B.fields()):
         assert rel_l2(x, y) <= tol_field

@@ -2,9 +2,11 @@
 (NDS_RESIDENT=0) on small meshes: the same method in another order of sums.
 FP64: equal iteration counts, iterates to 1e-9 relative (rounding amplified by
 the solves); FP32 state as the FP32 path against FP64; mixed and FP32 V-cycle:
-every solve meets its own target p_rtol = 1e-6, as do the fields.  Sizes: not
-multiples of the cluster's eight parts, fewer coarse rows than blocks, several
-cells per thread; the smoother's degrees 1 (Jacobi), 2, 3 and 4.
+every solve meets its own target p_rtol = 1e-6, as do the fields, in as many
+iterations give or take two.  Sizes: parts of equal and unequal length, fewer
+coarse rows than blocks, several cells per thread, and 10,296 cells, whose
+operators do not fit the shared memory; the smoother's degrees 1 (Jacobi), 2, 3
+and 4.  The profiler (whose runs are bitwise equal) shows which form ran.
 """
 from __future__ import annotations
 
@@ -29,12 +31,14 @@ CASES = {
     "mixed_half": (dict(SA, precision="mixed", amg_half=1), 1e-5, 1e-6),
     "mixed_half_wide": (dict(SA, precision="mixed", amg_half=1), 1e-5, 1e-6),
 }
-MESHES = [(2, 8, 6), (2, 8, 7), (3, 16, 12), (4, 24, 13)]
+MESHES = [(2, 8, 6), (2, 8, 7), (3, 24, 7), (3, 16, 12), (4, 24, 13)]  # 720, 840, 4,536, 4,608, 10,296 cells
+# coarse matrices over the form's 4 MB: the classical hierarchy keeps a quarter of the cells
+TOO_LARGE = {("jacobi", (3, 24, 7)), ("jacobi", (3, 16, 12)), ("jacobi", (4, 24, 13))}
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("mesh", MESHES, ids=["%d_%d_%d" % m for m in MESHES])
-@pytest.mark.parametrize("case", sorted(CASES))
+@pytest.mark.parametrize("case,mesh", [(c, m) for c in sorted(CASES) for m in MESHES if (c, m) not in TOO_LARGE],
+                         ids=lambda v: v if isinstance(v, str) else "%d_%d_%d" % v)
 def test_resident_pcg_matches_the_loop(native, monkeypatch, case, mesh):
     from nodals_b200 import meshgen
     kw, tol_cont, tol_field = CASES[case]
@@ -43,16 +47,18 @@ def test_resident_pcg_matches_the_loop(native, monkeypatch, case, mesh):
     P = native.Problem(m, **dict(CFG, **kw))
     if case.endswith("wide"):
         monkeypatch.setenv("NDS_SELL_COL32", "1")
-    monkeypatch.setenv("NDS_RESIDENT", "5000")  # also just above the size rule
+    monkeypatch.setenv("NDS_RESIDENT", "11000")  # also above the size rule
     A, A2 = native.Solver(P), native.Solver(P)
     monkeypatch.setenv("NDS_RESIDENT", "0")
     B = native.Solver(P)
+    A2.profile(True)
+    B.profile(True)
     for _ in range(4):
         a, a2, b = A.step(), A2.step(), B.step()
         assert (a.p_its, a.rel_cont, a.p_rel) == (a2.p_its, a2.rel_cont, a2.p_rel)  # reproducible
         assert abs(a.rel_cont - b.rel_cont) <= tol_cont * abs(b.rel_cont), (a.it, a.rel_cont, b.rel_cont)
-        if tol_field == 1e-9:
-            assert a.p_its == b.p_its
+        assert abs(a.p_its - b.p_its) <= (0 if tol_field == 1e-9 else 2), (a.it, a.p_its, b.p_its)
+    assert A2.profile_read()["pcg_resident"][0] > 0 and B.profile_read()["pcg_resident"][0] == 0
     for x, y in zip(A.fields(), B.fields()):
         assert rel_l2(x, y) <= tol_field
 

@@ -2032,7 +2032,12 @@ class Solver final : public ISolver {
   // none).  It is an ordinary launch, taken with graphs off and under the
   // profiler too, so that those runs have the same sums.
   static constexpr int kResidentCells = 4000;
-  static constexpr size_t kResidentDense = (size_t)4 << 20;
+  // The coarse matrix is read from L2 by the eight SMs, 64 rows a block of 512:
+  // with the classical hierarchy, which keeps a quarter of the cells, its rows
+  // set the line.  Loop / this: 500 rows FP64 30.4 / 29.5, FP32 30.3 / 24.1; 536
+  // rows 31.1 / 32.4, 30.9 / 29.5; 602 rows 32.4 / 34.8, 30.0 / 31.6; 834 rows
+  // 31.7 / 52.5, 30.1 / 40.8.  SA hierarchies have 244 rows at 4,000 cells.
+  static constexpr int kResidentRows = 512;
   // entries of n per block (at least 2: res_inverse)
   static int res_part(int n) { return std::max(2, (n + k::kResCluster - 1) / k::kResCluster); }
   void plan_resident() {
@@ -2043,7 +2048,7 @@ class Solver final : public ISolver {
     int cells = kResidentCells;
     if (const char* e = std::getenv("NDS_RESIDENT")) cells = std::atoi(e);
     const size_t ld = dense_ld(L_[0].n);
-    if (nc_ > cells || ld * (size_t)L_[0].n * sizeof(TA) > kResidentDense) return;
+    if (nc_ > cells || L_[0].n > kResidentRows) return;
     const int chunk = res_part(nc_), vchunk = res_part(svert_.n);
     res_smem_ = mixed_ ? k::res_smem<float, TA>(chunk, vchunk, (int)ld) : k::res_smem<T, TA>(chunk, vchunk, (int)ld);
     int most = 0;

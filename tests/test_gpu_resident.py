@@ -4,7 +4,7 @@ FP64: equal iteration counts, iterates to 1e-9 relative (rounding amplified by
 the solves); FP32 state as the FP32 path against FP64; mixed and FP32 V-cycle:
 every solve meets its own target p_rtol = 1e-6, as do the fields, in as many
 iterations give or take two.  Sizes: parts of equal and unequal length, fewer
-coarse rows than blocks, several cells per thread, and 10,296 cells, whose
+coarse rows than blocks, several cells per thread, and 7,680 cells, whose FP64
 operators do not fit the shared memory; the smoother's degrees 1 (Jacobi), 2, 3
 and 4.  The profiler (whose runs are bitwise equal) shows which form ran.
 """
@@ -31,9 +31,9 @@ CASES = {
     "mixed_half": (dict(SA, precision="mixed", amg_half=1), 1e-5, 1e-6),
     "mixed_half_wide": (dict(SA, precision="mixed", amg_half=1), 1e-5, 1e-6),
 }
-MESHES = [(2, 8, 6), (2, 8, 7), (3, 24, 7), (3, 16, 12), (4, 24, 13)]  # 720, 840, 4,536, 4,608, 10,296 cells
-# coarse matrices over the form's 4 MB: the classical hierarchy keeps a quarter of the cells
-TOO_LARGE = {("jacobi", (3, 24, 7)), ("jacobi", (3, 16, 12)), ("jacobi", (4, 24, 13))}
+MESHES = [(2, 8, 6), (2, 8, 7), (3, 24, 7), (3, 16, 12), (4, 16, 16)]  # 720, 840, 4,536, 4,608, 7,680 cells
+# more than the form's 512 coarse rows (the classical hierarchy keeps a quarter of the cells)
+TOO_LARGE = {("jacobi", (3, 24, 7)), ("jacobi", (3, 16, 12)), ("jacobi", (4, 16, 16))}
 
 
 @pytest.mark.gpu
@@ -47,7 +47,7 @@ def test_resident_pcg_matches_the_loop(native, monkeypatch, case, mesh):
     P = native.Problem(m, **dict(CFG, **kw))
     if case.endswith("wide"):
         monkeypatch.setenv("NDS_SELL_COL32", "1")
-    monkeypatch.setenv("NDS_RESIDENT", "11000")  # also above the size rule
+    monkeypatch.setenv("NDS_RESIDENT", "8000")  # also above the size rule
     A, A2 = native.Solver(P), native.Solver(P)
     monkeypatch.setenv("NDS_RESIDENT", "0")
     B = native.Solver(P)
@@ -83,3 +83,21 @@ def test_graphs_off_runs_the_same_solves(native, monkeypatch, case, mesh):
     assert (C.profile_read()["pcg_resident"][0] > 0) == (mesh[0] == 2)
     for x, y, z in zip(A.fields(), B.fields(), C.fields()):
         assert np.array_equal(x, y) and np.array_equal(x, z)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("mesh,rows,one_kernel", [((2, 16, 8), 500, True), ((3, 16, 6), 536, False),
+                                                  ((3, 16, 10), 834, False)])
+def test_coarse_rows_line(native, mesh, rows, one_kernel, precision):
+    """The form is taken up to 512 coarse rows, above which the loop of
+    kernels is faster."""
+    from nodals_b200 import meshgen
+    nr, nt, nz = mesh
+    m = native.Mesh.from_tetmesh(meshgen.pipe_mesh(nr=nr, ntheta=nt, nz=nz, length=0.5 * nz, jitter=0.05, seed=0))
+    P = native.Problem(m, **dict(CFG, **CASES["jacobi"][0], precision=precision, p_rtol=1e-4))
+    assert abs(P.array("amg.A0.row").size - 1 - rows) <= 10
+    S = native.Solver(P)
+    S.profile(True)
+    S.step()
+    assert (S.profile_read()["pcg_resident"][0] > 0) == one_kernel

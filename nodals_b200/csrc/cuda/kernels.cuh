@@ -1042,56 +1042,50 @@ struct SolveInit {
 };
 // End of the loop body: count the iteration and test ||r|| <= target the way
 // the host loop does (sqrt, then compare); stop on convergence, on any flag
-// or at max_its.  The loop always ends: every body pass runs this kernel and
-// the count reaches max_its.
-// max_its < 0: the cap is ctl[3] (set per solve by the host).  in_graph = 0:
-// launched outside a graph (host-driven loop), no condition to set.
+// or at the cap ctl[3], set per solve.  The loop always ends: every body pass
+// takes this step and the count reaches the cap.  in_graph = 0: launched
+// outside a graph (host-driven loop), no condition to set.
 __device__ __forceinline__ void pcg_check_step(const double* __restrict__ sc, int rn2_slot, int r0_slot,
                                                int target_slot, int* __restrict__ flags, int* __restrict__ ctl,
-                                               int max_its, cudaGraphConditionalHandle loop, int in_graph,
-                                               const HostWords& host) {
-  if (max_its < 0) max_its = ctl[3];
+                                               cudaGraphConditionalHandle loop, int in_graph, const HostWords& host) {
   const int it = ++ctl[0];
   ctl[2] = 0;
   const double rn = sqrt(sc[rn2_slot]);
   if (!isfinite(rn / fmax(sc[r0_slot], 1e-300))) *flags |= 4;
   const int conv = rn <= sc[target_slot];
   ctl[1] = conv;
-  const bool stop = conv || *flags != 0 || it >= max_its;
+  const bool stop = conv || *flags != 0 || it >= ctl[3];
   if (in_graph) cudaGraphSetConditional(loop, stop ? 0u : 1u);
   if (stop || !in_graph) host.put(it, conv, ctl[3], *flags, sc[rn2_slot]);
 }
-// A reduction of one value's block partials (as reduce_partials<1>) whose
-// thread 0 then takes the next scalar step of the device PCG: rho and beta
-// (PCG_RHO), alpha (PCG_ALPHA) or the stopping test (PCG_CHECK).  One launch
-// instead of two; the same sums and the same scalar arithmetic.
+// The scalar step taken with a reduction: rho and beta of PCG (PCG_RHO), alpha
+// (PCG_ALPHA), the stopping test (PCG_CHECK) or none (SUM_ONLY).
 enum { PCG_RHO = 1, PCG_ALPHA = 2, PCG_CHECK = 3, SUM_ONLY = 4 };
 struct PcgScalars {
   double* sc;
   int* flags;
   int* ctl;
-  int rn2_slot, r0_slot, target_slot, max_its;
+  int rn2_slot, r0_slot, target_slot;
   cudaGraphConditionalHandle loop;
   int in_graph;
   HostWords host;
 };
-template <int STEP>
-__global__ void reduce_pcg(const double* part, int nblocks, double* __restrict__ out, PcgScalars s) {
+// p.q from the block partials of a product that does not reduce them itself
+// (as reduce_partials<1>), and the step alpha
+__global__ void reduce_alpha(const double* part, int nblocks, double* sc, int* flags) {
   pdl_begin();
   double v[1] = {0.0};
   for (int b = threadIdx.x; b < nblocks; b += blockDim.x) v[0] += part[b];
   block_sum<1>(v);
   if (threadIdx.x == 0) {
-    out[0] = v[0];
-    if (STEP == PCG_RHO) pcg_rho_step(s.sc, s.flags, s.ctl);
-    else if (STEP == PCG_ALPHA) pcg_alpha_step(s.sc, s.flags);
-    else pcg_check_step(s.sc, s.rn2_slot, s.r0_slot, s.target_slot, s.flags, s.ctl, s.max_its, s.loop, s.in_graph, s.host);
+    sc[1] = v[0];
+    pcg_alpha_step(sc, flags);
   }
 }
 
 // The same reduction taken by the kernel that produced the values: every
 // block leaves its partial sum, and the block that finishes last (a ticket
-// counter) adds the partials in the fixed order of reduce_pcg and takes the
+// counter) adds the partials in the fixed order of reduce_partials and takes the
 // scalar step.  The order of the sums does not depend on which block that
 // is.  It saves a launch of 3 to 6 microseconds, a tenth of a PCG iteration
 // on small meshes.  blockDim.x = kBlock; every thread of the block calls it.
@@ -1123,7 +1117,7 @@ __device__ __forceinline__ void reduce_tail(double value, const ReduceTail& t) {
     if (STEP == PCG_RHO) pcg_rho_step(t.ps.sc, t.ps.flags, t.ps.ctl);
     else if (STEP == PCG_ALPHA) pcg_alpha_step(t.ps.sc, t.ps.flags);
     else if (STEP == PCG_CHECK)
-      pcg_check_step(t.ps.sc, t.ps.rn2_slot, t.ps.r0_slot, t.ps.target_slot, t.ps.flags, t.ps.ctl, t.ps.max_its,
+      pcg_check_step(t.ps.sc, t.ps.rn2_slot, t.ps.r0_slot, t.ps.target_slot, t.ps.flags, t.ps.ctl,
                      t.ps.loop, t.ps.in_graph, t.ps.host);
   }
 }
@@ -1254,9 +1248,8 @@ __global__ void prolong_add(int nf, int pw, const int32_t* __restrict__ pc, cons
 // j): a row of the level matrix is read once for all columns, and the columns
 // lie contiguous for the threads.
 // ---------------------------------------------------------------------------
-// epilogues of block_spmm: the modes of spmv / spmv_resid / spmv_smooth and
-// of the transfers
-enum { BLK_Y = 0, BLK_RESID = 1, BLK_SMOOTH = 2, BLK_ADD = 3 };
+// epilogues of block_spmm: the modes of spmv / spmv_resid / spmv_smooth
+enum { BLK_Y = 0, BLK_RESID = 1, BLK_SMOOTH = 2 };
 template <class T, class MT, class CT, int MODE>
 __global__ void __launch_bounds__(kBlock) block_spmm(int n, int m, const int32_t* __restrict__ rp,
                                                      const CT* __restrict__ ci, const MT* __restrict__ v, T vinv,
@@ -1270,7 +1263,6 @@ __global__ void __launch_bounds__(kBlock) block_spmm(int n, int m, const int32_t
     if constexpr (!std::is_same<MT, T>::value) s *= vinv;
     const size_t o = (size_t)i * m + j;
     if (MODE == BLK_Y) y[o] = s;
-    else if (MODE == BLK_ADD) y[o] += s;
     else if (MODE == BLK_RESID) y[o] = b[o] - s;
     else y[o] = x[o] + w * (b[o] - s) / den[i];
   }

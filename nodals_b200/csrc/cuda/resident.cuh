@@ -12,7 +12,8 @@
 // global memory costs an L2 round trip in every step: the operators' data is
 // copied to shared memory too, as far as it fits (the V-cycle's first: four
 // of five products).  Bound by the chain of latencies in a step (shared
-// memory, FP64 arithmetic and shuffles, barrier), about 1.5 us each.
+// memory, FP64 arithmetic and shuffles, barrier), about 1.5 us each.  512
+// threads of 128 registers: the FP64 forms spill 72 to 76 bytes there.
 // Microseconds of an iteration, loop of kernels / this: 720 cells FP64 35.5 /
 // 20, FP32 37 / 20; 2,400 cells FP64 38 / 24, mixed FP16 45 / 30; 4,608 cells
 // FP32 35 / 35.  One block instead of eight was tried: 34 at 720 cells, 93 at

@@ -975,8 +975,7 @@ class Solver final : public ISolver {
   enum { S_RHO = 0, S_PQ = 1, S_ALPHA = 2, S_RN2 = 3, S_RHON = 4, S_BETA = 5, S_R0 = 6, S_TARGET = 7, S_TMP = 8,
          S_TMP2 = 9, S_CONT2 = 10, S_WN = 11,
          S_AUDIT = 16, S_ST_T = 20, S_ST_V = 21,
-         S_GUESS = 24,  // 44 slots: Galerkin matrix (upper triangle) and right-hand side of the guess
-         S_COEF = 72 };  // 8 slots: guess coefficients
+         S_GUESS = 24 };  // 44 slots: Galerkin matrix (upper triangle) and right-hand side of the guess
 
   // CUDA graphs of fixed launch sequences (no host decisions inside)
   struct Graph {
@@ -1060,13 +1059,6 @@ class Solver final : public ISolver {
   template <int NV>
   void reduce_to(int nblocks, int slot) {
     pdl_launch(k::reduce_partials<NV>, 1, kBlock, 0, st_, part_.p, nblocks, sc_.p + slot);
-    NDS_LAUNCH();
-  }
-  // reduction of one value into sc[slot], then the PCG scalar step STEP
-  template <int STEP>
-  void reduce_pcg(int nblocks, int slot, int max_its = 0, cudaGraphConditionalHandle h = {}, int in_graph = 1) {
-    const k::PcgScalars ps{sc_.p, flags_.p, ctl_.p, S_RN2, S_R0, S_TARGET, max_its, h, in_graph, host_words()};
-    pdl_launch(k::reduce_pcg<STEP>, 1, kBlock, 0, st_, part_.p, nblocks, sc_.p + slot, ps);
     NDS_LAUNCH();
   }
   // a sum that the host needs: the reduction writes it to page-locked memory
@@ -1193,7 +1185,7 @@ class Solver final : public ISolver {
   // a reduction into sc[slot] taken by the producing kernel's last block
   k::ReduceTail tail(int slot, cudaGraphConditionalHandle h = {}) {
     return k::ReduceTail{tailpart_.p, ticket_.p, sc_.p + slot,
-                         k::PcgScalars{sc_.p, flags_.p, ctl_.p, S_RN2, S_R0, S_TARGET, -1, h, in_graph_, host_words()}};
+                         k::PcgScalars{sc_.p, flags_.p, ctl_.p, S_RN2, S_R0, S_TARGET, h, in_graph_, host_words()}};
   }
   template <int MODE, class V>
   void sell_launch(const OpView<V>& A, int grid, const V* x, const V* b, const V* den, double w, V* y, V* y2) {
@@ -1297,8 +1289,9 @@ class Solver final : public ISolver {
   // windows of a level's rows (FP64 levels): from kWinRows rows on, when a
   // window fits the block's share of shared memory.  The line: with fewer rows
   // than about two per lane group of the 296 blocks there is no next row to
-  // look ahead to and the copy of the window is not paid back.  At 74,540 rows
-  // a product takes 20 us on average over the explicit levels instead of 25.
+  // look ahead to.  Microseconds of a PCG iteration, a lane group a row / this:
+  // 12,419 rows 130.9 / 128.7, 17,736 rows 165.4 / 155.2, 23,192 rows 218.7 /
+  // 204.7, 74,540 rows 612 / 557 (a product there 25 / 20 us on average).
   static constexpr int kWinRows = 16384;
   static constexpr size_t kWinBytes = 72 * 1024;
   void level_windows(Level& Lv, const CsrHost& A) {
@@ -1596,7 +1589,10 @@ class Solver final : public ISolver {
   // restriction that feeds it (a polynomial smoother, not the terminal level)
   bool fuse_pre(int l) const { return o_.amg_smoother != NDS_SM_MCGS && l < (int)L_.size() - 1 && l != dense_level_; }
   // coarse rows from which the restriction streams: more than a wave of warps, so
-  // that there is a next row to load ahead (fewer rows: a lane group a row)
+  // that there is a next row to load ahead (fewer rows: a lane group a row).
+  // Microseconds of a PCG iteration, a lane group a row / streaming: 6,411 rows
+  // FP64 81.4 / 80.0, FP32 72.9 / 70.7; 12,419 rows 132.5 / 130.6, 102.9 / 101.7;
+  // 74,540 rows 569 / 556, 406 / 398.
   static constexpr int kStreamRows = 8192;
   // NDS_STREAM_ROWS overrides the row counts from which the streaming kernels
   // of the levels and the restriction are used
@@ -1937,8 +1933,11 @@ class Solver final : public ISolver {
   }
   // r.z taken by the V-cycle's last kernel up to this many cells: it saves a
   // launch there, but each of that kernel's blocks waits for its stores before
-  // it leaves its partial sum, which costs 12 us at 1.23M cells against 6 us
-  // for a pass of its own.
+  // it leaves its partial sum.  Microseconds of an iteration, a pass of its own /
+  // the tail: FP64 47,880 cells 58.6 / 56.9, 105,984 82.2 / 80.0, 205,320 131.0 /
+  // 130.9, 383,040 207.4 / 208.1; FP32 V-cycle 205,320 101.6 / 100.1, 383,040
+  // 149.8 / 152.1, 1.23M 400 / 407.  The line holds for the defect's norm too
+  // (fast configuration: 205,320 cells 99.7 / 98.7, 383,040 136.7 / 138.4).
   static constexpr int kRhoCells = 200000;
   // Vectors of a PCG solve in precision S (the preconditioner runs in TA):
   // rA the residual in TA when the precisions differ.
@@ -2000,7 +1999,8 @@ class Solver final : public ISolver {
         sell_launch<k::SELL_DOT, S>(A, g, v.p, nullptr, nullptr, 0.0, v.q, nullptr);
         NDS_LAUNCH();
       }
-      reduce_pcg<k::PCG_ALPHA>(g, S_PQ);
+      pdl_launch(k::reduce_alpha, 1, kBlock, 0, st_, part_.p, g, sc_.p, flags_.p);
+      NDS_LAUNCH();
     }
     const TA* den0 = nullptr;
     TA w0 = 0, *x1 = nullptr;
@@ -2027,8 +2027,10 @@ class Solver final : public ISolver {
   // kResidentCells cells whose vectors fit the cluster's shared memory.
   // Microseconds of an iteration, loop of kernels / this: 720 cells FP64 35.5 /
   // 19.9, FP32 37 / 20, mixed FP16 46 / 30; 2,688 cells 37 / 29, 35.5 / 25.5,
-  // 41 / 30.5; 4,608 cells 38 / 42, 35 / 35, 42 / 40; at 9,600 cells half as
-  // fast, as eight SMs no longer keep up.  NDS_RESIDENT overrides the line (0:
+  // 41 / 30.5; 3,840 to 4,032 cells of four shapes FP64 37 to 38.5 / 33 to 40,
+  // FP32 36 / 29 to 34, mixed FP16 38 to 40 / 31 to 36; 4,608 cells 38 / 42,
+  // 35 / 35, 42 / 40; at 9,600 cells half as fast, as eight SMs no longer keep
+  // up.  NDS_RESIDENT overrides the line (0:
   // none).  It is an ordinary launch, taken with graphs off and under the
   // profiler too, so that those runs have the same sums.
   static constexpr int kResidentCells = 4000;
@@ -2721,7 +2723,7 @@ class Solver final : public ISolver {
       NDS_LAUNCH();
       return;
     }
-    // cell blocks: a grid of 8 blocks per SM amortises the shared tensor load
+    // cell blocks: a grid of 4 blocks per SM amortises the load of the shared table
     k::SupgArgs sa{P_.setup.pipe.nu, o_.supg_tau_scale, o_.supg_magic};
     const int gc = std::min(grid_for(nc_, kBlock / 4), 4 * kSms);
     k::mom_cell_conv<T><<<gc, kBlock, 0, st_>>>(nc_, ref_.p, fixed_.p, uc(0), uc(1), uc(2), invJ_.p, det_.p,

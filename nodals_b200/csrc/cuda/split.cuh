@@ -12,7 +12,7 @@
 // of from assembled rows.  An assembled row of the pipe meshes has 69.5
 // entries (nearly all through the vertices: 24 cells around each), that is
 // 278 bytes a cell in FP16 with 16-bit column deltas, 417 in FP32 and 695 in
-// FP64; the two steps read 32 + 56, 64 + 84 and 112 + 136 bytes a cell, and
+// FP64; the two steps read 32 + 56, 64 + 76 and 112 + 128 bytes a cell, and
 // the refresh writes 4 tau a cell where the assembled form rewrites every
 // entry.  Smoothers that need the entries of a row (multicolour Gauss-Seidel,
 // L1-Jacobi) keep the assembled SELL form.

@@ -106,8 +106,10 @@ __global__ void deinterleave3(int n, const T* __restrict__ u, T* __restrict__ a0
 // of 1536, and a lane reads each of the 36 symmetric table records (its three
 // N and M, two 16-byte loads) once for both (a, m) and (m, a): 9 loads of a
 // warp per cell where the 8-lane form takes 48, which bound it (shared-memory
-// stalls).  Assembly at 1.23M cells 1.55 -> 1.31 ms, at 404k 0.50 -> 0.43, at
-// 40k 0.079 -> 0.070.
+// stalls).  Bound by the L1 / shared-memory pipe (80 % busy at 383k cells: the
+// records, then the scattered 8-value rows), with 16 warps of 128 registers an
+// SM; the FP64 pipe is 22 % busy, DRAM 23 %.  Assembly at 1.23M cells 1.55 ->
+// 1.31 ms, at 404k 0.50 -> 0.43, at 40k 0.079 -> 0.070.
 template <class T>
 __device__ __forceinline__ void conv_record(const T* __restrict__ t, T& n0, T& n1, T& n2, T& mm) {
   if constexpr (sizeof(T) == 8) {
@@ -220,9 +222,10 @@ __global__ void __launch_bounds__(kBlock, 2) mom_cell_conv(int nc, const int32_t
 // the four lanes of a cell each prepares every fourth point (velocity from
 // shared memory, square root and division), the lanes exchange the four
 // values, and lane i adds the columns of vertex i and of the bubble opposite
-// to it.  Bound by FP64 arithmetic: assembly with these terms at 35k
-// cells takes 0.132 ms, 0.288 when every lane of eight evaluated the basis
-// gradients at every point.
+// to it.  The FP64 pipe is 47 % busy at 35k cells, the rest is the latency of
+// its chains (16 warps of 124 registers an SM): assembly with these terms takes
+// 0.132 ms there, 0.288 when every lane of eight evaluated the basis gradients
+// at every point.
 struct SupgArgs {
   double nu, tau_scale, magic;
 };

@@ -26,9 +26,10 @@
 // thread issues 8 MMAs (M = 128, N = 64, K = 16) against the weight tile kept
 // in shared memory, and the accumulator (128 lanes x 64 columns of TMEM) is
 // read back with tcgen05.ld for the bias + ReLU epilogue, warp w taking lanes
-// 32 (w mod 4) and columns 16 (w / 4).  A layer on 403,680 nodes takes 70 us
-// (133 us with one thread a row); the 103 MB read and written would take 16
-// us, the rest is the latency of the gathers at 1,024 threads an SM.  Backward
+// 32 (w mod 4) and columns 16 (w / 4).  A layer on 403,680 nodes takes 68 us
+// (133 us with one thread a row), the first, which evaluates the encoder for
+// every neighbour, 131 us; the 103 MB read and written would take 16 us, the
+// rest is the latency of the gathers at 1,024 threads an SM.  Backward
 // uses the same tiles:
 // dX = delta W (M 128, N 128, K 64) and dW^T += X^T delta (M 128, N 64,
 // K = the 128 nodes of the tile, both operands read MN-major from the same
@@ -568,8 +569,8 @@ __global__ void scatter_bwd(int n, const int32_t* __restrict__ nbr, const float*
 // encoder backward: delta0 = dh0 (.) [h0 > 0]; partials of dWe (64 x 2), dbe
 // (64), FP64.  A thread keeps one unit and walks the rows, four rows of a
 // block at a time, so that a warp reads 32 consecutive gradients and the sums
-// stay in registers.  Bound by reading dh0 (103 MB at 403,680
-// nodes: 80 us; 782 us with 192 sums per thread, which spilled).
+// stay in registers.  It waits for its reads of dh0 (103 MB at 403,680 nodes in
+// 82 us, 1.3 TB/s; 782 us with 192 sums per thread, which spilled).
 __global__ void __launch_bounds__(kBlock) encoder_bwd(int n, const float2* __restrict__ f, const float* __restrict__ dh0,
                                                       const float* __restrict__ params, double* __restrict__ part) {
   constexpr int kRows = kBlock / kH;
@@ -619,8 +620,8 @@ __global__ void __launch_bounds__(kBlock) seg_loss(int lo, int hi, const float* 
 // The decoder's backward from g_i = dL/d out_i (functor): dh3 = g wd, and
 // partials of dwd (64), dbd, dcs in FP64.  Sixteen threads a row, four units
 // each: rows are read and written whole by half-warps and a thread keeps four
-// sums.  Bound by writing dh3 (128 us before at
-// 403,680 nodes, 64 us so).
+// sums.  It waits for its reads (long scoreboard; 64 us at 403,680 nodes for
+// 60 MB read and 103 MB written, 128 us with one thread a row).
 template <class G>
 __device__ __forceinline__ void decoder_rows(int n, const G& grad, const __nv_bfloat16* __restrict__ h3,
                                              const float2* __restrict__ f, const float* __restrict__ params,

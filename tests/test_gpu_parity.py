@@ -52,9 +52,10 @@ def test_gpu_matches_oracle(native, oracle_mod, meshes, case):
 
 
 @pytest.mark.gpu
-def test_gpu_fp32_close_to_fp64(native, meshes):
-    P64 = _make(native, meshes, "pipe_small", **ORACLE_CASES["sa_pcg"])
-    P32 = _make(native, meshes, "pipe_small", precision="fp32", **ORACLE_CASES["sa_pcg"])
+@pytest.mark.parametrize("case", ["sa_pcg", "sa_supg"])
+def test_gpu_fp32_close_to_fp64(native, meshes, case):
+    P64 = _make(native, meshes, "pipe_small", **ORACLE_CASES[case])
+    P32 = _make(native, meshes, "pipe_small", precision="fp32", **ORACLE_CASES[case])
     S64, S32 = native.Solver(P64), native.Solver(P32)
     for _ in range(10):
         a, b = S64.step(), S32.step()

@@ -133,11 +133,16 @@ def test_separate_post_vcycle_is_symmetric():
     assert gap({}) > 1e-3
 
 
+# degree 4 (default), 3 and 2 end in either buffer of the fused Chebyshev steps; 1 has no product
+SEPARATE = {**{n: VCYCLES[n] for n in ("cheb2", "cheb2_deg3_aggr", "jacobi_2sweeps")},
+            **{f"cheb2_deg{d}": ("exti_t60", dict(amg_cheb_degree=d), dict(cheb_degree=d)) for d in (1, 2)}}
+
+
 @pytest.mark.gpu
-@pytest.mark.parametrize("name", ["cheb2", "jacobi_2sweeps"])
+@pytest.mark.parametrize("name", sorted(SEPARATE))
 def test_device_separate_post_vcycle_matches_oracle(native, name):
     from oracle.hybrid_amg import VCycle
-    case, po, oo = VCYCLES[name]
+    case, po, oo = SEPARATE[name]
     v = np.load(VGOLD)
     nvel = native.hybrid_counts(MESH)[5]
     z = native.hybrid_amg_vcycle(MESH, _rau(nvel), v["b"], pressure_solver=1, amg_separate_post=1, **CASES[case],
